@@ -74,7 +74,7 @@ def _closure(root_files: list[Path], search: list[Path]) -> set[str]:
 def _stage_reference() -> Path | None:
     """Returns the directory to compile the reference from, staging it when
     the reference checkout is available."""
-    if REFERENCE.is_dir():
+    if (REFERENCE / "RadixSortLsdParallel.h").is_file():  # (an empty checkout is none)
         names = _closure([ORACLE / "ref_capi.cpp"], [ORACLE / "ref_stub", REFERENCE])
         REF_SRC_STAGE.mkdir(parents=True, exist_ok=True)
         for n in sorted(names):
