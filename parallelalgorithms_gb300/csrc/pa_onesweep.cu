@@ -9,9 +9,9 @@
 // (PermuteDerandomizedNew, :169-212) become a tile sorted by digit in shared
 // memory and written out in bin-contiguous runs.
 //
-// Per CTA (one tile of TILE = BLOCK * ITEMS keys):
-//   1. take the next tile ticket (tickets are handed out in launch order, so
-//      every tile a CTA waits on in step 5 is owned by a CTA already running);
+// Resident CTAs loop over tiles of TILE = BLOCK * ITEMS keys; per tile:
+//   1. take the next tile ticket (every tile a CTA waits on in step 5 has a
+//      lower ticket, so it is owned by a CTA already at work on it);
 //   2. bulk-copy the tile global -> shared with the TMA engine, completing on
 //      an mbarrier (plain loads for the <16-byte ragged end, or when a buffer
 //      is not 16-byte aligned);
@@ -33,6 +33,7 @@
 //      consecutive addresses.
 // Small inputs (at most small_sort_max_keys) are sorted whole by one CTA in
 // shared memory instead (small_sort_kernel).
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -55,28 +56,18 @@ __global__ void __launch_bounds__(BLOCK, MINB) onesweep_kernel(const OnesweepArg
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + G::kBarOff);
   uint32_t* s_tile_id = reinterpret_cast<uint32_t*>(smem + G::kTileIdOff);
-  // 1. tile ticket: tiles are taken in launch order
   if (threadIdx.x == 0) {
-    *s_tile_id = atomicAdd(args.tile_counter, 1u);
     mbar_init(s_bar, 1);
     mbar_fence_init();
-  }
-  __syncthreads();
-  const uint32_t tile = *s_tile_id;
-  // keys to move: args.n, or fewer counted on the device (tiles past them exit)
-  const size_t n = args.n_dev ? min((size_t)*args.n_dev, args.n) : args.n;
-  if ((size_t)tile >= (n + TILE - 1) / TILE) {
-    if (!args.n_dev && threadIdx.x == 0) raise_error(args.err, DEVERR_BAD_STATE);  // a ticket counter not reset
-    return;
   }
   TileJob<K, S> job;
   job.in = static_cast<const K*>(pc.src_is_tmp ? args.keys_b : args.keys_a);
   job.out = static_cast<K*>(pc.src_is_tmp ? args.keys_a : args.keys_b);
   job.vin = pc.src_is_tmp ? args.vals_b : args.vals_a;
   job.vout = pc.src_is_tmp ? args.vals_a : args.vals_b;
-  job.n = n;
-  job.out_n = args.out_n ? args.out_n : n;
-  job.tile = tile;
+  // keys to move: args.n, or fewer counted on the device (tiles past them are not taken)
+  job.n = args.n_dev ? min((size_t)*args.n_dev, args.n) : args.n;
+  job.out_n = args.out_n ? args.out_n : job.n;
   job.shift = args.shift;
   job.tin = args.is_float && pc.transform_in;
   job.tout = args.is_float && pc.transform_out;
@@ -88,10 +79,29 @@ __global__ void __launch_bounds__(BLOCK, MINB) onesweep_kernel(const OnesweepArg
   job.chunk_excl = args.chunk_excl;
   job.tiles_per_chunk = args.tiles_per_chunk;
   uint32_t parity = 0;
-  if constexpr (MULTISPLIT)
-    onesweep_tile_multisplit<K, HAS_VALS, BLOCK, ITEMS, S>(job, smem, s_bar, parity);
-  else
-    onesweep_tile<K, HAS_VALS, BLOCK, ITEMS, S>(job, smem, s_bar, parity);
+  for (;;) {
+    // 1. tile ticket: taken only when the CTA is ready for the tile, so every
+    // tile a look-back waits on is owned by a CTA already at work on it
+    if (threadIdx.x == 0) *s_tile_id = atomicAdd(args.tile_counter, 1u);
+    __syncthreads();
+    job.tile = *s_tile_id;
+    const size_t tiles = (job.n + TILE - 1) / TILE;
+    if ((size_t)job.tile >= tiles) {  // past the end: once per CTA, or the counter was not reset
+      if ((size_t)job.tile >= tiles + gridDim.x && !args.n_dev && threadIdx.x == 0)
+        raise_error(args.err, DEVERR_BAD_STATE);
+      return;
+    }
+    if constexpr (MULTISPLIT)
+      onesweep_tile_multisplit<K, HAS_VALS, BLOCK, ITEMS, S>(job, smem, s_bar, parity);
+    else
+      onesweep_tile<K, HAS_VALS, BLOCK, ITEMS, S>(job, smem, s_bar, parity);
+    // a grid of at least as many CTAs as tiles: each has had its one
+    if (gridDim.x >= tiles) return;
+    __syncthreads();
+    // a tile that gave up (it has published its words) ends its CTA, so that no
+    // copy still in flight can meet the next tile's
+    if (*reinterpret_cast<uint32_t*>(smem + G::kAbortOff)) return;
+  }
 }
 
 // Wide-digit pass (11-bit digits, 2048 bins): onesweep_tile_wide.
@@ -257,15 +267,19 @@ cudaError_t launch_g2(const OnesweepArgs& a, cudaStream_t stream) {
   if (e != cudaSuccess) return e;
   size_t tiles = ceil_div(a.n, (size_t)G::kTile);
   if (a.max_ctas && a.max_ctas < tiles) tiles = a.max_ctas;
+  // One grid of resident CTAs looping over tickets: a CTA per tile paid for
+  // 16-33 thousand CTA launches a pass (100M 64-bit keys with payloads, Zipf:
+  // 5.64 ms a sort against 6.03; twice or four times the resident CTAs 5.65).
+  tiles = std::min(tiles, (size_t)device_info().sm_count * MINB);
   kern<<<(unsigned)tiles, BLOCK, G::kBytes, stream>>>(a);
   return cudaGetLastError();
 }
 
 // Ranking method of a pass: the warp multisplit (default) or the in-tile
 // counting sort (PA_ONESWEEP_RANK=counting).  A persistent form of the
-// multisplit pass that copied each CTA's next tile in while it worked on the
-// current one was measured slower on GB300 (tickets taken early make
-// successors wait in the look-back) and is not built.
+// multisplit pass that took each CTA's next ticket and copied that tile in
+// while it worked on the current one was measured slower on GB300 (tickets
+// taken early make successors wait in the look-back) and is not built.
 bool use_multisplit() {
   static const bool v = [] {
     const char* e = std::getenv("PA_ONESWEEP_RANK");
