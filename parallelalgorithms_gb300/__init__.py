@@ -50,32 +50,47 @@ def _is_torch(x) -> bool:
     return type(x).__module__.startswith("torch")
 
 
+_torch_dtypes: dict = {}  # torch dtype -> numpy dtype, filled with the first tensor seen
+_raw_stream = None        # torch's current stream of a device, as a pointer
+
+
+def _torch_setup() -> None:
+    global _raw_stream
+    import torch
+    table = {torch.int32: np.uint32, torch.int64: np.uint64, torch.uint8: np.uint8,
+             torch.float32: np.float32, torch.int8: np.int8, torch.int16: np.int16,
+             torch.float64: np.float64}
+    for name in ("uint32", "uint64"):
+        if hasattr(torch, name):
+            table[getattr(torch, name)] = getattr(np, name)
+    _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if _raw_stream is None:
+        _raw_stream = lambda index: torch.cuda.current_stream(index).cuda_stream  # noqa: E731
+    _torch_dtypes.update((t, np.dtype(d)) for t, d in table.items())
+
+
 def _info(x):
-    """(pointer, element count, numpy dtype, stream or None) of a buffer."""
-    if _is_torch(x):
-        import torch
-        if not x.is_contiguous():
-            raise ValueError("tensor must be contiguous")
-        dt = {torch.int32: np.uint32, torch.int64: np.uint64, torch.uint8: np.uint8,
-              torch.float32: np.float32, torch.int8: np.int8, torch.int16: np.int16,
-              torch.float64: np.float64}.get(x.dtype)
-        if hasattr(torch, "uint32") and x.dtype == torch.uint32:
-            dt = np.uint32
-        if hasattr(torch, "uint64") and x.dtype == torch.uint64:
-            dt = np.uint64
-        if dt is None:
-            raise TypeError(f"unsupported tensor dtype {x.dtype}")
-        stream = torch.cuda.current_stream(x.device).cuda_stream if x.is_cuda else None
-        return x.data_ptr(), x.numel(), np.dtype(dt), stream
+    """(pointer, element count, numpy dtype, stream or None) of a buffer.  This
+    and the calls below are most of what a small call costs on the host: each
+    buffer is looked at once, and dtypes and functions come from tables."""
     if isinstance(x, np.ndarray):
         if not x.flags.c_contiguous:
             raise ValueError("array must be C-contiguous")
         return x.ctypes.data, x.size, x.dtype, None
+    if _is_torch(x):
+        if not _torch_dtypes:
+            _torch_setup()
+        if not x.is_contiguous():
+            raise ValueError("tensor must be contiguous")
+        dt = _torch_dtypes.get(x.dtype)
+        if dt is None:
+            raise TypeError(f"unsupported tensor dtype {x.dtype}")
+        return x.data_ptr(), x.numel(), dt, _raw_stream(x.device.index) if x.is_cuda else None
     raise TypeError(f"unsupported buffer type {type(x)}")
 
 
 def _ptr(x):
-    return ctypes.c_void_p(_info(x)[0]) if x is not None else None
+    return _info(x)[0] if x is not None else None
 
 
 def _opts(*bufs, digit_bits: int = 0):
@@ -89,20 +104,18 @@ def _opts(*bufs, digit_bits: int = 0):
 
 
 def _offset(x, elems: int, itemsize: int):
-    p = _info(x)[0]
-    return ctypes.c_void_p(p + elems * itemsize)
+    return _info(x)[0] + elems * itemsize
+
+
+_KINDS = {np.dtype(np.uint32): "u32", np.dtype(np.int32): "u32", np.dtype(np.uint64): "u64", np.dtype(np.int64): "u64",
+          np.dtype(np.float32): "f32", np.dtype(np.uint8): "u8"}
 
 
 def _kind(dt: np.dtype) -> str:
-    if dt == np.uint32 or dt == np.int32:
-        return "u32"
-    if dt == np.uint64 or dt == np.int64:
-        return "u64"
-    if dt == np.float32:
-        return "f32"
-    if dt == np.uint8:
-        return "u8"
-    raise TypeError(f"unsupported dtype {dt}")
+    k = _KINDS.get(dt)
+    if k is None:
+        raise TypeError(f"unsupported dtype {dt}")
+    return k
 
 
 # ---------------------------------------------------------------------------
@@ -113,18 +126,28 @@ def sort(keys, values=None, tmp_keys=None, tmp_values=None, n: int | None = None
     float32 keys, float32 by IEEE total order), moving an optional uint32
     payload with its key.  digit_bits: 8 (one pass per key byte, the
     reference's radix) or 11 (2048 bins, fewer passes; same result)."""
-    ptr, size, dt, _ = _info(keys)
+    ptr, size, dt, stream = _info(keys)
     n = size if n is None else n
     if n > size:
         raise ValueError("n exceeds the key buffer")
     k = _kind(dt)
-    o = _opts(keys, values, tmp_keys, tmp_values, digit_bits=0 if digit_bits == 8 else digit_bits)
+    rest = []  # the other buffers' pointers; the last one on a device decides the stream, as for the keys
+    for b in (values, tmp_keys, tmp_values):
+        p, m, _, s = _info(b) if b is not None else (None, 0, None, None)
+        rest.append((p, m))
+        stream = s if s is not None else stream
+    o = _native.opts(stream, digit_bits=0 if digit_bits == 8 else digit_bits)
+    (vals, nvals), (tmp, _), (tmp_vals, _) = rest
     if values is None:
-        call(f"pa_sort_{k}", ctypes.c_void_p(ptr), _ptr(tmp_keys), n, o)
+        call(_SORT[k], ptr, tmp, n, o)
     else:
-        if _info(values)[1] < n:
+        if nvals < n:
             raise ValueError("values shorter than n")
-        call(f"pa_sort_kv_{k}", ctypes.c_void_p(ptr), _ptr(values), _ptr(tmp_keys), _ptr(tmp_values), n, o)
+        call(_SORT_KV[k], ptr, vals, tmp, tmp_vals, n, o)
+
+
+_SORT = {k: f"pa_sort_{k}" for k in ("u32", "u64", "f32", "u8")}
+_SORT_KV = {k: f"pa_sort_kv_{k}" for k in ("u32", "u64", "f32", "u8")}
 
 
 def SortRadixPar(a, tmp_work_buff=None, a_size: int | None = None, parallelThreshold: int = 512 * 1024) -> None:
@@ -176,10 +199,8 @@ def HistogramByteComponentsParallel(inArray, l: int, r: int, parallelThreshold: 
         raise ValueError("only <256, 8> is defined (the reference's loop is hard-wired to 4 byte digits)")
     out = np.zeros((8, 256), np.uint64)
     n = r - l + 1 if l <= r else 0
-    body = np.zeros(4 * 256, np.uint64)
-    call("pa_hist_byte_components_u32", _offset(inArray, l, 4), n, ctypes.c_void_p(body.ctypes.data),
-         _opts(inArray))
-    out[:4] = body.reshape(4, 256)
+    ptr, _, _, stream = _info(inArray)
+    call("pa_hist_byte_components_u32", ptr + 4 * l, n, out.ctypes.data, _native.opts(stream))  # fills rows 0-3
     return out
 
 
@@ -190,16 +211,15 @@ def HistogramOneByteComponentParallel(inArray, l: int, r: int, shiftRight: int |
     uint8 input: HistogramParallel.h:17 HistogramOneByteComponentParallel<256>
     (a, l, r), r EXCLUSIVE, byte counts."""
     out = np.zeros(256, np.uint64)
-    k = _kind(_info(inArray)[2])
-    if k == "u8":
+    ptr, _, dt, stream = _info(inArray)
+    if _kind(dt) == "u8":
         n = max(0, r - l)
-        call("pa_hist_u8", _offset(inArray, l, 1), n, ctypes.c_void_p(out.ctypes.data), _opts(inArray))
+        call("pa_hist_u8", ptr + l, n, out.ctypes.data, _native.opts(stream))
     else:
         if shiftRight is None:
             raise TypeError("shiftRight is required for 32-bit input")
         n = r - l + 1 if l <= r else 0
-        call("pa_hist_one_byte_u32", _offset(inArray, l, 4), n, int(shiftRight), ctypes.c_void_p(out.ctypes.data),
-             _opts(inArray))
+        call("pa_hist_one_byte_u32", ptr + 4 * l, n, int(shiftRight), out.ctypes.data, _native.opts(stream))
     return out
 
 
@@ -252,26 +272,24 @@ def SelectRadix(a, *args) -> int:
 
 def select(a, k: int) -> int:
     """k-th smallest (0-based) of a uint32 or uint64 array; a is not modified."""
-    ptr, n, dt, _ = _info(a)
+    ptr, n, dt, stream = _info(a)
     kind = _kind(dt)
-    out = np.zeros(1, np.uint64 if kind == "u64" else np.uint32)
-    call(f"pa_select_{kind}", ctypes.c_void_p(ptr), n, k, ctypes.c_void_p(out.ctypes.data), _opts(a))
-    return int(out[0])
+    out = ctypes.c_uint64() if kind == "u64" else ctypes.c_uint32()
+    call(f"pa_select_{kind}", ptr, n, k, ctypes.byref(out), _native.opts(stream))
+    return out.value
 
 
 # ---------------------------------------------------------------------------
 # sum
 # ---------------------------------------------------------------------------
 def _sum(in_array, l: int, r: int) -> int:
-    dt = _info(in_array)[2]
+    ptr, _, dt, stream = _info(in_array)
     kind = _kind(dt)
     if kind not in ("u32", "u64"):
         raise TypeError("sum is defined for unsigned 32- and 64-bit arrays")
-    out = np.zeros(1, np.uint64)
-    isz = 4 if kind == "u32" else 8
-    call(f"pa_sum_{kind}", _offset(in_array, l, isz), max(0, r - l), ctypes.c_void_p(out.ctypes.data),
-         _opts(in_array))
-    return int(out[0])
+    out = ctypes.c_uint64()
+    call(f"pa_sum_{kind}", ptr + l * dt.itemsize, max(0, r - l), ctypes.byref(out), _native.opts(stream))
+    return out.value
 
 
 # element kinds of pa_sum_typed (PA_ELEM_* in include/pa_gpu.h)

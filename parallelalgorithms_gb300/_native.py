@@ -115,18 +115,36 @@ def status_name(status: int) -> str:
     return lib().pa_status_string(status).decode()
 
 
+_functions: dict[str, object] = {}
+
+
 def call(name: str, *args) -> None:
     """Calls a pa_* entry point and raises PaError on failure."""
-    rc = getattr(lib(), name)(*args)
+    fn = _functions.get(name)
+    if fn is None:
+        fn = _functions[name] = getattr(lib(), name)
+    rc = fn(*args)
     if rc != PA_OK:
         raise PaError(name, rc, lib().pa_last_error_message().decode())
 
 
 def opts(stream: int | None = None, async_device: bool = False, digit_bits: int = 0) -> ctypes.POINTER(PaOpts) | None:
-    if stream is None and not async_device and not digit_bits:
+    """The options block of a call (read by the library only, so blocks are kept
+    by value: building one costs more than the rest of a small call's arguments)."""
+    if not stream and not async_device and not digit_bits:
         return None
-    o = PaOpts()
-    o.stream = stream or None
-    o.async_device = 1 if async_device else 0
-    o.digit_bits = digit_bits
-    return ctypes.pointer(o)
+    key = (stream, async_device, digit_bits)
+    p = _opts_kept.get(key)
+    if p is None:
+        o = PaOpts()
+        o.stream = stream or None
+        o.async_device = 1 if async_device else 0
+        o.digit_bits = digit_bits
+        p = ctypes.pointer(o)
+        if len(_opts_kept) >= 64:
+            _opts_kept.clear()
+        _opts_kept[key] = p
+    return p
+
+
+_opts_kept: dict[tuple, object] = {}

@@ -81,11 +81,22 @@ constexpr int kPipeChunks = 8;   // host-buffer sort: copy-in chunks
 static_assert(kPipeChunks <= kMaxChunkRuns, "the bucket sort's chunk table holds every chunk");
 constexpr int kPipeGroups = 10;  // host-buffer sort: bucket groups sorted and copied out in turn
 
+constexpr size_t kReadBackWords = 2048;  // the largest small result: 8 digits' 256 counts
+struct HostBlock {
+  uint32_t err;       // error word of bounded waits, zero between calls
+  uint32_t unused;
+  uint64_t result;    // a select's or sum's result
+  uint64_t words[kReadBackWords];
+};
+
 struct Workspace {
   char* dev = nullptr;
   size_t dev_cap = 0;
-  uint32_t* err = nullptr;       // device error word, zero between calls
-  uint32_t* err_host = nullptr;  // pinned mirror for reading it back
+  // Page-locked and visible to the device, so that what a call reads back is
+  // there when its stream is done, without a copy of its own (4 to 10 us each):
+  HostBlock* host = nullptr;
+  uint32_t* err = nullptr;     // &host->err
+  uint32_t* ticket = nullptr;  // one device word, zero between calls (the sum's)
   cudaEvent_t ev[kMaxEvents] = {};  // phase timing (created on first use)
   // pipelined host-buffer sort (created on first use)
   cudaStream_t copy_stream = nullptr;
@@ -112,9 +123,11 @@ int get_workspace(cudaStream_t stream, Workspace** out) {
   PA_CUDA(cudaGetDevice(&dev));
   Workspace& ws = g_ws[{dev, stream}];
   if (!ws.err) {
-    PA_CUDA(cudaMalloc(&ws.err, 256));
-    PA_CUDA(cudaMemset(ws.err, 0, 256));
-    PA_CUDA(cudaMallocHost(&ws.err_host, sizeof(uint32_t)));
+    if (!ws.ticket) PA_CUDA(cudaMalloc(&ws.ticket, 256));
+    PA_CUDA(cudaMemset(ws.ticket, 0, 256));
+    if (!ws.host) PA_CUDA(cudaMallocHost(&ws.host, sizeof(HostBlock)));
+    ws.host->err = 0;
+    ws.err = &ws.host->err;
   }
   *out = &ws;
   return PA_OK;
@@ -168,12 +181,10 @@ int finish(Workspace* ws, cudaStream_t stream, bool async_ok) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
   if (async_ok) return PA_OK;
-  PA_CUDA(cudaMemcpyAsync(ws->err_host, ws->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
   PA_CUDA(cudaStreamSynchronize(stream));
-  const uint32_t err = *ws->err_host;
+  const uint32_t err = *const_cast<volatile uint32_t*>(ws->err);
   if (err) {
-    PA_CUDA(cudaMemsetAsync(ws->err, 0, sizeof(uint32_t), stream));
-    PA_CUDA(cudaStreamSynchronize(stream));
+    *const_cast<volatile uint32_t*>(ws->err) = 0;  // (the stream is idle)
     return set_error(PA_ERR_TIMEOUT, "device-side bounded wait gave up (code 0x%x); results are undefined", err);
   }
   return PA_OK;
@@ -741,8 +752,12 @@ int hist_impl(const void* a, size_t n, int kb, int num_digits, uint32_t shift0, 
   if (!in_dev && n) PA_CUDA(cudaMemcpyAsync(const_cast<void*>(d_in), a, n * kb, cudaMemcpyHostToDevice, stream));
   PA_CUDA(cudaMemsetAsync(d_out, 0, out_words * sizeof(uint64_t), stream));
   PA_CUDA(launch_digit_counts(d_in, n, kb, num_digits, 8, shift0, step, false, d_out, stream));
-  if (!out_dev) PA_CUDA(cudaMemcpyAsync(out, d_out, out_words * sizeof(uint64_t), cudaMemcpyDeviceToHost, stream));
-  return finish(ws, stream, opts && opts->async_device && in_dev && out_dev);
+  // (a copy to pageable memory would wait for the stream first)
+  if (!out_dev)
+    PA_CUDA(cudaMemcpyAsync(ws->host->words, d_out, out_words * sizeof(uint64_t), cudaMemcpyDeviceToHost, stream));
+  const int rc = finish(ws, stream, opts && opts->async_device && in_dev && out_dev);
+  if (!out_dev && rc == PA_OK) std::memcpy(out, ws->host->words, out_words * sizeof(uint64_t));
+  return rc;
 }
 
 // ---------------------------------------------------------------------------
@@ -769,7 +784,7 @@ int select_impl(const void* a, size_t n, size_t k, int kb, void* out, const pa_o
     d_in = in_dev ? a : c.take<char>(n * kb);
     cand = c.take<char>(cand_cap * kb);
     work = c.take<char>(select_state_bytes());
-    d_out = out_dev ? out : c.take<char>(8);
+    d_out = out_dev ? out : &ws->host->result;
   };
   Carve m{nullptr};
   layout(m);
@@ -778,8 +793,9 @@ int select_impl(const void* a, size_t n, size_t k, int kb, void* out, const pa_o
   layout(r);
   if (!in_dev) PA_CUDA(cudaMemcpyAsync(const_cast<void*>(d_in), a, n * kb, cudaMemcpyHostToDevice, stream));
   PA_CUDA(launch_select(d_in, n, k, kb, cand, cand_cap, work, d_out, ws->err, stream));
-  if (!out_dev) PA_CUDA(cudaMemcpyAsync(out, d_out, kb, cudaMemcpyDeviceToHost, stream));
-  return finish(ws, stream, opts && opts->async_device && in_dev && out_dev);
+  const int rc = finish(ws, stream, opts && opts->async_device && in_dev && out_dev);
+  if (!out_dev && rc == PA_OK) std::memcpy(out, &ws->host->result, kb);
+  return rc;
 }
 
 // ---------------------------------------------------------------------------
@@ -804,14 +820,15 @@ int sum_impl(const void* a, size_t n, int elem_kind, uint64_t* out, const pa_opt
   const bool sums_dev = chunk_sums && is_device_ptr(chunk_sums);
   const void* d_in = nullptr;
   unsigned long long* partials = nullptr;
-  uint32_t* ticket = nullptr;
   unsigned long long* d_out = nullptr;
   unsigned long long* d_sums = nullptr;
   auto layout = [&](Carve& c) {
     d_in = in_dev ? a : c.take<char>(n * kb);
     partials = c.take<unsigned long long>(sum_partials_needed());
-    ticket = c.take<uint32_t>(1);
-    d_out = out_dev ? reinterpret_cast<unsigned long long*>(out) : c.take<unsigned long long>(1);
+    if (out_dev)
+      d_out = reinterpret_cast<unsigned long long*>(out);
+    else  // (the per-chunk sums' total takes atomics)
+      d_out = chunk_sums ? c.take<unsigned long long>(1) : reinterpret_cast<unsigned long long*>(&ws->host->result);
     if (chunk_sums)
       d_sums = sums_dev ? reinterpret_cast<unsigned long long*>(chunk_sums) : c.take<unsigned long long>(nchunks);
   };
@@ -827,12 +844,14 @@ int sum_impl(const void* a, size_t n, int elem_kind, uint64_t* out, const pa_opt
     PA_CUDA(launch_sum_chunks(d_in, n, elem_kind, chunk, d_sums, d_out, stream));
     if (!sums_dev && nchunks)
       PA_CUDA(cudaMemcpyAsync(chunk_sums, d_sums, nchunks * sizeof(uint64_t), cudaMemcpyDeviceToHost, stream));
+    if (!out_dev)
+      PA_CUDA(cudaMemcpyAsync(&ws->host->result, d_out, sizeof(uint64_t), cudaMemcpyDeviceToHost, stream));
   } else {
-    PA_CUDA(cudaMemsetAsync(ticket, 0, sizeof(uint32_t), stream));
-    PA_CUDA(launch_sum(d_in, n, elem_kind, partials, ticket, d_out, ws->err, stream));
+    PA_CUDA(launch_sum(d_in, n, elem_kind, partials, ws->ticket, d_out, ws->err, stream));
   }
-  if (!out_dev) PA_CUDA(cudaMemcpyAsync(out, d_out, sizeof(uint64_t), cudaMemcpyDeviceToHost, stream));
-  return finish(ws, stream, opts && opts->async_device && in_dev && out_dev && (!chunk_sums || sums_dev));
+  const int rc = finish(ws, stream, opts && opts->async_device && in_dev && out_dev && (!chunk_sums || sums_dev));
+  if (!out_dev && rc == PA_OK) *out = ws->host->result;
+  return rc;
 }
 
 }  // namespace
@@ -1012,8 +1031,8 @@ int pa_release_workspaces(void) {
     cudaSetDevice(kv.first.first);
     cudaStreamSynchronize(kv.first.second);
     if (kv.second.dev) cudaFree(kv.second.dev);
-    if (kv.second.err) cudaFree(kv.second.err);
-    if (kv.second.err_host) cudaFreeHost(kv.second.err_host);
+    if (kv.second.ticket) cudaFree(kv.second.ticket);
+    if (kv.second.host) cudaFreeHost(kv.second.host);
   }
   g_ws.clear();
   cudaSetDevice(dev0);
