@@ -12,10 +12,10 @@ Printed as one JSON line (rank 0):
   value       keys/s over the device-resident sort (CUDA events per step)
   e2e         keys/s through the reference-facing C ABI (pa_sort_u32) with
               pinned HOST buffers: host->device copy, sort, device->host copy
-  roofline    the dominant kernel (one onesweep digit pass): algorithmic
-              bytes per launch (8 bytes/key: read + write each key once)
-              over its CUDA-event duration, against the measured HBM copy
-              bandwidth in MEASURED_PEAKS.json
+  roofline    the longest kernel (a partition pass or the sort of the
+              buckets): algorithmic bytes per launch (8 bytes/key: read +
+              write each key once) over its CUDA-event duration, against the
+              measured HBM copy bandwidth in MEASURED_PEAKS.json
   cpu_baseline the reference's own SortRadixPar (compiled unchanged, TBB
               stand-in thread pool) on this host's cores, same input
   extras      presorted / constant sorts, 64-bit key+payload and float32
@@ -53,7 +53,6 @@ UNIT = "keys/s"
 # (the reference README's table, its fastest published machine).
 PUBLISHED_KEYS_PER_S = 2.865e9
 PUBLISHED_SOURCE = "reference README: parallel LSD radix sort, 100M random uint32, 48-core AWS c7a.24xlarge"
-PROFILE_TRAFFIC = ROOT / "profiles" / "onesweep_pass_u32_100m_traffic.txt"
 
 
 def parse_args():
@@ -246,16 +245,6 @@ def measured_peak_gbs() -> tuple[float, str]:
     return 6800.0, "fallback"
 
 
-def profiled_traffic_per_launch() -> float | None:
-    """dram read+write bytes per onesweep launch from the committed ncu summary."""
-    if not PROFILE_TRAFFIC.exists():
-        return None
-    for line in PROFILE_TRAFFIC.read_text().splitlines():
-        if line.startswith("traffic_bytes_per_launch:"):
-            return float(line.split(":", 1)[1])
-    return None
-
-
 def dist_setup():
     world = int(os.environ.get("WORLD_SIZE", "1"))
     rank = int(os.environ.get("RANK", "0"))
@@ -422,22 +411,21 @@ def gb300_arm(args) -> None:
                      P(phases.ctypes.data), 16, _native.opts(stream.cuda_stream))
         acc += phases
     acc /= reps
-    hist_ms, scan_ms = float(acc[0]), float(acc[1])
-    pass_ms = [float(x) for x in acc[2:6]]
-    copy_ms = float(acc[6])
+    # keys alone are sorted by buckets: plan + counts, two partitions, the sort
+    # of each bucket; then the LSD launches, which find nothing to do
+    names = ["plan_and_count", "scan", "partition_high", "partition_low", "bucket_sort", "lsd_launches", "final_copy"]
+    phase = {name: float(x) for name, x in zip(names, acc)}
     peak, peak_kind = measured_peak_gbs()
-    pass_avg = statistics.mean(pass_ms)
-    achieved = 8.0 * n / (pass_avg / 1e3) / 1e9
-    traffic = profiled_traffic_per_launch()
-    roofline = {"bound": "hbm", "kernel": "onesweep digit pass (uint32 keys, 8-bit digit)", "achieved": achieved,
-                "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
+    top = max(("partition_high", "partition_low", "bucket_sort"), key=phase.get)
+    achieved = 8.0 * n / (phase[top] / 1e3) / 1e9
+    roofline = {"bound": "shared memory pipe", "kernel": f"{top} (uint32 keys)", "achieved": achieved,
+                "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": None,
                 "peak_source": f"{peak_kind} hbm_gbs (MEASURED_PEAKS.json)" if peak_kind == "measured"
                 else "fallback 6800 GB/s",
-                "bytes_per_launch": 8 * n, "launch_ms": pass_avg}
-    sort_bytes = 36.0 * n
-    whole = {"bytes_per_key": 36, "achieved_gbs": sort_bytes / (ms / 1e3) / 1e9,
-             "frac": sort_bytes / (ms / 1e3) / 1e9 / peak,
-             "phase_ms": {"histogram": hist_ms, "scan": scan_ms, "passes": pass_ms, "final_copy": copy_ms}}
+                "bytes_per_launch": 8 * n, "launch_ms": phase[top]}
+    sort_bytes = 28.0 * n
+    whole = {"bytes_per_key": 28, "achieved_gbs": sort_bytes / (ms / 1e3) / 1e9,
+             "frac": sort_bytes / (ms / 1e3) / 1e9 / peak, "phase_ms": phase}
 
     # end to end through the C ABI with pinned host buffers
     h_src = workloads.uniform_u32(n, pinned=True)

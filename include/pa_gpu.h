@@ -62,11 +62,12 @@ int pa_stream_check(void* stream);
 /* Releases the cached device and pinned workspaces of every stream. */
 int pa_release_workspaces(void);
 
-/* ---- LSD radix sort ------------------------------------------------------
+/* ---- radix sort ----------------------------------------------------------
  * Stable ascending sort of keys[0, n) in place.  tmp is caller scratch of n
  * keys whose contents are clobbered; tmp == NULL lets the library use its
- * own scratch.  The digit histograms of every pass are computed in one read
- * of the keys before the digit passes.
+ * own scratch.  LSD digit passes, the histograms of all of them computed in
+ * one read of the keys; keys alone, where the order equal keys were moved in
+ * cannot be seen, are sorted by buckets instead where that is faster.
  *
  * pa_sort_u32 replaces ParallelAlgorithms::SortRadixPar(unsigned* a,
  *   unsigned* tmp_work_buff, size_t a_size, size_t parallelThreshold)
@@ -102,7 +103,12 @@ int pa_sort_two_phase_u32(uint32_t* a, uint32_t* b, size_t n, const pa_opts* opt
  * and phase_ms[i] receives the device time in milliseconds of each kernel,
  * from CUDA events recorded between the launches: [0] the one-read digit
  * histogram, [1] the bin-offset scan, [2 + p] digit pass p (one per
- * digit), [2 + passes] the final copy.  phase_cap bounds the entries written.
+ * digit), [2 + passes] the final copy.  Keys alone of the sizes that are sorted
+ * by buckets (csrc/pa_buckets.cu): [0] the plan and the bucket counts, [2] and
+ * [3] the two partition passes, [4] the sort of each bucket, [5] every LSD
+ * launch behind them (nearly nothing, unless the keys were too unevenly spread
+ * for buckets; then [0] to [4] are), [2 + passes] the final copy, the others
+ * nothing.  phase_cap bounds the entries written.
  * GPU form of the per-phase timers the reference keeps commented out in its
  * sort (RadixSortLsdParallel.h:255-258, 287, 307-308). */
 enum { PA_KEY_U32 = 0, PA_KEY_U64 = 1, PA_KEY_F32 = 2 };

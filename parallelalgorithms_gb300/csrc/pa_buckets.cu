@@ -1,0 +1,1240 @@
+// Keys-only sorts by buckets (MSD): two partition passes, then one pass that
+// sorts every bucket in shared memory.
+//
+// A sort of keys alone has one result whatever the order equal keys were
+// moved in, so its passes need not be stable, and an unstable partition is
+// much cheaper than the stable digit pass of pa_onesweep.cu: a key's place in
+// its tile is the value a shared-memory atomic returns (no lane matching, no
+// per-warp counters), and a tile's place in a bin is one global atomic per bin
+// (no look-back).  Keys cross memory 1 + 2 + 2 + 2 times (count, partition,
+// partition, bucket sort) against 1 + 2 * 4 (1 + 2 * 8 for 64-bit keys).
+//
+//   bucket_plan_kernel     one cluster of 8 CTAs reads 16384 keys at even
+//                          strides, takes the range they span, and lays nb
+//                          equal buckets over it (BucketMap); counts the
+//                          sample per bucket to judge the fit: a sample that
+//                          crowds into few buckets leaves the sort to the LSD
+//                          passes, which do not mind how keys are spread;
+//   bucket_count_kernel    one read: exact keys per bucket; the last CTA turns
+//                          the counts into bucket starts and cursors;
+//   bucket_scatter_kernel  one tile at a time: rank, reserve, stage by bin,
+//                          write out in bin-contiguous runs.  First on the
+//                          bucket's high bits (keys -> tmp), then, bucket
+//                          group by bucket group, on its low bits (tmp ->
+//                          keys).  At most 256 buckets: one pass (keys -> tmp);
+//   bucket_finish_kernel   one CTA per bucket: the keys set bits of a bitmap of
+//                          their range, and a key's place is the number of bits
+//                          set below its own.
+//
+// The map is monotone in the key whatever the sample was, so the sample
+// decides only how evenly the buckets fill, never the result.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <cmath>
+
+#include "pa_common.cuh"
+#include "pa_kernels.cuh"
+#include "pa_onesweep_tile.cuh"
+
+namespace pa {
+namespace {
+
+namespace cg = cooperative_groups;
+
+constexpr uint32_t kFull = 0xFFFFFFFFu;
+constexpr int kPlanCtas = 8;
+constexpr int kPlanBlock = 1024;
+constexpr int kPlanPer = 2;  // sample keys per thread
+constexpr uint32_t kSample = (uint32_t)kPlanCtas * kPlanBlock * kPlanPer;
+constexpr uint32_t kGroups = 256;         // bins of a partition pass, at most
+constexpr uint32_t kBucketsMax = 32768;   // counters of the count kernel: 128 KB of shared memory
+constexpr uint32_t kBucketTarget = 3072;  // keys per bucket, at most, while more buckets can be had
+constexpr uint32_t kCells = 65536;        // cells of the finish kernel's bitmap
+constexpr uint32_t kBucketBins = 4096;    // bins of a bucket that is counted instead
+constexpr uint32_t kBucketBinMax = 64;    // keys of one bin that are still placed by comparing
+
+struct BucketArgs {
+  BucketMap* map;
+  SortCtrl* ctrl;
+  uint32_t* count;
+  uint32_t* start;
+  uint32_t* cursor;
+  uint32_t* group_cursor;
+  uint32_t* tile_first;
+  uint32_t nb;
+  uint32_t nb_bits;     // nb = 1 << nb_bits
+  uint32_t low_bits;
+  uint32_t tile;        // keys per partition tile
+  uint32_t tmp_align;   // scratch address modulo 16
+  uint32_t hot_above;   // sample keys above which a bucket looks too full
+  uint32_t max_sample;  // sample keys no bucket may exceed
+  uint32_t* err;
+  uint32_t* decided;    // where the plan tells the host whether the sort goes by buckets (may be null)
+};
+
+// t: the key's distance from the bottom of the map, in 32 bits.
+template <typename K>
+__device__ __forceinline__ uint32_t map_t(K key, K lo, uint32_t s) {
+  if constexpr (sizeof(K) == 4) {
+    (void)s;
+    return key > lo ? key - lo : 0u;
+  } else {
+    const K t = (key > lo ? key - lo : (K)0) >> s;
+    return t > (K)0xFFFFFFFFu ? 0xFFFFFFFFu : (uint32_t)t;
+  }
+}
+__device__ __forceinline__ uint32_t map_bucket(uint32_t t, uint32_t mult, uint32_t last) {
+  return min(__umulhi(t, mult), last);
+}
+
+// The key's top 32 bits: its distance from the bottom of a plain map.
+__device__ __forceinline__ uint32_t top_word(uint32_t key) { return key; }
+__device__ __forceinline__ uint32_t top_word(unsigned long long key) { return (uint32_t)(key >> 32); }
+
+// Elements from the 16-byte boundary at or below p to p.
+template <typename K>
+__device__ __forceinline__ uint32_t skew_of(const K* p) {
+  return (uint32_t)(reinterpret_cast<uintptr_t>(p) & 15u) / (uint32_t)sizeof(K);
+}
+
+template <typename K>
+__device__ __forceinline__ void warp_minmax(K& lo, K& hi) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const K a = __shfl_xor_sync(kFull, lo, o), b = __shfl_xor_sync(kFull, hi, o);
+    lo = a < lo ? a : lo;
+    hi = b > hi ? b : hi;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Plan.
+// ---------------------------------------------------------------------------
+// Latency only (about 16 K scattered sectors): one cluster instead of one CTA,
+// so that the sample's loads and its per-bucket counts (each CTA holds 1/8 of
+// them, reached through distributed shared memory) are spread over 8 SMs, and
+// cluster barriers instead of global tickets, so that nothing has to be zeroed
+// first.
+template <typename K>
+__global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
+    bucket_plan_kernel(const K* __restrict__ keys, size_t n, int is_float, BucketArgs a) {
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ uint32_t s_hist[kBucketsMax / kPlanCtas];
+  __shared__ K s_lo[32], s_hi[32];
+  __shared__ K s_cta_lo[kPlanCtas], s_cta_hi[kPlanCtas];
+  __shared__ uint32_t s_mult, s_s;
+  __shared__ K s_base;
+  __shared__ uint32_t s_max[kPlanCtas], s_hot[kPlanCtas];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t rank = cluster.block_rank();
+  K k[kPlanPer];
+  K lo = ~(K)0, hi = 0;
+#pragma unroll
+  for (int j = 0; j < kPlanPer; ++j) {
+    const size_t i = ((size_t)j * kPlanCtas + rank) * kPlanBlock + tid;
+    k[j] = to_ordered(keys[(size_t)(((unsigned long long)i * n) / kSample)], is_float != 0);
+    lo = min(lo, k[j]);
+    hi = max(hi, k[j]);
+  }
+  for (uint32_t i = tid; i < a.nb / kPlanCtas; i += kPlanBlock) s_hist[i] = 0;
+  warp_minmax(lo, hi);
+  if (lane == 0) {
+    s_lo[warp] = lo;
+    s_hi[warp] = hi;
+  }
+  cluster.sync();  // (every CTA of the cluster runs before its memory is written from another)
+  if (warp == 0) {
+    lo = s_lo[lane];
+    hi = s_hi[lane];
+    warp_minmax(lo, hi);
+    if (lane < (uint32_t)kPlanCtas) {
+      cluster.map_shared_rank(s_cta_lo, lane)[rank] = lo;
+      cluster.map_shared_rank(s_cta_hi, lane)[rank] = hi;
+    }
+  }
+  cluster.sync();
+  if (tid == 0) {
+    for (int c = 0; c < kPlanCtas; ++c) {
+      lo = min(lo, s_cta_lo[c]);
+      hi = max(hi, s_cta_hi[c]);
+    }
+    // widen by 1/1024 each way: about 16 keys of the sample's spacing, so that
+    // few keys of an even spread fall outside and crowd into the end buckets
+    const K pad = (hi - lo) >> 10;
+    lo -= min(lo, pad);
+    hi += min((K)(~(K)0 - hi), pad);
+    // keys over most of their type's range: the map is their top bits, which
+    // costs the partition passes a shift instead of a subtract and a multiply
+    if (hi - lo >= (~(K)0 >> 3) * 7) {
+      lo = 0;
+      hi = ~(K)0;
+    }
+    uint32_t s = 0;
+    if constexpr (sizeof(K) == 8) s = (uint32_t)max(0, 32 - __clzll((long long)(hi - lo)));
+    const unsigned long long range = (unsigned long long)((hi - lo) >> s) + 1;
+    const unsigned long long mult = ((unsigned long long)a.nb << 32) / range;
+    s_mult = mult > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)mult;
+    s_s = s;
+    s_base = lo;
+  }
+  __syncthreads();
+  const uint32_t mult = s_mult, s = s_s, last = a.nb - 1;
+  const K base = s_base;
+  const uint32_t per = a.nb / kPlanCtas;
+#pragma unroll
+  for (int j = 0; j < kPlanPer; ++j) {
+    const uint32_t b = map_bucket(map_t<K>(k[j], base, s), mult, last);
+    uint32_t* c = cluster.map_shared_rank(s_hist, b / per) + b % per;
+    if (__all_sync(kFull, b == __shfl_sync(kFull, b, 0))) {  // (constant keys: one add, not 32 in turn)
+      if (lane == 0) atomicAdd(c, 32u);
+    } else {
+      atomicAdd(c, 1u);
+    }
+  }
+  cluster.sync();
+  // the fullest bucket, and the keys of the sample in buckets that look fuller
+  // than the finish kernel holds
+  uint32_t mx = 0, hot = 0;
+  for (uint32_t i = tid; i < per; i += kPlanBlock) {
+    const uint32_t c = s_hist[i];
+    mx = max(mx, c);
+    hot += c > a.hot_above ? c : 0u;
+  }
+  mx = __reduce_max_sync(kFull, mx);
+  hot = __reduce_add_sync(kFull, hot);
+  __syncthreads();  // s_lo is free
+  uint32_t* w = reinterpret_cast<uint32_t*>(s_lo);
+  uint32_t* w2 = reinterpret_cast<uint32_t*>(s_hi);
+  if (lane == 0) {
+    w[warp] = mx;
+    w2[warp] = hot;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    mx = __reduce_max_sync(kFull, w[lane]);
+    hot = __reduce_add_sync(kFull, w2[lane]);
+    if (lane == 0) {
+      cluster.map_shared_rank(s_max, 0)[rank] = mx;
+      cluster.map_shared_rank(s_hot, 0)[rank] = hot;
+    }
+  }
+  cluster.sync();
+  if (rank == 0 && tid == 0) {
+    for (int c = 1; c < kPlanCtas; ++c) {
+      mx = max(mx, s_max[c]);
+      hot += s_hot[c];
+    }
+    const bool fits = mx <= a.max_sample && hot <= kSample / 64;
+    BucketMap m{};
+    m.on = fits ? 1u : 0u;
+    m.plain = base == 0 && mult == a.nb && s == 8 * sizeof(K) - 32 ? 1u : 0u;
+    m.mult = mult;
+    m.inv = (1ull << 63) / mult;
+    m.s = s;
+    m.lo = base;
+    // cells and bins of the finish kernel: the widest bucket spans
+    // ceil(2^32 / mult) values of t, 2^s keys each
+    const unsigned long long width = ((1ull << 32) + mult - 1) / mult;
+    uint32_t sh = 0;
+    while (((width - 1) >> sh) >= kCells) ++sh;
+    m.cell_shift = sh + s;
+    while (((width - 1) >> sh) >= kBucketBins) ++sh;
+    m.bin_shift = sh + s;
+    m.exact = m.bin_shift == 0 ? 1u : 0u;
+    *a.map = m;
+    if (fits) {  // the LSD passes enqueued behind this sort do nothing
+      for (int p = 0; p < kMaxPasses; ++p) a.ctrl->pass[p].skip = 1;
+      a.ctrl->final_in_tmp = 0;
+    }
+    if (a.decided) {  // page-locked host memory the caller polls
+      __threadfence_system();
+      *reinterpret_cast<volatile uint32_t*>(a.decided) = fits ? 1u : 0u;
+    }
+  }
+  // (last, so that no cluster barrier waits for these stores)
+  for (uint32_t i = rank * kPlanBlock + tid; i < a.nb; i += kPlanCtas * kPlanBlock) a.count[i] = 0;
+}
+
+// ---------------------------------------------------------------------------
+// Count.
+// ---------------------------------------------------------------------------
+// One read against a shared counter per bucket (up to 128 KB, so one CTA per
+// SM).  A thread's next four 16-byte loads are issued before the current ones
+// are counted: 32 warps alone left the SM waiting for loads half of the time.
+// 100M 32-bit keys: 0.105 ms, 3.8 TB/s (the digit histogram it replaces, with
+// its tile tables: 0.113 ms).
+constexpr int kCountBlock = 1024;
+
+template <typename K, bool FLT>
+__global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* __restrict__ keys, size_t n,
+                                                                      BucketArgs a) {
+  extern __shared__ __align__(16) uint32_t s_cnt[];
+  __shared__ uint32_t s_warp[kCountBlock / 32];
+  __shared__ uint32_t s_last;
+  constexpr int V = 16 / (int)sizeof(K);
+  const BucketMap m = *a.map;
+  if (!m.on) return;
+  const uint32_t tid = threadIdx.x;
+  for (uint32_t i = tid; i < a.nb; i += kCountBlock) s_cnt[i] = 0;
+  __syncthreads();
+  const uint32_t last = a.nb - 1;
+  auto count = [&](auto plainc) {
+    constexpr bool PLAIN = decltype(plainc)::value;
+    const K lo = (K)m.lo;
+    const uint32_t shift = 32u - a.nb_bits;
+    auto bucket = [&](K raw) {
+      const K key = to_ordered(raw, FLT);
+      if constexpr (PLAIN) return top_word(key) >> shift;
+      else return map_bucket(map_t<K>(key, lo, m.s), m.mult, last);
+    };
+    const uintptr_t addr = reinterpret_cast<uintptr_t>(keys);
+    size_t head = ((16u - (addr & 15u)) & 15u) / sizeof(K);
+    if (head > n) head = n;
+    const size_t nvec = (n - head) / V;
+    const size_t tail = head + nvec * V;
+    const uint4* vec = reinterpret_cast<const uint4*>(keys + head) + tid;
+    const size_t stride = (size_t)gridDim.x * kCountBlock;
+    constexpr int U = 4;
+    // whole rounds of U vectors per thread (every lane of a warp takes part),
+    // the next round's loads issued before this one's keys are counted
+    size_t i = (size_t)blockIdx.x * kCountBlock;
+    auto whole = [&](size_t at) { return at + (U - 1) * stride + kCountBlock <= nvec; };
+    uint4 q[U];
+    if (whole(i)) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) q[u] = ld_stream_v4(vec + i + u * stride);
+    }
+    while (whole(i)) {
+      const size_t nx = i + U * stride;
+      const bool more = whole(nx);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint4 w = q[u];
+        if (more) q[u] = ld_stream_v4(vec + nx + u * stride);
+        const K* k = reinterpret_cast<const K*>(&w);
+        const uint32_t d0 = bucket(k[0]);
+        bool one = d0 == __shfl_sync(kFull, d0, 0);
+        if (__all_sync(kFull, one)) {
+          // sorted or constant runs: one add for a warp that agrees, where its
+          // atomics would queue on one word
+#pragma unroll
+          for (int e = 1; e < V; ++e) one = one && bucket(k[e]) == d0;
+          if (__all_sync(kFull, one)) {
+            if ((tid & 31u) == 0) atomicAdd(s_cnt + d0, 32u * V);
+            continue;
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < V; ++e) atomicAdd(s_cnt + bucket(k[e]), 1u);
+      }
+      i = nx;
+    }
+    for (; i < nvec; i += stride) {
+      if (i + tid < nvec) {
+        const uint4 w = ld_stream_v4(vec + i);
+        const K* k = reinterpret_cast<const K*>(&w);
+#pragma unroll
+        for (int e = 0; e < V; ++e) atomicAdd(s_cnt + bucket(k[e]), 1u);
+      }
+    }
+    if (blockIdx.x == 0) {  // head and tail: fewer than 2 * V keys
+      const size_t rest = head + (n - tail);
+      for (size_t r = tid; r < rest; r += kCountBlock) atomicAdd(s_cnt + bucket(keys[r < head ? r : tail + (r - head)]), 1u);
+    }
+  };
+  if (m.plain) count(std::true_type{});
+  else count(std::false_type{});
+  __syncthreads();
+  // each CTA adds its counts starting at another place, so that CTAs that end
+  // together do not queue on the same words
+  const uint32_t off = (uint32_t)(((unsigned long long)blockIdx.x * a.nb) / gridDim.x);
+  for (uint32_t j = tid; j < a.nb; j += kCountBlock) {
+    const uint32_t b = (j + off) & last;
+    const uint32_t c = s_cnt[b];
+    if (c) atomicAdd(a.count + b, c);
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(&a.map->ticket, 1u) == gridDim.x - 1u ? 1u : 0u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  // The last CTA: bucket starts, cursors of both passes, and the second
+  // pass's tiles per group (tile_first).
+  const uint32_t per = max(1u, a.nb / kCountBlock);  // buckets per thread
+  if (a.nb >= (uint32_t)kCountBlock) {
+    for (uint32_t j = tid * 4; j < a.nb; j += kCountBlock * 4)
+      *reinterpret_cast<uint4*>(s_cnt + j) = __ldcg(reinterpret_cast<const uint4*>(a.count + j));
+  } else if (tid < a.nb) {
+    s_cnt[tid] = __ldcg(a.count + tid);
+  }
+  __syncthreads();
+  uint32_t local = 0;
+  if (tid * per < a.nb)
+    for (uint32_t j = 0; j < per; ++j) local += s_cnt[tid * per + ((j + tid) & (per - 1))];
+  uint32_t run = os::block_exclusive_scan<kCountBlock>(local, s_warp);
+  if (tid * per < a.nb) {
+    for (uint32_t j = 0; j < per; ++j) {
+      const uint32_t c = s_cnt[tid * per + j];
+      s_cnt[tid * per + j] = run;
+      run += c;
+    }
+  }
+  __syncthreads();
+  for (uint32_t j = tid; j < a.nb; j += kCountBlock) {
+    const uint32_t v = s_cnt[j];
+    a.start[j] = v;
+    a.cursor[j] = v;
+  }
+  if (tid == 0) a.start[a.nb] = (uint32_t)n;
+  const uint32_t groups = a.nb >> a.low_bits;
+  uint32_t tiles = 0;
+  if (tid < groups) {
+    const uint32_t g0 = s_cnt[tid << a.low_bits];
+    const uint32_t g1 = tid + 1 < groups ? s_cnt[(tid + 1) << a.low_bits] : (uint32_t)n;
+    a.group_cursor[tid] = g0;
+    // tiles start at 16-byte boundaries of the input (bucket_scatter_kernel)
+    const uint32_t head2 = (uint32_t)(((a.tmp_align + (size_t)g0 * sizeof(K)) & 15u) / sizeof(K));
+    tiles = g1 > g0 ? (g1 - g0 + head2 + a.tile - 1) / a.tile : 0;
+  }
+  __syncthreads();  // s_warp is reused
+  const uint32_t before = os::block_exclusive_scan<kCountBlock>(tiles, s_warp);
+  if (tid < groups) a.tile_first[tid] = before;
+  if (tid == groups - 1) a.tile_first[groups] = before + tiles;
+}
+
+// ---------------------------------------------------------------------------
+// Partition pass.
+// ---------------------------------------------------------------------------
+// Bound by the shared-memory / L1 data pipe (84 % of its cycles at 100M
+// uniform keys): per 32 keys one atomic, one look-up of the bin's start and one
+// store at random places (about 3 cycles each), the sequential read back, the
+// look-up of the bin's destination and the stores to global memory.  So what
+// counts is the number of shared accesses per key, not registers or occupancy
+// (two CTAs per SM measured as three).  A tile's next loads are issued before
+// it is written out, and a bin's reservation (a round trip to L2) passes while
+// the tile is staged.  100M uniform 32-bit keys: 0.208 ms for the first pass,
+// 0.240 ms for the grouped one, against 0.326 and 0.385 ms for a stable digit
+// pass with and without prepared offsets.
+constexpr int kScatterBlock = 512;
+constexpr int kScatterPerSm = 3;
+template <typename K>
+constexpr int kScatterItems = sizeof(K) == 4 ? 16 : 8;
+template <typename K>
+constexpr uint32_t kScatterTile = (uint32_t)kScatterBlock * kScatterItems<K>;
+
+// PLAIN: the map is the key's top bits (BucketMap::plain).
+template <typename K, bool GROUPED, bool FLT, bool PLAIN>
+__device__ __forceinline__ void scatter_tiles(const K* in, K* out, uint32_t n, const BucketArgs& a, const BucketMap& m,
+                                              K* s_keys, uint32_t* s_cnt, uint32_t* s_start, uint32_t* s_base,
+                                              uint32_t* s_warp, const uint32_t* s_first) {
+  constexpr int ITEMS = kScatterItems<K>;
+  constexpr uint32_t T = kScatterTile<K>;
+  constexpr int V = 16 / (int)sizeof(K);
+  constexpr int Q = ITEMS / V;  // 16-byte vectors per thread
+  const uint32_t tid = threadIdx.x, lane = tid & 31u;
+  const uint32_t groups = GROUPED ? a.nb >> a.low_bits : 1u;
+  const uint32_t bins = GROUPED ? 1u << a.low_bits : a.nb >> a.low_bits;
+  const uint32_t tiles = GROUPED ? s_first[groups] : (n + skew_of(in) + T - 1) / T;
+  const K lo = (K)m.lo;
+  const uint32_t last = a.nb - 1, mask = bins - 1, shift = GROUPED ? 32u - a.nb_bits : 32u - a.nb_bits + a.low_bits;
+  auto digit = [&](K key) {
+    if constexpr (PLAIN) {
+      const uint32_t d = top_word(key) >> shift;
+      return GROUPED ? d & mask : d;
+    } else {
+      const uint32_t b = map_bucket(map_t<K>(key, lo, m.s), m.mult, last);
+      return GROUPED ? b & mask : b >> a.low_bits;
+    }
+  };
+  uint32_t* cursor0 = GROUPED ? a.cursor : (a.low_bits ? a.group_cursor : a.cursor);
+  // The tile in hand: keys [g0, g1) of group g; the group's tiles start at the
+  // 16-byte boundary at or below g0.
+  uint32_t g = 0, g0 = 0, g1 = n;
+  long long tlo = 0;
+  bool full = false;
+  K k[ITEMS];
+  uint32_t valid = 0;  // bit j: item j is a key of the tile (not kept for a full tile)
+  auto load = [&](uint32_t tile) {
+    uint32_t t = tile;
+    if constexpr (GROUPED) {
+      uint32_t h = groups;  // g: the last group whose first tile is <= tile
+      g = 0;
+      while (h - g > 1) {
+        const uint32_t mid = (g + h) >> 1;
+        if (s_first[mid] <= tile) g = mid;
+        else h = mid;
+      }
+      t = tile - s_first[g];
+      g0 = a.start[g << a.low_bits];
+      g1 = a.start[(g + 1) << a.low_bits];
+    }
+    tlo = (long long)g0 - skew_of(in + g0) + (long long)t * T;
+    full = tlo >= (long long)g0 && tlo + (long long)T <= (long long)g1;
+    if (full) {
+      const uint4* src = reinterpret_cast<const uint4*>(in + tlo) + tid;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const uint4 v = src[q * kScatterBlock];
+        const K* e = reinterpret_cast<const K*>(&v);
+#pragma unroll
+        for (int i = 0; i < V; ++i) k[q * V + i] = e[i];
+      }
+    } else {
+      valid = 0;
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j) {
+        const long long x = tlo + (long long)j * kScatterBlock + tid;
+        const bool ok = x >= (long long)g0 && x < (long long)g1;
+        k[j] = ok ? in[x] : (K)0;
+        valid |= ok ? 1u << j : 0u;
+      }
+    }
+  };
+  if (blockIdx.x < tiles) load(blockIdx.x);
+  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    if (tid < kGroups) s_cnt[tid] = 0;
+    if constexpr (FLT) {
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j) k[j] = to_ordered(k[j], true);
+    }
+    __syncthreads();
+    uint32_t r[(ITEMS + 1) / 2];  // ranks in the tile's bins, two 16-bit halves per word
+#pragma unroll
+    for (int j = 0; j < (ITEMS + 1) / 2; ++j) r[j] = 0;
+    if (full) {
+      const uint32_t d0 = digit(k[0]);
+      if (__all_sync(kFull, d0 == __shfl_sync(kFull, d0, 0))) {
+        // Sorted or constant runs: the atomics of a warp that agrees would queue
+        // on one word, so where all of a vector's keys agree the warp adds once.
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const uint32_t dq = digit(k[q * V]);
+          bool one = dq == __shfl_sync(kFull, dq, 0);
+#pragma unroll
+          for (int i = 1; i < V; ++i) one = one && digit(k[q * V + i]) == dq;
+          if (__all_sync(kFull, one)) {
+            uint32_t x = 0;
+            if (lane == 0) x = atomicAdd(s_cnt + dq, 32u * V);
+            x = __shfl_sync(kFull, x, 0) + lane;
+#pragma unroll
+            for (int i = 0; i < V; ++i) r[(q * V + i) / 2] |= (x + 32u * i) << (16 * ((q * V + i) % 2));
+          } else {
+#pragma unroll
+            for (int j = q * V; j < q * V + V; ++j) r[j / 2] |= atomicAdd(s_cnt + digit(k[j]), 1u) << (16 * (j % 2));
+          }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j) r[j / 2] |= atomicAdd(s_cnt + digit(k[j]), 1u) << (16 * (j % 2));
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j)
+        if ((valid >> j) & 1u) r[j / 2] |= atomicAdd(s_cnt + digit(k[j]), 1u) << (16 * (j % 2));
+    }
+    __syncthreads();
+    uint32_t c = 0, at = 0;
+    if (tid < bins) {
+      c = s_cnt[tid];
+      if (c) at = atomicAdd(cursor0 + (size_t)g * bins + tid, c);
+    }
+    const uint32_t excl = os::block_exclusive_scan<kScatterBlock>(c, s_warp);
+    if (tid < bins) s_start[tid] = excl;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j)
+      if (full || ((valid >> j) & 1u)) s_keys[s_start[digit(k[j])] + ((r[j / 2] >> (16 * (j % 2))) & 0xFFFFu)] = k[j];
+    const bool was_full = full;
+    const uint32_t cnt = was_full ? T : (uint32_t)(min(tlo + (long long)T, (long long)g1) - max(tlo, (long long)g0));
+    if (tid < bins) s_base[tid] = at - excl;  // (the reservation's round trip passes during the staging)
+    // the next tile's keys are on their way while this one is written out
+    if (tile + gridDim.x < tiles) load(tile + gridDim.x);
+    __syncthreads();
+    if (was_full) {
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j) {
+        const uint32_t i = (uint32_t)j * kScatterBlock + tid;
+        const K key = s_keys[i];
+        const uint32_t o = s_base[digit(key)] + i;
+        if (o < n) out[o] = key;
+      }
+    } else {
+      for (uint32_t i = tid; i < cnt; i += kScatterBlock) {
+        const K key = s_keys[i];
+        const uint32_t o = s_base[digit(key)] + i;
+        if (o < n) out[o] = key;
+      }
+    }
+    // no barrier here: the next tile's writes to s_cnt, s_start / s_base and
+    // s_keys each come after a barrier that every thread reaches only past
+    // its last read of them
+  }
+}
+
+template <typename K, bool GROUPED, bool FLT>
+__global__ void __launch_bounds__(kScatterBlock, kScatterPerSm) bucket_scatter_kernel(const K* in, K* out, size_t n, BucketArgs a) {
+  __shared__ __align__(16) K s_keys[kScatterTile<K>];
+  __shared__ uint32_t s_cnt[kGroups], s_start[kGroups], s_base[kGroups];
+  __shared__ uint32_t s_warp[kScatterBlock / 32];
+  __shared__ uint32_t s_first[kGroups + 1];
+  const BucketMap m = *a.map;
+  if (!m.on) return;
+  if constexpr (GROUPED) {
+    for (uint32_t i = threadIdx.x; i <= (a.nb >> a.low_bits); i += kScatterBlock) s_first[i] = a.tile_first[i];
+    __syncthreads();
+  }
+  if (m.plain)
+    scatter_tiles<K, GROUPED, FLT, true>(in, out, (uint32_t)n, a, m, s_keys, s_cnt, s_start, s_base, s_warp, s_first);
+  else
+    scatter_tiles<K, GROUPED, FLT, false>(in, out, (uint32_t)n, a, m, s_keys, s_cnt, s_start, s_base, s_warp, s_first);
+}
+
+// ---------------------------------------------------------------------------
+// Finish: sort each bucket.
+// ---------------------------------------------------------------------------
+// A bucket's keys are spread over kCells cells of equal width, about twenty
+// cells per key, kept as a bitmap: one entry per 32 cells holds their bits and,
+// once scanned, the number of keys before them.  A key's place is that number
+// plus the set bits below its own: one atomic OR, one shared read, one popcount,
+// no comparing.  The few keys that find their cell taken (about m^2 / (2 kCells)
+// of m) are listed and counted beside the bits; they follow the entry's other
+// keys, and the thread of the entry's first such key sorts the entry's few keys
+// by comparing.  Buckets where that would be many (equal keys, clusters) are
+// counted per bin instead (finish_counted), and buckets larger than shared
+// memory, or crowded even there, take finish_slow.
+//
+// Bound by instruction issue and the shared-memory pipe together (about 60 %
+// of each): 100M uniform 32-bit keys in 0.328 ms.  On the way there (same
+// input): bins of one key on average and each key compared with its bin 0.80
+// ms; the bitmap with 512 threads and a branch per key 0.59; 256 threads and
+// more keys in flight 0.45; collisions listed instead of handled where they are
+// found 0.41; no branch per key, and the next bucket's job left to one thread,
+// 0.33.  Four CTAs per SM of 64 registers: five (48 registers) spill and lose
+// more than they hide; 512 threads with the keys re-read from shared memory
+// 0.41.  64-bit keys need 88 KB a CTA: two per SM.
+constexpr int kFinishBlock = 256;
+template <typename K>
+constexpr int kFinishPerSm = sizeof(K) == 4 ? 4 : 2;
+constexpr uint32_t kFinishCap = 4096;
+constexpr int kFinishItems = (int)kFinishCap / kFinishBlock;
+constexpr uint32_t kEntries = kCells / 32;
+constexpr uint32_t kEntryHits = 6;  // keys of one entry that found their cell taken, at most
+constexpr uint32_t kHits = 256;     // such keys of one bucket, at most
+
+// The least t with umulhi(t, mult) >= b (b < nb), from the rounded-down
+// reciprocal inv = 2^63 / mult: the estimate is at most two short.
+__device__ __forceinline__ uint32_t bucket_first_t(uint32_t b, const BucketMap& m) {
+  uint32_t t = (uint32_t)__umul64hi((unsigned long long)b << 33, m.inv);
+  while (__umulhi(t, m.mult) < b) ++t;
+  return t;
+}
+
+// Bin counters are padded by 4 words per 16, so that a thread's 16-byte reads
+// of its own run of bins in the scan touch every bank once per quarter warp.
+__device__ __forceinline__ uint32_t bin_at(uint32_t bin) { return bin + ((bin >> 4) << 2); }
+constexpr uint32_t kBinWords = kBucketBins + kBucketBins / 4;
+
+// bytes of the bitmap, or of the bins
+constexpr size_t kFinishAux = kEntries * 8 > (kBinWords + 4) * 4 ? kEntries * 8 : (kBinWords + 4) * 4;
+
+// A bucket too large for shared memory, or with many keys in one bin: stable
+// 8-bit LSD passes by the one CTA, a[0, m) and b[0, m) in turn; the result is
+// left in `a` when `into_a`, else in `b`.  Slow (a few hundred cycles per 512
+// keys and pass) and rare: the plan's sample bounds how large such a bucket
+// is likely to be, and the bits all its keys share are skipped.
+template <typename K>
+__device__ __noinline__ void finish_slow(K* a, K* b, uint32_t m, bool into_a, unsigned char* smem) {
+  constexpr int B = kFinishBlock, W = B / 32;
+  uint32_t* s_cur = reinterpret_cast<uint32_t*>(smem);                // [256]
+  uint32_t* s_wc = s_cur + 256;                                       // [W][256]
+  uint32_t* s_warp = s_wc + W * 256;                                  // [W]
+  K* s_mm = reinterpret_cast<K*>(s_warp + W);                         // [2 * W]
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  K lo = ~(K)0, hi = 0;
+  for (uint32_t i = tid; i < m; i += B) {
+    const K x = a[i];
+    lo = min(lo, x);
+    hi = max(hi, x);
+  }
+  warp_minmax(lo, hi);
+  __syncthreads();
+  if (lane == 0) {
+    s_mm[warp] = lo;
+    s_mm[W + warp] = hi;
+  }
+  __syncthreads();
+  for (int w = 0; w < W; ++w) {
+    lo = min(lo, s_mm[w]);
+    hi = max(hi, s_mm[W + w]);
+  }
+  const K diff = lo ^ hi;  // keys agree above its highest bit
+  K *src = a, *dst = b;
+  for (uint32_t sh = 0; sh < 8 * sizeof(K) && (diff >> sh) != 0; sh += 8) {
+    __syncthreads();
+    for (uint32_t i = tid; i < 256; i += B) s_cur[i] = 0;
+    __syncthreads();
+    for (uint32_t i = tid; i < m; i += B) atomicAdd(s_cur + ((uint32_t)(src[i] >> sh) & 255u), 1u);
+    __syncthreads();
+    const uint32_t c = tid < 256 ? s_cur[tid] : 0u;
+    const uint32_t e = os::block_exclusive_scan<B>(c, s_warp);
+    if (tid < 256) s_cur[tid] = e;
+    for (uint32_t base = 0; base < m; base += B) {
+      for (uint32_t i = tid; i < (uint32_t)W * 256; i += B) s_wc[i] = 0;
+      __syncthreads();
+      const uint32_t i = base + tid;
+      const bool ok = i < m;
+      const K x = ok ? src[i] : (K)0;
+      const uint32_t d = ok ? (uint32_t)(x >> sh) & 255u : 256u;
+      const uint32_t peers = __match_any_sync(kFull, d);
+      const uint32_t below = __popc(peers & lanemask_lt());
+      if (ok && below == 0) s_wc[warp * 256 + d] = __popc(peers);
+      __syncthreads();
+      if (tid < 256) {
+        uint32_t run = s_cur[tid];
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const uint32_t y = s_wc[w * 256 + tid];
+          s_wc[w * 256 + tid] = run;
+          run += y;
+        }
+        s_cur[tid] = run;
+      }
+      __syncthreads();
+      if (ok) {
+        const uint32_t o = s_wc[warp * 256 + d] + below;
+        if (o < m) dst[o] = x;
+      }
+      __syncthreads();
+    }
+    K* sw = src;
+    src = dst;
+    dst = sw;
+  }
+  __syncthreads();  // (this CTA's global writes are visible to its own threads after a barrier)
+  K* want = into_a ? a : b;
+  if (src != want)
+    for (uint32_t i = tid; i < m; i += B) want[i] = src[i];
+  __syncthreads();
+}
+
+// A bucket of at most CAP keys counted per bin ([first, first + 1 << shift)
+// and so on): keys placed by their bin's start and the atomic's return, then
+// each key compared with the others of its bin, unless every bin is one value
+// (`exact`).  Returns false, with nothing written, when a bin holds too many
+// different keys for that.
+template <typename K, bool FLT>
+__device__ __noinline__ bool finish_counted(const K* in, K* out, uint32_t cnt, K first, uint32_t shift, bool exact,
+                                            unsigned char* smem, uint32_t* s_warp) {
+  constexpr int B = kFinishBlock;
+  constexpr uint32_t CAP = kFinishCap;
+  constexpr int PER = (int)kBucketBins / B;  // bins per thread in the scan
+  static_assert(PER % 4 == 0, "a thread's bins are read as 16-byte vectors");
+  K* s_keys = reinterpret_cast<K*>(smem);
+  uint32_t* s_bin = reinterpret_cast<uint32_t*>(smem + (size_t)CAP * sizeof(K));
+  const uint32_t tid = threadIdx.x;
+  for (uint32_t i = tid * 4; i < kBinWords; i += B * 4)
+    *reinterpret_cast<uint4*>(s_bin + i) = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+  auto bin_of = [&](K key) {
+    const K x = (key > first ? key - first : (K)0) >> shift;
+    return x < (K)kBucketBins ? (uint32_t)x : kBucketBins - 1;
+  };
+  for (uint32_t i = tid; i < cnt; i += B) atomicAdd(s_bin + bin_at(bin_of(in[i])), 1u);
+  __syncthreads();
+  uint32_t c[PER];
+  uint32_t local = 0, mx = 0;
+#pragma unroll
+  for (int q = 0; q < PER / 4; ++q) {
+    const uint4 x = *reinterpret_cast<const uint4*>(s_bin + bin_at(tid * PER) + 4 * q);
+    c[4 * q] = x.x;
+    c[4 * q + 1] = x.y;
+    c[4 * q + 2] = x.z;
+    c[4 * q + 3] = x.w;
+  }
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    local += c[i];
+    mx = max(mx, c[i]);
+  }
+  uint32_t run = os::block_exclusive_scan<B>(local, s_warp);
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {  // the bins' ends, counted down to their starts below
+    run += c[i];
+    c[i] = run;
+  }
+#pragma unroll
+  for (int q = 0; q < PER / 4; ++q)
+    *reinterpret_cast<uint4*>(s_bin + bin_at(tid * PER) + 4 * q) =
+        make_uint4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
+  if (__syncthreads_or(!exact && mx > kBucketBinMax)) return false;
+  for (uint32_t i = tid; i < cnt; i += B) {
+    const K key = in[i];
+    s_keys[atomicSub(s_bin + bin_at(bin_of(key)), 1u) - 1u] = key;
+  }
+  __syncthreads();  // (s_bin: the bins' starts; every key of `in` has been read)
+  for (uint32_t p = tid; p < cnt; p += B) {
+    const K key = s_keys[p];
+    uint32_t o = p;
+    if (!exact) {
+      const uint32_t bin = bin_of(key);
+      const uint32_t s0 = s_bin[bin_at(bin)];
+      const uint32_t s1 = bin + 1 < kBucketBins ? s_bin[bin_at(bin + 1)] : cnt;
+      o = s0;
+      for (uint32_t i = s0; i < s1; ++i) {
+        const K x = s_keys[i];
+        o += (x < key || (x == key && i < p)) ? 1u : 0u;
+      }
+    }
+    out[o] = from_ordered(key, FLT);
+  }
+  return true;
+}
+
+// What thread 0 prepares of the next bucket while the CTA works on one.
+template <typename K>
+struct FinishJob {
+  K first;        // the bucket's least key: that of the least t with umulhi(t, mult) >= b
+  uint32_t at;    // its keys: [at, at + cnt)
+  uint32_t cnt;
+  uint32_t kind;  // 0: nothing to do, 1: cells, keys bulk-copied, 2: cells, plain loads, 3: counted or slow
+  uint32_t exact;
+};
+
+// in == out: buckets are sorted in place and `other` is scratch; else in is
+// the scratch array and other == out.
+template <typename K, bool FLT>
+__global__ void __launch_bounds__(kFinishBlock, kFinishPerSm<K>)
+    bucket_finish_kernel(K* in, K* out, K* other, size_t n, BucketArgs a) {
+  constexpr int ITEMS = kFinishItems;
+  constexpr uint32_t B = kFinishBlock;
+  constexpr uint32_t CAP = kFinishCap;
+  constexpr int C = 4;  // items handled together: their atomics in flight at once
+  constexpr int W = B / 32;
+  constexpr int U = (int)kEntries / (W * 64);  // 16-byte reads (two entries) per lane in the scan
+  constexpr uint32_t V = 16 / sizeof(K);
+  static_assert(U == 2 || U == 4, "runs of 64 entries per warp, scanned in pairs as 16-bit halves of one word");
+  static_assert(kHits <= B, "one listed key per thread");
+  extern __shared__ __align__(128) unsigned char smem[];
+  K* s_keys = reinterpret_cast<K*>(smem);                                           // [CAP + V]
+  uint2* s_entry = reinterpret_cast<uint2*>(smem + (CAP + V) * sizeof(K));          // [kEntries]
+  K* s_in = reinterpret_cast<K*>(smem + (CAP + V) * sizeof(K) + kFinishAux);        // [CAP + 2 * V]
+  K* s_hit = s_in + CAP + 2 * V;                                                    // [kHits]
+  __shared__ FinishJob<K> s_job[2];
+  __shared__ uint32_t s_warp[W];
+  __shared__ uint32_t s_nhit, s_over;
+  __shared__ __align__(8) uint64_t s_bar;
+  const BucketMap m = *a.map;
+  if (!m.on) return;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t cs = m.cell_shift;
+  auto entry_of = [&](K x) {  // (byte offset: the entry's number times 8)
+    return reinterpret_cast<uint2*>(reinterpret_cast<char*>(s_entry) + ((uint32_t)(x >> (cs + 2)) & ((kEntries - 1) * 8)));
+  };
+  auto cell_of = [&](K x) { return (uint32_t)(x >> cs) & 31u; };
+  // thread 0: bucket b's job, and its keys' bulk copy into s_in, from the
+  // 16-byte boundary at or below the first key to the one at or above the end
+  auto prepare = [&](uint32_t b, uint32_t at, uint32_t end, FinishJob<K>* job) {
+    const uint32_t cnt = end - at;
+    job->first = (K)m.lo + ((K)bucket_first_t(b, m) << m.s);
+    job->at = at;
+    job->cnt = cnt;
+    // (the first and last bucket also hold the keys outside the map)
+    const bool inner = b != 0 && b < a.nb - 1;
+    job->exact = m.exact && inner ? 1u : 0u;
+    uint32_t kind = 3;
+    if (cnt == 0 || (size_t)end > n) {
+      kind = 0;
+    } else if (inner && cnt <= CAP) {
+      const uint32_t skew = skew_of(in + at);
+      const uint32_t len = (skew + cnt + V - 1) / V * V;
+      kind = 2;
+      if (at >= skew && (size_t)at - skew + len <= n) {
+        kind = 1;
+        fence_proxy_async();
+        mbar_arrive_expect_tx(&s_bar, len * (uint32_t)sizeof(K));
+        bulk_load_g2s(s_in, in + at - skew, len * (uint32_t)sizeof(K), &s_bar);
+      }
+    }
+    job->kind = kind;
+  };
+  uint32_t at_next = 0, end_next = 0;  // (thread 0) the bucket after the prepared one
+  if (tid == 0) {
+    mbar_init(&s_bar, 1);
+    mbar_fence_init();
+    prepare(blockIdx.x, a.start[blockIdx.x], a.start[blockIdx.x + 1], &s_job[0]);
+    if (blockIdx.x + gridDim.x < a.nb) {
+      at_next = a.start[blockIdx.x + gridDim.x];
+      end_next = a.start[blockIdx.x + gridDim.x + 1];
+    }
+  }
+  uint32_t parity = 0, slot = 0;
+  for (uint32_t b = blockIdx.x; b < a.nb; b += gridDim.x, slot ^= 1u) {
+    if (tid == 0) {
+      s_nhit = 0;
+      s_over = 0;
+    }
+    for (uint32_t q = tid; q < kEntries / 2; q += B) reinterpret_cast<uint4*>(s_entry)[q] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();  // the job is there; everything of the last bucket is done with
+    const FinishJob<K> job = s_job[slot];
+    const uint32_t cnt = job.cnt;
+    const K first = job.first;
+    // thread 0, once s_in has been read: the next bucket
+    auto next = [&]() {
+      const uint32_t nx = b + gridDim.x;
+      if (tid == 0 && nx < a.nb) {
+        prepare(nx, at_next, end_next, &s_job[slot ^ 1u]);
+        if (nx + gridDim.x < a.nb) {
+          at_next = a.start[nx + gridDim.x];
+          end_next = a.start[nx + gridDim.x + 1];
+        }
+      }
+    };
+    bool done = job.kind == 0;
+    if (job.kind == 0 || job.kind == 3) next();
+    if (job.kind == 1 || job.kind == 2) {
+      const uint32_t skew_in = skew_of(in + job.at);
+      const K* src = s_in + skew_in + tid;
+      bool ok = true;
+      if (job.kind == 1) {
+        ok = mbar_wait_bounded(&s_bar, parity, a.err);
+        parity ^= 1u;
+      } else {
+        for (uint32_t i = tid; i < cnt; i += B) s_in[skew_in + i] = in[job.at + i];  // (read by the same thread)
+      }
+      K k[ITEMS];  // distances from `first`; past the end, whatever s_in holds
+      uint32_t hit = 0;   // bit j: key j found its cell taken
+      uint32_t skip = 0;  // bit j: that, or there is no key j
+#pragma unroll
+      for (int c = 0; c < ITEMS; c += C) {
+        if ((uint32_t)c * B >= cnt) break;
+        uint32_t old[C];
+        if ((uint32_t)(c + C) * B <= cnt) {
+#pragma unroll
+          for (int j = 0; j < C; ++j) {
+            k[c + j] = src[(uint32_t)(c + j) * B] - first;
+            old[j] = atomicOr(&entry_of(k[c + j])->x, 1u << cell_of(k[c + j]));
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < C; ++j) {
+            const bool has = (uint32_t)(c + j) * B + tid < cnt;
+            k[c + j] = src[(uint32_t)(c + j) * B] - first;
+            old[j] = atomicOr(&entry_of(k[c + j])->x, has ? 1u << cell_of(k[c + j]) : 0u);
+            skip |= has ? 0u : 1u << (c + j);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < C; ++j) hit |= ((old[j] >> cell_of(k[c + j])) & 1u) << (c + j);
+      }
+      hit &= ~skip;
+      skip |= hit;
+      if (hit) {
+        uint32_t p = atomicAdd(&s_nhit, (uint32_t)__popc(hit));
+        for (uint32_t h = hit; h; h &= h - 1u, ++p)
+          if (p < kHits) s_hit[p] = src[((uint32_t)__ffs((int)h) - 1u) * B] - first;
+      }
+      if (!ok) s_over = 2;
+      __syncthreads();
+      const uint32_t nhit = s_nhit;
+      if (s_over == 2) {  // the copy never came: wait it out once more, sort nothing further
+        mbar_wait_bounded(&s_bar, parity ^ 1u, a.err);
+        if (tid == 0) bulk_store_wait_all();
+        return;
+      }
+      next();
+      bool crowded = nhit > kHits;
+      K hx = 0;               // this thread's listed key
+      uint32_t turn = 0;      // its number among its entry's listed keys
+      uint32_t listed = 0, span = 0;  // how many those are; all of the entry's keys
+      if (nhit && !crowded) {
+        if (tid < nhit) {
+          hx = s_hit[tid];
+          turn = atomicAdd(&entry_of(hx)->y, 1u);
+          if (turn >= kEntryHits) s_over = 1;
+        }
+        __syncthreads();
+        crowded = s_over != 0;
+      }
+      if (!crowded) {
+        // Scan: warp w owns kEntries / W entries, lane l entries 2 l and 2 l + 1
+        // of each run of 64.  An entry's keys: its set bits and its listed keys.
+        uint4 q[U];
+        uint32_t c2[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          q[u] = reinterpret_cast<uint4*>(s_entry)[(warp * U + u) * 32 + lane];
+          q[u].y += __popc(q[u].x);
+          c2[u] = q[u].y + q[u].w + __popc(q[u].z);
+        }
+        if (tid < nhit) {
+          const uint2 e = *entry_of(hx);
+          listed = e.y;
+          span = e.y + __popc(e.x);
+        }
+        uint32_t p2[U / 2], t2[U / 2];
+#pragma unroll
+        for (int u = 0; u < U / 2; ++u) p2[u] = c2[2 * u] | (c2[2 * u + 1] << 16);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+          for (int u = 0; u < U / 2; ++u) {
+            const uint32_t x = __shfl_up_sync(kFull, p2[u], o);
+            if (lane >= (uint32_t)o) p2[u] += x;
+          }
+        }
+        uint32_t total = 0;
+#pragma unroll
+        for (int u = 0; u < U / 2; ++u) {
+          t2[u] = __shfl_sync(kFull, p2[u], 31);
+          total += (t2[u] & 0xFFFFu) + (t2[u] >> 16);
+        }
+        if (lane == 0) s_warp[warp] = total;
+        // (the last bucket's copy out of s_keys must have read it)
+        if (tid == 0) bulk_store_wait_read();
+        __syncthreads();
+        uint32_t before = __reduce_add_sync(kFull, lane < warp ? s_warp[lane & (W - 1)] : 0u);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const uint32_t run = before + (u & 1 ? p2[u / 2] >> 16 : p2[u / 2] & 0xFFFFu) - c2[u];
+          before += u & 1 ? t2[u / 2] >> 16 : t2[u / 2] & 0xFFFFu;
+          q[u].w = run + q[u].y;
+          q[u].y = run;
+          reinterpret_cast<uint4*>(s_entry)[(warp * U + u) * 32 + lane] = q[u];
+        }
+        __syncthreads();
+        // staged with the destination's own offset from a 16-byte boundary
+        K* dst = out + job.at;
+        const uint32_t skew = skew_of(dst);
+        K* stage = s_keys + skew;
+#pragma unroll
+        for (int c = 0; c < ITEMS; c += C) {
+          if ((uint32_t)c * B >= cnt) break;
+#pragma unroll
+          for (int j = c; j < c + C; ++j) {
+            const uint2 e = *entry_of(k[j]);
+            const uint32_t p = e.y + __popc(e.x & ((1u << cell_of(k[j])) - 1u));
+            if (!((skip >> j) & 1u)) stage[p & (CAP - 1)] = from_ordered((K)(k[j] + first), FLT);
+          }
+        }
+        if (nhit) {
+          uint32_t lo = 0, bits = 0;
+          if (tid < nhit) {
+            const uint2 e = *entry_of(hx);
+            lo = e.y;
+            bits = e.x;
+            if (listed > 1) stage[(lo + __popc(bits) + turn) & (CAP - 1)] = from_ordered((K)(hx + first), FLT);
+          }
+          __syncthreads();
+          if (listed == 1) {  // between the key it met and the next: those above move up by one
+            const uint32_t r = lo + __popc(bits & ((1u << cell_of(hx)) - 1u));
+            const uint32_t top = min(CAP, lo + span) - 1u;
+            for (uint32_t j = top; j > r + 1; --j) stage[j] = stage[j - 1];
+            const K x = from_ordered((K)(hx + first), FLT), y = stage[r];
+            const bool below = hx + first < to_ordered(y, FLT);
+            stage[r] = below ? x : y;
+            if (r < top) stage[r + 1] = below ? y : x;
+          } else if (listed > 1 && turn == 0) {  // several: the entry's keys are sorted
+            const uint32_t hi = min(CAP, lo + span);
+            for (uint32_t j = lo + 1; j < hi; ++j) {
+              const K x = stage[j];
+              uint32_t p = j;
+              while (p > lo) {
+                const K y = stage[p - 1];
+                if (to_ordered(y, FLT) <= to_ordered(x, FLT)) break;
+                stage[p] = y;
+                --p;
+              }
+              stage[p] = x;
+            }
+          }
+        }
+        // out: whole 16-byte units in one bulk copy, the keys before the first
+        // and after the last boundary singly
+        fence_proxy_async();
+        __syncthreads();
+        const uint32_t head = min(cnt, (V - skew) & (V - 1));
+        const uint32_t body = (cnt - head) / V * V;
+        if (tid == 0 && body) bulk_store_s2g(dst + head, stage + head, body * (uint32_t)sizeof(K));
+        if (tid >= 32 && tid < 32 + V) {  // (V - 1 keys at most each)
+          const uint32_t i = tid - 32;
+          if (i < head) dst[i] = stage[i];
+          if (head + body + i < cnt) dst[head + body + i] = stage[head + body + i];
+        }
+        done = true;
+      }
+    }
+    if (!done) {
+      if (tid == 0) bulk_store_wait_read();
+      __syncthreads();  // s_keys and s_entry are free
+      if (cnt <= CAP) done = finish_counted<K, FLT>(in + job.at, out + job.at, cnt, first, m.bin_shift, job.exact != 0, smem, s_warp);
+      if (!done) {
+        finish_slow<K>(in + job.at, other + job.at, cnt, in == out, smem);
+        if (FLT)
+          for (uint32_t i = tid; i < cnt; i += B) out[job.at + i] = from_ordered(out[job.at + i], true);
+      }
+      __syncthreads();
+    }
+  }
+  if (tid == 0) bulk_store_wait_all();
+}
+
+template <typename K>
+constexpr size_t finish_smem() {
+  constexpr size_t V = 16 / sizeof(K);
+  static_assert((256 + (kFinishBlock / 32) * 257) * 4 + 2 * (kFinishBlock / 32) * sizeof(K) <=
+                    kFinishCap * sizeof(K) + kFinishAux, "finish_slow fits");
+  return (2 * (size_t)kFinishCap + 3 * V + kHits) * sizeof(K) + kFinishAux;
+}
+
+template <typename K>
+BucketArgs make_args(const BucketScratch& s, const K* tmp, size_t n, SortCtrl* ctrl, uint32_t* err) {
+  BucketArgs a{};
+  a.map = s.map;
+  a.ctrl = ctrl;
+  a.err = err;
+  a.count = s.count;
+  a.start = s.start;
+  a.cursor = s.cursor;
+  a.group_cursor = s.group_cursor;
+  a.tile_first = s.tile_first;
+  a.nb = s.nb;
+  while ((1u << a.nb_bits) < s.nb) ++a.nb_bits;
+  a.low_bits = s.low_bits;
+  a.tile = kScatterTile<K>;
+  a.tmp_align = (uint32_t)(reinterpret_cast<uintptr_t>(tmp) & 15u);
+  // sample keys a bucket may hold: one that would be full, with room for chance
+  const double mean = (double)kSample / s.nb;
+  const double cap = (double)kFinishCap * (double)kSample / (double)n;
+  const double high = std::max(cap, mean + 6.0 * std::max(1.0, std::sqrt(mean)));
+  a.hot_above = (uint32_t)high;
+  a.max_sample = (uint32_t)(high + 4.0 + 2.0 * mean);
+  return a;
+}
+
+template <typename K>
+cudaError_t plan_t(const BucketArgs& a, const K* keys, size_t n, bool is_float, cudaStream_t stream) {
+  bucket_plan_kernel<K><<<kPlanCtas, kPlanBlock, 0, stream>>>(keys, n, is_float ? 1 : 0, a);
+  return cudaGetLastError();
+}
+
+template <typename K, bool FLT>
+cudaError_t sort_t(const BucketArgs& a, K* keys, K* tmp, size_t n, cudaStream_t stream,
+                   const std::function<cudaError_t()>& mark) {
+  const unsigned sms = (unsigned)device_info().sm_count;
+  auto m = [&]() { return mark ? mark() : cudaSuccess; };
+  cudaError_t e = cudaSuccess;
+  {
+    auto kern = bucket_count_kernel<K, FLT>;
+    const size_t smem = (size_t)std::max<uint32_t>(a.nb, 1024) * 4;
+    if ((e = ensure_dynamic_smem(kern, (size_t)kBucketsMax * 4)) != cudaSuccess) return e;
+    const size_t work = ceil_div(n, (size_t)kCountBlock * (16 / sizeof(K)) * 2);
+    kern<<<(unsigned)std::min<size_t>(std::max<size_t>(work, 1), sms), kCountBlock, smem, stream>>>(keys, n, a);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  if ((e = m()) != cudaSuccess) return e;
+  if ((e = m()) != cudaSuccess) return e;
+  const size_t tiles = ceil_div(n, (size_t)kScatterTile<K>) + 1;
+  bucket_scatter_kernel<K, false, FLT>
+      <<<(unsigned)std::min<size_t>(tiles, sms * kScatterPerSm), kScatterBlock, 0, stream>>>(keys, tmp, n, a);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if ((e = m()) != cudaSuccess) return e;
+  K* in = tmp;
+  if (a.low_bits) {
+    bucket_scatter_kernel<K, true, false>
+        <<<(unsigned)std::min<size_t>(tiles + kGroups, sms * kScatterPerSm), kScatterBlock, 0, stream>>>(tmp, keys, n, a);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    in = keys;
+  }
+  if ((e = m()) != cudaSuccess) return e;
+  auto kern = bucket_finish_kernel<K, FLT>;
+  if ((e = ensure_dynamic_smem(kern, finish_smem<K>())) != cudaSuccess) return e;
+  kern<<<std::min<unsigned>(a.nb, sms * kFinishPerSm<K>), kFinishBlock, finish_smem<K>(), stream>>>(
+      in, keys, a.low_bits ? tmp : keys, n, a);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  return m();
+}
+
+__global__ void clear_kernel(uint4* p, size_t words, uint32_t* tail, uint32_t tail_words, const uint32_t* off) {
+  if (off && *off) return;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (size_t i = i0; i < words; i += stride) p[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (i0 < tail_words) tail[i0] = 0;
+}
+
+}  // namespace
+
+cudaError_t launch_clear(void* p, size_t bytes, const uint32_t* off, cudaStream_t stream) {
+  if (bytes % 4 || (reinterpret_cast<uintptr_t>(p) & 15u)) return cudaErrorInvalidValue;
+  const size_t vec = bytes / 16;
+  const unsigned grid = (unsigned)std::min(ceil_div(vec, (size_t)256 * 4) + 1, (size_t)device_info().sm_count * 4);
+  clear_kernel<<<grid, 256, 0, stream>>>(static_cast<uint4*>(p), vec, reinterpret_cast<uint32_t*>(static_cast<uint4*>(p) + vec),
+                                         (uint32_t)(bytes % 16 / 4), off);
+  return cudaGetLastError();
+}
+
+// A synchronous call of n uniform keys, this sort against the LSD passes:
+// 32-bit 100 K 50 us against 68, 700 K 59 against 76, 2.2M 80 against 112, 10M
+// 144 against 233, 100M 918 against 1640; 64-bit 100 K 51 against 119, 1M 74
+// against 154, 10M 222 against 550.  Keys that the plan turns away pay for it,
+// about 18 us (32-bit, Zipf: 100 K 84 against 66, 1M 102 against 84), so 32-bit
+// keys come here from 2^19 on, where the gain is at least that much; 64-bit keys
+// have eight LSD passes to save and come from the smallest size on.  Above
+// kBucketsMax * kBucketTarget keys a bucket would no longer fit the finish
+// kernel with room for uneven filling.
+bool bucket_sort_supported(size_t n, int key_bytes) {
+  if (key_bytes != 4 && key_bytes != 8) return false;
+  const size_t least = key_bytes == 4 ? (size_t)1 << 19 : small_sort_max_keys(key_bytes, false) + 1;
+  return n >= least && n <= (size_t)kBucketsMax * kBucketTarget;
+}
+
+size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s) {
+  uint32_t nb = 256;
+  while (nb < kBucketsMax && n > (size_t)nb * kBucketTarget) nb *= 2;
+  uint32_t lb = 0;
+  while ((1u << lb) < nb) ++lb;
+  s->nb = nb;
+  s->low_bits = nb <= kGroups ? 0u : lb / 2;
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    off = (off + 255) & ~(size_t)255;
+    char* p = base + off;
+    off += bytes;
+    return p;
+  };
+  s->map = reinterpret_cast<BucketMap*>(take(sizeof(BucketMap)));
+  s->count = reinterpret_cast<uint32_t*>(take((size_t)nb * 4));
+  s->start = reinterpret_cast<uint32_t*>(take(((size_t)nb + 1) * 4));
+  s->cursor = reinterpret_cast<uint32_t*>(take((size_t)nb * 4));
+  s->group_cursor = reinterpret_cast<uint32_t*>(take(kGroups * 4));
+  s->tile_first = reinterpret_cast<uint32_t*>(take((kGroups + 1) * 4));
+  return off;
+}
+
+cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, const void* tmp, size_t n, int key_bytes,
+                                bool is_float, SortCtrl* ctrl, uint32_t* decided, cudaStream_t stream) {
+  if (key_bytes == 8) {
+    BucketArgs a = make_args(s, static_cast<const unsigned long long*>(tmp), n, ctrl, nullptr);
+    a.decided = decided;
+    return plan_t(a, static_cast<const unsigned long long*>(keys), n, false, stream);
+  }
+  BucketArgs a = make_args(s, static_cast<const uint32_t*>(tmp), n, ctrl, nullptr);
+  a.decided = decided;
+  return plan_t(a, static_cast<const uint32_t*>(keys), n, is_float, stream);
+}
+
+cudaError_t enqueue_bucket_sort(const BucketScratch& s, void* keys, void* tmp, size_t n, int key_bytes, bool is_float,
+                                SortCtrl* ctrl, uint32_t* err, cudaStream_t stream,
+                                const std::function<cudaError_t()>& mark) {
+  if (key_bytes == 8) {
+    auto *k = static_cast<unsigned long long*>(keys), *t = static_cast<unsigned long long*>(tmp);
+    return sort_t<unsigned long long, false>(make_args(s, t, n, ctrl, err), k, t, n, stream, mark);
+  }
+  auto *k = static_cast<uint32_t*>(keys), *t = static_cast<uint32_t*>(tmp);
+  const BucketArgs a = make_args(s, t, n, ctrl, err);
+  return is_float ? sort_t<uint32_t, true>(a, k, t, n, stream, mark) : sort_t<uint32_t, false>(a, k, t, n, stream, mark);
+}
+
+}  // namespace pa

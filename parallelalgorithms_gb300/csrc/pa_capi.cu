@@ -84,7 +84,7 @@ constexpr int kPipeGroups = 10;  // host-buffer sort: bucket groups sorted and c
 constexpr size_t kReadBackWords = 2048;  // the largest small result: 8 digits' 256 counts
 struct HostBlock {
   uint32_t err;       // error word of bounded waits, zero between calls
-  uint32_t unused;
+  uint32_t decided;   // a bucket plan's decision
   uint64_t result;    // a select's or sum's result
   uint64_t words[kReadBackWords];
 };
@@ -547,7 +547,9 @@ int sort_impl(void* keys, void* tmp, uint32_t* vals, uint32_t* tmp_vals, size_t 
     }
     return cudaEventRecord(ws->ev[nev++], stream);
   };
-  PA_CUDA(enqueue_sort(sc, d_keys, d_tmp, d_vals, d_tvals, n, kb, is_float, ws->err, stream, mark));
+  const bool sync_call = timed || !(opts && opts->async_device) || !keys_dev || (has_vals && !vals_dev);
+  PA_CUDA(enqueue_sort(sc, d_keys, d_tmp, d_vals, d_tvals, n, kb, is_float, ws->err, stream, mark,
+                       sync_call ? &ws->host->decided : nullptr));
   if (!keys_dev) PA_CUDA(cudaMemcpyAsync(keys, d_keys, key_bytes_total, cudaMemcpyDeviceToHost, stream));
   if (has_vals && !vals_dev)
     PA_CUDA(cudaMemcpyAsync(vals, d_vals, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
@@ -886,12 +888,43 @@ size_t sort_scratch_layout(char* base, size_t n, int kb, bool has_vals, SortScra
   s->tile_prefix = prepared ? c.take<uint32_t>(tiles * 256) : nullptr;
   s->chunk_tot = prepared ? c.take<uint32_t>((size_t)kTileCountMaxChunks * 256) : nullptr;
   s->chunk_excl = prepared ? c.take<uint32_t>((size_t)kTileCountMaxChunks * 256) : nullptr;
+  s->buckets = BucketScratch{};
+  if (!has_vals && radix_bits == 8 && bucket_sort_supported(n, kb)) {
+    const size_t bytes = bucket_scratch_layout(nullptr, n, &s->buckets);
+    char* b = c.take<char>(bytes);
+    bucket_scratch_layout(b, n, &s->buckets);
+  }
   return c.off;
 }
 
+namespace {
+
+// Without a host that waits for the plan, both sorts' launches are enqueued, and
+// those of the one not taken cost about 35 us: at most 2-3 % of these sizes.
+constexpr size_t kBucketAsyncMin32 = (size_t)1 << 26;
+constexpr size_t kBucketAsyncMin64 = (size_t)1 << 24;
+constexpr uint32_t kUndecided = 0xFFFFFFFFu;
+
+// Polls page-locked memory for the plan's decision; the stream is asked now
+// and then, so that a failed launch or earlier error ends the wait.
+cudaError_t wait_decided(const uint32_t* decided, cudaStream_t stream, uint32_t* value) {
+  const volatile uint32_t* p = decided;
+  for (;;) {
+    for (int i = 0; i < 4096; ++i)
+      if ((*value = *p) != kUndecided) return cudaSuccess;
+    const cudaError_t e = cudaStreamQuery(stream);
+    if (e == cudaErrorNotReady) continue;
+    if (e != cudaSuccess) return e;
+    *value = *p;  // everything enqueued has run
+    return *value == kUndecided ? cudaErrorUnknown : cudaSuccess;
+  }
+}
+
+}  // namespace
+
 cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32_t* d_vals, uint32_t* d_tvals,
                          size_t n, int kb, bool is_float, uint32_t* err, cudaStream_t stream,
-                         const std::function<cudaError_t()>& mark) {
+                         const std::function<cudaError_t()>& mark, uint32_t* decided) {
   const int rb = s.radix_bits;
   const int passes = s.passes;
   const size_t bins = (size_t)1 << rb;
@@ -906,8 +939,31 @@ cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32
     if (e == cudaSuccess) e = m();
     return e;
   }
-  cudaError_t e = cudaMemsetAsync(s.zero_begin, 0, s.zero_bytes, stream);
-  if (e == cudaSuccess) e = m();
+  cudaError_t e = cudaSuccess;
+  const uint32_t* off = nullptr;
+  // (float keys crowd into a few buckets of an even map: the plan would turn
+  // nearly all of them away)
+  if (s.buckets.nb && !has_vals && !is_float && (decided || n >= (kb == 4 ? kBucketAsyncMin32 : kBucketAsyncMin64))) {
+    e = m();
+    if (decided) *reinterpret_cast<volatile uint32_t*>(decided) = kUndecided;
+    if (e == cudaSuccess) e = enqueue_bucket_plan(s.buckets, d_keys, d_tmp, n, kb, is_float, s.ctrl, decided, stream);
+    uint32_t by_buckets = 1;
+    if (decided && e == cudaSuccess) e = wait_decided(decided, stream, &by_buckets);
+    if (by_buckets && e == cudaSuccess)
+      e = enqueue_bucket_sort(s.buckets, d_keys, d_tmp, n, kb, is_float, s.ctrl, err, stream, mark);
+    if (decided && by_buckets) {
+      for (int p = 3; p <= passes && e == cudaSuccess; ++p) e = m();  // (no LSD launches, no final copy)
+      return e;
+    }
+    // decided here: the LSD passes alone; on the device: behind the bucket
+    // sort, where they find `off` set and do nothing if it ran
+    off = decided ? nullptr : &s.buckets.map->on;
+    if (e == cudaSuccess) e = launch_clear(s.zero_begin, s.zero_bytes, off, stream);
+  } else {
+    e = cudaMemsetAsync(s.zero_begin, 0, s.zero_bytes, stream);
+    if (e == cudaSuccess) e = m();
+  }
+  auto lsd_mark = [&]() { return off ? cudaSuccess : m(); };
   // With the tables (and 16-byte aligned keys) the histogram also prepares
   // the first pass's tile offsets.
   const bool prepared = s.tile_prefix && kb == 4 && rb == 8 && !has_vals && n < ((size_t)1 << 30) &&
@@ -916,11 +972,12 @@ cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32
   if (e == cudaSuccess)
     e = prepared ? launch_tile_counts(static_cast<const uint32_t*>(d_keys), n, onesweep_tile_keys(kb, false, rb),
                                       is_float, s.counts, s.tile_prefix, s.chunk_tot, s.chunk_excl, s.tc_ticket, &tpc,
-                                      stream)
-                 : launch_digit_counts(d_keys, n, kb, passes, rb, 0, (uint32_t)rb, is_float, s.counts, stream);
-  if (e == cudaSuccess) e = m();
-  if (e == cudaSuccess) e = launch_scan_digits(s.counts, passes, rb, n, is_float, true, s.bin_start, s.ctrl, stream);
-  if (e == cudaSuccess) e = m();
+                                      stream, off)
+                 : launch_digit_counts(d_keys, n, kb, passes, rb, 0, (uint32_t)rb, is_float, s.counts, stream, off);
+  if (e == cudaSuccess) e = lsd_mark();
+  if (e == cudaSuccess)
+    e = launch_scan_digits(s.counts, passes, rb, n, is_float, true, s.bin_start, s.ctrl, stream, off);
+  if (e == cudaSuccess) e = lsd_mark();
   for (int p = 0; p < passes && e == cudaSuccess; ++p) {
     OnesweepArgs a{};
     a.keys_a = d_keys;
@@ -943,8 +1000,9 @@ cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32
       a.tiles_per_chunk = tpc;
     }
     e = launch_onesweep_pass(a, kb, has_vals, stream);
-    if (e == cudaSuccess) e = m();
+    if (e == cudaSuccess) e = lsd_mark();
   }
+  for (int p = 3; off && p < passes && e == cudaSuccess; ++p) e = m();  // (the passes' shares after the buckets' three)
   if (e == cudaSuccess) e = launch_final_copy(d_keys, d_tmp, d_vals, d_tvals, n, kb, s.ctrl, stream);
   if (e == cudaSuccess) e = m();
   return e;

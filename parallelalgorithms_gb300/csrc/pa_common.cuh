@@ -169,6 +169,18 @@ __device__ __forceinline__ void bulk_load_g2s(void* smem_dst, const void* gmem_s
       : "memory");
 }
 
+// Shared -> global bulk copy (same alignment rules), committed as a group of
+// its own; waits for the calling thread's groups: until the copies have read
+// shared memory, or until they are complete.
+__device__ __forceinline__ void bulk_store_s2g(void* gmem_dst, const void* smem_src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem_dst), "r"(smem_addr(smem_src)),
+               "r"(bytes)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // Streaming 16-byte load that does not allocate in L1.
 __device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
   uint4 v;

@@ -51,7 +51,9 @@ constexpr size_t hist_smem_bytes() {
 template <typename K, int ND, int RB, bool BYTES, bool FLT>
 __global__ void __launch_bounds__(kHistBlock, 1) digit_counts_kernel(const K* __restrict__ keys, size_t n,
                                                                        uint32_t shift0, uint32_t step,
-                                                                       unsigned long long* __restrict__ out) {
+                                                                       unsigned long long* __restrict__ out,
+                                                                       const uint32_t* off) {
+  if (off && *off) return;
   constexpr int R = 1 << RB;
   constexpr int V = kVec<K>;
   constexpr int L = kLanes<ND, RB>;
@@ -125,7 +127,7 @@ __global__ void __launch_bounds__(kHistBlock, 1) digit_counts_kernel(const K* __
 
 template <typename K, int ND, int RB, bool BYTES, bool FLT>
 cudaError_t launch_counts_k(const void* keys, size_t n, uint32_t shift0, uint32_t step, unsigned long long* out,
-                            cudaStream_t stream) {
+                            cudaStream_t stream, const uint32_t* off) {
   constexpr int V = kVec<K>;
   auto kern = digit_counts_kernel<K, ND, RB, BYTES, FLT>;
   constexpr size_t smem = hist_smem_bytes<ND, RB>();
@@ -134,19 +136,19 @@ cudaError_t launch_counts_k(const void* keys, size_t n, uint32_t shift0, uint32_
   const size_t work = ceil_div(ceil_div(n, (size_t)V), (size_t)kHistBlock * 4);
   size_t blocks = work < (size_t)device_info().sm_count ? work : (size_t)device_info().sm_count;
   if (blocks < 1) blocks = 1;
-  kern<<<(unsigned)blocks, kHistBlock, smem, stream>>>(static_cast<const K*>(keys), n, shift0, step, out);
+  kern<<<(unsigned)blocks, kHistBlock, smem, stream>>>(static_cast<const K*>(keys), n, shift0, step, out, off);
   return cudaGetLastError();
 }
 
 template <typename K, int ND, int RB>
 cudaError_t launch_counts_t(const void* keys, size_t n, uint32_t shift0, uint32_t step, bool is_float,
-                            unsigned long long* out, cudaStream_t stream) {
+                            unsigned long long* out, cudaStream_t stream, const uint32_t* off) {
   const bool bytes = RB == 8 && shift0 % 8 == 0 && (ND == 1 || step == 8) && (sizeof(K) > 1 || shift0 == 0);
   if (sizeof(K) == 4 && is_float)
-    return bytes ? launch_counts_k<K, ND, RB, true, true>(keys, n, shift0, step, out, stream)
-                 : launch_counts_k<K, ND, RB, false, true>(keys, n, shift0, step, out, stream);
-  return bytes ? launch_counts_k<K, ND, RB, true, false>(keys, n, shift0, step, out, stream)
-               : launch_counts_k<K, ND, RB, false, false>(keys, n, shift0, step, out, stream);
+    return bytes ? launch_counts_k<K, ND, RB, true, true>(keys, n, shift0, step, out, stream, off)
+                 : launch_counts_k<K, ND, RB, false, true>(keys, n, shift0, step, out, stream, off);
+  return bytes ? launch_counts_k<K, ND, RB, true, false>(keys, n, shift0, step, out, stream, off)
+               : launch_counts_k<K, ND, RB, false, false>(keys, n, shift0, step, out, stream, off);
 }
 
 // The 32-bit sort's histogram with the first pass's tile offsets
@@ -176,7 +178,8 @@ __global__ void __launch_bounds__(NT, 1) tile_counts_kernel(const uint32_t* __re
                                                               unsigned long long* __restrict__ out,
                                                               uint32_t* __restrict__ tile_prefix,
                                                               uint32_t* chunk_tot, uint32_t* __restrict__ chunk_excl,
-                                                              uint32_t* ticket) {
+                                                              uint32_t* ticket, const uint32_t* off) {
+  if (off && *off) return;
   constexpr uint32_t L = kTcLanes;
   extern __shared__ __align__(16) uint32_t s_tc[];
   uint32_t* s_hi = s_tc;                  // bytes 1..3: [3][256][L]
@@ -404,7 +407,8 @@ template <int R>
 __global__ void __launch_bounds__(kScanBlock) scan_digits_kernel(const unsigned long long* __restrict__ counts,
                                                                  int passes, size_t n, int is_float, int allow_skip,
                                                                  unsigned long long* __restrict__ bin_start,
-                                                                 SortCtrl* ctrl) {
+                                                                 SortCtrl* ctrl, const uint32_t* off) {
+  if (off && *off) return;
   constexpr int PER = R / kScanBlock;
   __shared__ unsigned long long s_warp[kScanBlock / 32];
   __shared__ uint32_t s_trivial[kMaxPasses];
@@ -469,7 +473,8 @@ bool tile_counts_supported(size_t tile_keys) { return tile_keys == 4096 || tile_
 
 cudaError_t launch_tile_counts(const uint32_t* keys, size_t n, size_t tile_keys, bool is_float,
                                unsigned long long* out, uint32_t* tile_prefix, uint32_t* chunk_tot,
-                               uint32_t* chunk_excl, uint32_t* ticket, uint32_t* tpc, cudaStream_t stream) {
+                               uint32_t* chunk_excl, uint32_t* ticket, uint32_t* tpc, cudaStream_t stream,
+                               const uint32_t* off) {
   if (n == 0 || n >= ((size_t)1 << 30) || !tile_counts_supported(tile_keys) ||
       (reinterpret_cast<uintptr_t>(keys) & 15u) != 0)
     return cudaErrorInvalidValue;
@@ -483,7 +488,7 @@ cudaError_t launch_tile_counts(const uint32_t* keys, size_t n, size_t tile_keys,
     if (e != cudaSuccess) return e;
     kern<<<(unsigned)grid, (unsigned)(tile_keys / 8), kTcSmemBytes, stream>>>(
         keys, n, (uint32_t)tile_keys, (uint32_t)tiles, (uint32_t)per, out, tile_prefix, chunk_tot, chunk_excl,
-        ticket);
+        ticket, off);
     *tpc = (uint32_t)per;
     return cudaGetLastError();
   };
@@ -494,26 +499,26 @@ cudaError_t launch_tile_counts(const uint32_t* keys, size_t n, size_t tile_keys,
 
 cudaError_t launch_digit_counts(const void* keys, size_t n, int key_bytes, int num_digits, int radix_bits,
                                 uint32_t shift0, uint32_t shift_step, bool is_float, unsigned long long* out,
-                                cudaStream_t stream) {
+                                cudaStream_t stream, const uint32_t* off) {
   if (n == 0) return cudaSuccess;
   if (radix_bits == 8) {
     if (key_bytes == 4) {
-      if (num_digits == 4) return launch_counts_t<uint32_t, 4, 8>(keys, n, shift0, shift_step, is_float, out, stream);
-      if (num_digits == 2) return launch_counts_t<uint32_t, 2, 8>(keys, n, shift0, shift_step, is_float, out, stream);
-      if (num_digits == 1) return launch_counts_t<uint32_t, 1, 8>(keys, n, shift0, shift_step, is_float, out, stream);
+      if (num_digits == 4) return launch_counts_t<uint32_t, 4, 8>(keys, n, shift0, shift_step, is_float, out, stream, off);
+      if (num_digits == 2) return launch_counts_t<uint32_t, 2, 8>(keys, n, shift0, shift_step, is_float, out, stream, off);
+      if (num_digits == 1) return launch_counts_t<uint32_t, 1, 8>(keys, n, shift0, shift_step, is_float, out, stream, off);
     } else if (key_bytes == 8) {
       if (num_digits == 8)
-        return launch_counts_t<unsigned long long, 8, 8>(keys, n, shift0, shift_step, false, out, stream);
+        return launch_counts_t<unsigned long long, 8, 8>(keys, n, shift0, shift_step, false, out, stream, off);
       if (num_digits == 1)
-        return launch_counts_t<unsigned long long, 1, 8>(keys, n, shift0, shift_step, false, out, stream);
+        return launch_counts_t<unsigned long long, 1, 8>(keys, n, shift0, shift_step, false, out, stream, off);
     } else if (key_bytes == 1 && num_digits == 1) {
-      return launch_counts_t<uint8_t, 1, 8>(keys, n, shift0, shift_step, false, out, stream);
+      return launch_counts_t<uint8_t, 1, 8>(keys, n, shift0, shift_step, false, out, stream, off);
     }
   } else if (radix_bits == 11) {
     if (key_bytes == 4 && num_digits == 3)
-      return launch_counts_t<uint32_t, 3, 11>(keys, n, shift0, shift_step, is_float, out, stream);
+      return launch_counts_t<uint32_t, 3, 11>(keys, n, shift0, shift_step, is_float, out, stream, off);
     if (key_bytes == 8 && num_digits == 6)
-      return launch_counts_t<unsigned long long, 6, 11>(keys, n, shift0, shift_step, false, out, stream);
+      return launch_counts_t<unsigned long long, 6, 11>(keys, n, shift0, shift_step, false, out, stream, off);
   }
   return cudaErrorInvalidValue;
 }
@@ -640,14 +645,14 @@ cudaError_t launch_counting_fill(uint8_t* a, size_t n, const unsigned long long*
 
 cudaError_t launch_scan_digits(const unsigned long long* counts, int passes, int radix_bits, size_t n,
                                bool is_float, bool allow_skip, unsigned long long* bin_start, SortCtrl* ctrl,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, const uint32_t* off) {
   if (passes < 1 || passes > kMaxPasses) return cudaErrorInvalidValue;
   if (radix_bits == 8)
     scan_digits_kernel<256><<<1, kScanBlock, 0, stream>>>(counts, passes, n, is_float ? 1 : 0, allow_skip ? 1 : 0,
-                                                           bin_start, ctrl);
+                                                           bin_start, ctrl, off);
   else if (radix_bits == 11)
     scan_digits_kernel<2048><<<1, kScanBlock, 0, stream>>>(counts, passes, n, is_float ? 1 : 0, allow_skip ? 1 : 0,
-                                                            bin_start, ctrl);
+                                                            bin_start, ctrl, off);
   else
     return cudaErrorInvalidValue;
   return cudaGetLastError();

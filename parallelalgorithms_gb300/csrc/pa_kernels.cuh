@@ -58,9 +58,11 @@ cudaError_t ensure_dynamic_smem(F* func, size_t bytes) {
 // Counts of `num_digits` digits of width `radix_bits` (digit d taken at bit
 // shift0 + d * shift_step of the ordered key) over keys[0, n), ADDED into
 // out[num_digits][1 << radix_bits] (unsigned 64-bit).  key_bytes is 1, 4 or 8.
+// Here and below, `off` (device memory, optional): the launch does nothing
+// when the word it points at is not zero.
 cudaError_t launch_digit_counts(const void* keys, size_t n, int key_bytes, int num_digits, int radix_bits,
                                 uint32_t shift0, uint32_t shift_step, bool is_float, unsigned long long* out,
-                                cudaStream_t stream);
+                                cudaStream_t stream, const uint32_t* off = nullptr);
 
 // The histogram of a 32-bit sort with 8-bit digits that also prepares its
 // first digit pass: one read of keys[0, n) (16-byte aligned, n < 2^30)
@@ -76,7 +78,8 @@ constexpr int kTileCountMaxChunks = 160;
 bool tile_counts_supported(size_t tile_keys);
 cudaError_t launch_tile_counts(const uint32_t* keys, size_t n, size_t tile_keys, bool is_float,
                                unsigned long long* out, uint32_t* tile_prefix, uint32_t* chunk_tot,
-                               uint32_t* chunk_excl, uint32_t* ticket, uint32_t* tpc, cudaStream_t stream);
+                               uint32_t* chunk_excl, uint32_t* ticket, uint32_t* tpc, cudaStream_t stream,
+                               const uint32_t* off = nullptr);
 
 // Several arrays' 256-bin histograms of (key >> shift) & 255 in one launch
 // (the serving loop's coalesced histogram requests).  jobs[0, njobs) in
@@ -114,7 +117,7 @@ cudaError_t launch_quanta_start_of_bins(const unsigned long long* counts, size_t
 // control block (skips, ping-pong direction, float transform placement).
 cudaError_t launch_scan_digits(const unsigned long long* counts, int passes, int radix_bits, size_t n,
                                bool is_float, bool allow_skip, unsigned long long* bin_start, SortCtrl* ctrl,
-                               cudaStream_t stream);
+                               cudaStream_t stream, const uint32_t* off = nullptr);
 
 // ---- onesweep digit pass (pa_onesweep.cu) --------------------------------
 struct OnesweepArgs {
@@ -195,6 +198,52 @@ cudaError_t launch_bucket_sort(const uint32_t* src, const ChunkRuns& chunks, con
 cudaError_t launch_final_copy(void* keys_a, const void* keys_b, uint32_t* vals_a, const uint32_t* vals_b,
                               size_t n, int key_bytes, const SortCtrl* ctrl, cudaStream_t stream);
 
+// ---- keys-only sorts by buckets (pa_buckets.cu) ----------------------------
+// Where a key goes: t = min(max(key - lo, 0) >> s, 2^32 - 1) and bucket =
+// min((t * mult) >> 32, nb - 1), written by the plan kernel.
+struct BucketMap {
+  uint32_t on;         // 1: this sort runs; 0: the sample did not fit, the LSD passes run
+  uint32_t plain;      // 1: the bucket is the key's top bits (lo = 0, mult = nb)
+  uint32_t mult;
+  uint32_t s;          // (0 for 32-bit keys)
+  uint32_t cell_shift;  // a bucket's keys are spread by (key - first) >> cell_shift
+  uint32_t bin_shift;   // or, counted per bin, by (key - first) >> bin_shift
+  uint32_t exact;       // 1: a bin holds one key value (outside the first and last bucket)
+  uint32_t ticket;     // CTAs of the count kernel that are done
+  unsigned long long lo;
+  unsigned long long inv;  // 2^63 / mult
+};
+struct BucketScratch {
+  uint32_t nb = 0;        // buckets (a power of two); 0: the sort does not go by buckets
+  uint32_t low_bits = 0;  // bucket bits of the second partition pass (0: one pass)
+  BucketMap* map = nullptr;
+  uint32_t* count = nullptr;         // [nb]
+  uint32_t* start = nullptr;         // [nb + 1]
+  uint32_t* cursor = nullptr;        // [nb]
+  uint32_t* group_cursor = nullptr;  // [nb >> low_bits]
+  uint32_t* tile_first = nullptr;    // [(nb >> low_bits) + 1] first tile of each group in the second pass
+};
+// Sizes this sort takes: more keys than the one-CTA sort, and few enough that
+// the most buckets there can be fit the finish kernel with room to spare.
+bool bucket_sort_supported(size_t n, int key_bytes);
+// Carves the scratch from `base` (nullptr measures); returns its size.
+size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s);
+// Enqueues the plan for keys[0, n): map->on says whether the sort goes by
+// buckets (when the keys are too unevenly spread it does not), and then ctrl
+// says "skip" for every LSD pass.  decided, when set, is page-locked host memory
+// that receives map->on as soon as it is known.
+cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, const void* tmp, size_t n, int key_bytes,
+                                bool is_float, SortCtrl* ctrl, uint32_t* decided, cudaStream_t stream);
+// Enqueues the planned sort (tmp: n keys of scratch; the result is in keys);
+// nothing is moved when map->on is 0.  `mark` runs after the count (twice:
+// there is no scan launch), after each of the two partitions and after the
+// sort of the buckets.
+cudaError_t enqueue_bucket_sort(const BucketScratch& s, void* keys, void* tmp, size_t n, int key_bytes, bool is_float,
+                                SortCtrl* ctrl, uint32_t* err, cudaStream_t stream,
+                                const std::function<cudaError_t()>& mark = {});
+// Zeroes bytes [p, p + bytes) (p 16-byte aligned) unless *off is not zero.
+cudaError_t launch_clear(void* p, size_t bytes, const uint32_t* off, cudaStream_t stream);
+
 // ---- whole sorts on device buffers (pa_capi.cu) ---------------------------
 // Per-call scratch of a device-resident sort: digit counts, tile tickets and
 // look-back words (zeroed by enqueue_sort), bin starts, pass control.
@@ -216,15 +265,21 @@ struct SortScratch {
   uint32_t* chunk_tot;
   uint32_t* chunk_excl;
   uint32_t* tc_ticket;  // zeroed with the counts
+  BucketScratch buckets;  // keys-only sorts with 8-bit digits of the sizes bucket_sort_supported takes
 };
 size_t sort_scratch_bytes(size_t n, int key_bytes, bool has_vals, int radix_bits = 8);
 // Carves the scratch from `base` (nullptr measures); returns its size.
 size_t sort_scratch_layout(char* base, size_t n, int key_bytes, bool has_vals, SortScratch* s, int radix_bits = 8);
-// Enqueues the whole sort (memset, histogram, scan, passes, final copy) of
-// device buffers on `stream`; `mark`, when set, runs between launches.
+// Enqueues the whole sort of device buffers on `stream` (the LSD chain: memset,
+// histogram, scan, passes, final copy; or by buckets, scratch and sizes
+// permitting); `mark`, when set, runs between launches.  decided (optional):
+// one word of page-locked host memory nothing else uses meanwhile; with it the
+// call waits for the bucket plan's decision and enqueues only what it takes,
+// without it (asynchronous callers) everything is enqueued and decides on the
+// device, which only large sorts do.
 cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32_t* d_vals, uint32_t* d_tvals,
                          size_t n, int key_bytes, bool is_float, uint32_t* err, cudaStream_t stream,
-                         const std::function<cudaError_t()>& mark = {});
+                         const std::function<cudaError_t()>& mark = {}, uint32_t* decided = nullptr);
 
 // ---- sum (pa_sum.cu) -------------------------------------------------------
 // Element kinds of the sums (the values of pa_gpu.h's PA_ELEM_*).
