@@ -1,11 +1,12 @@
 """Batched segmented sort and its autotuner.
 
 Many uint32 arrays of uneven size, stored back to back in one device buffer
-and described by offsets, are sorted independently in ONE persistent kernel
-launch (pa_segsort_plan_* in include/pa_gpu.h): segments up to a cutoff are
-sorted inside one CTA's shared memory, longer ones by the onesweep passes.
-A plan is built once per segmentation and replayed through a captured CUDA
-graph.
+and described by offsets, are sorted independently by one chain of launches
+that each cover all of them (pa_segsort_plan_* in include/pa_gpu.h): segments
+of at most 4096 keys are sorted inside one CTA's shared memory, longer ones are
+partitioned into buckets that are (or, where their keys crowd, by the onesweep
+passes).  A plan is built once per segmentation and replayed through a captured
+CUDA graph.
 
 The autotuner times every candidate configuration (small/large cutoff and
 digit width; the onesweep tile of 11-bit plans) on the caller's own data and

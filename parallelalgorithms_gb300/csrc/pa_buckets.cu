@@ -36,6 +36,7 @@
 #include "pa_common.cuh"
 #include "pa_kernels.cuh"
 #include "pa_onesweep_tile.cuh"
+#include "pa_segmented.cuh"
 
 namespace pa {
 namespace {
@@ -50,9 +51,9 @@ constexpr uint32_t kSample = (uint32_t)kPlanCtas * kPlanBlock * kPlanPer;
 constexpr uint32_t kGroups = 256;         // bins of a partition pass, at most
 constexpr uint32_t kBucketsMax = 32768;   // counters of the count kernel: 128 KB of shared memory
 constexpr uint32_t kBucketTarget = 3072;  // keys per bucket, at most, while more buckets can be had
-constexpr uint32_t kCells = 65536;        // cells of the finish kernel's bitmap
-constexpr uint32_t kBucketBins = 4096;    // bins of a bucket that is counted instead
-constexpr uint32_t kBucketBinMax = 64;    // keys of one bin that are still placed by comparing
+constexpr int kCellBits = 16, kBinBits = 12;
+constexpr uint32_t kCells = 1u << kCellBits;      // cells of the finish kernel's bitmap
+constexpr uint32_t kBucketBins = 1u << kBinBits;  // values a crowded bucket may span to be counted instead
 
 struct BucketArgs {
   BucketMap* map;
@@ -62,6 +63,7 @@ struct BucketArgs {
   uint32_t* cursor;
   uint32_t* group_cursor;
   uint32_t* tile_first;
+  uint32_t* rare;
   uint32_t nb;
   uint32_t nb_bits;     // nb = 1 << nb_bits
   uint32_t low_bits;
@@ -233,16 +235,14 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
     m.inv = (1ull << 63) / mult;
     m.s = s;
     m.lo = base;
-    // cells and bins of the finish kernel: the widest bucket spans
-    // ceil(2^32 / mult) values of t, 2^s keys each
+    // cells of the finish kernel: the widest bucket spans ceil(2^32 / mult)
+    // values of t, 2^s keys each
     const unsigned long long width = ((1ull << 32) + mult - 1) / mult;
     uint32_t sh = 0;
     while (((width - 1) >> sh) >= kCells) ++sh;
     m.cell_shift = sh + s;
-    while (((width - 1) >> sh) >= kBucketBins) ++sh;
-    m.bin_shift = sh + s;
-    m.exact = m.bin_shift == 0 ? 1u : 0u;
     *a.map = m;
+    a.rare[0] = 0;
     if (fits) {  // the LSD passes enqueued behind this sort do nothing
       for (int p = 0; p < kMaxPasses; ++p) a.ctrl->pass[p].skip = 1;
       a.ctrl->final_in_tmp = 0;
@@ -601,9 +601,8 @@ __global__ void __launch_bounds__(kScatterBlock, kScatterPerSm) bucket_scatter_k
 // no comparing.  The few keys that find their cell taken (about m^2 / (2 kCells)
 // of m) are listed and counted beside the bits; they follow the entry's other
 // keys, and the thread of the entry's first such key sorts the entry's few keys
-// by comparing.  Buckets where that would be many (equal keys, clusters) are
-// counted per bin instead (finish_counted), and buckets larger than shared
-// memory, or crowded even there, take finish_slow.
+// by comparing.  Buckets where that would be many (equal keys, clusters), and
+// buckets larger than shared memory, are listed for a launch of their own.
 //
 // Bound by instruction issue and the shared-memory pipe together (about 60 %
 // of each): 100M uniform 32-bit keys in 0.328 ms.  On the way there (same
@@ -625,19 +624,326 @@ constexpr uint32_t kHits = 256;     // such keys of one bucket, at most
 
 // The least t with umulhi(t, mult) >= b (b < nb), from the rounded-down
 // reciprocal inv = 2^63 / mult: the estimate is at most two short.
-__device__ __forceinline__ uint32_t bucket_first_t(uint32_t b, const BucketMap& m) {
-  uint32_t t = (uint32_t)__umul64hi((unsigned long long)b << 33, m.inv);
-  while (__umulhi(t, m.mult) < b) ++t;
+__device__ __forceinline__ uint32_t bucket_first_t(uint32_t b, uint32_t mult, unsigned long long inv) {
+  uint32_t t = (uint32_t)__umul64hi((unsigned long long)b << 33, inv);
+  while (__umulhi(t, mult) < b) ++t;
   return t;
 }
 
+constexpr size_t kFinishAux = kEntries * 8;  // bytes of the bitmap
+
+// What thread 0 prepares of the next bucket while the CTA works on one.
+enum : uint32_t {
+  kJobSkip = 0,   // nothing to do
+  kJobBulk = 1,   // cells, keys bulk-copied in
+  kJobLoads = 2,  // cells, plain loads (a copy would reach past the array's ends)
+  kJobLarge = 3   // more keys than shared memory holds
+};
+template <typename K>
+struct FinishJob {
+  K* src;         // its keys, sorted into dst; other: scratch of as many keys beside src (dst, unless in place)
+  K* dst;
+  K* other;
+  K first;        // no key of the bucket is below it
+  uint32_t cnt;
+  uint32_t kind;
+  uint32_t edge;  // 1: the bucket's range is not known (it holds keys outside the map): found here
+  uint32_t cell_shift;  // cells of (key - first)
+  const K *lo, *hi;     // the array src lies in
+};
+
+// Cells and bins of keys that span `range`.
+template <typename K>
+__device__ __forceinline__ void spread_of(K range, uint32_t& cell_shift, uint32_t& bin_shift) {
+  const int bits = 8 * (int)sizeof(K) - (sizeof(K) == 4 ? __clz((int)(uint32_t)range) : __clzll((long long)range));
+  cell_shift = (uint32_t)max(0, bits - kCellBits);
+  bin_shift = (uint32_t)max(0, bits - kBinBits);
+}
+
+// Sorts buckets blockIdx.x, blockIdx.x + gridDim.x, ... below nb.  next(b, job)
+// (thread 0) fills all of a bucket's job but its kind.  Buckets that this is not
+// for are listed (rare[0]: how many, rare[1...]: which) and sorted by
+// rare_buckets: their code here would cost the main path its registers (0.51 ms
+// against 0.35 at 100M keys).
+template <typename K, bool FLT, typename Next>
+__device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint32_t* err, Next&& next) {
+  constexpr int ITEMS = kFinishItems;
+  constexpr uint32_t B = kFinishBlock;
+  constexpr uint32_t CAP = kFinishCap;
+  constexpr int C = 4;  // items handled together: their atomics in flight at once
+  constexpr int W = B / 32;
+  constexpr int U = (int)kEntries / (W * 64);  // 16-byte reads (two entries) per lane in the scan
+  constexpr uint32_t V = 16 / sizeof(K);
+  static_assert(U == 2 || U == 4, "runs of 64 entries per warp, scanned in pairs as 16-bit halves of one word");
+  static_assert(kHits <= B, "one listed key per thread");
+  extern __shared__ __align__(128) unsigned char smem[];
+  K* s_keys = reinterpret_cast<K*>(smem);                                           // [CAP + V]
+  uint2* s_entry = reinterpret_cast<uint2*>(smem + (CAP + V) * sizeof(K));          // [kEntries]
+  K* s_in = reinterpret_cast<K*>(smem + (CAP + V) * sizeof(K) + kFinishAux);        // [CAP + 2 * V]
+  K* s_hit = s_in + CAP + 2 * V;                                                    // [kHits]
+  __shared__ FinishJob<K> s_job[2];
+  __shared__ K s_edge[2 * W];
+  __shared__ uint32_t s_warp[W];
+  __shared__ uint32_t s_nhit, s_over;
+  __shared__ __align__(8) uint64_t s_bar;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  uint32_t cs = 0;
+  auto entry_of = [&](K x) {  // (byte offset: the entry's number times 8)
+    return reinterpret_cast<uint2*>(reinterpret_cast<char*>(s_entry) + ((uint32_t)(x >> (cs + 2)) & ((kEntries - 1) * 8)));
+  };
+  auto cell_of = [&](K x) { return (uint32_t)(x >> cs) & 31u; };
+  // thread 0: bucket b's job, and its keys' bulk copy into s_in, from the
+  // 16-byte boundary at or below the first key to the one at or above the end
+  auto prepare = [&](uint32_t b, FinishJob<K>* job) {
+    FinishJob<K> j;
+    next(b, j);
+    j.kind = j.cnt == 0 ? kJobSkip : kJobLarge;
+    if (j.cnt != 0 && j.cnt <= CAP) {
+      const uint32_t skew = skew_of(j.src);
+      const uint32_t len = (skew + j.cnt + V - 1) / V * V;
+      j.kind = kJobLoads;
+      if (j.src - skew >= j.lo && j.src - skew + len <= j.hi) {
+        j.kind = kJobBulk;
+        fence_proxy_async();
+        mbar_arrive_expect_tx(&s_bar, len * (uint32_t)sizeof(K));
+        bulk_load_g2s(s_in, j.src - skew, len * (uint32_t)sizeof(K), &s_bar);
+      }
+    }
+    *job = j;
+  };
+  if (tid == 0) {
+    mbar_init(&s_bar, 1);
+    mbar_fence_init();
+    if (blockIdx.x < nb) prepare(blockIdx.x, &s_job[0]);
+  }
+  uint32_t parity = 0, slot = 0;
+  for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x, slot ^= 1u) {
+    if (tid == 0) {
+      s_nhit = 0;
+      s_over = 0;
+    }
+    for (uint32_t q = tid; q < kEntries / 2; q += B) reinterpret_cast<uint4*>(s_entry)[q] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();  // the job is there; everything of the last bucket is done with
+    const FinishJob<K>& job = s_job[slot];  // (read where needed: its pointers need no registers meanwhile)
+    const uint32_t cnt = job.cnt;
+    K first = 0;
+    // thread 0, once s_in has been read: the next bucket
+    auto go_on = [&]() {
+      if (tid == 0 && b + gridDim.x < nb) prepare(b + gridDim.x, &s_job[slot ^ 1u]);
+    };
+    bool done = job.kind == kJobSkip;
+    if (job.kind == kJobSkip || job.kind == kJobLarge) go_on();
+    if (job.kind == kJobBulk || job.kind == kJobLoads) {
+      const uint32_t skew_in = skew_of(job.src);
+      const K* src = s_in + skew_in + tid;
+      bool ok = true;
+      if (job.kind == kJobBulk) {
+        ok = mbar_wait_bounded(&s_bar, parity, err);
+        parity ^= 1u;
+      } else {
+        for (uint32_t i = tid; i < cnt; i += B) s_in[skew_in + i] = job.src[i];  // (read by the same thread)
+      }
+      first = job.first;
+      cs = job.cell_shift;
+      if (job.edge) {  // the bucket's own range
+        K lo = ~(K)0, hi = 0;
+        for (uint32_t i = 0; i + tid < cnt; i += B) {
+          lo = min(lo, src[i]);
+          hi = max(hi, src[i]);
+        }
+        warp_minmax(lo, hi);
+        if (lane == 0) {
+          s_edge[warp] = lo;
+          s_edge[W + warp] = hi;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          lo = min(lo, s_edge[w]);
+          hi = max(hi, s_edge[W + w]);
+        }
+        uint32_t bins;
+        first = lo;
+        spread_of<K>((K)(hi - lo), cs, bins);
+      }
+      K k[ITEMS];  // distances from `first`; past the end, whatever s_in holds
+      uint32_t hit = 0;   // bit j: key j found its cell taken
+      uint32_t skip = 0;  // bit j: that, or there is no key j
+#pragma unroll
+      for (int c = 0; c < ITEMS; c += C) {
+        if ((uint32_t)c * B >= cnt) break;
+        uint32_t old[C];
+        if ((uint32_t)(c + C) * B <= cnt) {
+#pragma unroll
+          for (int j = 0; j < C; ++j) {
+            k[c + j] = src[(uint32_t)(c + j) * B] - first;
+            old[j] = atomicOr(&entry_of(k[c + j])->x, 1u << cell_of(k[c + j]));
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < C; ++j) {
+            const bool has = (uint32_t)(c + j) * B + tid < cnt;
+            k[c + j] = src[(uint32_t)(c + j) * B] - first;
+            old[j] = atomicOr(&entry_of(k[c + j])->x, has ? 1u << cell_of(k[c + j]) : 0u);
+            skip |= has ? 0u : 1u << (c + j);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < C; ++j) hit |= ((old[j] >> cell_of(k[c + j])) & 1u) << (c + j);
+      }
+      hit &= ~skip;
+      skip |= hit;
+      if (hit) {
+        uint32_t p = atomicAdd(&s_nhit, (uint32_t)__popc(hit));
+        for (uint32_t h = hit; h; h &= h - 1u, ++p)
+          if (p < kHits) s_hit[p] = src[((uint32_t)__ffs((int)h) - 1u) * B] - first;
+      }
+      if (!ok) s_over = 2;
+      __syncthreads();
+      const uint32_t nhit = s_nhit;
+      if (s_over == 2) {  // the copy never came: wait it out once more, sort nothing further
+        mbar_wait_bounded(&s_bar, parity ^ 1u, err);
+        if (tid == 0) bulk_store_wait_all();
+        return;
+      }
+      go_on();
+      bool crowded = nhit > kHits;
+      K hx = 0;               // this thread's listed key
+      uint32_t turn = 0;      // its number among its entry's listed keys
+      uint32_t listed = 0, span = 0;  // how many those are; all of the entry's keys
+      if (nhit && !crowded) {
+        if (tid < nhit) {
+          hx = s_hit[tid];
+          turn = atomicAdd(&entry_of(hx)->y, 1u);
+          if (turn >= kEntryHits) s_over = 1;
+        }
+        __syncthreads();
+        crowded = s_over != 0;
+      }
+      if (!crowded) {
+        // Scan: warp w owns kEntries / W entries, lane l entries 2 l and 2 l + 1
+        // of each run of 64.  An entry's keys: its set bits and its listed keys.
+        uint4 q[U];
+        uint32_t c2[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          q[u] = reinterpret_cast<uint4*>(s_entry)[(warp * U + u) * 32 + lane];
+          q[u].y += __popc(q[u].x);
+          c2[u] = q[u].y + q[u].w + __popc(q[u].z);
+        }
+        if (tid < nhit) {
+          const uint2 e = *entry_of(hx);
+          listed = e.y;
+          span = e.y + __popc(e.x);
+        }
+        uint32_t p2[U / 2], t2[U / 2];
+#pragma unroll
+        for (int u = 0; u < U / 2; ++u) p2[u] = c2[2 * u] | (c2[2 * u + 1] << 16);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+          for (int u = 0; u < U / 2; ++u) {
+            const uint32_t x = __shfl_up_sync(kFull, p2[u], o);
+            if (lane >= (uint32_t)o) p2[u] += x;
+          }
+        }
+        uint32_t total = 0;
+#pragma unroll
+        for (int u = 0; u < U / 2; ++u) {
+          t2[u] = __shfl_sync(kFull, p2[u], 31);
+          total += (t2[u] & 0xFFFFu) + (t2[u] >> 16);
+        }
+        if (lane == 0) s_warp[warp] = total;
+        // (the last bucket's copy out of s_keys must have read it)
+        if (tid == 0) bulk_store_wait_read();
+        __syncthreads();
+        uint32_t before = __reduce_add_sync(kFull, lane < warp ? s_warp[lane & (W - 1)] : 0u);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const uint32_t run = before + (u & 1 ? p2[u / 2] >> 16 : p2[u / 2] & 0xFFFFu) - c2[u];
+          before += u & 1 ? t2[u / 2] >> 16 : t2[u / 2] & 0xFFFFu;
+          q[u].w = run + q[u].y;
+          q[u].y = run;
+          reinterpret_cast<uint4*>(s_entry)[(warp * U + u) * 32 + lane] = q[u];
+        }
+        __syncthreads();
+        // staged with the destination's own offset from a 16-byte boundary
+        K* dst = job.dst;
+        const uint32_t skew = skew_of(dst);
+        K* stage = s_keys + skew;
+#pragma unroll
+        for (int c = 0; c < ITEMS; c += C) {
+          if ((uint32_t)c * B >= cnt) break;
+#pragma unroll
+          for (int j = c; j < c + C; ++j) {
+            const uint2 e = *entry_of(k[j]);
+            const uint32_t p = e.y + __popc(e.x & ((1u << cell_of(k[j])) - 1u));
+            if (!((skip >> j) & 1u)) stage[p & (CAP - 1)] = from_ordered((K)(k[j] + first), FLT);
+          }
+        }
+        if (nhit) {
+          uint32_t lo = 0, bits = 0;
+          if (tid < nhit) {
+            const uint2 e = *entry_of(hx);
+            lo = e.y;
+            bits = e.x;
+            if (listed > 1) stage[(lo + __popc(bits) + turn) & (CAP - 1)] = from_ordered((K)(hx + first), FLT);
+          }
+          __syncthreads();
+          if (listed == 1) {  // between the key it met and the next: those above move up by one
+            const uint32_t r = lo + __popc(bits & ((1u << cell_of(hx)) - 1u));
+            const uint32_t top = min(CAP, lo + span) - 1u;
+            for (uint32_t j = top; j > r + 1; --j) stage[j] = stage[j - 1];
+            const K x = from_ordered((K)(hx + first), FLT), y = stage[r];
+            const bool below = hx + first < to_ordered(y, FLT);
+            stage[r] = below ? x : y;
+            if (r < top) stage[r + 1] = below ? y : x;
+          } else if (listed > 1 && turn == 0) {  // several: the entry's keys are sorted
+            const uint32_t hi = min(CAP, lo + span);
+            for (uint32_t j = lo + 1; j < hi; ++j) {
+              const K x = stage[j];
+              uint32_t p = j;
+              while (p > lo) {
+                const K y = stage[p - 1];
+                if (to_ordered(y, FLT) <= to_ordered(x, FLT)) break;
+                stage[p] = y;
+                --p;
+              }
+              stage[p] = x;
+            }
+          }
+        }
+        // out: whole 16-byte units in one bulk copy, the keys before the first
+        // and after the last boundary singly
+        fence_proxy_async();
+        __syncthreads();
+        const uint32_t head = min(cnt, (V - skew) & (V - 1));
+        const uint32_t body = (cnt - head) / V * V;
+        if (tid == 0 && body) bulk_store_s2g(dst + head, stage + head, body * (uint32_t)sizeof(K));
+        if (tid >= 32 && tid < 32 + V) {  // (V - 1 keys at most each)
+          const uint32_t i = tid - 32;
+          if (i < head) dst[i] = stage[i];
+          if (head + body + i < cnt) dst[head + body + i] = stage[head + body + i];
+        }
+        done = true;
+      }
+    }
+    if (!done && tid == 0) rare[1 + atomicAdd(rare, 1u)] = b;
+  }
+  if (tid == 0) bulk_store_wait_all();
+}
+
+// ---------------------------------------------------------------------------
+// The listed buckets: equal keys, clusters, more keys than shared memory holds.
+// ---------------------------------------------------------------------------
+constexpr int kRareBlock = 512;
+constexpr int kRareItems = (int)kFinishCap / kRareBlock;
 // Bin counters are padded by 4 words per 16, so that a thread's 16-byte reads
 // of its own run of bins in the scan touch every bank once per quarter warp.
 __device__ __forceinline__ uint32_t bin_at(uint32_t bin) { return bin + ((bin >> 4) << 2); }
 constexpr uint32_t kBinWords = kBucketBins + kBucketBins / 4;
-
-// bytes of the bitmap, or of the bins
-constexpr size_t kFinishAux = kEntries * 8 > (kBinWords + 4) * 4 ? kEntries * 8 : (kBinWords + 4) * 4;
+// bytes of the bins, or of the 4-bit passes' counters
+constexpr size_t kRareAux = std::max<size_t>((size_t)(kBinWords + 4) * 4, (size_t)os::kNibbleBins * (kRareBlock + 32) * 4);
 
 // A bucket too large for shared memory, or with many keys in one bin: stable
 // 8-bit LSD passes by the one CTA, a[0, m) and b[0, m) in turn; the result is
@@ -645,8 +951,8 @@ constexpr size_t kFinishAux = kEntries * 8 > (kBinWords + 4) * 4 ? kEntries * 8 
 // keys and pass) and rare: the plan's sample bounds how large such a bucket
 // is likely to be, and the bits all its keys share are skipped.
 template <typename K>
-__device__ __noinline__ void finish_slow(K* a, K* b, uint32_t m, bool into_a, unsigned char* smem) {
-  constexpr int B = kFinishBlock, W = B / 32;
+__device__ void finish_slow(K* a, K* b, uint32_t m, bool into_a, unsigned char* smem) {
+  constexpr int B = kRareBlock, W = B / 32;
   uint32_t* s_cur = reinterpret_cast<uint32_t*>(smem);                // [256]
   uint32_t* s_wc = s_cur + 256;                                       // [W][256]
   uint32_t* s_warp = s_wc + W * 256;                                  // [W]
@@ -719,32 +1025,24 @@ __device__ __noinline__ void finish_slow(K* a, K* b, uint32_t m, bool into_a, un
   __syncthreads();
 }
 
-// A bucket of at most CAP keys counted per bin ([first, first + 1 << shift)
-// and so on): keys placed by their bin's start and the atomic's return, then
-// each key compared with the others of its bin, unless every bin is one value
-// (`exact`).  Returns false, with nothing written, when a bin holds too many
-// different keys for that.
+// A bucket of at most CAP keys that span fewer than kBucketBins values from
+// `first` on: counted per value, and placed from each value's end down.
 template <typename K, bool FLT>
-__device__ __noinline__ bool finish_counted(const K* in, K* out, uint32_t cnt, K first, uint32_t shift, bool exact,
-                                            unsigned char* smem, uint32_t* s_warp) {
-  constexpr int B = kFinishBlock;
-  constexpr uint32_t CAP = kFinishCap;
-  constexpr int PER = (int)kBucketBins / B;  // bins per thread in the scan
-  static_assert(PER % 4 == 0, "a thread's bins are read as 16-byte vectors");
+__device__ void finish_counted(const K* in, K* out, uint32_t cnt, K first, unsigned char* smem, uint32_t* s_warp) {
+  constexpr int B = kRareBlock;
+  constexpr int PER = (int)kBucketBins / B;  // values per thread in the scan
+  static_assert(PER % 4 == 0, "a thread's counters are read as 16-byte vectors");
   K* s_keys = reinterpret_cast<K*>(smem);
-  uint32_t* s_bin = reinterpret_cast<uint32_t*>(smem + (size_t)CAP * sizeof(K));
+  uint32_t* s_bin = reinterpret_cast<uint32_t*>(smem + (size_t)kFinishCap * sizeof(K));
   const uint32_t tid = threadIdx.x;
   for (uint32_t i = tid * 4; i < kBinWords; i += B * 4)
     *reinterpret_cast<uint4*>(s_bin + i) = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
-  auto bin_of = [&](K key) {
-    const K x = (key > first ? key - first : (K)0) >> shift;
-    return x < (K)kBucketBins ? (uint32_t)x : kBucketBins - 1;
-  };
+  auto bin_of = [&](K key) { return min((uint32_t)(key - first), kBucketBins - 1); };
   for (uint32_t i = tid; i < cnt; i += B) atomicAdd(s_bin + bin_at(bin_of(in[i])), 1u);
   __syncthreads();
   uint32_t c[PER];
-  uint32_t local = 0, mx = 0;
+  uint32_t local = 0;
 #pragma unroll
   for (int q = 0; q < PER / 4; ++q) {
     const uint4 x = *reinterpret_cast<const uint4*>(s_bin + bin_at(tid * PER) + 4 * q);
@@ -754,13 +1052,10 @@ __device__ __noinline__ bool finish_counted(const K* in, K* out, uint32_t cnt, K
     c[4 * q + 3] = x.w;
   }
 #pragma unroll
-  for (int i = 0; i < PER; ++i) {
-    local += c[i];
-    mx = max(mx, c[i]);
-  }
+  for (int i = 0; i < PER; ++i) local += c[i];
   uint32_t run = os::block_exclusive_scan<B>(local, s_warp);
 #pragma unroll
-  for (int i = 0; i < PER; ++i) {  // the bins' ends, counted down to their starts below
+  for (int i = 0; i < PER; ++i) {  // the values' ends, counted down below
     run += c[i];
     c[i] = run;
   }
@@ -768,323 +1063,135 @@ __device__ __noinline__ bool finish_counted(const K* in, K* out, uint32_t cnt, K
   for (int q = 0; q < PER / 4; ++q)
     *reinterpret_cast<uint4*>(s_bin + bin_at(tid * PER) + 4 * q) =
         make_uint4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
-  if (__syncthreads_or(!exact && mx > kBucketBinMax)) return false;
+  __syncthreads();
   for (uint32_t i = tid; i < cnt; i += B) {
     const K key = in[i];
-    s_keys[atomicSub(s_bin + bin_at(bin_of(key)), 1u) - 1u] = key;
+    s_keys[(atomicSub(s_bin + bin_at(bin_of(key)), 1u) - 1u) & (kFinishCap - 1)] = key;
   }
-  __syncthreads();  // (s_bin: the bins' starts; every key of `in` has been read)
-  for (uint32_t p = tid; p < cnt; p += B) {
-    const K key = s_keys[p];
-    uint32_t o = p;
-    if (!exact) {
-      const uint32_t bin = bin_of(key);
-      const uint32_t s0 = s_bin[bin_at(bin)];
-      const uint32_t s1 = bin + 1 < kBucketBins ? s_bin[bin_at(bin + 1)] : cnt;
-      o = s0;
-      for (uint32_t i = s0; i < s1; ++i) {
-        const K x = s_keys[i];
-        o += (x < key || (x == key && i < p)) ? 1u : 0u;
-      }
-    }
-    out[o] = from_ordered(key, FLT);
-  }
-  return true;
+  __syncthreads();  // (every key of `in` has been read)
+  for (uint32_t i = tid; i < cnt; i += B) out[i] = from_ordered(s_keys[i], FLT);
 }
 
-// What thread 0 prepares of the next bucket while the CTA works on one.
+// A bucket of at most CAP keys, crowded (many keys equal or nearly so): stable
+// 4-bit counting passes over the bits its keys differ in (diff: the least and
+// greatest key's), in shared memory.
+template <typename K, bool FLT>
+__device__ void finish_nibbles(const K* in, K* out, uint32_t cnt, K diff, unsigned char* smem, uint32_t* s_warp) {
+  constexpr int B = kRareBlock, ITEMS = kRareItems;
+  static_assert((size_t)os::kNibbleBins * (B + 32) * 4 <= kRareAux, "the nibble counters fit beside the keys");
+  K* s_keys = reinterpret_cast<K*>(smem);
+  uint32_t* s_cnt = reinterpret_cast<uint32_t*>(smem + (size_t)kFinishCap * sizeof(K));
+  const uint32_t tid = threadIdx.x;
+  for (uint32_t i = tid; i < kFinishCap; i += B) s_keys[i] = i < cnt ? in[i] : ~(K)0;  // (padding sorts behind every key)
+  __syncthreads();
+  K k[ITEMS];
+  uint32_t unused[1];
+  for (uint32_t sh = 0; sh < 8 * sizeof(K) && (diff >> sh) != 0; sh += 4) {
+    os::load_run<K, false, ITEMS>(k, unused, s_keys, nullptr);
+    os::nibble_pass<K, false, B, ITEMS>(k, unused, sh, s_keys, nullptr, s_cnt, s_warp);  // ends with a barrier
+  }
+  for (uint32_t i = tid; i < cnt; i += B) out[i] = from_ordered(s_keys[i], FLT);
+}
+
+// job_of(b): bucket b's job.
+template <typename K, bool FLT, typename JobOf>
+__device__ __forceinline__ void rare_buckets(const uint32_t* rare, JobOf&& job_of) {
+  constexpr int W = kRareBlock / 32;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ uint32_t s_warp[W];
+  __shared__ K s_edge[2 * W];
+  const uint32_t num = rare[0], tid = threadIdx.x;
+  for (uint32_t i = blockIdx.x; i < num; i += gridDim.x) {
+    FinishJob<K> job{};
+    job_of(rare[1 + i], job);
+    if (job.cnt <= kFinishCap) {
+      K lo = ~(K)0, hi = 0;
+      for (uint32_t j = tid; j < job.cnt; j += kRareBlock) {
+        const K x = job.src[j];
+        lo = min(lo, x);
+        hi = max(hi, x);
+      }
+      warp_minmax(lo, hi);
+      if ((tid & 31u) == 0) {
+        s_edge[tid >> 5] = lo;
+        s_edge[W + (tid >> 5)] = hi;
+      }
+      __syncthreads();
+      for (int w = 0; w < W; ++w) {
+        lo = min(lo, s_edge[w]);
+        hi = max(hi, s_edge[W + w]);
+      }
+      uint32_t cells, bins;
+      spread_of<K>((K)(hi - lo), cells, bins);
+      if (bins == 0)
+        finish_counted<K, FLT>(job.src, job.dst, job.cnt, lo, smem, s_warp);
+      else
+        finish_nibbles<K, FLT>(job.src, job.dst, job.cnt, lo ^ hi, smem, s_warp);
+    } else {
+      finish_slow<K>(job.src, job.other, job.cnt, job.src == job.dst, smem);
+      if (FLT)
+        for (uint32_t j = tid; j < job.cnt; j += kRareBlock) job.dst[j] = from_ordered(job.dst[j], true);
+    }
+    __syncthreads();
+  }
+}
+
 template <typename K>
-struct FinishJob {
-  K first;        // the bucket's least key: that of the least t with umulhi(t, mult) >= b
-  uint32_t at;    // its keys: [at, at + cnt)
-  uint32_t cnt;
-  uint32_t kind;  // 0: nothing to do, 1: cells, keys bulk-copied, 2: cells, plain loads, 3: counted or slow
-  uint32_t exact;
-};
+constexpr size_t rare_smem() {
+  static_assert((256 + (kRareBlock / 32) * 257) * 4 + 2 * (kRareBlock / 32) * sizeof(K) <= kFinishCap * sizeof(K) + kRareAux,
+                "finish_slow fits");
+  return (size_t)kFinishCap * sizeof(K) + kRareAux;
+}
 
 // in == out: buckets are sorted in place and `other` is scratch; else in is
 // the scratch array and other == out.
+template <typename K>
+__device__ __forceinline__ void plain_job(const BucketArgs& a, const BucketMap& m, uint32_t b, uint32_t at, uint32_t end,
+                                          K* in, K* out, K* other, size_t n, FinishJob<K>& job) {
+  job.src = in + at;
+  job.dst = out + at;
+  job.other = other + at;
+  job.lo = in;
+  job.hi = in + n;
+  job.first = (K)m.lo + ((K)bucket_first_t(b, m.mult, m.inv) << m.s);
+  job.cnt = (size_t)end <= n ? end - at : 0u;
+  // the first and last bucket also hold the keys outside the map
+  job.edge = b == 0 || b == a.nb - 1 ? 1u : 0u;
+  job.cell_shift = m.cell_shift;
+}
+
 template <typename K, bool FLT>
 __global__ void __launch_bounds__(kFinishBlock, kFinishPerSm<K>)
     bucket_finish_kernel(K* in, K* out, K* other, size_t n, BucketArgs a) {
-  constexpr int ITEMS = kFinishItems;
-  constexpr uint32_t B = kFinishBlock;
-  constexpr uint32_t CAP = kFinishCap;
-  constexpr int C = 4;  // items handled together: their atomics in flight at once
-  constexpr int W = B / 32;
-  constexpr int U = (int)kEntries / (W * 64);  // 16-byte reads (two entries) per lane in the scan
-  constexpr uint32_t V = 16 / sizeof(K);
-  static_assert(U == 2 || U == 4, "runs of 64 entries per warp, scanned in pairs as 16-bit halves of one word");
-  static_assert(kHits <= B, "one listed key per thread");
-  extern __shared__ __align__(128) unsigned char smem[];
-  K* s_keys = reinterpret_cast<K*>(smem);                                           // [CAP + V]
-  uint2* s_entry = reinterpret_cast<uint2*>(smem + (CAP + V) * sizeof(K));          // [kEntries]
-  K* s_in = reinterpret_cast<K*>(smem + (CAP + V) * sizeof(K) + kFinishAux);        // [CAP + 2 * V]
-  K* s_hit = s_in + CAP + 2 * V;                                                    // [kHits]
-  __shared__ FinishJob<K> s_job[2];
-  __shared__ uint32_t s_warp[W];
-  __shared__ uint32_t s_nhit, s_over;
-  __shared__ __align__(8) uint64_t s_bar;
   const BucketMap m = *a.map;
   if (!m.on) return;
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  const uint32_t cs = m.cell_shift;
-  auto entry_of = [&](K x) {  // (byte offset: the entry's number times 8)
-    return reinterpret_cast<uint2*>(reinterpret_cast<char*>(s_entry) + ((uint32_t)(x >> (cs + 2)) & ((kEntries - 1) * 8)));
-  };
-  auto cell_of = [&](K x) { return (uint32_t)(x >> cs) & 31u; };
-  // thread 0: bucket b's job, and its keys' bulk copy into s_in, from the
-  // 16-byte boundary at or below the first key to the one at or above the end
-  auto prepare = [&](uint32_t b, uint32_t at, uint32_t end, FinishJob<K>* job) {
-    const uint32_t cnt = end - at;
-    job->first = (K)m.lo + ((K)bucket_first_t(b, m) << m.s);
-    job->at = at;
-    job->cnt = cnt;
-    // (the first and last bucket also hold the keys outside the map)
-    const bool inner = b != 0 && b < a.nb - 1;
-    job->exact = m.exact && inner ? 1u : 0u;
-    uint32_t kind = 3;
-    if (cnt == 0 || (size_t)end > n) {
-      kind = 0;
-    } else if (inner && cnt <= CAP) {
-      const uint32_t skew = skew_of(in + at);
-      const uint32_t len = (skew + cnt + V - 1) / V * V;
-      kind = 2;
-      if (at >= skew && (size_t)at - skew + len <= n) {
-        kind = 1;
-        fence_proxy_async();
-        mbar_arrive_expect_tx(&s_bar, len * (uint32_t)sizeof(K));
-        bulk_load_g2s(s_in, in + at - skew, len * (uint32_t)sizeof(K), &s_bar);
-      }
-    }
-    job->kind = kind;
-  };
-  uint32_t at_next = 0, end_next = 0;  // (thread 0) the bucket after the prepared one
-  if (tid == 0) {
-    mbar_init(&s_bar, 1);
-    mbar_fence_init();
-    prepare(blockIdx.x, a.start[blockIdx.x], a.start[blockIdx.x + 1], &s_job[0]);
-    if (blockIdx.x + gridDim.x < a.nb) {
-      at_next = a.start[blockIdx.x + gridDim.x];
-      end_next = a.start[blockIdx.x + gridDim.x + 1];
-    }
+  // (thread 0) start[b] and start[b + 1] of the next bucket, read a bucket ahead
+  uint32_t at = 0, end = 0;
+  if (threadIdx.x == 0 && blockIdx.x < a.nb) {
+    at = a.start[blockIdx.x];
+    end = a.start[blockIdx.x + 1];
   }
-  uint32_t parity = 0, slot = 0;
-  for (uint32_t b = blockIdx.x; b < a.nb; b += gridDim.x, slot ^= 1u) {
-    if (tid == 0) {
-      s_nhit = 0;
-      s_over = 0;
+  finish_buckets<K, FLT>(a.nb, a.rare, a.err, [&](uint32_t b, FinishJob<K>& job) {
+    plain_job<K>(a, m, b, at, end, in, out, other, n, job);
+    if (b + gridDim.x < a.nb) {
+      at = a.start[b + gridDim.x];
+      end = a.start[b + gridDim.x + 1];
     }
-    for (uint32_t q = tid; q < kEntries / 2; q += B) reinterpret_cast<uint4*>(s_entry)[q] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();  // the job is there; everything of the last bucket is done with
-    const FinishJob<K> job = s_job[slot];
-    const uint32_t cnt = job.cnt;
-    const K first = job.first;
-    // thread 0, once s_in has been read: the next bucket
-    auto next = [&]() {
-      const uint32_t nx = b + gridDim.x;
-      if (tid == 0 && nx < a.nb) {
-        prepare(nx, at_next, end_next, &s_job[slot ^ 1u]);
-        if (nx + gridDim.x < a.nb) {
-          at_next = a.start[nx + gridDim.x];
-          end_next = a.start[nx + gridDim.x + 1];
-        }
-      }
-    };
-    bool done = job.kind == 0;
-    if (job.kind == 0 || job.kind == 3) next();
-    if (job.kind == 1 || job.kind == 2) {
-      const uint32_t skew_in = skew_of(in + job.at);
-      const K* src = s_in + skew_in + tid;
-      bool ok = true;
-      if (job.kind == 1) {
-        ok = mbar_wait_bounded(&s_bar, parity, a.err);
-        parity ^= 1u;
-      } else {
-        for (uint32_t i = tid; i < cnt; i += B) s_in[skew_in + i] = in[job.at + i];  // (read by the same thread)
-      }
-      K k[ITEMS];  // distances from `first`; past the end, whatever s_in holds
-      uint32_t hit = 0;   // bit j: key j found its cell taken
-      uint32_t skip = 0;  // bit j: that, or there is no key j
-#pragma unroll
-      for (int c = 0; c < ITEMS; c += C) {
-        if ((uint32_t)c * B >= cnt) break;
-        uint32_t old[C];
-        if ((uint32_t)(c + C) * B <= cnt) {
-#pragma unroll
-          for (int j = 0; j < C; ++j) {
-            k[c + j] = src[(uint32_t)(c + j) * B] - first;
-            old[j] = atomicOr(&entry_of(k[c + j])->x, 1u << cell_of(k[c + j]));
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < C; ++j) {
-            const bool has = (uint32_t)(c + j) * B + tid < cnt;
-            k[c + j] = src[(uint32_t)(c + j) * B] - first;
-            old[j] = atomicOr(&entry_of(k[c + j])->x, has ? 1u << cell_of(k[c + j]) : 0u);
-            skip |= has ? 0u : 1u << (c + j);
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < C; ++j) hit |= ((old[j] >> cell_of(k[c + j])) & 1u) << (c + j);
-      }
-      hit &= ~skip;
-      skip |= hit;
-      if (hit) {
-        uint32_t p = atomicAdd(&s_nhit, (uint32_t)__popc(hit));
-        for (uint32_t h = hit; h; h &= h - 1u, ++p)
-          if (p < kHits) s_hit[p] = src[((uint32_t)__ffs((int)h) - 1u) * B] - first;
-      }
-      if (!ok) s_over = 2;
-      __syncthreads();
-      const uint32_t nhit = s_nhit;
-      if (s_over == 2) {  // the copy never came: wait it out once more, sort nothing further
-        mbar_wait_bounded(&s_bar, parity ^ 1u, a.err);
-        if (tid == 0) bulk_store_wait_all();
-        return;
-      }
-      next();
-      bool crowded = nhit > kHits;
-      K hx = 0;               // this thread's listed key
-      uint32_t turn = 0;      // its number among its entry's listed keys
-      uint32_t listed = 0, span = 0;  // how many those are; all of the entry's keys
-      if (nhit && !crowded) {
-        if (tid < nhit) {
-          hx = s_hit[tid];
-          turn = atomicAdd(&entry_of(hx)->y, 1u);
-          if (turn >= kEntryHits) s_over = 1;
-        }
-        __syncthreads();
-        crowded = s_over != 0;
-      }
-      if (!crowded) {
-        // Scan: warp w owns kEntries / W entries, lane l entries 2 l and 2 l + 1
-        // of each run of 64.  An entry's keys: its set bits and its listed keys.
-        uint4 q[U];
-        uint32_t c2[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          q[u] = reinterpret_cast<uint4*>(s_entry)[(warp * U + u) * 32 + lane];
-          q[u].y += __popc(q[u].x);
-          c2[u] = q[u].y + q[u].w + __popc(q[u].z);
-        }
-        if (tid < nhit) {
-          const uint2 e = *entry_of(hx);
-          listed = e.y;
-          span = e.y + __popc(e.x);
-        }
-        uint32_t p2[U / 2], t2[U / 2];
-#pragma unroll
-        for (int u = 0; u < U / 2; ++u) p2[u] = c2[2 * u] | (c2[2 * u + 1] << 16);
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-          for (int u = 0; u < U / 2; ++u) {
-            const uint32_t x = __shfl_up_sync(kFull, p2[u], o);
-            if (lane >= (uint32_t)o) p2[u] += x;
-          }
-        }
-        uint32_t total = 0;
-#pragma unroll
-        for (int u = 0; u < U / 2; ++u) {
-          t2[u] = __shfl_sync(kFull, p2[u], 31);
-          total += (t2[u] & 0xFFFFu) + (t2[u] >> 16);
-        }
-        if (lane == 0) s_warp[warp] = total;
-        // (the last bucket's copy out of s_keys must have read it)
-        if (tid == 0) bulk_store_wait_read();
-        __syncthreads();
-        uint32_t before = __reduce_add_sync(kFull, lane < warp ? s_warp[lane & (W - 1)] : 0u);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const uint32_t run = before + (u & 1 ? p2[u / 2] >> 16 : p2[u / 2] & 0xFFFFu) - c2[u];
-          before += u & 1 ? t2[u / 2] >> 16 : t2[u / 2] & 0xFFFFu;
-          q[u].w = run + q[u].y;
-          q[u].y = run;
-          reinterpret_cast<uint4*>(s_entry)[(warp * U + u) * 32 + lane] = q[u];
-        }
-        __syncthreads();
-        // staged with the destination's own offset from a 16-byte boundary
-        K* dst = out + job.at;
-        const uint32_t skew = skew_of(dst);
-        K* stage = s_keys + skew;
-#pragma unroll
-        for (int c = 0; c < ITEMS; c += C) {
-          if ((uint32_t)c * B >= cnt) break;
-#pragma unroll
-          for (int j = c; j < c + C; ++j) {
-            const uint2 e = *entry_of(k[j]);
-            const uint32_t p = e.y + __popc(e.x & ((1u << cell_of(k[j])) - 1u));
-            if (!((skip >> j) & 1u)) stage[p & (CAP - 1)] = from_ordered((K)(k[j] + first), FLT);
-          }
-        }
-        if (nhit) {
-          uint32_t lo = 0, bits = 0;
-          if (tid < nhit) {
-            const uint2 e = *entry_of(hx);
-            lo = e.y;
-            bits = e.x;
-            if (listed > 1) stage[(lo + __popc(bits) + turn) & (CAP - 1)] = from_ordered((K)(hx + first), FLT);
-          }
-          __syncthreads();
-          if (listed == 1) {  // between the key it met and the next: those above move up by one
-            const uint32_t r = lo + __popc(bits & ((1u << cell_of(hx)) - 1u));
-            const uint32_t top = min(CAP, lo + span) - 1u;
-            for (uint32_t j = top; j > r + 1; --j) stage[j] = stage[j - 1];
-            const K x = from_ordered((K)(hx + first), FLT), y = stage[r];
-            const bool below = hx + first < to_ordered(y, FLT);
-            stage[r] = below ? x : y;
-            if (r < top) stage[r + 1] = below ? y : x;
-          } else if (listed > 1 && turn == 0) {  // several: the entry's keys are sorted
-            const uint32_t hi = min(CAP, lo + span);
-            for (uint32_t j = lo + 1; j < hi; ++j) {
-              const K x = stage[j];
-              uint32_t p = j;
-              while (p > lo) {
-                const K y = stage[p - 1];
-                if (to_ordered(y, FLT) <= to_ordered(x, FLT)) break;
-                stage[p] = y;
-                --p;
-              }
-              stage[p] = x;
-            }
-          }
-        }
-        // out: whole 16-byte units in one bulk copy, the keys before the first
-        // and after the last boundary singly
-        fence_proxy_async();
-        __syncthreads();
-        const uint32_t head = min(cnt, (V - skew) & (V - 1));
-        const uint32_t body = (cnt - head) / V * V;
-        if (tid == 0 && body) bulk_store_s2g(dst + head, stage + head, body * (uint32_t)sizeof(K));
-        if (tid >= 32 && tid < 32 + V) {  // (V - 1 keys at most each)
-          const uint32_t i = tid - 32;
-          if (i < head) dst[i] = stage[i];
-          if (head + body + i < cnt) dst[head + body + i] = stage[head + body + i];
-        }
-        done = true;
-      }
-    }
-    if (!done) {
-      if (tid == 0) bulk_store_wait_read();
-      __syncthreads();  // s_keys and s_entry are free
-      if (cnt <= CAP) done = finish_counted<K, FLT>(in + job.at, out + job.at, cnt, first, m.bin_shift, job.exact != 0, smem, s_warp);
-      if (!done) {
-        finish_slow<K>(in + job.at, other + job.at, cnt, in == out, smem);
-        if (FLT)
-          for (uint32_t i = tid; i < cnt; i += B) out[job.at + i] = from_ordered(out[job.at + i], true);
-      }
-      __syncthreads();
-    }
-  }
-  if (tid == 0) bulk_store_wait_all();
+  });
+}
+
+template <typename K, bool FLT>
+__global__ void __launch_bounds__(kRareBlock) bucket_rare_kernel(K* in, K* out, K* other, size_t n, BucketArgs a) {
+  const BucketMap m = *a.map;
+  if (!m.on) return;
+  rare_buckets<K, FLT>(a.rare, [&](uint32_t b, FinishJob<K>& job) {
+    plain_job<K>(a, m, b, a.start[b], a.start[b + 1], in, out, other, n, job);
+  });
 }
 
 template <typename K>
 constexpr size_t finish_smem() {
   constexpr size_t V = 16 / sizeof(K);
-  static_assert((256 + (kFinishBlock / 32) * 257) * 4 + 2 * (kFinishBlock / 32) * sizeof(K) <=
-                    kFinishCap * sizeof(K) + kFinishAux, "finish_slow fits");
   return (2 * (size_t)kFinishCap + 3 * V + kHits) * sizeof(K) + kFinishAux;
 }
 
@@ -1099,6 +1206,7 @@ BucketArgs make_args(const BucketScratch& s, const K* tmp, size_t n, SortCtrl* c
   a.cursor = s.cursor;
   a.group_cursor = s.group_cursor;
   a.tile_first = s.tile_first;
+  a.rare = s.rare;
   a.nb = s.nb;
   while ((1u << a.nb_bits) < s.nb) ++a.nb_bits;
   a.low_bits = s.low_bits;
@@ -1153,7 +1261,388 @@ cudaError_t sort_t(const BucketArgs& a, K* keys, K* tmp, size_t n, cudaStream_t 
   kern<<<std::min<unsigned>(a.nb, sms * kFinishPerSm<K>), kFinishBlock, finish_smem<K>(), stream>>>(
       in, keys, a.low_bits ? tmp : keys, n, a);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  auto rare = bucket_rare_kernel<K, FLT>;
+  if ((e = ensure_dynamic_smem(rare, rare_smem<K>())) != cudaSuccess) return e;
+  rare<<<std::min<unsigned>(a.nb, sms * 2), kRareBlock, rare_smem<K>(), stream>>>(in, keys, a.low_bits ? tmp : keys, n, a);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   return m();
+}
+
+// ---------------------------------------------------------------------------
+// Many segments at once (the batched sort's plans, 32-bit keys).
+// ---------------------------------------------------------------------------
+// The same steps per segment: a map from a sample, counts, one partition pass
+// (up to 2048 bins, so that every segment needs one only: a second pass would
+// cross memory once more, while short runs cost the stores about a third of a
+// pass), and all segments' buckets through the finish kernel.
+using seg::BucketSeg;
+using seg::PlanDev;
+using seg::SegBucketJob;
+using seg::SegBucketsDev;
+using seg::SegMap;
+using seg::SegTileJob;
+using seg::kSegBinsLog2;
+using seg::kSegTile;
+constexpr uint32_t kSegBins = 1u << kSegBinsLog2;
+
+__device__ __forceinline__ uint32_t seg_bucket(uint32_t key, uint32_t lo, uint32_t mult, uint32_t nb_bits) {
+  return mult == 0 ? key >> (32u - nb_bits) : map_bucket(map_t<uint32_t>(key, lo, 0u), mult, (1u << nb_bits) - 1u);
+}
+
+// One CTA per segment of several buckets: the range a sample of 1024 keys spans.
+constexpr int kSegPlanBlock = 256;
+__global__ void __launch_bounds__(kSegPlanBlock) seg_map_kernel(const uint32_t* __restrict__ keys, SegBucketsDev sb) {
+  __shared__ uint32_t s_lo[kSegPlanBlock / 32], s_hi[kSegPlanBlock / 32];
+  __shared__ uint32_t s_cnt[kSegBins];
+  const BucketSeg g = sb.seg[blockIdx.x];
+  uint32_t lo = 0xFFFFFFFFu, hi = 0;
+  uint32_t k[4];
+#pragma unroll
+  for (uint32_t j = 0; j < 4; ++j) {
+    const uint32_t i = j * kSegPlanBlock + threadIdx.x;
+    k[j] = keys[g.base + (((unsigned long long)i * g.len) >> 10)];
+    lo = min(lo, k[j]);
+    hi = max(hi, k[j]);
+  }
+  for (uint32_t i = threadIdx.x; i < (1u << g.nb_bits); i += kSegPlanBlock) s_cnt[i] = 0;
+  lo = __reduce_min_sync(kFull, lo);
+  hi = __reduce_max_sync(kFull, hi);
+  if ((threadIdx.x & 31u) == 0) {
+    s_lo[threadIdx.x >> 5] = lo;
+    s_hi[threadIdx.x >> 5] = hi;
+  }
+  __syncthreads();
+  for (int w = 0; w < kSegPlanBlock / 32; ++w) {
+    lo = min(lo, s_lo[w]);
+    hi = max(hi, s_hi[w]);
+  }
+  const uint32_t pad = (hi - lo) >> 7;  // (about eight keys of the sample's spacing)
+  lo -= min(lo, pad);
+  hi += min(0xFFFFFFFFu - hi, pad);
+  if (hi - lo >= 0xE0000000u) {
+    lo = 0;
+    hi = 0xFFFFFFFFu;
+  }
+  const unsigned long long range = (unsigned long long)(hi - lo) + 1;
+  const uint32_t mult = (uint32_t)min(0xFFFFFFFFull, ((unsigned long long)1 << (32 + g.nb_bits)) / range);
+  // The fullest bucket of the sample: a segment with one far beyond the finish
+  // kernel is left to the digit passes before its keys are counted.
+  uint32_t mx = 0;
+#pragma unroll
+  for (uint32_t j = 0; j < 4; ++j)
+    mx = max(mx, atomicAdd(s_cnt + map_bucket(map_t<uint32_t>(k[j], lo, 0u), mult, (1u << g.nb_bits) - 1u), 1u) + 1u);
+  const uint32_t most = 12u + (uint32_t)(((unsigned long long)(4 * kFinishCap) << 10) / g.len);
+  const bool off = __syncthreads_or(mx > most) != 0;
+  if (threadIdx.x != 0) return;
+  SegMap m{};
+  m.off = off ? 1u : 0u;
+  m.lo = lo;
+  m.mult = mult;
+  m.plain = lo == 0 && hi == 0xFFFFFFFFu ? 1u : 0u;
+  m.inv = (1ull << 63) / mult;
+  const unsigned long long width = ((1ull << 32) + mult - 1) / mult;
+  while (((width - 1) >> m.cell_shift) >= kCells) ++m.cell_shift;
+  sb.map[blockIdx.x] = m;
+}
+
+// Counts per bucket: chunks of 64 K keys, dealt out round robin.
+constexpr int kSegCountBlock = 512;
+__global__ void __launch_bounds__(kSegCountBlock, 3) seg_count_kernel(const PlanDev P) {
+  __shared__ uint32_t s_cnt[kSegBins];
+  for (uint32_t c = blockIdx.x; c < P.sb.chunks; c += gridDim.x) {
+    const seg::Item it = P.items[c];
+    const uint32_t s = P.sb.of_large[it.seg];
+    if (s == 0xFFFFFFFFu) continue;
+    const BucketSeg g = P.sb.seg[s];
+    const SegMap m = P.sb.map[s];
+    if (m.off) continue;
+    const uint32_t nb = 1u << g.nb_bits, mult = m.plain ? 0u : m.mult;
+    for (uint32_t i = threadIdx.x; i < nb; i += kSegCountBlock) s_cnt[i] = 0;
+    __syncthreads();
+    const uint32_t lo = it.idx * seg::kHistChunk;
+    const uint32_t len = min(seg::kHistChunk, g.len - lo);
+    const uint32_t* src = P.keys + g.base + lo;
+    const uint32_t head = min(len, (4u - skew_of(src)) & 3u);
+    const uint32_t nvec = (len - head) / 4u, tail = head + nvec * 4u;
+    const uint4* vec = reinterpret_cast<const uint4*>(src + head);
+    auto add = [&](uint32_t key) { atomicAdd(s_cnt + seg_bucket(key, m.lo, mult, g.nb_bits), 1u); };
+    constexpr uint32_t U = 4;
+    uint32_t v = threadIdx.x;
+    for (; v + (U - 1) * kSegCountBlock < nvec; v += U * kSegCountBlock) {
+      uint4 q[U];
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) q[u] = ld_stream_v4(vec + v + u * kSegCountBlock);
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) {
+        add(q[u].x);
+        add(q[u].y);
+        add(q[u].z);
+        add(q[u].w);
+      }
+    }
+    for (; v < nvec; v += kSegCountBlock) {
+      const uint4 q = ld_stream_v4(vec + v);
+      add(q.x);
+      add(q.y);
+      add(q.z);
+      add(q.w);
+    }
+    if (threadIdx.x < head) add(src[threadIdx.x]);
+    if (threadIdx.x < len - tail) add(src[tail + threadIdx.x]);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < nb; i += kSegCountBlock)
+      if (s_cnt[i]) atomicAdd(P.sb.count + g.first_bucket + i, s_cnt[i]);
+    __syncthreads();
+  }
+}
+
+// One CTA per large segment: its counts become cursors and jobs, or it is
+// declined: no bucket map (longer than the bins allow), or too many of its keys
+// in buckets beyond the finish kernel's shared memory.
+constexpr int kSegScanBlock = 256;
+__global__ void __launch_bounds__(kSegScanBlock) seg_jobs_kernel(const PlanDev P) {
+  __shared__ uint32_t s_warp[kSegScanBlock / 32];
+  __shared__ uint32_t s_over, s_first, s_job0, s_tile0;
+  const uint32_t L = blockIdx.x, tid = threadIdx.x;
+  const uint32_t s = P.sb.of_large[L];
+  bool off = s == 0xFFFFFFFFu;
+  if (!off) {
+    const BucketSeg g = P.sb.seg[s];
+    const SegMap m = P.sb.map[s];
+    const uint32_t nb = 1u << g.nb_bits;
+    uint32_t* cnt = P.sb.count + g.first_bucket;
+    if (tid == 0) s_over = 0;
+    __syncthreads();
+    uint32_t over = 0;
+    for (uint32_t i = tid; i < nb; i += kSegScanBlock) {
+      const uint32_t c = cnt[i];
+      if (c > kFinishCap) over += c > 4 * kFinishCap ? g.len : c;
+    }
+    if (over) atomicAdd(&s_over, min(over, g.len));
+    __syncthreads();
+    off = m.off || s_over > g.len / 32;
+    if (!off) {
+      // room for its jobs behind those of the segments before it
+      const uint32_t tiles = (g.len + 3u + kSegTile - 1u) / kSegTile;
+      if (tid == 0) {
+        s_job0 = P.sb.whole + atomicAdd(&P.declined[seg::kJobBuckets], nb);
+        s_tile0 = atomicAdd(&P.declined[seg::kJobTiles], tiles);
+      }
+      __syncthreads();
+      const uint32_t job0 = s_job0, tile0 = s_tile0;
+      const uint32_t per = (nb + kSegScanBlock - 1) / kSegScanBlock;
+      uint32_t local = 0;
+      for (uint32_t i = tid * per; i < min(nb, (tid + 1) * per); ++i) local += cnt[i];
+      uint32_t run = os::block_exclusive_scan<kSegScanBlock>(local, s_warp);
+      for (uint32_t i = tid * per; i < min(nb, (tid + 1) * per); ++i) {
+        const uint32_t c = cnt[i];
+        SegBucketJob j;
+        j.at = g.base + run;
+        j.cnt = c;
+        j.first = m.plain ? i << (32u - g.nb_bits) : m.lo + bucket_first_t(i, m.mult, m.inv);
+        j.in_keys = 0;
+        j.edge = i == 0 || i == nb - 1 ? 1u : 0u;
+        j.cell_shift = m.cell_shift;
+        P.sb.bucket_job[job0 + i] = j;
+        cnt[i] = run;
+        run += c;
+      }
+      for (uint32_t t = tid; t < tiles; t += kSegScanBlock) {
+        SegTileJob j;
+        j.base = g.base;
+        j.len = g.len;
+        j.tile = t;
+        j.first_bucket = g.first_bucket;
+        j.nb_bits = g.nb_bits;
+        j.lo = m.lo;
+        j.mult = m.plain ? 0u : m.mult;
+        P.sb.tile_job[tile0 + t] = j;
+      }
+    }
+  }
+  if (off) {
+    if (tid == 0) {
+      P.declined[seg::kDeclinedHead + atomicAdd(&P.declined[seg::kDeclinedSegs], 1u)] = L;
+      s_first = atomicAdd(&P.declined[seg::kDeclinedTiles], (P.large[L].len + seg::kPassTile - 1) / seg::kPassTile);
+      P.declined_first[L] = s_first;
+    }
+    __syncthreads();
+    const uint32_t tiles = (P.large[L].len + seg::kPassTile - 1) / seg::kPassTile;
+    for (uint32_t t = tid; t < tiles; t += kSegScanBlock) P.declined_tile[s_first + t] = L;
+  }
+}
+
+// The partition pass (bucket_scatter_kernel's steps) with up to kSegBins bins.
+// A tile's job is copied in a tile ahead, its keys while the tile before it is
+// written out.
+struct SegScatterSmem {
+  uint32_t keys[kSegTile];
+  uint32_t cnt[kSegBins], start[kSegBins], base[kSegBins];
+  SegTileJob job[2];
+  uint32_t warp[kScatterBlock / 32];
+};
+
+__global__ void __launch_bounds__(kScatterBlock, kScatterPerSm) seg_scatter_kernel(const PlanDev P) {
+  constexpr int ITEMS = kScatterItems<uint32_t>;
+  constexpr int Q = ITEMS / 4;
+  constexpr int BPT = (int)kSegBins / kScatterBlock;  // bins per thread
+  static_assert(BPT == 4, "a thread's bins are read as one 16-byte vector");
+  static_assert(kScatterTile<uint32_t> == kSegTile, "one tile geometry");
+  extern __shared__ __align__(16) unsigned char raw[];
+  SegScatterSmem& sm = *reinterpret_cast<SegScatterSmem*>(raw);
+  const uint32_t tid = threadIdx.x;
+  const uint32_t tiles = P.declined[seg::kJobTiles];
+  auto fetch_job = [&](uint32_t tile, uint32_t slot) {  // thread 0
+    if (tile >= tiles) return;
+    const char* src = reinterpret_cast<const char*>(P.sb.tile_job + tile);
+#pragma unroll
+    for (uint32_t i = 0; i < sizeof(SegTileJob); i += 16)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(&sm.job[slot]) + i), "l"(src + i) : "memory");
+  };
+  auto jobs_here = [&]() { asm volatile("cp.async.wait_all;" ::: "memory"); };
+  uint32_t k[ITEMS];
+  uint32_t valid = 0;
+  long long tlo = 0;  // the tile's first place, counted from its segment's first key
+  bool full = false;
+  uint32_t nb_bits = 0, lo = 0, mult = 0, first_bucket = 0, seg_len = 0;
+  unsigned long long seg_base = 0;
+  auto load = [&](uint32_t slot) {
+    const SegTileJob j = sm.job[slot];
+    seg_base = j.base;
+    seg_len = j.len;
+    nb_bits = j.nb_bits;
+    lo = j.lo;
+    mult = j.mult;
+    first_bucket = j.first_bucket;
+    const uint32_t* in = P.keys + seg_base;
+    tlo = (long long)j.tile * kSegTile - skew_of(in);
+    full = tlo >= 0 && tlo + (long long)kSegTile <= (long long)seg_len;
+    if (full) {
+      const uint4* src = reinterpret_cast<const uint4*>(in + tlo) + tid;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const uint4 v = src[q * kScatterBlock];
+        k[4 * q] = v.x;
+        k[4 * q + 1] = v.y;
+        k[4 * q + 2] = v.z;
+        k[4 * q + 3] = v.w;
+      }
+    } else {
+      valid = 0;
+#pragma unroll
+      for (int i = 0; i < ITEMS; ++i) {
+        const long long x = tlo + (long long)i * kScatterBlock + tid;
+        const bool ok = x >= 0 && x < (long long)seg_len;
+        k[i] = ok ? in[x] : 0u;
+        valid |= ok ? 1u << i : 0u;
+      }
+    }
+  };
+  uint32_t slot = 0;
+  if (tid == 0) {
+    fetch_job(blockIdx.x, 0);
+    fetch_job(blockIdx.x + gridDim.x, 1);
+    jobs_here();
+  }
+  __syncthreads();
+  if (blockIdx.x < tiles) load(0);
+  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, slot ^= 1u) {
+    // (the next tile's job is in slot ^ 1; this tile's slot is read: the one after goes there)
+    reinterpret_cast<uint4*>(sm.cnt)[tid] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    if (tid == 0) fetch_job(tile + 2 * gridDim.x, slot);
+    const uint32_t bins = 1u << nb_bits;
+    const uint32_t bits = nb_bits, at0 = first_bucket, l0 = lo, mu = mult, len = seg_len;
+    uint32_t* out = P.tmp + seg_base;
+    const bool was_full = full;
+    // (a segment's last tile is empty when its first key's place in a 16-byte unit left no need for it)
+    const uint32_t cnt = (uint32_t)max(0ll, min(tlo + (long long)kSegTile, (long long)len) - max(tlo, 0ll));
+    auto digit = [&](uint32_t key) { return seg_bucket(key, l0, mu, bits); };
+    uint32_t r[ITEMS / 2];
+#pragma unroll
+    for (int j = 0; j < ITEMS / 2; ++j) r[j] = 0;
+    if (full) {
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j) r[j / 2] |= atomicAdd(sm.cnt + digit(k[j]), 1u) << (16 * (j % 2));
+    } else {
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j)
+        if ((valid >> j) & 1u) r[j / 2] |= atomicAdd(sm.cnt + digit(k[j]), 1u) << (16 * (j % 2));
+    }
+    __syncthreads();
+    const uint4 c4 = reinterpret_cast<const uint4*>(sm.cnt)[tid];
+    uint32_t at[BPT];
+#pragma unroll
+    for (int q = 0; q < BPT; ++q) {  // (consecutive threads, consecutive words)
+      const uint32_t b = (uint32_t)q * kScatterBlock + tid;
+      at[q] = 0;
+      if (b < bins) {
+        const uint32_t c = sm.cnt[b];
+        if (c) at[q] = atomicAdd(P.sb.count + at0 + b, c);
+      }
+    }
+    const uint32_t excl = os::block_exclusive_scan<kScatterBlock>(c4.x + c4.y + c4.z + c4.w, sm.warp);
+    reinterpret_cast<uint4*>(sm.start)[tid] = make_uint4(excl, excl + c4.x, excl + c4.x + c4.y, excl + c4.x + c4.y + c4.z);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j)
+      if (was_full || ((valid >> j) & 1u))
+        sm.keys[sm.start[digit(k[j])] + ((r[j / 2] >> (16 * (j % 2))) & 0xFFFFu)] = k[j];
+#pragma unroll
+    for (int q = 0; q < BPT; ++q) {
+      const uint32_t b = (uint32_t)q * kScatterBlock + tid;
+      if (b < bins) sm.base[b] = at[q] - sm.start[b];
+    }
+    if (tile + gridDim.x < tiles) load(slot ^ 1u);
+    if (tid == 0) jobs_here();
+    __syncthreads();
+    if (was_full) {
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j) {
+        const uint32_t i = (uint32_t)j * kScatterBlock + tid;
+        const uint32_t key = sm.keys[i];
+        const uint32_t o = sm.base[digit(key)] + i;
+        if (o < len) out[o] = key;
+      }
+    } else {
+      for (uint32_t i = tid; i < cnt; i += kScatterBlock) {
+        const uint32_t key = sm.keys[i];
+        const uint32_t o = sm.base[digit(key)] + i;
+        if (o < len) out[o] = key;
+      }
+    }
+    // (no barrier: as in scatter_tiles)
+  }
+}
+
+// Both arrays have `total` keys: a copy that stays inside one of them is safe.
+__device__ __forceinline__ void seg_job(const PlanDev& P, size_t total, const SegBucketJob& j, FinishJob<uint32_t>& job) {
+  job.src = (j.in_keys ? P.keys : P.tmp) + j.at;
+  job.dst = P.keys + j.at;
+  job.other = (j.in_keys ? P.tmp : P.keys) + j.at;
+  job.lo = j.in_keys ? P.keys : P.tmp;
+  job.hi = job.lo + total;
+  job.first = j.first;
+  job.cnt = j.cnt;
+  job.edge = j.edge;
+  job.cell_shift = j.cell_shift;
+}
+
+__global__ void __launch_bounds__(kFinishBlock, kFinishPerSm<uint32_t>) seg_finish_kernel(const PlanDev P, size_t total) {
+  // (thread 0) the next bucket's job, read a bucket ahead
+  const uint32_t jobs = P.sb.whole + P.declined[seg::kJobBuckets];
+  SegBucketJob nj{};
+  if (threadIdx.x == 0 && blockIdx.x < jobs) nj = P.sb.bucket_job[blockIdx.x];
+  finish_buckets<uint32_t, false>(jobs, P.sb.rare, P.err, [&](uint32_t b, FinishJob<uint32_t>& job) {
+    seg_job(P, total, nj, job);
+    if (b + gridDim.x < jobs) nj = P.sb.bucket_job[b + gridDim.x];
+  });
+}
+
+__global__ void __launch_bounds__(kRareBlock) seg_rare_kernel(const PlanDev P, size_t total) {
+  rare_buckets<uint32_t, false>(P.sb.rare, [&](uint32_t b, FinishJob<uint32_t>& job) {
+    seg_job(P, total, P.sb.bucket_job[b], job);
+  });
 }
 
 __global__ void clear_kernel(uint4* p, size_t words, uint32_t* tail, uint32_t tail_words, const uint32_t* off) {
@@ -1210,6 +1699,7 @@ size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s) {
   s->cursor = reinterpret_cast<uint32_t*>(take((size_t)nb * 4));
   s->group_cursor = reinterpret_cast<uint32_t*>(take(kGroups * 4));
   s->tile_first = reinterpret_cast<uint32_t*>(take((kGroups + 1) * 4));
+  s->rare = reinterpret_cast<uint32_t*>(take(((size_t)nb + 1) * 4));
   return off;
 }
 
@@ -1237,4 +1727,37 @@ cudaError_t enqueue_bucket_sort(const BucketScratch& s, void* keys, void* tmp, s
   return is_float ? sort_t<uint32_t, true>(a, k, t, n, stream, mark) : sort_t<uint32_t, false>(a, k, t, n, stream, mark);
 }
 
+namespace seg {
+
+cudaError_t launch_seg_buckets(const PlanDev& pd, size_t total_keys, cudaStream_t s) {
+  const unsigned sms = (unsigned)device_info().sm_count;
+  cudaError_t e = cudaSuccess;
+  if (pd.sb.num) {
+    seg_map_kernel<<<pd.sb.num, kSegPlanBlock, 0, s>>>(pd.keys, pd.sb);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    seg_count_kernel<<<std::min(pd.sb.chunks, sms * 3), kSegCountBlock, 0, s>>>(pd);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  if (pd.num_large) {
+    seg_jobs_kernel<<<pd.num_large, kSegScanBlock, 0, s>>>(pd);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  if (pd.sb.tiles) {
+    if ((e = ensure_dynamic_smem(seg_scatter_kernel, sizeof(SegScatterSmem))) != cudaSuccess) return e;
+    seg_scatter_kernel<<<std::min(pd.sb.tiles, sms * kScatterPerSm), kScatterBlock, sizeof(SegScatterSmem), s>>>(pd);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  if (pd.sb.buckets) {
+    if ((e = ensure_dynamic_smem(seg_finish_kernel, finish_smem<uint32_t>())) != cudaSuccess) return e;
+    seg_finish_kernel<<<std::min(pd.sb.buckets, sms * kFinishPerSm<uint32_t>), kFinishBlock, finish_smem<uint32_t>(), s>>>(
+        pd, total_keys);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = ensure_dynamic_smem(seg_rare_kernel, rare_smem<uint32_t>())) != cudaSuccess) return e;
+    seg_rare_kernel<<<std::min(pd.sb.buckets, sms * 4), kRareBlock, rare_smem<uint32_t>(), s>>>(pd, total_keys);
+    e = cudaGetLastError();
+  }
+  return e;
+}
+
+}  // namespace seg
 }  // namespace pa

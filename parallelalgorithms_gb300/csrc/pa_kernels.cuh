@@ -207,8 +207,6 @@ struct BucketMap {
   uint32_t mult;
   uint32_t s;          // (0 for 32-bit keys)
   uint32_t cell_shift;  // a bucket's keys are spread by (key - first) >> cell_shift
-  uint32_t bin_shift;   // or, counted per bin, by (key - first) >> bin_shift
-  uint32_t exact;       // 1: a bin holds one key value (outside the first and last bucket)
   uint32_t ticket;     // CTAs of the count kernel that are done
   unsigned long long lo;
   unsigned long long inv;  // 2^63 / mult
@@ -222,6 +220,7 @@ struct BucketScratch {
   uint32_t* cursor = nullptr;        // [nb]
   uint32_t* group_cursor = nullptr;  // [nb >> low_bits]
   uint32_t* tile_first = nullptr;    // [(nb >> low_bits) + 1] first tile of each group in the second pass
+  uint32_t* rare = nullptr;          // [1 + nb] buckets left to a launch of their own
 };
 // Sizes this sort takes: more keys than the one-CTA sort, and few enough that
 // the most buckets there can be fit the finish kernel with room to spare.

@@ -1,6 +1,18 @@
 // Batched segmented sort: thousands of uint32 arrays of uneven size, each
-// sorted independently (stable, ascending), in ONE persistent kernel launch
-// fed by a device work queue, launched through a captured CUDA graph.
+// sorted independently (stable, ascending), through a captured CUDA graph.
+//
+// Public plans with 8-bit digits sort by buckets (launch_seg_buckets,
+// pa_buckets.cu); only the segments that declines go through the digit passes
+// here (declined_*_kernel, seg_pass_kernel over a list made on the device).  4096
+// arrays of 1 K to 4 M uniform keys, 2.0 G keys: 15.9 ms against 36.0 with four
+// digit passes; 64 arrays of 1 K to 50 K keys 39 us against 58.  Skewed keys pay
+// for the maps and counts they are declined on (the 2.0 G keys skewed: 37.9 ms
+// against 36.1; 300 arrays of up to 1 M keys 1.01 ms against 0.86; the 64 small
+// arrays 97 us against 58, most of it launches).
+//
+// 11-bit plans, and the plans other sorts build for their groups, run ONE
+// persistent kernel fed by a device work queue (8-bit ones then a launch per
+// digit pass):
 //
 // No reference counterpart: the reference sorts one array per call
 // (SortRadixPar, RadixSortLsdParallel.h:367); its nearest idea is bundling
@@ -229,38 +241,83 @@ __global__ void __launch_bounds__(kPassBlock, 3) seg_pass_kernel(const PlanDev P
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + PassGeometry::kBarOff);
   uint32_t* s_tile = reinterpret_cast<uint32_t*>(smem + PassGeometry::kTileIdOff);
+  // all large segments' tiles, or those of the segments the bucket sort declined
+  const uint32_t tiles = P.by_buckets ? P.declined[kDeclinedTiles] : P.pass_tiles;
+  if (tiles == 0) return;
   if (threadIdx.x == 0) {
-    *s_tile = atomicAdd(P.pass_ticket, 1u);
     mbar_init(s_bar, 1);
     mbar_fence_init();
   }
-  __syncthreads();
-  const uint32_t g = *s_tile;
-  if (g >= P.pass_tiles) {  // a ticket counter that was not cleared
-    if (threadIdx.x == 0) raise_error(P.err, DEVERR_BAD_STATE);
-    return;
-  }
-  const uint32_t seg = P.tile_seg[g];
-  const LargeSeg L = P.large[seg];
-  const bool even = (pass & 1u) == 0;
-  TileJob<uint32_t, uint32_t> job;
-  job.in = (even ? P.keys : P.tmp) + L.base;
-  job.out = (even ? P.tmp : P.keys) + L.base;
-  job.vin = nullptr;
-  job.vout = nullptr;
-  job.n = L.len;
-  job.out_n = L.len;
-  job.tile = g - L.ptile_base;
-  job.shift = 8u * pass;
-  job.tin = false;
-  job.tout = false;
-  job.bin_start = P.bin_start + (size_t)seg * 4 * 256 + pass * 256;
-  job.status = P.pass_status + (size_t)L.ptile_base * 256;
-  job.err = P.err;
-  job.spin_limit = kSpinLimit;
   uint32_t parity = 0;
-  onesweep_tile_multisplit<uint32_t, false, kPassBlock, kPassItems, uint32_t>(job, smem, s_bar, parity);
+  for (;;) {  // resident CTAs take tickets until the tiles are used up
+    if (threadIdx.x == 0) *s_tile = atomicAdd(P.pass_ticket + pass, 1u);
+    __syncthreads();
+    const uint32_t g = *s_tile;
+    if (g >= tiles) {
+      if (g >= tiles + gridDim.x && threadIdx.x == 0) raise_error(P.err, DEVERR_BAD_STATE);  // a counter not cleared
+      return;
+    }
+    const uint32_t seg = P.by_buckets ? P.declined_tile[g] : P.tile_seg[g];
+    const LargeSeg L = P.large[seg];
+    const uint32_t first = P.by_buckets ? P.declined_first[seg] : L.ptile_base;
+    const bool even = (pass & 1u) == 0;
+    TileJob<uint32_t, uint32_t> job;
+    job.in = (even ? P.keys : P.tmp) + L.base;
+    job.out = (even ? P.tmp : P.keys) + L.base;
+    job.vin = nullptr;
+    job.vout = nullptr;
+    job.n = L.len;
+    job.out_n = L.len;
+    job.tile = g - first;
+    job.shift = 8u * pass;
+    job.tin = false;
+    job.tout = false;
+    job.bin_start = P.bin_start + (size_t)seg * 4 * 256 + pass * 256;
+    job.status = P.pass_status + ((size_t)first + (P.by_buckets && P.status_sets > 1 ? (size_t)pass * P.pass_tiles : 0)) * 256;
+    job.err = P.err;
+    job.spin_limit = kSpinLimit;
+    onesweep_tile_multisplit<uint32_t, false, kPassBlock, kPassItems, uint32_t>(job, smem, s_bar, parity);
+    __syncthreads();
+    // (a tile that gave up ends its CTA, as in the plain pass)
+    if (*reinterpret_cast<uint32_t*>(smem + PassGeometry::kAbortOff)) return;
+  }
 }
+
+// The segments the bucket sort declined: their tiles' look-back words cleared
+// (sets: passes to clear for), their digit counts (each CTA takes every
+// gridDim.x-th chunk of each) and bin starts.
+__device__ __forceinline__ void clear_status(const PlanDev& P, uint32_t sets) {
+  const size_t words = (size_t)P.declined[kDeclinedTiles] * 64;  // 16-byte words: 256 counters a tile
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (uint32_t p = 0; p < sets; ++p) {
+    uint4* q = reinterpret_cast<uint4*>(P.pass_status + (size_t)p * P.pass_tiles * 256);
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += stride) q[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+
+__global__ void __launch_bounds__(kBlock, 2) declined_counts_kernel(const PlanDev P) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  const uint32_t num = P.declined[kDeclinedSegs];
+  if (num == 0) return;
+  clear_status(P, P.status_sets);
+  for (uint32_t d = 0; d < num; ++d) {
+    const uint32_t seg = P.declined[kDeclinedHead + d];
+    const uint32_t chunks = P.large[seg].hist_chunks;
+    for (uint32_t c = (blockIdx.x + d * 61u) % gridDim.x; c < chunks; c += gridDim.x) {
+      hist_item<8>(P, Item{ITEM_HIST, 0, seg, c}, smem);
+      __syncthreads();
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kBlock) declined_scan_kernel(const PlanDev P) {
+  __shared__ __align__(16) unsigned char s_scan[kBlock / 32 * 4];
+  const uint32_t num = P.declined[kDeclinedSegs];
+  for (uint32_t d = blockIdx.x; d < num; d += gridDim.x)
+    scan_item<8>(P, Item{ITEM_SCAN, 0, P.declined[kDeclinedHead + d], 0}, s_scan);
+}
+
+__global__ void __launch_bounds__(256) declined_clear_kernel(const PlanDev P) { clear_status(P, 1); }
 
 // ---- host side ---------------------------------------------------------------
 template <int PI, int SI, int RB>
@@ -298,8 +355,10 @@ bool pick_kernel(int tile_keys, int small_cutoff, int radix_bits, KernelChoice* 
 }
 
 // ---- host-side planning --------------------------------------------------------
+constexpr uint32_t kStatusSetTiles = 16384;  // 64 MB of look-back words for four passes
+
 int build_host_plan(const uint64_t* off_host, size_t num_segments, const pa_segsort_config* cfg, HostPlan* hp,
-                    int passes) {
+                    int passes, bool by_buckets) {
   if (passes < 1 || passes > kPasses) return record_error(PA_ERR_ARG, "a batched plan runs 1 to 4 digit passes");
   pa_segsort_config c{};
   if (cfg) c = *cfg;
@@ -327,6 +386,11 @@ int build_host_plan(const uint64_t* off_host, size_t num_segments, const pa_segs
   hp->split = c.digit_bits == 8;
   hp->tile_seg.clear();
   hp->pass_tiles = 0;
+  hp->by_buckets = by_buckets && hp->split && passes == kPasses;
+  hp->bsegs.clear();
+  hp->of_large.clear();
+  hp->bjobs.clear();
+  hp->buckets = hp->part_tiles = 0;
   hp->off.assign(off, off + num_segments + 1);
   hp->items.clear();
   hp->large.clear();
@@ -335,7 +399,9 @@ int build_host_plan(const uint64_t* off_host, size_t num_segments, const pa_segs
   for (size_t i = 0; i < num_segments; ++i) {
     const uint64_t len = off[i + 1] - off[i];
     if (len == 0 || (len == 1 && (passes % 2) == 0)) continue;  // (an odd pass count moves even single keys to tmp)
-    if (len <= (uint64_t)kc.small_tile && len <= (uint64_t)c.small_cutoff) {
+    const bool small = hp->by_buckets ? len <= (uint64_t)kBucketSegKeys
+                                      : len <= (uint64_t)kc.small_tile && len <= (uint64_t)c.small_cutoff;
+    if (small) {
       small_ids.push_back((uint32_t)i);
     } else {
       LargeSeg L{};
@@ -345,6 +411,18 @@ int build_host_plan(const uint64_t* off_host, size_t num_segments, const pa_segs
       L.hist_chunks = (uint32_t)((len + kHistChunk - 1) / kHistChunk);
       L.tile_base = total_tiles;
       total_tiles += L.tiles;
+      if (hp->by_buckets) {
+        uint32_t bits = 1;  // about 1500 to 3072 keys a bucket
+        while (bits < kSegBinsLog2 && (len >> bits) > 3072) ++bits;
+        if (len > kBucketSegMax) {
+          hp->of_large.push_back(0xFFFFFFFFu);
+        } else {
+          hp->of_large.push_back((uint32_t)hp->bsegs.size());
+          hp->bsegs.push_back({off[i], (uint32_t)len, bits, hp->buckets, hp->part_tiles, (uint32_t)hp->large.size(), 0});
+          hp->buckets += 1u << bits;
+          hp->part_tiles += (uint32_t)((len + 3 + kSegTile - 1) / kSegTile);
+        }
+      }
       if (hp->split) {
         const uint32_t pt = (uint32_t)((len + kPassTile - 1) / kPassTile);
         L.ptile_base = hp->pass_tiles;
@@ -368,6 +446,12 @@ int build_host_plan(const uint64_t* off_host, size_t num_segments, const pa_segs
   const uint32_t nlarge = (uint32_t)hp->large.size();
   for (uint32_t l = 0; l < nlarge; ++l)
     for (uint32_t ch = 0; ch < hp->large[l].hist_chunks; ++ch) items.push_back({ITEM_HIST, 0, l, ch});
+  hp->hist_items = (uint32_t)items.size();
+  if (hp->by_buckets) {  // a small segment is one bucket, sorted in place
+    for (uint32_t i : small_ids)
+      hp->bjobs.push_back({off[i], (uint32_t)(off[i + 1] - off[i]), 0u, 1u, 1u, 0u, 0u});
+    hp->buckets += (uint32_t)hp->bjobs.size();
+  }
   add_small(1);
   for (uint32_t l = 0; l < nlarge; ++l) items.push_back({ITEM_SCAN, 0, l, 0});
   add_small(2);
@@ -401,9 +485,25 @@ int build_host_plan(const uint64_t* off_host, size_t num_segments, const pa_segs
   hp->o_head = take(256);  // everything from here on is cleared per run
   hp->o_done = take(nl * kStages * 4);
   hp->o_hist = take(nl * per_seg * 4);
+  if (hp->by_buckets) {
+    hp->o_count = take((size_t)std::max<uint32_t>(hp->buckets, 1) * 4);
+    hp->o_decl = take((kDeclinedHead + nl) * 4);
+    hp->o_rare = take(((size_t)hp->buckets + 1) * 4);
+  }
   hp->o_status = take(hp->split ? 0 : (size_t)passes * std::max<uint32_t>(total_tiles, 1) * seg_bins(hp->radix_bits) * 4);
   hp->o_pticket = take(256);
-  hp->o_pstatus = take((size_t)std::max<uint32_t>(hp->pass_tiles, 1) * 256 * 4);
+  // (a plan by buckets: the passes' words all at once where that is little memory)
+  hp->status_sets = hp->by_buckets && hp->pass_tiles <= kStatusSetTiles ? (uint32_t)passes : 1u;
+  hp->o_pstatus = take((size_t)std::max<uint32_t>(hp->pass_tiles, 1) * 256 * 4 * hp->status_sets);
+  if (hp->by_buckets) {  // (not cleared)
+    hp->o_bseg = take(std::max<size_t>(hp->bsegs.size(), 1) * sizeof(BucketSeg));
+    hp->o_of_large = take(nl * 4);
+    hp->o_map = take(std::max<size_t>(hp->bsegs.size(), 1) * sizeof(SegMap));
+    hp->o_bjob = take((size_t)std::max<uint32_t>(hp->buckets, 1) * sizeof(SegBucketJob));
+    hp->o_tjob = take((size_t)std::max<uint32_t>(hp->part_tiles, 1) * sizeof(SegTileJob));
+    hp->o_dtile = take((size_t)std::max<uint32_t>(hp->pass_tiles, 1) * 4);
+    hp->o_dfirst = take(nl * 4);
+  }
   hp->bytes = o;
   return PA_OK;
 }
@@ -429,6 +529,26 @@ PlanDev device_view(const HostPlan& hp, char* dev, uint32_t* keys, uint32_t* tmp
   d.pass_tiles = hp.pass_tiles;
   d.pass_ticket = reinterpret_cast<uint32_t*>(dev + hp.o_pticket);
   d.pass_status = reinterpret_cast<uint32_t*>(dev + hp.o_pstatus);
+  d.by_buckets = hp.by_buckets ? 1u : 0u;
+  d.num_large = hp.num_large;
+  if (hp.by_buckets) {
+    d.status_sets = hp.status_sets;
+    d.sb.whole = (uint32_t)hp.bjobs.size();
+    d.declined = reinterpret_cast<uint32_t*>(dev + hp.o_decl);
+    d.declined_tile = reinterpret_cast<uint32_t*>(dev + hp.o_dtile);
+    d.declined_first = reinterpret_cast<uint32_t*>(dev + hp.o_dfirst);
+    d.sb.rare = reinterpret_cast<uint32_t*>(dev + hp.o_rare);
+    d.sb.num = (uint32_t)hp.bsegs.size();
+    d.sb.buckets = hp.buckets;
+    d.sb.tiles = hp.part_tiles;
+    d.sb.chunks = hp.hist_items;
+    d.sb.seg = reinterpret_cast<const BucketSeg*>(dev + hp.o_bseg);
+    d.sb.of_large = reinterpret_cast<const uint32_t*>(dev + hp.o_of_large);
+    d.sb.map = reinterpret_cast<SegMap*>(dev + hp.o_map);
+    d.sb.count = reinterpret_cast<uint32_t*>(dev + hp.o_count);
+    d.sb.tile_job = reinterpret_cast<SegTileJob*>(dev + hp.o_tjob);
+    d.sb.bucket_job = reinterpret_cast<SegBucketJob*>(dev + hp.o_bjob);
+  }
   return d;
 }
 
@@ -436,6 +556,7 @@ size_t plan_image_bytes(const HostPlan& hp) { return hp.o_tile_seg + std::max<si
 
 cudaError_t upload_plan(const HostPlan& hp, char* dev, cudaStream_t s, void* pinned_staging) {
   cudaError_t e = cudaSuccess;
+  if (pinned_staging && hp.by_buckets) return cudaErrorInvalidValue;  // (its tables are not in the image)
   if (pinned_staging) {
     char* img = static_cast<char*>(pinned_staging);
     const size_t bytes = plan_image_bytes(hp);
@@ -457,6 +578,13 @@ cudaError_t upload_plan(const HostPlan& hp, char* dev, cudaStream_t s, void* pin
                         cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && !hp.tile_seg.empty())
     e = cudaMemcpyAsync(dev + hp.o_tile_seg, hp.tile_seg.data(), hp.tile_seg.size() * 4, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess && !hp.bsegs.empty())
+    e = cudaMemcpyAsync(dev + hp.o_bseg, hp.bsegs.data(), hp.bsegs.size() * sizeof(BucketSeg), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess && !hp.of_large.empty())
+    e = cudaMemcpyAsync(dev + hp.o_of_large, hp.of_large.data(), hp.of_large.size() * 4, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess && !hp.bjobs.empty())  // (the partitioned segments' jobs, behind them, are written by each run)
+    e = cudaMemcpyAsync(dev + hp.o_bjob, hp.bjobs.data(), hp.bjobs.size() * sizeof(SegBucketJob),
+                        cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(dev + hp.o_err, 0, 256, s);
   return e;
 }
@@ -476,17 +604,37 @@ unsigned plan_grid(const HostPlan& hp) {
 }
 
 cudaError_t launch_plan(const HostPlan& hp, const PlanDev& pd, char* dev, unsigned grid, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(dev + hp.o_head, 0, hp.o_pticket - hp.o_head, s);
+  cudaError_t e = cudaMemsetAsync(dev + hp.o_head, 0, hp.o_pticket + 256 - hp.o_head, s);
   if (e != cudaSuccess) return e;
+  const unsigned sms = (unsigned)device_info().sm_count;
+  const unsigned pass_grid = std::min<unsigned>(hp.pass_tiles, sms * 3);
+  if (hp.by_buckets) {
+    e = launch_seg_buckets(pd, hp.off.empty() ? 0 : (size_t)hp.off.back(), s);
+    if (e != cudaSuccess || hp.pass_tiles == 0) return e;
+    // the declined segments' digit passes (launches that return at once when
+    // there are none)
+    const size_t hist_smem = (size_t)4 * 256 * hist_lanes<8>() * 4;
+    declined_counts_kernel<<<sms * 2, kBlock, hist_smem, s>>>(pd);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    declined_scan_kernel<<<std::min<unsigned>(hp.num_large, sms), kBlock, 0, s>>>(pd);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    for (uint32_t p = 0; p < hp.passes && e == cudaSuccess; ++p) {
+      if (p > 0 && hp.status_sets == 1) declined_clear_kernel<<<sms * 4, 256, 0, s>>>(pd);
+      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+      seg_pass_kernel<<<pass_grid, kPassBlock, PassGeometry::kBytes, s>>>(pd, p);
+      e = cudaGetLastError();
+    }
+    return e;
+  }
   if (!hp.items.empty()) {
     hp.kc.fn<<<grid, kBlock, hp.kc.smem, s>>>(pd);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   if (!hp.split || hp.pass_tiles == 0) return cudaSuccess;
   for (uint32_t p = 0; p < hp.passes && e == cudaSuccess; ++p) {
-    e = cudaMemsetAsync(dev + hp.o_pticket, 0, hp.bytes - hp.o_pticket, s);
+    e = cudaMemsetAsync(dev + hp.o_pstatus, 0, (size_t)hp.pass_tiles * 256 * 4, s);
     if (e == cudaSuccess) {
-      seg_pass_kernel<<<hp.pass_tiles, kPassBlock, PassGeometry::kBytes, s>>>(pd, p);
+      seg_pass_kernel<<<pass_grid, kPassBlock, PassGeometry::kBytes, s>>>(pd, p);
       e = cudaGetLastError();
     }
   }
@@ -579,7 +727,7 @@ int pa_segsort_plan_create(const uint64_t* seg_offsets, size_t num_segments, con
     std::memcpy(off.data(), seg_offsets, off.size() * 8);
   }
   auto* p = new pa_segsort_plan();
-  if (int rc = build_host_plan(off.data(), num_segments, cfg, &p->hp)) {
+  if (int rc = build_host_plan(off.data(), num_segments, cfg, &p->hp, kPasses, true)) {
     delete p;
     return rc;
   }

@@ -40,6 +40,67 @@ struct LargeSeg {
   uint32_t pad;
 };
 
+// Plans that sort by buckets (pa_buckets.cu): a segment of at most
+// kBucketSegKeys keys is one bucket; a longer one of up to kBucketSegMax keys is
+// counted and partitioned into a power of two of buckets in one pass; longer
+// ones, and those whose keys crowd into few buckets, are left to the digit
+// passes (declined).
+constexpr uint32_t kBucketSegKeys = 4096;
+constexpr uint32_t kSegBinsLog2 = 11;  // most buckets of a segment
+constexpr uint32_t kSegTile = 8192;    // keys per partition tile
+constexpr uint32_t kBucketSegMax = (1u << kSegBinsLog2) * 3072u;
+
+struct BucketSeg {
+  unsigned long long base;
+  uint32_t len;
+  uint32_t nb_bits;       // 1 << nb_bits buckets
+  uint32_t first_bucket;  // of all segments' buckets
+  uint32_t first_tile;    // of all partition tiles (segments of several buckets)
+  uint32_t large;         // its LargeSeg
+  uint32_t pad;
+};
+// Device side, written by each run: a segment's map (as BucketMap), a tile's
+// and a bucket's job.
+struct SegMap {
+  uint32_t lo, mult, plain, off;  // off: left to the digit passes
+  unsigned long long inv;
+  uint32_t cell_shift, pad;
+};
+struct __align__(16) SegTileJob {
+  unsigned long long base;  // first key of its segment
+  uint32_t len;             // keys of its segment
+  uint32_t tile;            // its number in the segment
+  uint32_t first_bucket;
+  uint32_t nb_bits;
+  uint32_t lo, mult;        // mult 0: a plain map
+};
+struct __align__(16) SegBucketJob {
+  unsigned long long at;  // first key
+  uint32_t cnt;
+  uint32_t first;
+  uint32_t in_keys;   // 1: the bucket is a whole segment, still in the key array
+  uint32_t edge;
+  uint32_t cell_shift, pad;
+};
+// Words of PlanDev::declined, zeroed per run: declined segments and their pass
+// tiles; jobs of the others' buckets (behind the whole segments') and tiles;
+// then the declined segments.
+enum : uint32_t { kDeclinedSegs = 0, kDeclinedTiles = 1, kJobBuckets = 2, kJobTiles = 3, kDeclinedHead = 4 };
+struct SegBucketsDev {
+  uint32_t num;                 // segments of several buckets
+  uint32_t whole;               // segments that are one bucket: the first jobs, uploaded with the plan
+  uint32_t buckets;             // of all segments
+  uint32_t tiles;               // partition tiles
+  uint32_t chunks;              // count chunks: the plan's first `chunks` HIST items
+  const BucketSeg* seg;         // [num]
+  const uint32_t* of_large;     // [large] BucketSeg of a large segment, all ones: declined
+  SegMap* map;                  // [num]
+  uint32_t* count;              // [buckets] zeroed per run; then the partition's cursors
+  SegTileJob* tile_job;         // [tiles]
+  SegBucketJob* bucket_job;     // [buckets]
+  uint32_t* rare;               // [1 + buckets] buckets left to a launch of their own; [0] zeroed per run
+};
+
 // 8-bit plans run their digit passes as separate launches after the
 // persistent kernel: one onesweep launch per pass over every large
 // segment's tiles (the plain sort's pass geometry), look-back within each
@@ -70,6 +131,15 @@ struct PlanDev {
   uint32_t pass_tiles;
   uint32_t* pass_ticket;           // zeroed before each pass
   uint32_t* pass_status;           // [pass_tiles][256], zeroed before each pass
+  // Plans that sort by buckets: the digit passes' segments are listed on the
+  // device (`by_buckets` not zero).
+  uint32_t by_buckets;
+  uint32_t num_large;
+  uint32_t* declined;              // [kDeclinedHead + large]
+  uint32_t status_sets;            // look-back words for that many passes (one: cleared between passes)
+  uint32_t* declined_tile;         // [pass_tiles] segment of each of their tiles
+  uint32_t* declined_first;        // [large] a segment's first tile among them
+  SegBucketsDev sb;
 };
 
 // Digits of a 32-bit key and bins per digit for a digit width.
@@ -101,6 +171,14 @@ struct HostPlan {
   bool split = false;              // digit passes as separate launches (8-bit plans)
   uint32_t pass_tiles = 0;
   std::vector<uint32_t> tile_seg;
+  // plans that sort by buckets
+  bool by_buckets = false;
+  std::vector<BucketSeg> bsegs;
+  std::vector<uint32_t> of_large;
+  std::vector<SegBucketJob> bjobs;
+  uint32_t hist_items = 0, buckets = 0, part_tiles = 0, status_sets = 1;
+  size_t o_bseg = 0, o_of_large = 0, o_bjob = 0, o_map = 0, o_count = 0, o_tjob = 0, o_decl = 0, o_rare = 0, o_dtile = 0,
+         o_dfirst = 0;
   size_t o_items = 0, o_off = 0, o_large = 0, o_tile_seg = 0, o_bins = 0, o_err = 0, o_head = 0, o_done = 0,
          o_hist = 0, o_status = 0, o_pticket = 0, o_pstatus = 0, bytes = 0;
 };
@@ -110,8 +188,13 @@ struct HostPlan {
 // segments whose higher bytes are constant); results then end in tmp when
 // `passes` is odd (result_buffer).  With cfg->digit_bits = 11 the plan runs
 // three 11-bit passes (and `passes` is ignored).
+// by_buckets: 8-bit plans of four passes sort by buckets where they can (more
+// device memory: 64 bytes a bucket and 32 a tile).
 int build_host_plan(const uint64_t* off_host, size_t num_segments, const pa_segsort_config* cfg, HostPlan* hp,
-                    int passes = kPasses);
+                    int passes = kPasses, bool by_buckets = false);
+// The bucket part of a run (pa_buckets.cu): maps, counts, partition and the
+// sort of every bucket; segments it declines are listed in pd.declined.
+cudaError_t launch_seg_buckets(const PlanDev& pd, size_t total_keys, cudaStream_t s);
 // Pointers of a device block laid out by `hp` (keys / tmp: the batch's keys).
 PlanDev device_view(const HostPlan& hp, char* dev, uint32_t* keys, uint32_t* tmp);
 // Where a run of `pd` leaves the sorted keys: keys after an even number of
