@@ -618,9 +618,7 @@ template <typename K>
 constexpr int kFinishPerSm = sizeof(K) == 4 ? 4 : 2;
 constexpr uint32_t kFinishCap = 4096;
 constexpr int kFinishItems = (int)kFinishCap / kFinishBlock;
-constexpr uint32_t kEntries = kCells / 32;
 constexpr uint32_t kEntryHits = 6;  // keys of one entry that found their cell taken, at most
-constexpr uint32_t kHits = 256;     // such keys of one bucket, at most
 
 // The least t with umulhi(t, mult) >= b (b < nb), from the rounded-down
 // reciprocal inv = 2^63 / mult: the estimate is at most two short.
@@ -630,7 +628,6 @@ __device__ __forceinline__ uint32_t bucket_first_t(uint32_t b, uint32_t mult, un
   return t;
 }
 
-constexpr size_t kFinishAux = kEntries * 8;  // bytes of the bitmap
 
 // What thread 0 prepares of the next bucket while the CTA works on one.
 enum : uint32_t {
@@ -652,12 +649,11 @@ struct FinishJob {
   const K *lo, *hi;     // the array src lies in
 };
 
-// Cells and bins of keys that span `range`.
+// The shift that leaves at most `keep` bits of distances up to `range`.
 template <typename K>
-__device__ __forceinline__ void spread_of(K range, uint32_t& cell_shift, uint32_t& bin_shift) {
+__device__ __forceinline__ uint32_t spread_of(K range, int keep) {
   const int bits = 8 * (int)sizeof(K) - (sizeof(K) == 4 ? __clz((int)(uint32_t)range) : __clzll((long long)range));
-  cell_shift = (uint32_t)max(0, bits - kCellBits);
-  bin_shift = (uint32_t)max(0, bits - kBinBits);
+  return (uint32_t)max(0, bits - keep);
 }
 
 // Sorts buckets blockIdx.x, blockIdx.x + gridDim.x, ... below nb.  next(b, job)
@@ -665,21 +661,25 @@ __device__ __forceinline__ void spread_of(K range, uint32_t& cell_shift, uint32_
 // for are listed (rare[0]: how many, rare[1...]: which) and sorted by
 // rare_buckets: their code here would cost the main path its registers (0.51 ms
 // against 0.35 at 100M keys).
-template <typename K, bool FLT, typename Next>
+// RAW: float keys are read as they are stored, not in ordered form.
+template <typename K, bool FLT, int BLOCK = kFinishBlock, uint32_t CAP = kFinishCap, int CELL_BITS = kCellBits,
+          bool RAW = false, typename Next>
 __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint32_t* err, Next&& next) {
-  constexpr int ITEMS = kFinishItems;
-  constexpr uint32_t B = kFinishBlock;
-  constexpr uint32_t CAP = kFinishCap;
+  constexpr uint32_t B = BLOCK;
+  constexpr int ITEMS = (int)CAP / BLOCK;
+  constexpr uint32_t kEntries = 1u << (CELL_BITS - 5);
+  constexpr uint32_t kHits = B;  // one listed key per thread
+  constexpr size_t kAux = kEntries * 8;
   constexpr int C = 4;  // items handled together: their atomics in flight at once
   constexpr int W = B / 32;
   constexpr int U = (int)kEntries / (W * 64);  // 16-byte reads (two entries) per lane in the scan
   constexpr uint32_t V = 16 / sizeof(K);
   static_assert(U == 2 || U == 4, "runs of 64 entries per warp, scanned in pairs as 16-bit halves of one word");
-  static_assert(kHits <= B, "one listed key per thread");
+  static_assert((CAP & (CAP - 1)) == 0 && ITEMS <= 16 && ITEMS % C == 0, "whole groups of items; places are masked");
   extern __shared__ __align__(128) unsigned char smem[];
   K* s_keys = reinterpret_cast<K*>(smem);                                           // [CAP + V]
   uint2* s_entry = reinterpret_cast<uint2*>(smem + (CAP + V) * sizeof(K));          // [kEntries]
-  K* s_in = reinterpret_cast<K*>(smem + (CAP + V) * sizeof(K) + kFinishAux);        // [CAP + 2 * V]
+  K* s_in = reinterpret_cast<K*>(smem + (CAP + V) * sizeof(K) + kAux);              // [CAP + 2 * V]
   K* s_hit = s_in + CAP + 2 * V;                                                    // [kHits]
   __shared__ FinishJob<K> s_job[2];
   __shared__ K s_edge[2 * W];
@@ -748,8 +748,9 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
       if (job.edge) {  // the bucket's own range
         K lo = ~(K)0, hi = 0;
         for (uint32_t i = 0; i + tid < cnt; i += B) {
-          lo = min(lo, src[i]);
-          hi = max(hi, src[i]);
+          const K x = to_ordered(src[i], RAW);
+          lo = min(lo, x);
+          hi = max(hi, x);
         }
         warp_minmax(lo, hi);
         if (lane == 0) {
@@ -762,9 +763,8 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
           lo = min(lo, s_edge[w]);
           hi = max(hi, s_edge[W + w]);
         }
-        uint32_t bins;
         first = lo;
-        spread_of<K>((K)(hi - lo), cs, bins);
+        cs = spread_of<K>((K)(hi - lo), CELL_BITS);
       }
       K k[ITEMS];  // distances from `first`; past the end, whatever s_in holds
       uint32_t hit = 0;   // bit j: key j found its cell taken
@@ -776,14 +776,14 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
         if ((uint32_t)(c + C) * B <= cnt) {
 #pragma unroll
           for (int j = 0; j < C; ++j) {
-            k[c + j] = src[(uint32_t)(c + j) * B] - first;
+            k[c + j] = to_ordered(src[(uint32_t)(c + j) * B], RAW) - first;
             old[j] = atomicOr(&entry_of(k[c + j])->x, 1u << cell_of(k[c + j]));
           }
         } else {
 #pragma unroll
           for (int j = 0; j < C; ++j) {
             const bool has = (uint32_t)(c + j) * B + tid < cnt;
-            k[c + j] = src[(uint32_t)(c + j) * B] - first;
+            k[c + j] = to_ordered(src[(uint32_t)(c + j) * B], RAW) - first;
             old[j] = atomicOr(&entry_of(k[c + j])->x, has ? 1u << cell_of(k[c + j]) : 0u);
             skip |= has ? 0u : 1u << (c + j);
           }
@@ -796,7 +796,7 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
       if (hit) {
         uint32_t p = atomicAdd(&s_nhit, (uint32_t)__popc(hit));
         for (uint32_t h = hit; h; h &= h - 1u, ++p)
-          if (p < kHits) s_hit[p] = src[((uint32_t)__ffs((int)h) - 1u) * B] - first;
+          if (p < kHits) s_hit[p] = to_ordered(src[((uint32_t)__ffs((int)h) - 1u) * B], RAW) - first;
       }
       if (!ok) s_over = 2;
       __syncthreads();
@@ -937,13 +937,35 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
 // The listed buckets: equal keys, clusters, more keys than shared memory holds.
 // ---------------------------------------------------------------------------
 constexpr int kRareBlock = 512;
-constexpr int kRareItems = (int)kFinishCap / kRareBlock;
 // Bin counters are padded by 4 words per 16, so that a thread's 16-byte reads
 // of its own run of bins in the scan touch every bank once per quarter warp.
 __device__ __forceinline__ uint32_t bin_at(uint32_t bin) { return bin + ((bin >> 4) << 2); }
 constexpr uint32_t kBinWords = kBucketBins + kBucketBins / 4;
 // bytes of the bins, or of the 4-bit passes' counters
 constexpr size_t kRareAux = std::max<size_t>((size_t)(kBinWords + 4) * 4, (size_t)os::kNibbleBins * (kRareBlock + 32) * 4);
+
+// The least and greatest of a[0, m) (in ordered form; raw: a holds floats as
+// stored), in every thread.  s_ends: two words a warp.
+template <typename K, int B>
+__device__ __forceinline__ void block_minmax(const K* a, uint32_t m, bool raw, K* s_ends, K& lo, K& hi) {
+  lo = ~(K)0;
+  hi = 0;
+  for (uint32_t i = threadIdx.x; i < m; i += B) {
+    const K x = to_ordered(a[i], raw);
+    lo = min(lo, x);
+    hi = max(hi, x);
+  }
+  warp_minmax(lo, hi);
+  if ((threadIdx.x & 31u) == 0) {
+    s_ends[threadIdx.x >> 5] = lo;
+    s_ends[B / 32 + (threadIdx.x >> 5)] = hi;
+  }
+  __syncthreads();
+  for (int w = 0; w < B / 32; ++w) {
+    lo = min(lo, s_ends[w]);
+    hi = max(hi, s_ends[B / 32 + w]);
+  }
+}
 
 // A bucket too large for shared memory, or with many keys in one bin: stable
 // 8-bit LSD passes by the one CTA, a[0, m) and b[0, m) in turn; the result is
@@ -958,23 +980,9 @@ __device__ void finish_slow(K* a, K* b, uint32_t m, bool into_a, unsigned char* 
   uint32_t* s_warp = s_wc + W * 256;                                  // [W]
   K* s_mm = reinterpret_cast<K*>(s_warp + W);                         // [2 * W]
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  K lo = ~(K)0, hi = 0;
-  for (uint32_t i = tid; i < m; i += B) {
-    const K x = a[i];
-    lo = min(lo, x);
-    hi = max(hi, x);
-  }
-  warp_minmax(lo, hi);
+  K lo, hi;
   __syncthreads();
-  if (lane == 0) {
-    s_mm[warp] = lo;
-    s_mm[W + warp] = hi;
-  }
-  __syncthreads();
-  for (int w = 0; w < W; ++w) {
-    lo = min(lo, s_mm[w]);
-    hi = max(hi, s_mm[W + w]);
-  }
+  block_minmax<K, B>(a, m, false, s_mm, lo, hi);
   const K diff = lo ^ hi;  // keys agree above its highest bit
   K *src = a, *dst = b;
   for (uint32_t sh = 0; sh < 8 * sizeof(K) && (diff >> sh) != 0; sh += 8) {
@@ -1075,14 +1083,13 @@ __device__ void finish_counted(const K* in, K* out, uint32_t cnt, K first, unsig
 // A bucket of at most CAP keys, crowded (many keys equal or nearly so): stable
 // 4-bit counting passes over the bits its keys differ in (diff: the least and
 // greatest key's), in shared memory.
-template <typename K, bool FLT>
+template <typename K, bool FLT, int B = kRareBlock, uint32_t CAP = kFinishCap, bool RAW = false>
 __device__ void finish_nibbles(const K* in, K* out, uint32_t cnt, K diff, unsigned char* smem, uint32_t* s_warp) {
-  constexpr int B = kRareBlock, ITEMS = kRareItems;
-  static_assert((size_t)os::kNibbleBins * (B + 32) * 4 <= kRareAux, "the nibble counters fit beside the keys");
+  constexpr int ITEMS = (int)CAP / B;
   K* s_keys = reinterpret_cast<K*>(smem);
-  uint32_t* s_cnt = reinterpret_cast<uint32_t*>(smem + (size_t)kFinishCap * sizeof(K));
+  uint32_t* s_cnt = reinterpret_cast<uint32_t*>(smem + (size_t)CAP * sizeof(K));
   const uint32_t tid = threadIdx.x;
-  for (uint32_t i = tid; i < kFinishCap; i += B) s_keys[i] = i < cnt ? in[i] : ~(K)0;  // (padding sorts behind every key)
+  for (uint32_t i = tid; i < CAP; i += B) s_keys[i] = i < cnt ? to_ordered(in[i], RAW) : ~(K)0;  // (padding sorts behind every key)
   __syncthreads();
   K k[ITEMS];
   uint32_t unused[1];
@@ -1105,25 +1112,9 @@ __device__ __forceinline__ void rare_buckets(const uint32_t* rare, JobOf&& job_o
     FinishJob<K> job{};
     job_of(rare[1 + i], job);
     if (job.cnt <= kFinishCap) {
-      K lo = ~(K)0, hi = 0;
-      for (uint32_t j = tid; j < job.cnt; j += kRareBlock) {
-        const K x = job.src[j];
-        lo = min(lo, x);
-        hi = max(hi, x);
-      }
-      warp_minmax(lo, hi);
-      if ((tid & 31u) == 0) {
-        s_edge[tid >> 5] = lo;
-        s_edge[W + (tid >> 5)] = hi;
-      }
-      __syncthreads();
-      for (int w = 0; w < W; ++w) {
-        lo = min(lo, s_edge[w]);
-        hi = max(hi, s_edge[W + w]);
-      }
-      uint32_t cells, bins;
-      spread_of<K>((K)(hi - lo), cells, bins);
-      if (bins == 0)
+      K lo, hi;
+      block_minmax<K, kRareBlock>(job.src, job.cnt, false, s_edge, lo, hi);
+      if (hi - lo < (K)kBucketBins)
         finish_counted<K, FLT>(job.src, job.dst, job.cnt, lo, smem, s_warp);
       else
         finish_nibbles<K, FLT>(job.src, job.dst, job.cnt, lo ^ hi, smem, s_warp);
@@ -1190,9 +1181,61 @@ __global__ void __launch_bounds__(kRareBlock) bucket_rare_kernel(K* in, K* out, 
 }
 
 template <typename K>
-constexpr size_t finish_smem() {
-  constexpr size_t V = 16 / sizeof(K);
-  return (2 * (size_t)kFinishCap + 3 * V + kHits) * sizeof(K) + kFinishAux;
+constexpr size_t finish_smem(int block = kFinishBlock, size_t cap = kFinishCap, int cell_bits = kCellBits) {
+  return (2 * cap + (size_t)block + 3 * (16 / sizeof(K))) * sizeof(K) + ((size_t)8 << (cell_bits - 5));
+}
+
+// ---------------------------------------------------------------------------
+// A few keys: the whole sort by one CTA.
+// ---------------------------------------------------------------------------
+// The array is one bucket of unknown range.  Latency only: about ten barriers
+// and a dozen shared accesses per key, where eight (64-bit keys: sixteen) 4-bit
+// passes take three barriers and about eight accesses each; those still sort
+// keys that crowd, and payloads.  In a stream of them 4096 uniform 32-bit keys
+// take 8 us against 27, 8192 8 us against 23; between events 4096 keys 13 us
+// against 29 (Zipf, which crowds: 22 against 29), 64-bit 14 against 33.
+template <typename K, bool FLT, int BLOCK, uint32_t CAP, int CELL_BITS>
+__global__ void __launch_bounds__(BLOCK, 1) small_cells_kernel(K* keys, uint32_t n, uint32_t* err) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ uint32_t s_rare[2];
+  __shared__ uint32_t s_warp[BLOCK / 32];
+  __shared__ K s_ends[2 * BLOCK / 32];
+  if (threadIdx.x == 0) s_rare[0] = 0;
+  finish_buckets<K, FLT, BLOCK, CAP, CELL_BITS, FLT>(1, s_rare, err, [&](uint32_t, FinishJob<K>& job) {
+    job.src = job.dst = job.other = keys;
+    job.lo = keys;
+    job.hi = keys + n;
+    job.first = 0;
+    job.cnt = n;
+    job.edge = 1;
+    job.cell_shift = 0;
+  });
+  __syncthreads();
+  if (s_rare[0]) {
+    K lo, hi;
+    block_minmax<K, BLOCK>(keys, n, FLT, s_ends, lo, hi);
+    finish_nibbles<K, FLT, BLOCK, CAP, FLT>(keys, keys, n, lo ^ hi, smem, s_warp);
+  }
+}
+
+template <typename K, bool FLT, int BLOCK, uint32_t CAP, int CELL_BITS>
+cudaError_t small_cells_t(K* keys, size_t n, uint32_t* err, cudaStream_t stream) {
+  constexpr size_t nibbles = (size_t)CAP * sizeof(K) + (size_t)os::kNibbleBins * (BLOCK + 32) * 4;
+  const size_t smem = std::max(finish_smem<K>(BLOCK, CAP, CELL_BITS), nibbles);
+  auto kern = small_cells_kernel<K, FLT, BLOCK, CAP, CELL_BITS>;
+  cudaError_t e = ensure_dynamic_smem(kern, smem);
+  if (e != cudaSuccess) return e;
+  kern<<<1, BLOCK, smem, stream>>>(keys, (uint32_t)n, err);
+  return cudaGetLastError();
+}
+
+// Fewer than 2048 keys leave most of 512 threads' items empty; 8192 need twice
+// the cells for the same share of collisions.
+template <typename K, bool FLT>
+cudaError_t small_cells_k(K* keys, size_t n, uint32_t* err, cudaStream_t stream) {
+  if (n <= 4096) return small_cells_t<K, FLT, 512, 4096, 16>(keys, n, err, stream);
+  if constexpr (sizeof(K) == 4) return small_cells_t<K, FLT, 512, 8192, 17>(keys, n, err, stream);
+  return cudaErrorInvalidValue;
 }
 
 template <typename K>
@@ -1654,6 +1697,14 @@ __global__ void clear_kernel(uint4* p, size_t words, uint32_t* tail, uint32_t ta
 }
 
 }  // namespace
+
+cudaError_t launch_small_keys(void* keys, size_t n, int key_bytes, bool is_float, uint32_t* err, cudaStream_t stream) {
+  if (n == 0) return cudaSuccess;
+  if (n > small_sort_max_keys(key_bytes, false)) return cudaErrorInvalidValue;
+  if (key_bytes == 8) return small_cells_k<unsigned long long, false>(static_cast<unsigned long long*>(keys), n, err, stream);
+  return is_float ? small_cells_k<uint32_t, true>(static_cast<uint32_t*>(keys), n, err, stream)
+                  : small_cells_k<uint32_t, false>(static_cast<uint32_t*>(keys), n, err, stream);
+}
 
 cudaError_t launch_clear(void* p, size_t bytes, const uint32_t* off, cudaStream_t stream) {
   if (bytes % 4 || (reinterpret_cast<uintptr_t>(p) & 15u)) return cudaErrorInvalidValue;

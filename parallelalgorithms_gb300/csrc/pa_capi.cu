@@ -931,11 +931,10 @@ cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32
   const bool has_vals = d_vals != nullptr;
   auto m = [&]() { return mark ? mark() : cudaSuccess; };
   if (n <= small_sort_max_keys(kb, has_vals)) {  // one CTA, one launch
-    (void)d_tmp;
-    (void)d_tvals;
-    (void)err;
     cudaError_t e = m();
-    if (e == cudaSuccess) e = launch_small_sort(d_keys, d_vals, n, kb, is_float, stream);
+    if (e == cudaSuccess)
+      e = has_vals ? launch_small_sort(d_keys, d_vals, n, kb, is_float, stream)
+                   : launch_small_keys(d_keys, n, kb, is_float, err, stream);
     if (e == cudaSuccess) e = m();
     return e;
   }

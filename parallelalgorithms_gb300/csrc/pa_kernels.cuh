@@ -240,6 +240,10 @@ cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, const 
 cudaError_t enqueue_bucket_sort(const BucketScratch& s, void* keys, void* tmp, size_t n, int key_bytes, bool is_float,
                                 SortCtrl* ctrl, uint32_t* err, cudaStream_t stream,
                                 const std::function<cudaError_t()>& mark = {});
+// Whole sort of n <= small_sort_max_keys(key_bytes, false) keys by one CTA, in
+// place (launch_small_sort's result; a bulk-copy wait that gives up raises a bit
+// in *err).
+cudaError_t launch_small_keys(void* keys, size_t n, int key_bytes, bool is_float, uint32_t* err, cudaStream_t stream);
 // Zeroes bytes [p, p + bytes) (p 16-byte aligned) unless *off is not zero.
 cudaError_t launch_clear(void* p, size_t bytes, const uint32_t* off, cudaStream_t stream);
 

@@ -63,6 +63,50 @@ def test_u64(pa, port, name, n):
     np.testing.assert_array_equal(got, want)
 
 
+SMALL = [1, 2, 3, 31, 511, 512, 513, 2047, 4095, 4096, 4097, 8191, 8192]
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("kind", ["uniform", "constant", "few", "sorted", "pairs", "outlier", "offset"])
+def test_few_keys(pa, port, torch_cuda, bits, kind):
+    """Whole sorts by one CTA: every size at which its steps change, in place on
+    a buffer that need not start at a 16-byte boundary."""
+    dt, signed = (np.uint32, np.int32) if bits == 32 else (np.uint64, np.int64)
+    rng = np.random.default_rng(bits)
+    for n in SMALL:
+        a = rng.integers(0, 1 << bits, n, dtype=dt)
+        if kind == "constant":
+            a[:] = a[0]
+        elif kind == "few":
+            a = a[rng.integers(0, min(n, 5), n)]
+        elif kind == "sorted":
+            a = np.arange(n, dtype=dt)
+        elif kind == "pairs":  # every value twice: one collision each
+            a[n // 2:2 * (n // 2)] = a[:n // 2]
+        elif kind == "outlier":
+            a %= dt(1000)
+            a[n // 2] = dt((1 << bits) - 1)
+        want, _ = port.sort(a)
+        skip = 1 if kind == "offset" else 0
+        buf = torch_cuda.zeros(n + 8, dtype=torch_cuda.int32 if bits == 32 else torch_cuda.int64, device="cuda")
+        keys = buf[skip:skip + n]
+        keys.copy_(torch_cuda.from_numpy(a.view(signed)))
+        pa.sort(keys)
+        np.testing.assert_array_equal(keys.cpu().numpy().view(dt), want, err_msg=f"n = {n}")
+        assert not buf[:skip].any() and not buf[skip + n:].any()
+
+
+@pytest.mark.parametrize("n", SMALL)
+def test_few_floats(pa, port, n):
+    a = np.random.default_rng(n).integers(0, 1 << 32, n, dtype=np.uint32)
+    a[:n // 3] = np.random.default_rng(n).standard_normal(n // 3).astype(np.float32).view(np.uint32)
+    flip = lambda b: b ^ np.where(b >> 31, 0xFFFFFFFF, 0x80000000).astype(np.uint32)  # noqa: E731
+    want, _ = port.sort(flip(a))
+    got = a.view(np.float32).copy()
+    pa.sort(got)
+    np.testing.assert_array_equal(flip(got.view(np.uint32)), want)
+
+
 @pytest.mark.parametrize("kind", ["range", "normal", "signs"])
 def test_f32(pa, port, kind):
     rng = np.random.default_rng(7)
