@@ -514,6 +514,8 @@ int sort_impl(void* keys, void* tmp, uint32_t* vals, uint32_t* tmp_vals, size_t 
   }
   const bool vals_dev = has_vals && is_device_ptr(vals);
   const bool tvals_dev = has_vals && is_device_ptr(tmp_vals);
+  const bool timed = phase_ms && phase_cap > 0;
+  const bool sync_call = timed || !(opts && opts->async_device) || !keys_dev || (has_vals && !vals_dev);
   void *d_keys = nullptr, *d_tmp = nullptr;
   uint32_t *d_vals = nullptr, *d_tvals = nullptr;
   SortScratch sc{};
@@ -537,7 +539,6 @@ int sort_impl(void* keys, void* tmp, uint32_t* vals, uint32_t* tmp_vals, size_t 
   if (!keys_dev) PA_CUDA(cudaMemcpyAsync(d_keys, keys, key_bytes_total, cudaMemcpyHostToDevice, stream));
   if (has_vals && !vals_dev)
     PA_CUDA(cudaMemcpyAsync(d_vals, vals, n * sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
-  const bool timed = phase_ms && phase_cap > 0;
   int nev = 0;
   auto mark = [&]() -> cudaError_t {
     if (!timed || nev >= kMaxEvents) return cudaSuccess;
@@ -547,14 +548,23 @@ int sort_impl(void* keys, void* tmp, uint32_t* vals, uint32_t* tmp_vals, size_t 
     }
     return cudaEventRecord(ws->ev[nev++], stream);
   };
-  const bool sync_call = timed || !(opts && opts->async_device) || !keys_dev || (has_vals && !vals_dev);
   PA_CUDA(enqueue_sort(sc, d_keys, d_tmp, d_vals, d_tvals, n, kb, is_float, ws->err, stream, mark,
                        sync_call ? &ws->host->decided : nullptr));
-  if (!keys_dev) PA_CUDA(cudaMemcpyAsync(keys, d_keys, key_bytes_total, cudaMemcpyDeviceToHost, stream));
-  if (has_vals && !vals_dev)
-    PA_CUDA(cudaMemcpyAsync(vals, d_vals, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-  const bool all_dev = keys_dev && (!has_vals || vals_dev);
-  int rc = finish(ws, stream, !timed && opts && opts->async_device && all_dev);
+  auto copy_out = [&]() -> int {
+    if (!keys_dev) PA_CUDA(cudaMemcpyAsync(keys, d_keys, key_bytes_total, cudaMemcpyDeviceToHost, stream));
+    if (has_vals && !vals_dev)
+      PA_CUDA(cudaMemcpyAsync(vals, d_vals, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+    return PA_OK;
+  };
+  if (int rc = copy_out()) return rc;
+  int rc = finish(ws, stream, !sync_call);
+  if (rc == PA_OK && sync_call && sc.window.state && ws->host->decided == kSortAgain) {
+    sc.buckets = BucketScratch{};
+    sc.window = WindowScratch{};
+    PA_CUDA(enqueue_sort(sc, d_keys, d_tmp, d_vals, d_tvals, n, kb, is_float, ws->err, stream, {}, &ws->host->decided));
+    if (int rc2 = copy_out()) return rc2;
+    rc = finish(ws, stream, false);
+  }
   if (rc == PA_OK && timed) {
     for (int i = 0; i + 1 < nev && i < phase_cap; ++i) {
       float ms = 0.f;
@@ -879,6 +889,7 @@ size_t sort_scratch_layout(char* base, size_t n, int kb, bool has_vals, SortScra
   s->zero_begin = reinterpret_cast<char*>(s->counts);
   s->tile_ctr = c.take<uint32_t>((size_t)passes + 1);
   s->tc_ticket = s->tile_ctr + passes;
+  WindowState* wstate = c.take<WindowState>(1);
   s->status = c.take<char>((size_t)passes * tiles * bins * sb);
   s->zero_bytes = (size_t)(base + c.off - s->zero_begin);
   s->bin_start = c.take<unsigned long long>((size_t)passes * bins);
@@ -894,6 +905,8 @@ size_t sort_scratch_layout(char* base, size_t n, int kb, bool has_vals, SortScra
     char* b = c.take<char>(bytes);
     bucket_scratch_layout(b, n, &s->buckets);
   }
+  s->window = WindowScratch{};
+  if (radix_bits == 8 && window_sort_supported(n, kb)) s->window = window_scratch(n, s->status, 2 * tiles * bins * sb, wstate);
   return c.off;
 }
 
@@ -963,6 +976,8 @@ cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32
     if (e == cudaSuccess) e = m();
   }
   auto lsd_mark = [&]() { return off ? cudaSuccess : m(); };
+  const bool window = s.window.state && decided && kb == 8 && rb == 8;
+  if (decided) *reinterpret_cast<volatile uint32_t*>(decided) = 0;  // (kSortAgain comes after the passes)
   // With the tables (and 16-byte aligned keys) the histogram also prepares
   // the first pass's tile offsets.
   const bool prepared = s.tile_prefix && kb == 4 && rb == 8 && !has_vals && n < ((size_t)1 << 30) &&
@@ -976,6 +991,7 @@ cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32
   if (e == cudaSuccess) e = lsd_mark();
   if (e == cudaSuccess)
     e = launch_scan_digits(s.counts, passes, rb, n, is_float, true, s.bin_start, s.ctrl, stream, off);
+  if (e == cudaSuccess && window) e = enqueue_window_test(s.window, d_keys, d_tmp, n, s.ctrl, stream);
   if (e == cudaSuccess) e = lsd_mark();
   for (int p = 0; p < passes && e == cudaSuccess; ++p) {
     OnesweepArgs a{};
@@ -1003,6 +1019,11 @@ cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32
   }
   for (int p = 3; off && p < passes && e == cudaSuccess; ++p) e = m();  // (the passes' shares after the buckets' three)
   if (e == cudaSuccess) e = launch_final_copy(d_keys, d_tmp, d_vals, d_tvals, n, kb, s.ctrl, stream);
+  if (e == cudaSuccess && window) {
+    WindowScratch w = s.window;
+    w.fail = decided;
+    e = enqueue_window_mend(w, d_keys, d_tmp, d_vals, d_tvals, n, stream);
+  }
   if (e == cudaSuccess) e = m();
   return e;
 }

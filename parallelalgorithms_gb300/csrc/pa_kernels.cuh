@@ -244,6 +244,38 @@ cudaError_t enqueue_bucket_sort(const BucketScratch& s, void* keys, void* tmp, s
 // place (launch_small_sort's result; a bulk-copy wait that gives up raises a bit
 // in *err).
 cudaError_t launch_small_keys(void* keys, size_t n, int key_bytes, bool is_float, uint32_t* err, cudaStream_t stream);
+// ---- 64-bit LSD sorts by their leading digits (pa_window.cu) ---------------
+// Least keys (pairs, all passes -> by the leading digits, us): 524288 156 -> 151,
+// 1M 173 -> 159, 2M 240 -> 201, 20M 1296 -> 787; below, the test and the mending
+// cost what four passes do (262144: 134 -> 149).
+constexpr size_t kWindowLeastKeys = (size_t)1 << 19;
+struct WindowState {
+  uint32_t shift;   // bits below the window; 0: all passes run
+  uint32_t runs;    // long runs
+  uint32_t fail;    // all passes run after all
+  uint32_t ticket;
+  uint32_t hits;    // pairs of the sample that agree in the window alone
+};
+struct WindowScratch {
+  WindowState* state = nullptr;  // zeroed before, as the marks and the set; nullptr: not used
+  uint32_t* claim = nullptr;     // a bit per key: first keys of runs that are being mended
+  uint32_t slots_log2 = 0;
+  uint32_t* set = nullptr;       // long runs, by their first key
+  uint32_t* run = nullptr;       // their first and end
+  uint32_t* fail = nullptr;      // page-locked word set to kSortAgain when the passes must all run after all
+};
+bool window_sort_supported(size_t n, int key_bytes);
+// `skipped`: zeroed words of the lowest two passes, which are left out whenever
+// the window is used.
+WindowScratch window_scratch(size_t n, char* skipped, size_t skipped_bytes, WindowState* state);
+// Behind the scan: leaves out the passes below the window when a sample says
+// that its digits tell the keys apart.  Writes to tmp.
+cudaError_t enqueue_window_test(const WindowScratch& s, const void* keys, void* tmp, size_t n, SortCtrl* ctrl,
+                                cudaStream_t stream);
+// Behind the passes: puts in order what the passes left out would have.
+cudaError_t enqueue_window_mend(const WindowScratch& s, void* keys, void* tmp, uint32_t* vals, uint32_t* tvals, size_t n,
+                                cudaStream_t stream);
+
 // Zeroes bytes [p, p + bytes) (p 16-byte aligned) unless *off is not zero.
 cudaError_t launch_clear(void* p, size_t bytes, const uint32_t* off, cudaStream_t stream);
 
@@ -269,17 +301,21 @@ struct SortScratch {
   uint32_t* chunk_excl;
   uint32_t* tc_ticket;  // zeroed with the counts
   BucketScratch buckets;  // keys-only sorts with 8-bit digits of the sizes bucket_sort_supported takes
+  WindowScratch window;   // 64-bit sorts with 8-bit digits of the sizes window_sort_supported takes
 };
 size_t sort_scratch_bytes(size_t n, int key_bytes, bool has_vals, int radix_bits = 8);
 // Carves the scratch from `base` (nullptr measures); returns its size.
 size_t sort_scratch_layout(char* base, size_t n, int key_bytes, bool has_vals, SortScratch* s, int radix_bits = 8);
+constexpr uint32_t kSortAgain = 2;  // (not a value of the bucket plan)
 // Enqueues the whole sort of device buffers on `stream` (the LSD chain: memset,
 // histogram, scan, passes, final copy; or by buckets, scratch and sizes
 // permitting); `mark`, when set, runs between launches.  decided (optional):
 // one word of page-locked host memory nothing else uses meanwhile; with it the
 // call waits for the bucket plan's decision and enqueues only what it takes,
 // without it (asynchronous callers) everything is enqueued and decides on the
-// device, which only large sorts do.
+// device, which only large sorts do.  A 64-bit sort by its leading digits may
+// leave kSortAgain in *decided once the stream is done: the caller then enqueues
+// the sort again with s.buckets and s.window cleared.
 cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32_t* d_vals, uint32_t* d_tvals,
                          size_t n, int key_bytes, bool is_float, uint32_t* err, cudaStream_t stream,
                          const std::function<cudaError_t()>& mark = {}, uint32_t* decided = nullptr);
