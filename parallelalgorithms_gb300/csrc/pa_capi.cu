@@ -804,8 +804,15 @@ int select_impl(const void* a, size_t n, size_t k, int kb, void* out, const pa_o
   Carve r{ws->dev};
   layout(r);
   if (!in_dev) PA_CUDA(cudaMemcpyAsync(const_cast<void*>(d_in), a, n * kb, cudaMemcpyHostToDevice, stream));
-  PA_CUDA(launch_select(d_in, n, k, kb, cand, cand_cap, work, d_out, ws->err, stream));
-  const int rc = finish(ws, stream, opts && opts->async_device && in_dev && out_dev);
+  const bool async = opts && opts->async_device && in_dev && out_dev;
+  if (!async) *reinterpret_cast<volatile uint32_t*>(&ws->host->decided) = 0;
+  PA_CUDA(launch_select(d_in, n, k, kb, cand, cand_cap, work, d_out, stream, async ? SelectPart::kAll : SelectPart::kFast,
+                        async ? nullptr : &ws->host->decided));
+  int rc = finish(ws, stream, async);
+  if (!async && rc == PA_OK && ws->host->decided != 1) {
+    PA_CUDA(launch_select(d_in, n, k, kb, cand, cand_cap, work, d_out, stream, SelectPart::kRest));
+    rc = finish(ws, stream, false);
+  }
   if (!out_dev && rc == PA_OK) std::memcpy(out, &ws->host->result, kb);
   return rc;
 }
@@ -1269,7 +1276,7 @@ int pa_partition_radix_u32(uint32_t* a, size_t n, const size_t* k, size_t k_len,
   layout(r);
   if (!dev) PA_CUDA(cudaMemcpyAsync(d_a, a, n * 4, cudaMemcpyHostToDevice, stream));
   for (size_t i = 0; i < k_len; ++i)
-    PA_CUDA(launch_select(d_a, n, k[i], 4, cand, cand_cap, work, piv + i, ws->err, stream));
+    PA_CUDA(launch_select(d_a, n, k[i], 4, cand, cand_cap, work, piv + i, stream));
   PA_CUDA(launch_partition(d_a, tmp, n, piv, (int)k_len, counts, stream));
   PA_CUDA(cudaMemcpyAsync(a, tmp, n * 4, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, stream));
   return finish(ws, stream, dev && opts && opts->async_device);
@@ -1386,7 +1393,7 @@ int pa_select_radix_u32(uint32_t* a, size_t start, size_t length, size_t k, uint
   Carve r{ws->dev};
   layout(r);
   if (!in_dev) PA_CUDA(cudaMemcpyAsync(d_in, base, n * 4, cudaMemcpyHostToDevice, stream));
-  PA_CUDA(launch_select(d_in, n, kk, 4, cand, cand_cap, work, d_val, ws->err, stream));
+  PA_CUDA(launch_select(d_in, n, kk, 4, cand, cand_cap, work, d_val, stream));
   // The reference rearranges the range and leaves the answer at a[k]; here
   // the answer is swapped with a[k] from the first place that holds it, so
   // the range stays a permutation of its input.

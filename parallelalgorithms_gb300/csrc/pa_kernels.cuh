@@ -378,11 +378,15 @@ cudaError_t launch_inplace_partition(uint32_t* keys, size_t n, uint32_t shift, c
 // ---- select (pa_select.cu) -------------------------------------------------
 struct SelectState;
 size_t select_state_bytes();
-// k-th smallest (0-based) of keys[0, n) into *out (device).  cand holds
-// cand_cap keys; work is select_state_bytes() of scratch (initialised by the
-// launcher).
+// k-th smallest (0-based) of keys[0, n) into *out (device or page-locked).  cand
+// holds cand_cap keys; work is select_state_bytes() of scratch (initialised by
+// the launcher).  A caller that waits enqueues kFast with `decided`, one word of
+// page-locked host memory it has set to 0, and kRest behind it only if the word
+// is not 1 once the stream is done.
+enum class SelectPart { kAll, kFast, kRest };
 cudaError_t launch_select(const void* keys, size_t n, size_t k, int key_bytes, void* cand, size_t cand_cap,
-                          void* work, void* out, uint32_t* err, cudaStream_t stream);
+                          void* work, void* out, cudaStream_t stream, SelectPart part = SelectPart::kAll,
+                          uint32_t* decided = nullptr);
 // *idx = k when keys[k] == *value, else the smallest index of a key equal to
 // *value in keys[0, n) (all ones if none).
 cudaError_t launch_find_key(const uint32_t* keys, size_t n, size_t k, const uint32_t* value, unsigned long long* idx,

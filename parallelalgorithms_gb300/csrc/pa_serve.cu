@@ -329,7 +329,7 @@ class GpuBackend {
         off += align256(cap * kb);
         void* work = base + off;
         off += align256(select_state_bytes());
-        if (run && e == cudaSuccess) e = launch_select(keys, r->n, q->k, (int)kb, cand, cap, work, results + i * slot, err, s);
+        if (run && e == cudaSuccess) e = launch_select(keys, r->n, q->k, (int)kb, cand, cap, work, results + i * slot, s);
       } else {
         hj.push_back({keys, (unsigned long long)r->n, reinterpret_cast<unsigned long long*>(results + i * slot),
                       q->shift, chunks});
