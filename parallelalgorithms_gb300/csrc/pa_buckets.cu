@@ -51,6 +51,7 @@ constexpr uint32_t kSample = (uint32_t)kPlanCtas * kPlanBlock * kPlanPer;
 constexpr uint32_t kGroups = 256;         // bins of a partition pass, at most
 constexpr uint32_t kBucketsMax = 32768;   // counters of the count kernel: 128 KB of shared memory
 constexpr uint32_t kBucketTarget = 3072;  // keys per bucket, at most, while more buckets can be had
+static_assert(kBucketMostKeys == (size_t)kBucketsMax * kBucketTarget, "the declared limit");
 constexpr int kCellBits = 16, kBinBits = 12;
 constexpr uint32_t kCells = 1u << kCellBits;      // cells of the finish kernel's bitmap
 constexpr uint32_t kBucketBins = 1u << kBinBits;  // values a crowded bucket may span to be counted instead
@@ -1727,7 +1728,7 @@ cudaError_t launch_clear(void* p, size_t bytes, const uint32_t* off, cudaStream_
 bool bucket_sort_supported(size_t n, int key_bytes) {
   if (key_bytes != 4 && key_bytes != 8) return false;
   const size_t least = key_bytes == 4 ? (size_t)1 << 19 : small_sort_max_keys(key_bytes, false) + 1;
-  return n >= least && n <= (size_t)kBucketsMax * kBucketTarget;
+  return n >= least && n <= kBucketMostKeys;
 }
 
 size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s) {

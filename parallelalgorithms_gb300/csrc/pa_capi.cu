@@ -876,8 +876,12 @@ int sum_impl(const void* a, size_t n, int elem_kind, uint64_t* out, const pa_opt
 }  // namespace
 
 size_t sort_scratch_bytes(size_t n, int kb, bool has_vals, int radix_bits) {
+  // enough for any part of the keys too: above the bucket sort's sizes, for the
+  // largest part that it takes
   SortScratch s{};
-  return sort_scratch_layout(nullptr, n, kb, has_vals, &s, radix_bits);
+  const size_t all = sort_scratch_layout(nullptr, n, kb, has_vals, &s, radix_bits);
+  return n <= kBucketMostKeys ? all
+                              : std::max(all, sort_scratch_layout(nullptr, kBucketMostKeys, kb, has_vals, &s, radix_bits));
 }
 
 size_t sort_scratch_layout(char* base, size_t n, int kb, bool has_vals, SortScratch* s, int radix_bits) {

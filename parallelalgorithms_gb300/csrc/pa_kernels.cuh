@@ -224,6 +224,7 @@ struct BucketScratch {
 };
 // Sizes this sort takes: more keys than the one-CTA sort, and few enough that
 // the most buckets there can be fit the finish kernel with room to spare.
+constexpr size_t kBucketMostKeys = (size_t)32768 * 3072;
 bool bucket_sort_supported(size_t n, int key_bytes);
 // Carves the scratch from `base` (nullptr measures); returns its size.
 size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s);
@@ -303,6 +304,7 @@ struct SortScratch {
   BucketScratch buckets;  // keys-only sorts with 8-bit digits of the sizes bucket_sort_supported takes
   WindowScratch window;   // 64-bit sorts with 8-bit digits of the sizes window_sort_supported takes
 };
+// Scratch for n keys, or any part of them.
 size_t sort_scratch_bytes(size_t n, int key_bytes, bool has_vals, int radix_bits = 8);
 // Carves the scratch from `base` (nullptr measures); returns its size.
 size_t sort_scratch_layout(char* base, size_t n, int key_bytes, bool has_vals, SortScratch* s, int radix_bits = 8);
