@@ -587,12 +587,18 @@ int sort_impl(void* keys, void* tmp, uint32_t* vals, uint32_t* tmp_vals, size_t 
 // segmented sort, with the scratch as its second buffer; larger buckets are
 // partitioned again on the next digit.  A range whose keys all share the
 // digit is not moved.
+//
+// A call that waits (`decided`: its page-locked word) sorts up to S keys, and
+// groups whose digits are evenly filled, by buckets where the plan finds them
+// fit (pa_buckets.cu).  Calls on uniform keys, by digit passes
+// alone and a longer host path -> now (us): 100M 3261 -> 2673, 30M 1043 -> 891;
+// 10M (within the scratch) 257 -> 155.
 constexpr size_t kInplaceDefaultScratch = (size_t)1 << 24;  // keys
 constexpr size_t kInplaceMinScratch = (size_t)1 << 16;
 
 int inplace_levels(Workspace* ws, cudaStream_t stream, uint32_t* a, size_t n, size_t S, uint32_t* buf,
                    InplaceState* st, void* status, unsigned long long* hist, char* plan_dev, size_t plan_cap,
-                   char* sort_base) {
+                   char* sort_base, uint32_t* decided) {
   struct Range {
     size_t lo, len;
     uint32_t shift;
@@ -621,6 +627,8 @@ int inplace_levels(Workspace* ws, cudaStream_t stream, uint32_t* a, size_t n, si
     struct Group {
       size_t lo;
       std::vector<uint64_t> off;
+      int first, last;  // digits
+      size_t most;      // keys of the fullest
     };
     std::vector<Group> groups;
     size_t at = rg.lo;
@@ -633,9 +641,11 @@ int inplace_levels(Workspace* ws, cudaStream_t stream, uint32_t* a, size_t n, si
         open = false;
       } else {
         if (!open || groups.back().off.back() + c > S) {
-          groups.push_back({at, {0}});
+          groups.push_back({at, {0}, b, b, 0});
           open = true;
         }
+        groups.back().last = b;
+        groups.back().most = std::max(groups.back().most, c);
         groups.back().off.push_back(groups.back().off.back() + c);
       }
       at += c;
@@ -643,9 +653,16 @@ int inplace_levels(Workspace* ws, cudaStream_t stream, uint32_t* a, size_t n, si
     std::vector<seg::HostPlan> plans(groups.size());
     std::vector<bool> planned(groups.size(), false);
     std::vector<size_t> image_off(groups.size() + 1, 0);
+    // Evenly filled: the fullest digit has at most 5/4 of the group's mean (the
+    // bucket plan turns away what crowds inside a digit, and the group is then
+    // sorted as one array).
+    auto by_buckets = [&](const Group& gr) {
+      const size_t len = (size_t)gr.off.back();
+      return decided && bucket_sort_supported(len, 4) && gr.most * (size_t)(gr.last - gr.first + 1) * 4 <= len * 5;
+    };
     for (size_t g = 0; g < groups.size(); ++g) {
       size_t bytes = 0;
-      if (groups[g].off.back() > 1) {
+      if (groups[g].off.back() > 1 && !by_buckets(groups[g])) {
         pa_segsort_config cfg{};
         cfg.small_cutoff = 4096;
         cfg.tile_keys = 8192;
@@ -674,7 +691,7 @@ int inplace_levels(Workspace* ws, cudaStream_t stream, uint32_t* a, size_t n, si
       } else {  // the group as one array: its buckets are already in order
         SortScratch sc{};
         sort_scratch_layout(sort_base, glen, 4, false, &sc);
-        PA_CUDA(enqueue_sort(sc, ga, buf, nullptr, nullptr, glen, 4, false, ws->err, stream));
+        PA_CUDA(enqueue_sort(sc, ga, buf, nullptr, nullptr, glen, 4, false, ws->err, stream, {}, decided));
       }
     }
   }
@@ -718,12 +735,13 @@ int inplace_impl(uint32_t* keys, size_t n, size_t scratch_keys, const pa_opts* o
   Carve real{ws->dev};
   layout(real);
   if (!keys_dev) PA_CUDA(cudaMemcpyAsync(d_keys, keys, n * sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
+  uint32_t* decided = opts && opts->async_device && keys_dev ? nullptr : &ws->host->decided;
   if (n <= S) {
     SortScratch sc{};
     sort_scratch_layout(sort_base, n, 4, false, &sc);
-    PA_CUDA(enqueue_sort(sc, d_keys, buf, nullptr, nullptr, n, 4, false, ws->err, stream));
+    PA_CUDA(enqueue_sort(sc, d_keys, buf, nullptr, nullptr, n, 4, false, ws->err, stream, {}, decided));
   } else if (int rc = inplace_levels(ws, stream, d_keys, n, S, buf, st, status, hist, plan_dev, plan_cap,
-                                     sort_base)) {
+                                     sort_base, decided)) {
     cudaStreamSynchronize(stream);
     cudaGetLastError();
     return rc;
