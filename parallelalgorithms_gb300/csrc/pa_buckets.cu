@@ -415,8 +415,10 @@ __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* _
 // counts is the number of shared accesses per key, not registers or occupancy
 // (two CTAs per SM measured as three).  A tile's next loads are issued before
 // it is written out, and a bin's reservation (a round trip to L2) passes while
-// the tile is staged.  100M uniform 32-bit keys: 0.208 ms for the first pass,
-// 0.240 ms for the grouped one, against 0.326 and 0.385 ms for a stable digit
+// the tile is staged.  100M uniform 32-bit keys: 0.214 ms for the first pass,
+// 0.235 ms for the grouped one (sorted keys 0.179 and 0.305; 0.241 and 0.365 while
+// tiles of one bin were shuffled like the others and a warp's vectors added one
+// after the other), against 0.326 and 0.385 ms for a stable digit
 // pass with and without prepared offsets.
 constexpr int kScatterBlock = 512;
 constexpr int kScatterPerSm = 3;
@@ -429,7 +431,7 @@ constexpr uint32_t kScatterTile = (uint32_t)kScatterBlock * kScatterItems<K>;
 template <typename K, bool GROUPED, bool FLT, bool PLAIN>
 __device__ __forceinline__ void scatter_tiles(const K* in, K* out, uint32_t n, const BucketArgs& a, const BucketMap& m,
                                               K* s_keys, uint32_t* s_cnt, uint32_t* s_start, uint32_t* s_base,
-                                              uint32_t* s_warp, const uint32_t* s_first) {
+                                              uint32_t* s_warp, uint32_t* s_one, const uint32_t* s_first) {
   constexpr int ITEMS = kScatterItems<K>;
   constexpr uint32_t T = kScatterTile<K>;
   constexpr int V = 16 / (int)sizeof(K);
@@ -496,6 +498,7 @@ __device__ __forceinline__ void scatter_tiles(const K* in, K* out, uint32_t n, c
   if (blockIdx.x < tiles) load(blockIdx.x);
   for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     if (tid < kGroups) s_cnt[tid] = 0;
+    if (tid == 0) *s_one = 0;
     if constexpr (FLT) {
 #pragma unroll
       for (int j = 0; j < ITEMS; ++j) k[j] = to_ordered(k[j], true);
@@ -509,18 +512,24 @@ __device__ __forceinline__ void scatter_tiles(const K* in, K* out, uint32_t n, c
       if (__all_sync(kFull, d0 == __shfl_sync(kFull, d0, 0))) {
         // Sorted or constant runs: the atomics of a warp that agrees would queue
         // on one word, so where all of a vector's keys agree the warp adds once.
+        uint32_t ones = 0, dl = 0;  // bit q: vector q agrees; lane q: its digit
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
           const uint32_t dq = digit(k[q * V]);
           bool one = dq == __shfl_sync(kFull, dq, 0);
 #pragma unroll
           for (int i = 1; i < V; ++i) one = one && digit(k[q * V + i]) == dq;
-          if (__all_sync(kFull, one)) {
-            uint32_t x = 0;
-            if (lane == 0) x = atomicAdd(s_cnt + dq, 32u * V);
-            x = __shfl_sync(kFull, x, 0) + lane;
+          ones |= __all_sync(kFull, one) ? 1u << q : 0u;
+          if (lane == (uint32_t)q) dl = dq;
+        }
+        uint32_t x = 0;
+        if ((ones >> lane) & 1u) x = atomicAdd(s_cnt + dl, 32u * V);
 #pragma unroll
-            for (int i = 0; i < V; ++i) r[(q * V + i) / 2] |= (x + 32u * i) << (16 * ((q * V + i) % 2));
+        for (int q = 0; q < Q; ++q) {
+          const uint32_t y = __shfl_sync(kFull, x, q) + lane;
+          if ((ones >> q) & 1u) {
+#pragma unroll
+            for (int i = 0; i < V; ++i) r[(q * V + i) / 2] |= (y + 32u * i) << (16 * ((q * V + i) % 2));
           } else {
 #pragma unroll
             for (int j = q * V; j < q * V + V; ++j) r[j / 2] |= atomicAdd(s_cnt + digit(k[j]), 1u) << (16 * (j % 2));
@@ -540,13 +549,27 @@ __device__ __forceinline__ void scatter_tiles(const K* in, K* out, uint32_t n, c
     if (tid < bins) {
       c = s_cnt[tid];
       if (c) at = atomicAdd(cursor0 + (size_t)g * bins + tid, c);
+      if (c == T) *s_one = 1;
     }
     const uint32_t excl = os::block_exclusive_scan<kScatterBlock>(c, s_warp);
     if (tid < bins) s_start[tid] = excl;
     __syncthreads();
+    if (*s_one) {
+      // One bin takes the whole tile (sorted keys): in their order, so that the
+      // second pass finds sorted runs again and not this pass's shuffled ones.
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j)
-      if (full || ((valid >> j) & 1u)) s_keys[s_start[digit(k[j])] + ((r[j / 2] >> (16 * (j % 2))) & 0xFFFFu)] = k[j];
+      for (int q = 0; q < Q; ++q) {
+        uint4 v;
+        K* e = reinterpret_cast<K*>(&v);
+#pragma unroll
+        for (int x = 0; x < V; ++x) e[x] = k[q * V + x];
+        reinterpret_cast<uint4*>(s_keys)[q * kScatterBlock + tid] = v;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < ITEMS; ++j)
+        if (full || ((valid >> j) & 1u)) s_keys[s_start[digit(k[j])] + ((r[j / 2] >> (16 * (j % 2))) & 0xFFFFu)] = k[j];
+    }
     const bool was_full = full;
     const uint32_t cnt = was_full ? T : (uint32_t)(min(tlo + (long long)T, (long long)g1) - max(tlo, (long long)g0));
     if (tid < bins) s_base[tid] = at - excl;  // (the reservation's round trip passes during the staging)
@@ -579,6 +602,7 @@ __global__ void __launch_bounds__(kScatterBlock, kScatterPerSm) bucket_scatter_k
   __shared__ __align__(16) K s_keys[kScatterTile<K>];
   __shared__ uint32_t s_cnt[kGroups], s_start[kGroups], s_base[kGroups];
   __shared__ uint32_t s_warp[kScatterBlock / 32];
+  __shared__ uint32_t s_one;
   __shared__ uint32_t s_first[kGroups + 1];
   const BucketMap m = *a.map;
   if (!m.on) return;
@@ -587,9 +611,9 @@ __global__ void __launch_bounds__(kScatterBlock, kScatterPerSm) bucket_scatter_k
     __syncthreads();
   }
   if (m.plain)
-    scatter_tiles<K, GROUPED, FLT, true>(in, out, (uint32_t)n, a, m, s_keys, s_cnt, s_start, s_base, s_warp, s_first);
+    scatter_tiles<K, GROUPED, FLT, true>(in, out, (uint32_t)n, a, m, s_keys, s_cnt, s_start, s_base, s_warp, &s_one, s_first);
   else
-    scatter_tiles<K, GROUPED, FLT, false>(in, out, (uint32_t)n, a, m, s_keys, s_cnt, s_start, s_base, s_warp, s_first);
+    scatter_tiles<K, GROUPED, FLT, false>(in, out, (uint32_t)n, a, m, s_keys, s_cnt, s_start, s_base, s_warp, &s_one, s_first);
 }
 
 // ---------------------------------------------------------------------------
@@ -606,7 +630,7 @@ __global__ void __launch_bounds__(kScatterBlock, kScatterPerSm) bucket_scatter_k
 // buckets larger than shared memory, are listed for a launch of their own.
 //
 // Bound by instruction issue and the shared-memory pipe together (about 60 %
-// of each): 100M uniform 32-bit keys in 0.328 ms.  On the way there (same
+// of each): 100M uniform 32-bit keys in 0.353 ms.  On the way there (same
 // input): bins of one key on average and each key compared with its bin 0.80
 // ms; the bitmap with 512 threads and a branch per key 0.59; 256 threads and
 // more keys in flight 0.45; collisions listed instead of handled where they are
