@@ -54,6 +54,7 @@ constexpr uint32_t kBucketTarget = 3072;  // keys per bucket, at most, while mor
 static_assert(kBucketMostKeys == (size_t)kBucketsMax * kBucketTarget, "the declared limit");
 constexpr int kCellBits = 16, kBinBits = 12;
 constexpr uint32_t kCells = 1u << kCellBits;      // cells of the finish kernel's bitmap
+constexpr uint32_t kCountSpan = 1u << (kCellBits - 3);  // values a counted bucket may span
 constexpr uint32_t kBucketBins = 1u << kBinBits;  // values a crowded bucket may span to be counted instead
 
 struct BucketArgs {
@@ -70,6 +71,7 @@ struct BucketArgs {
   uint32_t low_bits;
   uint32_t tile;        // keys per partition tile
   uint32_t tmp_align;   // scratch address modulo 16
+  size_t keys;          // of the sort
   uint32_t hot_above;   // sample keys above which a bucket looks too full
   uint32_t max_sample;  // sample keys no bucket may exceed
   uint32_t* err;
@@ -157,6 +159,7 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
     }
   }
   cluster.sync();
+  K raw = 0;  // (thread 0) the sample's range
   if (tid == 0) {
     for (int c = 0; c < kPlanCtas; ++c) {
       lo = min(lo, s_cta_lo[c]);
@@ -164,7 +167,11 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
     }
     // widen by 1/1024 each way: about 16 keys of the sample's spacing, so that
     // few keys of an even spread fall outside and crowd into the end buckets
-    const K pad = (hi - lo) >> 10;
+    // (unless that made the buckets too wide to be counted)
+    raw = hi - lo;
+    K pad = raw >> 10;
+    const K most = (K)kCountSpan * a.nb;
+    if (raw < most && raw + 2 * pad >= most) pad = 0;
     lo -= min(lo, pad);
     hi += min((K)(~(K)0 - hi), pad);
     // keys over most of their type's range: the map is their top bits, which
@@ -228,9 +235,8 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
       mx = max(mx, s_max[c]);
       hot += s_hot[c];
     }
-    const bool fits = mx <= a.max_sample && hot <= kSample / 64;
+    bool fits = mx <= a.max_sample && hot <= kSample / 64;
     BucketMap m{};
-    m.on = fits ? 1u : 0u;
     m.plain = base == 0 && mult == a.nb && s == 8 * sizeof(K) - 32 ? 1u : 0u;
     m.mult = mult;
     m.inv = (1ull << 63) / mult;
@@ -242,6 +248,15 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
     uint32_t sh = 0;
     while (((width - 1) >> sh) >= kCells) ++sh;
     m.cell_shift = sh + s;
+    m.counts = s == 0 && width <= kCountSpan ? 1u : 0u;
+    // Buckets of few values are counted.  Where they span too many for that and too
+    // few for the bitmap (200 of m keys meet another), the LSD passes run, as they
+    // do for ranges of two digits whose counters would see every value hundreds of
+    // times (100M keys of 16 bits: 922 us by digits, 1275 by buckets).
+    const unsigned long long per = a.keys / a.nb;
+    if (!m.counts && s < 16 && per * per > (400 * width) << s) fits = false;
+    if (m.counts && raw < 65536 && a.keys / ((unsigned long long)raw + 1) > 512) fits = false;
+    m.on = fits ? 1u : 0u;
     *a.map = m;
     a.rare[0] = 0;
     if (fits) {  // the LSD passes enqueued behind this sort do nothing
@@ -671,6 +686,7 @@ struct FinishJob {
   uint32_t kind;
   uint32_t edge;  // 1: the bucket's range is not known (it holds keys outside the map): found here
   uint32_t cell_shift;  // cells of (key - first)
+  uint32_t number;      // listed if the bucket is left to rare_buckets
   const K *lo, *hi;     // the array src lies in
 };
 
@@ -687,8 +703,16 @@ __device__ __forceinline__ uint32_t spread_of(K range, int keep) {
 // rare_buckets: their code here would cost the main path its registers (0.51 ms
 // against 0.35 at 100M keys).
 // RAW: float keys are read as they are stored, not in ordered form.
+// COUNTS: for buckets that span at most kCountSpan values (keys that repeat, as
+// floats of one octave do: 2^23 values): a 16-bit counter per value in place of
+// the bitmap.  The atomic add gives a key's place among its equals, and the
+// scanned counters its value's place: no key meets another.  100M 32-bit keys of
+// 20 to 26 bits: 0.99 ms for the sort (by digits 1.48 to 1.66); 28 bits, whose
+// bitmaps are full of keys that meet and left nearly all buckets to rare_buckets,
+// 2.17 -> 1.04.  Sorted 64-bit keys, one value each: 0.223 -> 0.183 ms for this
+// kernel at 33M; 32-bit 0.304 -> 0.321 at 100M.
 template <typename K, bool FLT, int BLOCK = kFinishBlock, uint32_t CAP = kFinishCap, int CELL_BITS = kCellBits,
-          bool RAW = false, typename Next>
+          bool RAW = false, bool COUNTS = false, typename Next>
 __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint32_t* err, Next&& next) {
   constexpr uint32_t B = BLOCK;
   constexpr int ITEMS = (int)CAP / BLOCK;
@@ -752,6 +776,7 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
     const FinishJob<K>& job = s_job[slot];  // (read where needed: its pointers need no registers meanwhile)
     const uint32_t cnt = job.cnt;
     K first = 0;
+    [[maybe_unused]] K edge_hi = 0;  // greatest key of a job of unknown range
     // thread 0, once s_in has been read: the next bucket
     auto go_on = [&]() {
       if (tid == 0 && b + gridDim.x < nb) prepare(b + gridDim.x, &s_job[slot ^ 1u]);
@@ -789,157 +814,15 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
           hi = max(hi, s_edge[W + w]);
         }
         first = lo;
+        edge_hi = hi;
         cs = spread_of<K>((K)(hi - lo), CELL_BITS);
       }
-      K k[ITEMS];  // distances from `first`; past the end, whatever s_in holds
-      uint32_t hit = 0;   // bit j: key j found its cell taken
-      uint32_t skip = 0;  // bit j: that, or there is no key j
-#pragma unroll
-      for (int c = 0; c < ITEMS; c += C) {
-        if ((uint32_t)c * B >= cnt) break;
-        uint32_t old[C];
-        if ((uint32_t)(c + C) * B <= cnt) {
-#pragma unroll
-          for (int j = 0; j < C; ++j) {
-            k[c + j] = to_ordered(src[(uint32_t)(c + j) * B], RAW) - first;
-            old[j] = atomicOr(&entry_of(k[c + j])->x, 1u << cell_of(k[c + j]));
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < C; ++j) {
-            const bool has = (uint32_t)(c + j) * B + tid < cnt;
-            k[c + j] = to_ordered(src[(uint32_t)(c + j) * B], RAW) - first;
-            old[j] = atomicOr(&entry_of(k[c + j])->x, has ? 1u << cell_of(k[c + j]) : 0u);
-            skip |= has ? 0u : 1u << (c + j);
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < C; ++j) hit |= ((old[j] >> cell_of(k[c + j])) & 1u) << (c + j);
-      }
-      hit &= ~skip;
-      skip |= hit;
-      if (hit) {
-        uint32_t p = atomicAdd(&s_nhit, (uint32_t)__popc(hit));
-        for (uint32_t h = hit; h; h &= h - 1u, ++p)
-          if (p < kHits) s_hit[p] = to_ordered(src[((uint32_t)__ffs((int)h) - 1u) * B], RAW) - first;
-      }
-      if (!ok) s_over = 2;
-      __syncthreads();
-      const uint32_t nhit = s_nhit;
-      if (s_over == 2) {  // the copy never came: wait it out once more, sort nothing further
-        mbar_wait_bounded(&s_bar, parity ^ 1u, err);
-        if (tid == 0) bulk_store_wait_all();
-        return;
-      }
-      go_on();
-      bool crowded = nhit > kHits;
-      K hx = 0;               // this thread's listed key
-      uint32_t turn = 0;      // its number among its entry's listed keys
-      uint32_t listed = 0, span = 0;  // how many those are; all of the entry's keys
-      if (nhit && !crowded) {
-        if (tid < nhit) {
-          hx = s_hit[tid];
-          turn = atomicAdd(&entry_of(hx)->y, 1u);
-          if (turn >= kEntryHits) s_over = 1;
-        }
-        __syncthreads();
-        crowded = s_over != 0;
-      }
-      if (!crowded) {
-        // Scan: warp w owns kEntries / W entries, lane l entries 2 l and 2 l + 1
-        // of each run of 64.  An entry's keys: its set bits and its listed keys.
-        uint4 q[U];
-        uint32_t c2[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          q[u] = reinterpret_cast<uint4*>(s_entry)[(warp * U + u) * 32 + lane];
-          q[u].y += __popc(q[u].x);
-          c2[u] = q[u].y + q[u].w + __popc(q[u].z);
-        }
-        if (tid < nhit) {
-          const uint2 e = *entry_of(hx);
-          listed = e.y;
-          span = e.y + __popc(e.x);
-        }
-        uint32_t p2[U / 2], t2[U / 2];
-#pragma unroll
-        for (int u = 0; u < U / 2; ++u) p2[u] = c2[2 * u] | (c2[2 * u + 1] << 16);
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-          for (int u = 0; u < U / 2; ++u) {
-            const uint32_t x = __shfl_up_sync(kFull, p2[u], o);
-            if (lane >= (uint32_t)o) p2[u] += x;
-          }
-        }
-        uint32_t total = 0;
-#pragma unroll
-        for (int u = 0; u < U / 2; ++u) {
-          t2[u] = __shfl_sync(kFull, p2[u], 31);
-          total += (t2[u] & 0xFFFFu) + (t2[u] >> 16);
-        }
-        if (lane == 0) s_warp[warp] = total;
-        // (the last bucket's copy out of s_keys must have read it)
-        if (tid == 0) bulk_store_wait_read();
-        __syncthreads();
-        uint32_t before = __reduce_add_sync(kFull, lane < warp ? s_warp[lane & (W - 1)] : 0u);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const uint32_t run = before + (u & 1 ? p2[u / 2] >> 16 : p2[u / 2] & 0xFFFFu) - c2[u];
-          before += u & 1 ? t2[u / 2] >> 16 : t2[u / 2] & 0xFFFFu;
-          q[u].w = run + q[u].y;
-          q[u].y = run;
-          reinterpret_cast<uint4*>(s_entry)[(warp * U + u) * 32 + lane] = q[u];
-        }
-        __syncthreads();
-        // staged with the destination's own offset from a 16-byte boundary
-        K* dst = job.dst;
+      // out of s_keys, where the keys lie with the destination's own offset from a
+      // 16-byte boundary: whole 16-byte units in one bulk copy, the keys before
+      // the first and after the last boundary singly
+      auto write_out = [&](K* dst) {
         const uint32_t skew = skew_of(dst);
         K* stage = s_keys + skew;
-#pragma unroll
-        for (int c = 0; c < ITEMS; c += C) {
-          if ((uint32_t)c * B >= cnt) break;
-#pragma unroll
-          for (int j = c; j < c + C; ++j) {
-            const uint2 e = *entry_of(k[j]);
-            const uint32_t p = e.y + __popc(e.x & ((1u << cell_of(k[j])) - 1u));
-            if (!((skip >> j) & 1u)) stage[p & (CAP - 1)] = from_ordered((K)(k[j] + first), FLT);
-          }
-        }
-        if (nhit) {
-          uint32_t lo = 0, bits = 0;
-          if (tid < nhit) {
-            const uint2 e = *entry_of(hx);
-            lo = e.y;
-            bits = e.x;
-            if (listed > 1) stage[(lo + __popc(bits) + turn) & (CAP - 1)] = from_ordered((K)(hx + first), FLT);
-          }
-          __syncthreads();
-          if (listed == 1) {  // between the key it met and the next: those above move up by one
-            const uint32_t r = lo + __popc(bits & ((1u << cell_of(hx)) - 1u));
-            const uint32_t top = min(CAP, lo + span) - 1u;
-            for (uint32_t j = top; j > r + 1; --j) stage[j] = stage[j - 1];
-            const K x = from_ordered((K)(hx + first), FLT), y = stage[r];
-            const bool below = hx + first < to_ordered(y, FLT);
-            stage[r] = below ? x : y;
-            if (r < top) stage[r + 1] = below ? y : x;
-          } else if (listed > 1 && turn == 0) {  // several: the entry's keys are sorted
-            const uint32_t hi = min(CAP, lo + span);
-            for (uint32_t j = lo + 1; j < hi; ++j) {
-              const K x = stage[j];
-              uint32_t p = j;
-              while (p > lo) {
-                const K y = stage[p - 1];
-                if (to_ordered(y, FLT) <= to_ordered(x, FLT)) break;
-                stage[p] = y;
-                --p;
-              }
-              stage[p] = x;
-            }
-          }
-        }
-        // out: whole 16-byte units in one bulk copy, the keys before the first
-        // and after the last boundary singly
         fence_proxy_async();
         __syncthreads();
         const uint32_t head = min(cnt, (V - skew) & (V - 1));
@@ -951,9 +834,252 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
           if (head + body + i < cnt) dst[head + body + i] = stage[head + body + i];
         }
         done = true;
+      };
+      if constexpr (COUNTS) {
+        uint32_t* s_half = reinterpret_cast<uint32_t*>(s_entry);
+        constexpr uint32_t kWords = kEntries * 2;
+        if (job.edge) {  // (its range is known only now)
+          const bool wide = first > (K)~(K)0 - (kCountSpan - 1) ? false : edge_hi > first + (kCountSpan - 1);
+          if (wide && tid == 0) s_over = 1;
+        }
+        K k[ITEMS];
+        uint32_t r[ITEMS / 2];
+#pragma unroll
+        for (int c = 0; c < ITEMS / 2; ++c) r[c] = 0;
+#pragma unroll
+        for (int c = 0; c < ITEMS; c += C) {
+          if ((uint32_t)c * B >= cnt) break;
+#pragma unroll
+          for (int j = c; j < c + C; ++j) {
+            const bool has = (uint32_t)j * B + tid < cnt;
+            k[j] = to_ordered(src[(uint32_t)j * B], RAW) - first;
+            const uint32_t sh = ((uint32_t)k[j] & 1u) * 16u;
+            const uint32_t old = atomicAdd(s_half + ((uint32_t)(k[j] >> 1) & (kWords - 1)), has ? 1u << sh : 0u);
+            r[j / 2] |= ((old >> sh) & 0xFFFFu) << (16 * (j % 2));
+          }
+        }
+        if (!ok) s_over = 2;
+        __syncthreads();
+        if (s_over == 2) {  // (as below)
+          mbar_wait_bounded(&s_bar, parity ^ 1u, err);
+          if (tid == 0) bulk_store_wait_all();
+          return;
+        }
+        go_on();
+        if (s_over == 0) {
+          uint4 q[U];
+          uint32_t c2[U];
+          auto both = [](uint32_t w) { return (w & 0xFFFFu) + (w >> 16); };
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            q[u] = reinterpret_cast<uint4*>(s_half)[(warp * U + u) * 32 + lane];
+            c2[u] = both(q[u].x) + both(q[u].y) + both(q[u].z) + both(q[u].w);
+          }
+          uint32_t p2[U / 2], t2[U / 2];
+#pragma unroll
+          for (int u = 0; u < U / 2; ++u) p2[u] = c2[2 * u] | (c2[2 * u + 1] << 16);
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+            for (int u = 0; u < U / 2; ++u) {
+              const uint32_t x = __shfl_up_sync(kFull, p2[u], o);
+              if (lane >= (uint32_t)o) p2[u] += x;
+            }
+          }
+          uint32_t total = 0;
+#pragma unroll
+          for (int u = 0; u < U / 2; ++u) {
+            t2[u] = __shfl_sync(kFull, p2[u], 31);
+            total += (t2[u] & 0xFFFFu) + (t2[u] >> 16);
+          }
+          if (lane == 0) s_warp[warp] = total;
+          // (the last bucket's copy out of s_keys must have read it)
+          if (tid == 0) bulk_store_wait_read();
+          __syncthreads();
+          uint32_t before = __reduce_add_sync(kFull, lane < warp ? s_warp[lane & (W - 1)] : 0u);
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            uint32_t run = before + (u & 1 ? p2[u / 2] >> 16 : p2[u / 2] & 0xFFFFu) - c2[u];
+            before += u & 1 ? t2[u / 2] >> 16 : t2[u / 2] & 0xFFFFu;
+            auto start = [&](uint32_t w) {
+              const uint32_t at = run | ((run + (w & 0xFFFFu)) << 16);
+              run += both(w);
+              return at;
+            };
+            uint4 p;
+            p.x = start(q[u].x);
+            p.y = start(q[u].y);
+            p.z = start(q[u].z);
+            p.w = start(q[u].w);
+            reinterpret_cast<uint4*>(s_half)[(warp * U + u) * 32 + lane] = p;
+          }
+          __syncthreads();
+          K* stage = s_keys + skew_of(job.dst);
+#pragma unroll
+          for (int c = 0; c < ITEMS; c += C) {
+            if ((uint32_t)c * B >= cnt) break;
+#pragma unroll
+            for (int j = c; j < c + C; ++j) {
+              const uint32_t w = s_half[(uint32_t)(k[j] >> 1) & (kWords - 1)];
+              const uint32_t p = ((w >> (((uint32_t)k[j] & 1u) * 16u)) & 0xFFFFu) + ((r[j / 2] >> (16 * (j % 2))) & 0xFFFFu);
+              if ((uint32_t)j * B + tid < cnt) stage[p & (CAP - 1)] = from_ordered((K)(k[j] + first), FLT);
+            }
+          }
+          write_out(job.dst);
+        }
+      } else {
+        K k[ITEMS];  // distances from `first`; past the end, whatever s_in holds
+        uint32_t hit = 0;   // bit j: key j found its cell taken
+        uint32_t skip = 0;  // bit j: that, or there is no key j
+#pragma unroll
+        for (int c = 0; c < ITEMS; c += C) {
+          if ((uint32_t)c * B >= cnt) break;
+          uint32_t old[C];
+          if ((uint32_t)(c + C) * B <= cnt) {
+#pragma unroll
+            for (int j = 0; j < C; ++j) {
+              k[c + j] = to_ordered(src[(uint32_t)(c + j) * B], RAW) - first;
+              old[j] = atomicOr(&entry_of(k[c + j])->x, 1u << cell_of(k[c + j]));
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < C; ++j) {
+              const bool has = (uint32_t)(c + j) * B + tid < cnt;
+              k[c + j] = to_ordered(src[(uint32_t)(c + j) * B], RAW) - first;
+              old[j] = atomicOr(&entry_of(k[c + j])->x, has ? 1u << cell_of(k[c + j]) : 0u);
+              skip |= has ? 0u : 1u << (c + j);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < C; ++j) hit |= ((old[j] >> cell_of(k[c + j])) & 1u) << (c + j);
+        }
+        hit &= ~skip;
+        skip |= hit;
+        if (hit) {
+          uint32_t p = atomicAdd(&s_nhit, (uint32_t)__popc(hit));
+          for (uint32_t h = hit; h; h &= h - 1u, ++p)
+            if (p < kHits) s_hit[p] = to_ordered(src[((uint32_t)__ffs((int)h) - 1u) * B], RAW) - first;
+        }
+        if (!ok) s_over = 2;
+        __syncthreads();
+        const uint32_t nhit = s_nhit;
+        if (s_over == 2) {  // the copy never came: wait it out once more, sort nothing further
+          mbar_wait_bounded(&s_bar, parity ^ 1u, err);
+          if (tid == 0) bulk_store_wait_all();
+          return;
+        }
+        go_on();
+        bool crowded = nhit > kHits;
+        K hx = 0;               // this thread's listed key
+        uint32_t turn = 0;      // its number among its entry's listed keys
+        uint32_t listed = 0, span = 0;  // how many those are; all of the entry's keys
+        if (nhit && !crowded) {
+          if (tid < nhit) {
+            hx = s_hit[tid];
+            turn = atomicAdd(&entry_of(hx)->y, 1u);
+            if (turn >= kEntryHits) s_over = 1;
+          }
+          __syncthreads();
+          crowded = s_over != 0;
+        }
+        if (!crowded) {
+          // Scan: warp w owns kEntries / W entries, lane l entries 2 l and 2 l + 1
+          // of each run of 64.  An entry's keys: its set bits and its listed keys.
+          uint4 q[U];
+          uint32_t c2[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            q[u] = reinterpret_cast<uint4*>(s_entry)[(warp * U + u) * 32 + lane];
+            q[u].y += __popc(q[u].x);
+            c2[u] = q[u].y + q[u].w + __popc(q[u].z);
+          }
+          if (tid < nhit) {
+            const uint2 e = *entry_of(hx);
+            listed = e.y;
+            span = e.y + __popc(e.x);
+          }
+          uint32_t p2[U / 2], t2[U / 2];
+#pragma unroll
+          for (int u = 0; u < U / 2; ++u) p2[u] = c2[2 * u] | (c2[2 * u + 1] << 16);
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+            for (int u = 0; u < U / 2; ++u) {
+              const uint32_t x = __shfl_up_sync(kFull, p2[u], o);
+              if (lane >= (uint32_t)o) p2[u] += x;
+            }
+          }
+          uint32_t total = 0;
+#pragma unroll
+          for (int u = 0; u < U / 2; ++u) {
+            t2[u] = __shfl_sync(kFull, p2[u], 31);
+            total += (t2[u] & 0xFFFFu) + (t2[u] >> 16);
+          }
+          if (lane == 0) s_warp[warp] = total;
+          // (the last bucket's copy out of s_keys must have read it)
+          if (tid == 0) bulk_store_wait_read();
+          __syncthreads();
+          uint32_t before = __reduce_add_sync(kFull, lane < warp ? s_warp[lane & (W - 1)] : 0u);
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const uint32_t run = before + (u & 1 ? p2[u / 2] >> 16 : p2[u / 2] & 0xFFFFu) - c2[u];
+            before += u & 1 ? t2[u / 2] >> 16 : t2[u / 2] & 0xFFFFu;
+            q[u].w = run + q[u].y;
+            q[u].y = run;
+            reinterpret_cast<uint4*>(s_entry)[(warp * U + u) * 32 + lane] = q[u];
+          }
+          __syncthreads();
+          // staged with the destination's own offset from a 16-byte boundary
+          K* dst = job.dst;
+          const uint32_t skew = skew_of(dst);
+          K* stage = s_keys + skew;
+#pragma unroll
+          for (int c = 0; c < ITEMS; c += C) {
+            if ((uint32_t)c * B >= cnt) break;
+#pragma unroll
+            for (int j = c; j < c + C; ++j) {
+              const uint2 e = *entry_of(k[j]);
+              const uint32_t p = e.y + __popc(e.x & ((1u << cell_of(k[j])) - 1u));
+              if (!((skip >> j) & 1u)) stage[p & (CAP - 1)] = from_ordered((K)(k[j] + first), FLT);
+            }
+          }
+          if (nhit) {
+            uint32_t lo = 0, bits = 0;
+            if (tid < nhit) {
+              const uint2 e = *entry_of(hx);
+              lo = e.y;
+              bits = e.x;
+              if (listed > 1) stage[(lo + __popc(bits) + turn) & (CAP - 1)] = from_ordered((K)(hx + first), FLT);
+            }
+            __syncthreads();
+            if (listed == 1) {  // between the key it met and the next: those above move up by one
+              const uint32_t r = lo + __popc(bits & ((1u << cell_of(hx)) - 1u));
+              const uint32_t top = min(CAP, lo + span) - 1u;
+              for (uint32_t j = top; j > r + 1; --j) stage[j] = stage[j - 1];
+              const K x = from_ordered((K)(hx + first), FLT), y = stage[r];
+              const bool below = hx + first < to_ordered(y, FLT);
+              stage[r] = below ? x : y;
+              if (r < top) stage[r + 1] = below ? y : x;
+            } else if (listed > 1 && turn == 0) {  // several: the entry's keys are sorted
+              const uint32_t hi = min(CAP, lo + span);
+              for (uint32_t j = lo + 1; j < hi; ++j) {
+                const K x = stage[j];
+                uint32_t p = j;
+                while (p > lo) {
+                  const K y = stage[p - 1];
+                  if (to_ordered(y, FLT) <= to_ordered(x, FLT)) break;
+                  stage[p] = y;
+                  --p;
+                }
+                stage[p] = x;
+              }
+            }
+          }
+          write_out(dst);
+        }
       }
     }
-    if (!done && tid == 0) rare[1 + atomicAdd(rare, 1u)] = b;
+    if (!done && tid == 0) rare[1 + atomicAdd(rare, 1u)] = job.number;
   }
   if (tid == 0) bulk_store_wait_all();
 }
@@ -1174,6 +1300,7 @@ __device__ __forceinline__ void plain_job(const BucketArgs& a, const BucketMap& 
   // the first and last bucket also hold the keys outside the map
   job.edge = b == 0 || b == a.nb - 1 ? 1u : 0u;
   job.cell_shift = m.cell_shift;
+  job.number = b;
 }
 
 template <typename K, bool FLT>
@@ -1187,13 +1314,17 @@ __global__ void __launch_bounds__(kFinishBlock, kFinishPerSm<K>)
     at = a.start[blockIdx.x];
     end = a.start[blockIdx.x + 1];
   }
-  finish_buckets<K, FLT>(a.nb, a.rare, a.err, [&](uint32_t b, FinishJob<K>& job) {
+  auto next = [&](uint32_t b, FinishJob<K>& job) {
     plain_job<K>(a, m, b, at, end, in, out, other, n, job);
     if (b + gridDim.x < a.nb) {
       at = a.start[b + gridDim.x];
       end = a.start[b + gridDim.x + 1];
     }
-  });
+  };
+  if (m.counts)
+    finish_buckets<K, FLT, kFinishBlock, kFinishCap, kCellBits, false, true>(a.nb, a.rare, a.err, next);
+  else
+    finish_buckets<K, FLT>(a.nb, a.rare, a.err, next);
 }
 
 template <typename K, bool FLT>
@@ -1234,6 +1365,7 @@ __global__ void __launch_bounds__(BLOCK, 1) small_cells_kernel(K* keys, uint32_t
     job.cnt = n;
     job.edge = 1;
     job.cell_shift = 0;
+    job.number = 0;
   });
   __syncthreads();
   if (s_rare[0]) {
@@ -1278,6 +1410,7 @@ BucketArgs make_args(const BucketScratch& s, const K* tmp, size_t n, SortCtrl* c
   a.nb = s.nb;
   while ((1u << a.nb_bits) < s.nb) ++a.nb_bits;
   a.low_bits = s.low_bits;
+  a.keys = n;
   a.tile = kScatterTile<K>;
   a.tmp_align = (uint32_t)(reinterpret_cast<uintptr_t>(tmp) & 15u);
   // sample keys a bucket may hold: one that would be full, with room for chance
@@ -1384,7 +1517,9 @@ __global__ void __launch_bounds__(kSegPlanBlock) seg_map_kernel(const uint32_t* 
     lo = min(lo, s_lo[w]);
     hi = max(hi, s_hi[w]);
   }
-  const uint32_t pad = (hi - lo) >> 7;  // (about eight keys of the sample's spacing)
+  uint32_t pad = (hi - lo) >> 7;  // (about eight keys of the sample's spacing)
+  const uint32_t most_values = kCountSpan << g.nb_bits;  // (as in bucket_plan_kernel)
+  if (hi - lo < most_values && hi - lo + 2 * pad >= most_values) pad = 0;
   lo -= min(lo, pad);
   hi += min(0xFFFFFFFFu - hi, pad);
   if (hi - lo >= 0xE0000000u) {
@@ -1400,7 +1535,9 @@ __global__ void __launch_bounds__(kSegPlanBlock) seg_map_kernel(const uint32_t* 
   for (uint32_t j = 0; j < 4; ++j)
     mx = max(mx, atomicAdd(s_cnt + map_bucket(map_t<uint32_t>(k[j], lo, 0u), mult, (1u << g.nb_bits) - 1u), 1u) + 1u);
   const uint32_t most = 12u + (uint32_t)(((unsigned long long)(4 * kFinishCap) << 10) / g.len);
-  const bool off = __syncthreads_or(mx > most) != 0;
+  const unsigned long long width = ((1ull << 32) + mult - 1) / mult, per = g.len >> g.nb_bits;
+  // (few values a bucket, but too many to count: as in bucket_plan_kernel)
+  const bool off = __syncthreads_or(mx > most || (width > kCountSpan && per * per > 400 * width)) != 0;
   if (threadIdx.x != 0) return;
   SegMap m{};
   m.off = off ? 1u : 0u;
@@ -1408,7 +1545,6 @@ __global__ void __launch_bounds__(kSegPlanBlock) seg_map_kernel(const uint32_t* 
   m.mult = mult;
   m.plain = lo == 0 && hi == 0xFFFFFFFFu ? 1u : 0u;
   m.inv = (1ull << 63) / mult;
-  const unsigned long long width = ((1ull << 32) + mult - 1) / mult;
   while (((width - 1) >> m.cell_shift) >= kCells) ++m.cell_shift;
   sb.map[blockIdx.x] = m;
 }
@@ -1492,8 +1628,11 @@ __global__ void __launch_bounds__(kSegScanBlock) seg_jobs_kernel(const PlanDev P
     if (!off) {
       // room for its jobs behind those of the segments before it
       const uint32_t tiles = (g.len + 3u + kSegTile - 1u) / kSegTile;
+      // (a bucket's values, at most: ceil(2^32 / mult))
+      const bool counted = ((1ull << 32) + m.mult - 1) / m.mult <= kCountSpan;
       if (tid == 0) {
-        s_job0 = P.sb.whole + atomicAdd(&P.declined[seg::kJobBuckets], nb);
+        s_job0 = counted ? P.sb.buckets - nb - atomicAdd(&P.declined[seg::kJobCounted], nb)
+                         : P.sb.whole + atomicAdd(&P.declined[seg::kJobBuckets], nb);
         s_tile0 = atomicAdd(&P.declined[seg::kJobTiles], tiles);
       }
       __syncthreads();
@@ -1696,15 +1835,33 @@ __device__ __forceinline__ void seg_job(const PlanDev& P, size_t total, const Se
   job.cell_shift = j.cell_shift;
 }
 
-__global__ void __launch_bounds__(kFinishBlock, kFinishPerSm<uint32_t>) seg_finish_kernel(const PlanDev P, size_t total) {
+// Whole segments and buckets at the job array's front, then the counted ones at
+// its end.
+template <bool FLT, typename Make>
+__device__ __forceinline__ void seg_finish(const PlanDev& P, Make&& make) {
   // (thread 0) the next bucket's job, read a bucket ahead
   const uint32_t jobs = P.sb.whole + P.declined[seg::kJobBuckets];
   SegBucketJob nj{};
   if (threadIdx.x == 0 && blockIdx.x < jobs) nj = P.sb.bucket_job[blockIdx.x];
-  finish_buckets<uint32_t, false>(jobs, P.sb.rare, P.err, [&](uint32_t b, FinishJob<uint32_t>& job) {
-    seg_job(P, total, nj, job);
+  finish_buckets<uint32_t, FLT>(jobs, P.sb.rare, P.err, [&](uint32_t b, FinishJob<uint32_t>& job) {
+    make(nj, job);
+    job.number = b;
     if (b + gridDim.x < jobs) nj = P.sb.bucket_job[b + gridDim.x];
   });
+  const uint32_t counted = P.declined[seg::kJobCounted], first = P.sb.buckets - counted;
+  if (counted == 0) return;
+  __syncthreads();
+  if (threadIdx.x == 0 && blockIdx.x < counted) nj = P.sb.bucket_job[first + blockIdx.x];
+  finish_buckets<uint32_t, FLT, kFinishBlock, kFinishCap, kCellBits, false, true>(
+      counted, P.sb.rare, P.err, [&](uint32_t b, FinishJob<uint32_t>& job) {
+        make(nj, job);
+        job.number = first + b;
+        if (b + gridDim.x < counted) nj = P.sb.bucket_job[first + b + gridDim.x];
+      });
+}
+
+__global__ void __launch_bounds__(kFinishBlock, kFinishPerSm<uint32_t>) seg_finish_kernel(const PlanDev P, size_t total) {
+  seg_finish<false>(P, [&](const SegBucketJob& j, FinishJob<uint32_t>& job) { seg_job(P, total, j, job); });
 }
 
 __global__ void __launch_bounds__(kRareBlock) seg_rare_kernel(const PlanDev P, size_t total) {

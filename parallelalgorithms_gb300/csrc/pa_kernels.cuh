@@ -208,6 +208,8 @@ struct BucketMap {
   uint32_t s;          // (0 for 32-bit keys)
   uint32_t cell_shift;  // a bucket's keys are spread by (key - first) >> cell_shift
   uint32_t ticket;     // CTAs of the count kernel that are done
+  uint32_t counts;     // 1: buckets span few values, which the finish kernel counts
+  uint32_t pad;
   unsigned long long lo;
   unsigned long long inv;  // 2^63 / mult
 };

@@ -83,9 +83,9 @@ struct __align__(16) SegBucketJob {
   uint32_t cell_shift, pad;
 };
 // Words of PlanDev::declined, zeroed per run: declined segments and their pass
-// tiles; jobs of the others' buckets (behind the whole segments') and tiles;
-// then the declined segments.
-enum : uint32_t { kDeclinedSegs = 0, kDeclinedTiles = 1, kJobBuckets = 2, kJobTiles = 3, kDeclinedHead = 4 };
+// tiles; jobs of the others' buckets (behind the whole segments') and tiles; jobs
+// of counted buckets (from the job array's end on); then the declined segments.
+enum : uint32_t { kDeclinedSegs = 0, kDeclinedTiles = 1, kJobBuckets = 2, kJobTiles = 3, kJobCounted = 4, kDeclinedHead = 5 };
 struct SegBucketsDev {
   uint32_t num;                 // segments of several buckets
   uint32_t whole;               // segments that are one bucket: the first jobs, uploaded with the plan
