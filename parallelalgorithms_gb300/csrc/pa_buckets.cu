@@ -657,7 +657,6 @@ constexpr int kFinishBlock = 256;
 template <typename K>
 constexpr int kFinishPerSm = sizeof(K) == 4 ? 4 : 2;
 constexpr uint32_t kFinishCap = 4096;
-constexpr int kFinishItems = (int)kFinishCap / kFinishBlock;
 constexpr uint32_t kEntryHits = 6;  // keys of one entry that found their cell taken, at most
 
 // The least t with umulhi(t, mult) >= b (b < nb), from the rounded-down
@@ -1130,7 +1129,7 @@ __device__ void finish_slow(K* a, K* b, uint32_t m, bool into_a, unsigned char* 
   uint32_t* s_wc = s_cur + 256;                                       // [W][256]
   uint32_t* s_warp = s_wc + W * 256;                                  // [W]
   K* s_mm = reinterpret_cast<K*>(s_warp + W);                         // [2 * W]
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t tid = threadIdx.x, warp = tid >> 5;
   K lo, hi;
   __syncthreads();
   block_minmax<K, B>(a, m, false, s_mm, lo, hi);
@@ -1429,19 +1428,23 @@ cudaError_t plan_t(const BucketArgs& a, const K* keys, size_t n, bool is_float, 
 }
 
 template <typename K, bool FLT>
+cudaError_t count_t(const BucketArgs& a, const K* keys, size_t n, cudaStream_t stream) {
+  auto kern = bucket_count_kernel<K, FLT>;
+  const size_t smem = (size_t)std::max<uint32_t>(a.nb, 1024) * 4;
+  cudaError_t e = ensure_dynamic_smem(kern, (size_t)kBucketsMax * 4);
+  if (e != cudaSuccess) return e;
+  const size_t work = ceil_div(n, (size_t)kCountBlock * (16 / sizeof(K)) * 2);
+  const size_t grid = std::min<size_t>(std::max<size_t>(work, 1), (size_t)device_info().sm_count);
+  kern<<<(unsigned)grid, kCountBlock, smem, stream>>>(keys, n, a);
+  return cudaGetLastError();
+}
+
+template <typename K, bool FLT>
 cudaError_t sort_t(const BucketArgs& a, K* keys, K* tmp, size_t n, cudaStream_t stream,
                    const std::function<cudaError_t()>& mark) {
   const unsigned sms = (unsigned)device_info().sm_count;
   auto m = [&]() { return mark ? mark() : cudaSuccess; };
   cudaError_t e = cudaSuccess;
-  {
-    auto kern = bucket_count_kernel<K, FLT>;
-    const size_t smem = (size_t)std::max<uint32_t>(a.nb, 1024) * 4;
-    if ((e = ensure_dynamic_smem(kern, (size_t)kBucketsMax * 4)) != cudaSuccess) return e;
-    const size_t work = ceil_div(n, (size_t)kCountBlock * (16 / sizeof(K)) * 2);
-    kern<<<(unsigned)std::min<size_t>(std::max<size_t>(work, 1), sms), kCountBlock, smem, stream>>>(keys, n, a);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  }
   if ((e = m()) != cudaSuccess) return e;
   if ((e = m()) != cudaSuccess) return e;
   const size_t tiles = ceil_div(n, (size_t)kScatterTile<K>) + 1;
@@ -1941,11 +1944,16 @@ cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, const 
   if (key_bytes == 8) {
     BucketArgs a = make_args(s, static_cast<const unsigned long long*>(tmp), n, ctrl, nullptr);
     a.decided = decided;
-    return plan_t(a, static_cast<const unsigned long long*>(keys), n, false, stream);
+    const auto* k = static_cast<const unsigned long long*>(keys);
+    const cudaError_t e = plan_t(a, k, n, false, stream);
+    return e != cudaSuccess ? e : count_t<unsigned long long, false>(a, k, n, stream);
   }
   BucketArgs a = make_args(s, static_cast<const uint32_t*>(tmp), n, ctrl, nullptr);
   a.decided = decided;
-  return plan_t(a, static_cast<const uint32_t*>(keys), n, is_float, stream);
+  const auto* k = static_cast<const uint32_t*>(keys);
+  const cudaError_t e = plan_t(a, k, n, is_float, stream);
+  if (e != cudaSuccess) return e;
+  return is_float ? count_t<uint32_t, true>(a, k, n, stream) : count_t<uint32_t, false>(a, k, n, stream);
 }
 
 cudaError_t enqueue_bucket_sort(const BucketScratch& s, void* keys, void* tmp, size_t n, int key_bytes, bool is_float,
