@@ -1900,19 +1900,17 @@ cudaError_t launch_clear(void* p, size_t bytes, const uint32_t* off, cudaStream_
   return cudaGetLastError();
 }
 
-// A synchronous call of n uniform keys, this sort against the LSD passes:
-// 32-bit 100 K 50 us against 68, 700 K 59 against 76, 2.2M 80 against 112, 10M
-// 144 against 233, 100M 918 against 1640; 64-bit 100 K 51 against 119, 1M 74
-// against 154, 10M 222 against 550.  Keys that the plan turns away pay for it,
-// about 18 us (32-bit, Zipf: 100 K 84 against 66, 1M 102 against 84), so 32-bit
-// keys come here from 2^19 on, where the gain is at least that much; 64-bit keys
-// have eight LSD passes to save and come from the smallest size on.  Above
-// kBucketsMax * kBucketTarget keys a bucket would no longer fit the finish
+// A synchronous call of n uniform keys, this sort against the LSD passes (us):
+// 32-bit 8193 52 against 67, 100 K 50 against 69, 400 K 54 against 75, 2.2M 80
+// against 112, 10M 144 against 233, 100M 918 against 1640; 64-bit 100 K 51 against
+// 119, 1M 74 against 154, 10M 222 against 550.  Keys that the plan turns away pay
+// for it, 12 to 18 us (32-bit Zipf keys: 100 K 83 against 67, 1M 104 against 84;
+// constant ones 62 against 49), so every size beyond the one-CTA sort comes here.
+// Above kBucketsMax * kBucketTarget keys a bucket would no longer fit the finish
 // kernel with room for uneven filling.
 bool bucket_sort_supported(size_t n, int key_bytes) {
   if (key_bytes != 4 && key_bytes != 8) return false;
-  const size_t least = key_bytes == 4 ? (size_t)1 << 19 : small_sort_max_keys(key_bytes, false) + 1;
-  return n >= least && n <= kBucketMostKeys;
+  return n > small_sort_max_keys(key_bytes, false) && n <= kBucketMostKeys;
 }
 
 size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s) {

@@ -595,6 +595,7 @@ int sort_impl(void* keys, void* tmp, uint32_t* vals, uint32_t* tmp_vals, size_t 
 // 10M (within the scratch) 257 -> 155.
 constexpr size_t kInplaceDefaultScratch = (size_t)1 << 24;  // keys
 constexpr size_t kInplaceMinScratch = (size_t)1 << 16;
+constexpr size_t kInplaceBucketKeys = (size_t)1 << 19;  // (smaller groups do not pay for a wait each)
 
 int inplace_levels(Workspace* ws, cudaStream_t stream, uint32_t* a, size_t n, size_t S, uint32_t* buf,
                    InplaceState* st, void* status, unsigned long long* hist, char* plan_dev, size_t plan_cap,
@@ -658,7 +659,7 @@ int inplace_levels(Workspace* ws, cudaStream_t stream, uint32_t* a, size_t n, si
     // sorted as one array).
     auto by_buckets = [&](const Group& gr) {
       const size_t len = (size_t)gr.off.back();
-      return decided && bucket_sort_supported(len, 4) && gr.most * (size_t)(gr.last - gr.first + 1) * 4 <= len * 5;
+      return decided && len >= kInplaceBucketKeys && bucket_sort_supported(len, 4) && gr.most * (size_t)(gr.last - gr.first + 1) * 4 <= len * 5;
     };
     for (size_t g = 0; g < groups.size(); ++g) {
       size_t bytes = 0;

@@ -234,9 +234,9 @@ size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s);
 // buckets (when the keys are too unevenly spread it does not), and then ctrl
 // says "skip" for every LSD pass; and the count behind it, which runs while a
 // caller that waits for the decision learns it and enqueues the rest (1M uniform
-// 32-bit keys 75 -> 70 us a call, 600 K 62 -> 56; keys turned away find one more launch that
-// returns).  decided, when set, is page-locked host memory that receives map->on
-// as soon as it is known.
+// 32-bit keys 75 -> 70 us a call, 600 K 62 -> 56; keys turned away find one more
+// launch that returns).  decided, when set, is page-locked host memory that
+// receives map->on as soon as it is known.
 cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, const void* tmp, size_t n, int key_bytes,
                                 bool is_float, SortCtrl* ctrl, uint32_t* decided, cudaStream_t stream);
 // Enqueues the planned sort (tmp: n keys of scratch; the result is in keys);
