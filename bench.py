@@ -83,8 +83,10 @@ def profile_op(a) -> None:
     """Runs one operation of the path `a.reps` times with nothing else on the
     GPU, so that an ncu launch filter (-k regex:... -s <skip> -c <count>)
     lands on known launches.  The seeded input is generated once and kept
-    device-resident.  Per sort: the workspace memset, one digit histogram,
-    one scan, one onesweep launch per key byte, one final copy.
+    device-resident.  Per sort by buckets: plan, count, one or two
+    partitions, the sort of the buckets and of the rare ones; by digits: the
+    workspace memset, one digit histogram, one scan, one onesweep launch per key
+    byte, one final copy.
     `sort_u32_host` sorts a page-locked host copy through the C ABI instead
     (the pipelined host-buffer path); `sort_u32_inplace` is the bounded-scratch
     in-place sort, `partition_u32` PartitionRadix around k = n/2 and n - 21,
