@@ -149,6 +149,7 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
     s_hi[warp] = hi;
   }
   cluster.sync();  // (every CTA of the cluster runs before its memory is written from another)
+  chain_next();
   if (warp == 0) {
     lo = s_lo[lane];
     hi = s_hi[lane];
@@ -289,10 +290,12 @@ __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* _
   __shared__ uint32_t s_warp[kCountBlock / 32];
   __shared__ uint32_t s_last;
   constexpr int V = 16 / (int)sizeof(K);
-  const BucketMap m = *a.map;
-  if (!m.on) return;
   const uint32_t tid = threadIdx.x;
   for (uint32_t i = tid; i < a.nb; i += kCountBlock) s_cnt[i] = 0;
+  chain_wait();
+  chain_next();
+  const BucketMap m = *a.map;
+  if (!m.on) return;
   __syncthreads();
   const uint32_t last = a.nb - 1;
   auto count = [&](auto plainc) {
@@ -619,6 +622,8 @@ __global__ void __launch_bounds__(kScatterBlock, kScatterPerSm) bucket_scatter_k
   __shared__ uint32_t s_warp[kScatterBlock / 32];
   __shared__ uint32_t s_one;
   __shared__ uint32_t s_first[kGroups + 1];
+  chain_wait();
+  chain_next();
   const BucketMap m = *a.map;
   if (!m.on) return;
   if constexpr (GROUPED) {
@@ -1305,6 +1310,8 @@ __device__ __forceinline__ void plain_job(const BucketArgs& a, const BucketMap& 
 template <typename K, bool FLT>
 __global__ void __launch_bounds__(kFinishBlock, kFinishPerSm<K>)
     bucket_finish_kernel(K* in, K* out, K* other, size_t n, BucketArgs a) {
+  chain_wait();
+  chain_next();
   const BucketMap m = *a.map;
   if (!m.on) return;
   // (thread 0) start[b] and start[b + 1] of the next bucket, read a bucket ahead
@@ -1328,6 +1335,7 @@ __global__ void __launch_bounds__(kFinishBlock, kFinishPerSm<K>)
 
 template <typename K, bool FLT>
 __global__ void __launch_bounds__(kRareBlock) bucket_rare_kernel(K* in, K* out, K* other, size_t n, BucketArgs a) {
+  chain_wait();
   const BucketMap m = *a.map;
   if (!m.on) return;
   rare_buckets<K, FLT>(a.rare, [&](uint32_t b, FinishJob<K>& job) {
@@ -1435,8 +1443,7 @@ cudaError_t count_t(const BucketArgs& a, const K* keys, size_t n, cudaStream_t s
   if (e != cudaSuccess) return e;
   const size_t work = ceil_div(n, (size_t)kCountBlock * (16 / sizeof(K)) * 2);
   const size_t grid = std::min<size_t>(std::max<size_t>(work, 1), (size_t)device_info().sm_count);
-  kern<<<(unsigned)grid, kCountBlock, smem, stream>>>(keys, n, a);
-  return cudaGetLastError();
+  return launch_chained(kern, (unsigned)grid, kCountBlock, smem, stream, keys, n, a);
 }
 
 template <typename K, bool FLT>
@@ -1448,27 +1455,29 @@ cudaError_t sort_t(const BucketArgs& a, K* keys, K* tmp, size_t n, cudaStream_t 
   if ((e = m()) != cudaSuccess) return e;
   if ((e = m()) != cudaSuccess) return e;
   const size_t tiles = ceil_div(n, (size_t)kScatterTile<K>) + 1;
-  bucket_scatter_kernel<K, false, FLT>
-      <<<(unsigned)std::min<size_t>(tiles, sms * kScatterPerSm), kScatterBlock, 0, stream>>>(keys, tmp, n, a);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  e = launch_chained(bucket_scatter_kernel<K, false, FLT>, (unsigned)std::min<size_t>(tiles, sms * kScatterPerSm),
+                     kScatterBlock, 0, stream, keys, tmp, n, a);
+  if (e != cudaSuccess) return e;
   if ((e = m()) != cudaSuccess) return e;
   K* in = tmp;
   if (a.low_bits) {
-    bucket_scatter_kernel<K, true, false>
-        <<<(unsigned)std::min<size_t>(tiles + kGroups, sms * kScatterPerSm), kScatterBlock, 0, stream>>>(tmp, keys, n, a);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = launch_chained(bucket_scatter_kernel<K, true, false>,
+                       (unsigned)std::min<size_t>(tiles + kGroups, sms * kScatterPerSm), kScatterBlock, 0, stream, tmp, keys, n,
+                       a);
+    if (e != cudaSuccess) return e;
     in = keys;
   }
   if ((e = m()) != cudaSuccess) return e;
   auto kern = bucket_finish_kernel<K, FLT>;
   if ((e = ensure_dynamic_smem(kern, finish_smem<K>())) != cudaSuccess) return e;
-  kern<<<std::min<unsigned>(a.nb, sms * kFinishPerSm<K>), kFinishBlock, finish_smem<K>(), stream>>>(
-      in, keys, a.low_bits ? tmp : keys, n, a);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  e = launch_chained(kern, std::min<unsigned>(a.nb, sms * kFinishPerSm<K>), kFinishBlock, finish_smem<K>(), stream, in, keys,
+                     a.low_bits ? tmp : keys, n, a);
+  if (e != cudaSuccess) return e;
   auto rare = bucket_rare_kernel<K, FLT>;
   if ((e = ensure_dynamic_smem(rare, rare_smem<K>())) != cudaSuccess) return e;
-  rare<<<std::min<unsigned>(a.nb, sms * 2), kRareBlock, rare_smem<K>(), stream>>>(in, keys, a.low_bits ? tmp : keys, n, a);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  e = launch_chained(rare, std::min<unsigned>(a.nb, sms * 2), kRareBlock, rare_smem<K>(), stream, in, keys,
+                     a.low_bits ? tmp : keys, n, a);
+  if (e != cudaSuccess) return e;
   return m();
 }
 
