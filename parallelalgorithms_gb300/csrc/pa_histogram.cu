@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(kHistBlock, 1) digit_counts_kernel(const K* __
                                                                        uint32_t shift0, uint32_t step,
                                                                        unsigned long long* __restrict__ out,
                                                                        const uint32_t* off) {
+  chain_next();
   if (off && *off) return;
   constexpr int R = 1 << RB;
   constexpr int V = kVec<K>;
@@ -179,6 +180,7 @@ __global__ void __launch_bounds__(NT, 1) tile_counts_kernel(const uint32_t* __re
                                                               uint32_t* __restrict__ tile_prefix,
                                                               uint32_t* chunk_tot, uint32_t* __restrict__ chunk_excl,
                                                               uint32_t* ticket, const uint32_t* off) {
+  chain_next();
   if (off && *off) return;
   constexpr uint32_t L = kTcLanes;
   extern __shared__ __align__(16) uint32_t s_tc[];
@@ -408,6 +410,8 @@ __global__ void __launch_bounds__(kScanBlock) scan_digits_kernel(const unsigned 
                                                                  int passes, size_t n, int is_float, int allow_skip,
                                                                  unsigned long long* __restrict__ bin_start,
                                                                  SortCtrl* ctrl, const uint32_t* off) {
+  chain_wait();
+  chain_next();
   if (off && *off) return;
   constexpr int PER = R / kScanBlock;
   __shared__ unsigned long long s_warp[kScanBlock / 32];
@@ -648,14 +652,12 @@ cudaError_t launch_scan_digits(const unsigned long long* counts, int passes, int
                                cudaStream_t stream, const uint32_t* off) {
   if (passes < 1 || passes > kMaxPasses) return cudaErrorInvalidValue;
   if (radix_bits == 8)
-    scan_digits_kernel<256><<<1, kScanBlock, 0, stream>>>(counts, passes, n, is_float ? 1 : 0, allow_skip ? 1 : 0,
-                                                           bin_start, ctrl, off);
-  else if (radix_bits == 11)
-    scan_digits_kernel<2048><<<1, kScanBlock, 0, stream>>>(counts, passes, n, is_float ? 1 : 0, allow_skip ? 1 : 0,
-                                                            bin_start, ctrl, off);
-  else
-    return cudaErrorInvalidValue;
-  return cudaGetLastError();
+    return launch_chained(scan_digits_kernel<256>, 1, kScanBlock, 0, stream, counts, passes, n, is_float ? 1 : 0,
+                          allow_skip ? 1 : 0, bin_start, ctrl, off);
+  if (radix_bits == 11)
+    return launch_chained(scan_digits_kernel<2048>, 1, kScanBlock, 0, stream, counts, passes, n, is_float ? 1 : 0,
+                          allow_skip ? 1 : 0, bin_start, ctrl, off);
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace pa

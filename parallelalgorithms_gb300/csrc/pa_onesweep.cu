@@ -51,6 +51,8 @@ template <typename K, bool HAS_VALS, int BLOCK, int ITEMS, int MINB, typename S,
 __global__ void __launch_bounds__(BLOCK, MINB) onesweep_kernel(const OnesweepArgs args) {
   using G = Geometry<K, HAS_VALS, BLOCK, ITEMS>;
   constexpr int TILE = G::kTile;
+  chain_wait();
+  chain_next();  // (the next pass starts once every CTA of this one has, so none waits for a tile not begun)
   const PassCtrl pc = args.ctrl->pass[args.pass];
   if (pc.skip) return;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -193,6 +195,7 @@ cudaError_t launch_small_t(void* keys, uint32_t* vals, size_t n, bool is_float, 
 template <typename K>
 __global__ void final_copy_kernel(K* keys_a, const K* keys_b, uint32_t* vals_a, const uint32_t* vals_b, size_t n,
                                   const SortCtrl* ctrl) {
+  chain_wait();
   if (!ctrl->final_in_tmp) return;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -271,8 +274,7 @@ cudaError_t launch_g2(const OnesweepArgs& a, cudaStream_t stream) {
   // 16-33 thousand CTA launches a pass (100M 64-bit keys with payloads, Zipf:
   // 5.64 ms a sort against 6.03; twice or four times the resident CTAs 5.65).
   tiles = std::min(tiles, (size_t)device_info().sm_count * MINB);
-  kern<<<(unsigned)tiles, BLOCK, G::kBytes, stream>>>(a);
-  return cudaGetLastError();
+  return launch_chained(kern, (unsigned)tiles, BLOCK, G::kBytes, stream, a);
 }
 
 // Ranking method of a pass: the warp multisplit (default) or the in-tile
@@ -434,14 +436,11 @@ cudaError_t launch_final_copy(void* keys_a, const void* keys_b, uint32_t* vals_a
   const int block = 256;
   const unsigned grid = (unsigned)min(ceil_div(n, (size_t)block), (size_t)device_info().sm_count * 8);
   if (key_bytes == 4)
-    final_copy_kernel<uint32_t><<<grid, block, 0, stream>>>(static_cast<uint32_t*>(keys_a),
-                                                            static_cast<const uint32_t*>(keys_b), vals_a, vals_b, n,
-                                                            ctrl);
-  else
-    final_copy_kernel<unsigned long long><<<grid, block, 0, stream>>>(
-        static_cast<unsigned long long*>(keys_a), static_cast<const unsigned long long*>(keys_b), vals_a, vals_b, n,
-        ctrl);
-  return cudaGetLastError();
+    return launch_chained(final_copy_kernel<uint32_t>, grid, block, 0, stream, static_cast<uint32_t*>(keys_a),
+                          static_cast<const uint32_t*>(keys_b), vals_a, vals_b, n, ctrl);
+  return launch_chained(final_copy_kernel<unsigned long long>, grid, block, 0, stream,
+                        static_cast<unsigned long long*>(keys_a), static_cast<const unsigned long long*>(keys_b), vals_a,
+                        vals_b, n, ctrl);
 }
 
 }  // namespace pa
