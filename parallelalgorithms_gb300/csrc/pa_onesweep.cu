@@ -196,6 +196,7 @@ template <typename K>
 __global__ void final_copy_kernel(K* keys_a, const K* keys_b, uint32_t* vals_a, const uint32_t* vals_b, size_t n,
                                   const SortCtrl* ctrl) {
   chain_wait();
+  chain_next();
   if (!ctrl->final_in_tmp) return;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {

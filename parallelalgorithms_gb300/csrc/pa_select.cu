@@ -218,6 +218,7 @@ __global__ void __cluster_dims__(kSampleCtas, 1, 1) __launch_bounds__(kSampleThr
   for (uint32_t i = j0; i < (uint32_t)kLinBins; i += kSample) st->lin_bins[i] = 0;
   for (uint32_t i = j0; i < 256u; i += kSample) st->hist[i] = 0;
   cluster.sync();  // (the first CTA runs before its memory is written)
+  chain_next();
   if (j0 < ns) cluster.map_shared_rank(s, 0)[j0] = mine;
   cluster.sync();
   if (cluster.block_rank() != 0) return;
@@ -463,6 +464,8 @@ __global__ void __launch_bounds__(kSelBlock, 1) select_range_kernel(const K* key
   const uint32_t tid = threadIdx.x;
   for (uint32_t i = tid; i < (uint32_t)kLinBins; i += kSelBlock) s_bins[i] = 0;
   if (tid == 0) s_cnt[0] = s_cnt[1] = s_cnt[2] = 0;
+  chain_wait();
+  chain_next();
   const K lo = (K)st->lo, hi = (K)st->hi;
   const bool dup = st->dup != 0;
   const LinMap lin = lin_map(lo, hi);
@@ -676,6 +679,7 @@ __global__ void __launch_bounds__(kSelBlock, 1) select_linear_kernel(const K* ca
                                                                      SelectState* st, K* out, uint32_t* decided) {
   extern __shared__ __align__(128) unsigned char lin_smem[];
   __shared__ bool s_last;
+  chain_wait();
   if (!st->lin) return;
   const uint32_t tid = threadIdx.x, lane = tid & 31u;
   const K lo = (K)st->lo;
@@ -873,12 +877,13 @@ cudaError_t launch_select_t(const K* keys, size_t n, unsigned long long k, K* ca
     if (n <= (size_t)kSample) return cudaSuccess;  // the answer is written
     e = ensure_dynamic_smem(select_range_kernel<K>, kStreamSmem);
     if (e != cudaSuccess) return e;
-    select_range_kernel<K><<<grid, kSelBlock, kStreamSmem, stream>>>(keys, n, cand_a, cap_a, cap_b, st, out, decided);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = launch_chained(select_range_kernel<K>, grid, kSelBlock, kStreamSmem, stream, keys, n, cand_a, cap_a, cap_b, st, out,
+                       decided);
+    if (e != cudaSuccess) return e;
     e = ensure_dynamic_smem(select_linear_kernel<K>, kLinSmem);
     if (e != cudaSuccess) return e;
-    select_linear_kernel<K><<<grid, kSelBlock, kLinSmem, stream>>>(cand_a, cand_b, cap_b, st, out, decided);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = launch_chained(select_linear_kernel<K>, grid, kSelBlock, kLinSmem, stream, cand_a, cand_b, cap_b, st, out, decided);
+    if (e != cudaSuccess) return e;
   }
   if (part == SelectPart::kFast) return cudaSuccess;
   e = ensure_dynamic_smem(select_step_kernel<K>, kStreamSmem);

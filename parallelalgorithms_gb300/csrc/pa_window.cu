@@ -163,6 +163,8 @@ __device__ __noinline__ void mend_run(K* keys, uint32_t* vals, size_t n, size_t 
 // marked by then.)
 constexpr int kFindRows = 8;
 __global__ void __launch_bounds__(256) window_mend_kernel(K* keys, uint32_t* vals, size_t n, WindowScratch s) {
+  chain_wait();
+  chain_next();
   const uint32_t shift = s.state->shift;
   if (shift == 0) return;
   const uint32_t lane = lane_id();
@@ -191,6 +193,7 @@ __global__ void __launch_bounds__(kLongBlock) window_long_kernel(K* keys, K* tke
                                                                   WindowScratch s) {
   constexpr int B = kLongBlock, W = B / 32;
   __shared__ uint32_t s_cur[256], s_wc[W * 256], s_warp[W];
+  chain_wait();
   const uint32_t shift = s.state->shift;
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
   if (shift == 0 || s.state->fail) {
@@ -306,12 +309,10 @@ cudaError_t enqueue_window_mend(const WindowScratch& s, void* keys, void* tmp, u
                                 cudaStream_t stream) {
   const unsigned sms = (unsigned)device_info().sm_count;
   K* k = static_cast<K*>(keys);
-  window_mend_kernel<<<(unsigned)std::min(ceil_div(n, (size_t)256 * kFindRows), (size_t)sms * 8), 256, 0, stream>>>(k, vals,
-                                                                                                                n, s);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_chained(
+      window_mend_kernel, (unsigned)std::min(ceil_div(n, (size_t)256 * kFindRows), (size_t)sms * 8), 256, 0, stream, k, vals, n, s);
   if (e != cudaSuccess) return e;
-  window_long_kernel<<<sms, kLongBlock, 0, stream>>>(k, static_cast<K*>(tmp), vals, tvals, s);
-  return cudaGetLastError();
+  return launch_chained(window_long_kernel, sms, kLongBlock, 0, stream, k, static_cast<K*>(tmp), vals, tvals, s);
 }
 
 }  // namespace pa
