@@ -36,7 +36,7 @@
 // the remaining digits in shared memory.
 //
 // Median of 100M uniform 32-bit keys, kernels one by one (us): sample 9, range 72
-// (59 of it the read at the measured copy rate), linear 16; a call that waits 109.
+// (59 of it the read at the measured copy rate), linear 16; a call that waits 106.
 // Before (a ticketed sample of exact bounds 12, both bounds' keys always counted
 // and a five-sigma bracket 81, digit steps over the candidates 16 and 11, three
 // launches that only returned or cleared 7): 144.  Shared memory for the linear
