@@ -844,7 +844,7 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
         constexpr uint32_t kWords = kEntries * 2;
         if (job.edge) {  // (its range is known only now)
           const bool wide = first > (K)~(K)0 - (kCountSpan - 1) ? false : edge_hi > first + (kCountSpan - 1);
-          if (wide && tid == 0) s_over = 1;
+          if (wide && tid == 0) atomicMax(&s_over, 1u);  // (not over the 2 of a copy that never came)
         }
         K k[ITEMS];
         uint32_t r[ITEMS / 2];
@@ -1083,7 +1083,12 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
         }
       }
     }
-    if (!done && tid == 0) rare[1 + atomicAdd(rare, 1u)] = job.number;
+    if (!done) {
+      if (tid == 0) rare[1 + atomicAdd(rare, 1u)] = job.number;
+      // every thread has read s_nhit and s_over, which say which barriers it
+      // takes part in, before thread 0 clears them (write_out has a barrier too)
+      __syncthreads();
+    }
   }
   if (tid == 0) bulk_store_wait_all();
 }
