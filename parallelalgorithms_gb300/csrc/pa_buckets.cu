@@ -9,8 +9,8 @@
 // (no look-back).  Keys cross memory 1 + 2 + 2 + 2 times (count, partition,
 // partition, bucket sort) against 1 + 2 * 4 (1 + 2 * 8 for 64-bit keys).
 //
-//   bucket_plan_kernel     one cluster of 8 CTAs reads 16384 keys at even
-//                          strides, takes the range they span, and lays nb
+//   bucket_plan_kernel     one cluster of 8 CTAs reads 16384 keys, one at a
+//                          random place of each stride, takes the range they span, and lays nb
 //                          equal buckets over it (BucketMap); counts the
 //                          sample per bucket to judge the fit: a sample that
 //                          crowds into few buckets leaves the sort to the LSD
@@ -47,7 +47,9 @@ constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr int kPlanCtas = 8;
 constexpr int kPlanBlock = 1024;
 constexpr int kPlanPer = 2;  // sample keys per thread
-constexpr uint32_t kSample = (uint32_t)kPlanCtas * kPlanBlock * kPlanPer;
+constexpr int kSampleLog2 = 14;
+constexpr uint32_t kSample = 1u << kSampleLog2;
+static_assert(kSample == (uint32_t)kPlanCtas * kPlanBlock * kPlanPer, "a key per thread and round");
 constexpr uint32_t kGroups = 256;         // bins of a partition pass, at most
 constexpr uint32_t kBucketsMax = 32768;   // counters of the count kernel: 128 KB of shared memory
 constexpr uint32_t kBucketTarget = 3072;  // keys per bucket, at most, while more buckets can be had
@@ -113,6 +115,19 @@ __device__ __forceinline__ void warp_minmax(K& lo, K& hi) {
   }
 }
 
+// The place of sample key i of 1 << log2 in an array of n keys: somewhere in the
+// i-th stride.  At even places keys that repeat a pattern whose period divides the
+// stride (a matrix, records, channels) would be seen in one phase only: 2^24 keys,
+// every second one small, looked evenly spread and 31 ms went into one bucket.
+__device__ __forceinline__ size_t sample_place(uint32_t i, int log2, size_t n) {
+  const size_t lo = (size_t)(((unsigned long long)i * n) >> log2);
+  const size_t hi = (size_t)((((unsigned long long)i + 1) * n) >> log2);
+  uint32_t h = i * 0x9E3779B9u;  // (2^32 / golden ratio; its product folded, twice)
+  h = (h ^ (h >> 15)) * 0x9E3779B9u;
+  h ^= h >> 13;
+  return lo + (size_t)__umul64hi((unsigned long long)h << 32, hi - lo);
+}
+
 // ---------------------------------------------------------------------------
 // Plan.
 // ---------------------------------------------------------------------------
@@ -137,8 +152,8 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
   K lo = ~(K)0, hi = 0;
 #pragma unroll
   for (int j = 0; j < kPlanPer; ++j) {
-    const size_t i = ((size_t)j * kPlanCtas + rank) * kPlanBlock + tid;
-    k[j] = to_ordered(keys[(size_t)(((unsigned long long)i * n) / kSample)], is_float != 0);
+    const uint32_t i = ((uint32_t)j * kPlanCtas + rank) * kPlanBlock + tid;
+    k[j] = to_ordered(keys[sample_place(i, kSampleLog2, n)], is_float != 0);
     lo = min(lo, k[j]);
     hi = max(hi, k[j]);
   }
@@ -1518,7 +1533,7 @@ __global__ void __launch_bounds__(kSegPlanBlock) seg_map_kernel(const uint32_t* 
 #pragma unroll
   for (uint32_t j = 0; j < 4; ++j) {
     const uint32_t i = j * kSegPlanBlock + threadIdx.x;
-    k[j] = keys[g.base + (((unsigned long long)i * g.len) >> 10)];
+    k[j] = keys[g.base + sample_place(i, 10, g.len)];
     lo = min(lo, k[j]);
     hi = max(hi, k[j]);
   }
