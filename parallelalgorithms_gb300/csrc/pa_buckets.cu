@@ -51,9 +51,16 @@ constexpr int kSampleLog2 = 14;
 constexpr uint32_t kSample = 1u << kSampleLog2;
 static_assert(kSample == (uint32_t)kPlanCtas * kPlanBlock * kPlanPer, "a key per thread and round");
 constexpr uint32_t kGroups = 256;         // bins of a partition pass, at most
+constexpr uint32_t kPlanParts = 64;       // parts of the buckets whose shares of the sample the plan looks at
+// Keys in buckets beyond the finish kernel, which go through bucket_rare_kernel at
+// about 27 us a million (100M keys, all of them in such buckets: 3.6 ms against
+// 1.66 by digits and 0.93 without): up to an eighth of the keys, what a bucket sort
+// gains over the digit passes (8.6 us a million) pays for several times over.
+constexpr uint32_t kOverShare = 8;
 constexpr uint32_t kBucketsMax = 32768;   // counters of the count kernel: 128 KB of shared memory
 constexpr uint32_t kBucketTarget = 3072;  // keys per bucket, at most, while more buckets can be had
 static_assert(kBucketMostKeys == (size_t)kBucketsMax * kBucketTarget, "the declared limit");
+constexpr uint32_t kFinishCap = 4096;     // keys of a bucket the finish kernel holds
 constexpr int kCellBits = 16, kBinBits = 12;
 constexpr uint32_t kCells = 1u << kCellBits;      // cells of the finish kernel's bitmap
 constexpr uint32_t kCountSpan = 1u << (kCellBits - 3);  // values a counted bucket may span
@@ -77,7 +84,15 @@ struct BucketArgs {
   uint32_t hot_above;   // sample keys above which a bucket looks too full
   uint32_t max_sample;  // sample keys no bucket may exceed
   uint32_t* err;
-  uint32_t* decided;    // where the plan tells the host whether the sort goes by buckets (may be null)
+  SortWords* words;     // where plan and count tell a host that waits (may be null)
+};
+
+// What plan and count turn a sort away for, besides.  (Not in BucketArgs: words
+// more there cost the partition passes 1 % at 100M keys.)
+struct BucketLimits {
+  uint32_t dense_above;  // sample keys above which a 64th of the buckets looks too full
+  uint32_t most_keys;   // keys no bucket may exceed
+  uint32_t most_over;   // keys that may lie in buckets beyond the finish kernel
 };
 
 // t: the key's distance from the bottom of the map, in 32 bits.
@@ -138,14 +153,14 @@ __device__ __forceinline__ size_t sample_place(uint32_t i, int log2, size_t n) {
 // first.
 template <typename K>
 __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
-    bucket_plan_kernel(const K* __restrict__ keys, size_t n, int is_float, BucketArgs a) {
+    bucket_plan_kernel(const K* __restrict__ keys, size_t n, int is_float, BucketArgs a, BucketLimits most) {
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ uint32_t s_hist[kBucketsMax / kPlanCtas];
   __shared__ K s_lo[32], s_hi[32];
   __shared__ K s_cta_lo[kPlanCtas], s_cta_hi[kPlanCtas];
   __shared__ uint32_t s_mult, s_s;
   __shared__ K s_base;
-  __shared__ uint32_t s_max[kPlanCtas], s_hot[kPlanCtas];
+  __shared__ uint32_t s_max[kPlanCtas], s_hot[kPlanCtas], s_dense;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t rank = cluster.block_rank();
   K k[kPlanPer];
@@ -158,6 +173,7 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
     hi = max(hi, k[j]);
   }
   for (uint32_t i = tid; i < a.nb / kPlanCtas; i += kPlanBlock) s_hist[i] = 0;
+  if (tid == 0) s_dense = 0;
   warp_minmax(lo, hi);
   if (lane == 0) {
     s_lo[warp] = lo;
@@ -219,6 +235,16 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
     }
   }
   cluster.sync();
+  // the keys of the sample in 64ths of the buckets that look fuller than the
+  // finish kernel holds on average: the sample tells a 64th's keys to a sixteenth,
+  // a bucket's not at all where there are more buckets than sample keys
+  if (warp < kPlanParts / kPlanCtas) {
+    const uint32_t part = a.nb / kPlanParts;
+    uint32_t c = 0;
+    for (uint32_t i = lane; i < part; i += 32) c += s_hist[warp * part + i];
+    c = __reduce_add_sync(kFull, c);
+    if (lane == 0 && c > most.dense_above) atomicAdd(cluster.map_shared_rank(&s_dense, 0), c);
+  }
   // the fullest bucket, and the keys of the sample in buckets that look fuller
   // than the finish kernel holds
   uint32_t mx = 0, hot = 0;
@@ -251,7 +277,7 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
       mx = max(mx, s_max[c]);
       hot += s_hot[c];
     }
-    bool fits = mx <= a.max_sample && hot <= kSample / 64;
+    bool fits = mx <= a.max_sample && hot <= kSample / 64 && s_dense <= kSample / kOverShare;
     BucketMap m{};
     m.plain = base == 0 && mult == a.nb && s == 8 * sizeof(K) - 32 ? 1u : 0u;
     m.mult = mult;
@@ -279,9 +305,9 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
       for (int p = 0; p < kMaxPasses; ++p) a.ctrl->pass[p].skip = 1;
       a.ctrl->final_in_tmp = 0;
     }
-    if (a.decided) {  // page-locked host memory the caller polls
+    if (a.words) {  // (the caller polls it)
       __threadfence_system();
-      *reinterpret_cast<volatile uint32_t*>(a.decided) = fits ? 1u : 0u;
+      *reinterpret_cast<volatile uint32_t*>(&a.words->decided) = fits ? 1u : 0u;
     }
   }
   // (last, so that no cluster barrier waits for these stores)
@@ -300,13 +326,14 @@ constexpr int kCountBlock = 1024;
 
 template <typename K, bool FLT>
 __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* __restrict__ keys, size_t n,
-                                                                      BucketArgs a) {
+                                                                      BucketArgs a, BucketLimits most) {
   extern __shared__ __align__(16) uint32_t s_cnt[];
   __shared__ uint32_t s_warp[kCountBlock / 32];
-  __shared__ uint32_t s_last;
+  __shared__ uint32_t s_last, s_over;
   constexpr int V = 16 / (int)sizeof(K);
   const uint32_t tid = threadIdx.x;
   for (uint32_t i = tid; i < a.nb; i += kCountBlock) s_cnt[i] = 0;
+  if (tid == 0) s_over = 0;
   chain_wait();
   chain_next();
   const BucketMap m = *a.map;
@@ -394,8 +421,8 @@ __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* _
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  // The last CTA: bucket starts, cursors of both passes, and the second
-  // pass's tiles per group (tile_first).
+  // The last CTA: whether the buckets fit after all, their starts, cursors of both
+  // passes, and the second pass's tiles per group (tile_first).
   const uint32_t per = max(1u, a.nb / kCountBlock);  // buckets per thread
   if (a.nb >= (uint32_t)kCountBlock) {
     for (uint32_t j = tid * 4; j < a.nb; j += kCountBlock * 4)
@@ -404,9 +431,23 @@ __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* _
     s_cnt[tid] = __ldcg(a.count + tid);
   }
   __syncthreads();
-  uint32_t local = 0;
+  uint32_t local = 0, over = 0;
+  bool large = false;
   if (tid * per < a.nb)
-    for (uint32_t j = 0; j < per; ++j) local += s_cnt[tid * per + ((j + tid) & (per - 1))];
+    for (uint32_t j = 0; j < per; ++j) {
+      const uint32_t c = s_cnt[tid * per + ((j + tid) & (per - 1))];
+      local += c;
+      over += c > kFinishCap ? c : 0u;
+      large |= c > most.most_keys;
+    }
+  if (over) atomicAdd(&s_over, over);
+  if (__syncthreads_or(large) || s_over > most.most_over) {
+    if (tid == 0) {
+      a.map->on = 0;  // (every other CTA is past its look at it; the launches behind find nothing to do)
+      if (a.words) *reinterpret_cast<volatile uint32_t*>(&a.words->again) = kAgainByDigits;
+    }
+    return;
+  }
   uint32_t run = os::block_exclusive_scan<kCountBlock>(local, s_warp);
   if (tid * per < a.nb) {
     for (uint32_t j = 0; j < per; ++j) {
@@ -676,7 +717,6 @@ __global__ void __launch_bounds__(kScatterBlock, kScatterPerSm) bucket_scatter_k
 constexpr int kFinishBlock = 256;
 template <typename K>
 constexpr int kFinishPerSm = sizeof(K) == 4 ? 4 : 2;
-constexpr uint32_t kFinishCap = 4096;
 constexpr uint32_t kEntryHits = 6;  // keys of one entry that found their cell taken, at most
 
 // The least t with umulhi(t, mult) >= b (b < nb), from the rounded-down
@@ -1449,9 +1489,20 @@ BucketArgs make_args(const BucketScratch& s, const K* tmp, size_t n, SortCtrl* c
   return a;
 }
 
+BucketLimits make_limits(uint32_t nb, size_t n) {
+  BucketLimits m{};
+  m.dense_above = (uint32_t)((double)kFinishCap * (nb / kPlanParts) * (double)kSample / (double)n);
+  // One CTA sorts such a bucket, at about 2 ns a key and byte; by then the count
+  // has been paid for, a fifteenth of the digit passes: n / 1024 keys, 0.6 ms at
+  // 100M, are still the shorter way, and where calls are short, 8192.
+  m.most_keys = (uint32_t)std::max<size_t>(2 * kFinishCap, n / 1024);
+  m.most_over = (uint32_t)(n / kOverShare);
+  return m;
+}
+
 template <typename K>
 cudaError_t plan_t(const BucketArgs& a, const K* keys, size_t n, bool is_float, cudaStream_t stream) {
-  bucket_plan_kernel<K><<<kPlanCtas, kPlanBlock, 0, stream>>>(keys, n, is_float ? 1 : 0, a);
+  bucket_plan_kernel<K><<<kPlanCtas, kPlanBlock, 0, stream>>>(keys, n, is_float ? 1 : 0, a, make_limits(a.nb, n));
   return cudaGetLastError();
 }
 
@@ -1463,7 +1514,7 @@ cudaError_t count_t(const BucketArgs& a, const K* keys, size_t n, cudaStream_t s
   if (e != cudaSuccess) return e;
   const size_t work = ceil_div(n, (size_t)kCountBlock * (16 / sizeof(K)) * 2);
   const size_t grid = std::min<size_t>(std::max<size_t>(work, 1), (size_t)device_info().sm_count);
-  return launch_chained(kern, (unsigned)grid, kCountBlock, smem, stream, keys, n, a);
+  return launch_chained(kern, (unsigned)grid, kCountBlock, smem, stream, keys, n, a, make_limits(a.nb, n));
 }
 
 template <typename K, bool FLT>
@@ -1967,16 +2018,16 @@ size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s) {
 }
 
 cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, const void* tmp, size_t n, int key_bytes,
-                                bool is_float, SortCtrl* ctrl, uint32_t* decided, cudaStream_t stream) {
+                                bool is_float, SortCtrl* ctrl, SortWords* words, cudaStream_t stream) {
   if (key_bytes == 8) {
     BucketArgs a = make_args(s, static_cast<const unsigned long long*>(tmp), n, ctrl, nullptr);
-    a.decided = decided;
+    a.words = words;
     const auto* k = static_cast<const unsigned long long*>(keys);
     const cudaError_t e = plan_t(a, k, n, false, stream);
     return e != cudaSuccess ? e : count_t<unsigned long long, false>(a, k, n, stream);
   }
   BucketArgs a = make_args(s, static_cast<const uint32_t*>(tmp), n, ctrl, nullptr);
-  a.decided = decided;
+  a.words = words;
   const auto* k = static_cast<const uint32_t*>(keys);
   const cudaError_t e = plan_t(a, k, n, is_float, stream);
   if (e != cudaSuccess) return e;

@@ -82,11 +82,14 @@ static_assert(kPipeChunks <= kMaxChunkRuns, "the bucket sort's chunk table holds
 constexpr int kPipeGroups = 10;  // host-buffer sort: bucket groups sorted and copied out in turn
 
 constexpr size_t kReadBackWords = 2048;  // the largest small result: 8 digits' 256 counts
+constexpr size_t kInplaceWaits = 1024;   // groups of an in-place sort that may go by buckets
 struct HostBlock {
   uint32_t err;       // error word of bounded waits, zero between calls
-  uint32_t decided;   // a bucket plan's decision
+  uint32_t decided;   // a select's: the result is written
+  SortWords sort;
   uint64_t result;    // a select's or sum's result
   uint64_t words[kReadBackWords];
+  SortWords groups[kInplaceWaits];
 };
 
 struct Workspace {
@@ -480,6 +483,8 @@ int pipelined_host_sort(Workspace* ws, cudaStream_t stream, void* keys, size_t n
   return PA_OK;
 }
 
+uint32_t sort_again(const SortWords& w) { return *const_cast<const volatile uint32_t*>(&w.again); }
+
 // phase_ms (optional, phase_cap entries): device time of each kernel of the
 // sort from CUDA events recorded between launches on the call's stream:
 // [0] digit histogram, [1] scan, [2 + p] digit pass p, [2 + passes] final
@@ -549,7 +554,7 @@ int sort_impl(void* keys, void* tmp, uint32_t* vals, uint32_t* tmp_vals, size_t 
     return cudaEventRecord(ws->ev[nev++], stream);
   };
   PA_CUDA(enqueue_sort(sc, d_keys, d_tmp, d_vals, d_tvals, n, kb, is_float, ws->err, stream, mark,
-                       sync_call ? &ws->host->decided : nullptr));
+                       sync_call ? &ws->host->sort : nullptr));
   auto copy_out = [&]() -> int {
     if (!keys_dev) PA_CUDA(cudaMemcpyAsync(keys, d_keys, key_bytes_total, cudaMemcpyDeviceToHost, stream));
     if (has_vals && !vals_dev)
@@ -558,10 +563,11 @@ int sort_impl(void* keys, void* tmp, uint32_t* vals, uint32_t* tmp_vals, size_t 
   };
   if (int rc = copy_out()) return rc;
   int rc = finish(ws, stream, !sync_call);
-  if (rc == PA_OK && sync_call && sc.window.state && ws->host->decided == kSortAgain) {
+  while (rc == PA_OK && sync_call && sort_again(ws->host->sort)) {  // (at most twice)
     sc.buckets = BucketScratch{};
-    sc.window = WindowScratch{};
-    PA_CUDA(enqueue_sort(sc, d_keys, d_tmp, d_vals, d_tvals, n, kb, is_float, ws->err, stream, {}, &ws->host->decided));
+    if (sort_again(ws->host->sort) == kAgainAllDigits) sc.window = WindowScratch{};
+    nev = 0;  // (the phases of the run that sorts)
+    PA_CUDA(enqueue_sort(sc, d_keys, d_tmp, d_vals, d_tvals, n, kb, is_float, ws->err, stream, mark, &ws->host->sort));
     if (int rc2 = copy_out()) return rc2;
     rc = finish(ws, stream, false);
   }
@@ -588,9 +594,10 @@ int sort_impl(void* keys, void* tmp, uint32_t* vals, uint32_t* tmp_vals, size_t 
 // partitioned again on the next digit.  A range whose keys all share the
 // digit is not moved.
 //
-// A call that waits (`decided`: its page-locked word) sorts up to S keys, and
+// A call that waits (`words`: kInplaceWaits of them) sorts up to S keys, and
 // groups whose digits are evenly filled, by buckets where the plan finds them
-// fit (pa_buckets.cu).  Calls on uniform keys, by digit passes
+// fit (pa_buckets.cu); `waits` lists their keys, in the order of the words, for
+// those that are to be sorted again once the stream is done.  Calls on uniform keys, by digit passes
 // alone and a longer host path -> now (us): 100M 3261 -> 2673, 30M 1043 -> 891;
 // 10M (within the scratch) 257 -> 155.
 constexpr size_t kInplaceDefaultScratch = (size_t)1 << 24;  // keys
@@ -599,7 +606,7 @@ constexpr size_t kInplaceBucketKeys = (size_t)1 << 19;  // (smaller groups do no
 
 int inplace_levels(Workspace* ws, cudaStream_t stream, uint32_t* a, size_t n, size_t S, uint32_t* buf,
                    InplaceState* st, void* status, unsigned long long* hist, char* plan_dev, size_t plan_cap,
-                   char* sort_base, uint32_t* decided) {
+                   char* sort_base, SortWords* words, std::vector<std::pair<uint32_t*, size_t>>* waits) {
   struct Range {
     size_t lo, len;
     uint32_t shift;
@@ -659,7 +666,8 @@ int inplace_levels(Workspace* ws, cudaStream_t stream, uint32_t* a, size_t n, si
     // sorted as one array).
     auto by_buckets = [&](const Group& gr) {
       const size_t len = (size_t)gr.off.back();
-      return decided && len >= kInplaceBucketKeys && bucket_sort_supported(len, 4) && gr.most * (size_t)(gr.last - gr.first + 1) * 4 <= len * 5;
+      return words && waits->size() + groups.size() <= kInplaceWaits && len >= kInplaceBucketKeys &&
+             bucket_sort_supported(len, 4) && gr.most * (size_t)(gr.last - gr.first + 1) * 4 <= len * 5;
     };
     for (size_t g = 0; g < groups.size(); ++g) {
       size_t bytes = 0;
@@ -692,7 +700,9 @@ int inplace_levels(Workspace* ws, cudaStream_t stream, uint32_t* a, size_t n, si
       } else {  // the group as one array: its buckets are already in order
         SortScratch sc{};
         sort_scratch_layout(sort_base, glen, 4, false, &sc);
-        PA_CUDA(enqueue_sort(sc, ga, buf, nullptr, nullptr, glen, 4, false, ws->err, stream, {}, decided));
+        SortWords* w = words && waits->size() < kInplaceWaits ? words + waits->size() : nullptr;
+        if (w) waits->push_back({ga, glen});
+        PA_CUDA(enqueue_sort(sc, ga, buf, nullptr, nullptr, glen, 4, false, ws->err, stream, {}, w));
       }
     }
   }
@@ -736,19 +746,38 @@ int inplace_impl(uint32_t* keys, size_t n, size_t scratch_keys, const pa_opts* o
   Carve real{ws->dev};
   layout(real);
   if (!keys_dev) PA_CUDA(cudaMemcpyAsync(d_keys, keys, n * sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
-  uint32_t* decided = opts && opts->async_device && keys_dev ? nullptr : &ws->host->decided;
+  const bool async = opts && opts->async_device && keys_dev;
+  SortWords* words = async ? nullptr : ws->host->groups;
+  std::vector<std::pair<uint32_t*, size_t>> waits;  // keys sorted with words[0], words[1], ...
   if (n <= S) {
     SortScratch sc{};
     sort_scratch_layout(sort_base, n, 4, false, &sc);
-    PA_CUDA(enqueue_sort(sc, d_keys, buf, nullptr, nullptr, n, 4, false, ws->err, stream, {}, decided));
+    if (words) waits.push_back({d_keys, n});
+    PA_CUDA(enqueue_sort(sc, d_keys, buf, nullptr, nullptr, n, 4, false, ws->err, stream, {}, words));
   } else if (int rc = inplace_levels(ws, stream, d_keys, n, S, buf, st, status, hist, plan_dev, plan_cap,
-                                     sort_base, decided)) {
+                                     sort_base, words, &waits)) {
     cudaStreamSynchronize(stream);
     cudaGetLastError();
     return rc;
   }
-  if (!keys_dev) PA_CUDA(cudaMemcpyAsync(keys, d_keys, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-  return finish(ws, stream, opts && opts->async_device && keys_dev);
+  auto copy_out = [&]() -> int {
+    if (!keys_dev) PA_CUDA(cudaMemcpyAsync(keys, d_keys, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
+    return PA_OK;
+  };
+  if (int rc = copy_out()) return rc;
+  int rc = finish(ws, stream, async);
+  bool again = false;
+  for (size_t w = 0; rc == PA_OK && w < waits.size(); ++w) {
+    if (!sort_again(words[w])) continue;
+    again = true;
+    SortScratch sc{};
+    sort_scratch_layout(sort_base, waits[w].second, 4, false, &sc);
+    sc.buckets = BucketScratch{};
+    PA_CUDA(enqueue_sort(sc, waits[w].first, buf, nullptr, nullptr, waits[w].second, 4, false, ws->err, stream));
+  }
+  if (!again) return rc;
+  if (int rc2 = copy_out()) return rc2;
+  return finish(ws, stream, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -967,12 +996,13 @@ cudaError_t wait_decided(const uint32_t* decided, cudaStream_t stream, uint32_t*
 
 cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32_t* d_vals, uint32_t* d_tvals,
                          size_t n, int kb, bool is_float, uint32_t* err, cudaStream_t stream,
-                         const std::function<cudaError_t()>& mark, uint32_t* decided) {
+                         const std::function<cudaError_t()>& mark, SortWords* words) {
   const int rb = s.radix_bits;
   const int passes = s.passes;
   const size_t bins = (size_t)1 << rb;
   const bool has_vals = d_vals != nullptr;
   auto m = [&]() { return mark ? mark() : cudaSuccess; };
+  if (words) *const_cast<volatile uint32_t*>(&words->again) = 0;
   if (n <= small_sort_max_keys(kb, has_vals)) {  // one CTA, one launch
     cudaError_t e = m();
     if (e == cudaSuccess)
@@ -985,29 +1015,28 @@ cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32
   const uint32_t* off = nullptr;
   // (float keys crowd into a few buckets of an even map: the plan would turn
   // nearly all of them away)
-  if (s.buckets.nb && !has_vals && !is_float && (decided || n >= (kb == 4 ? kBucketAsyncMin32 : kBucketAsyncMin64))) {
+  if (s.buckets.nb && !has_vals && !is_float && (words || n >= (kb == 4 ? kBucketAsyncMin32 : kBucketAsyncMin64))) {
     e = m();
-    if (decided) *reinterpret_cast<volatile uint32_t*>(decided) = kUndecided;
-    if (e == cudaSuccess) e = enqueue_bucket_plan(s.buckets, d_keys, d_tmp, n, kb, is_float, s.ctrl, decided, stream);
+    if (words) *const_cast<volatile uint32_t*>(&words->decided) = kUndecided;
+    if (e == cudaSuccess) e = enqueue_bucket_plan(s.buckets, d_keys, d_tmp, n, kb, is_float, s.ctrl, words, stream);
     uint32_t by_buckets = 1;
-    if (decided && e == cudaSuccess) e = wait_decided(decided, stream, &by_buckets);
+    if (words && e == cudaSuccess) e = wait_decided(&words->decided, stream, &by_buckets);
     if (by_buckets && e == cudaSuccess)
       e = enqueue_bucket_sort(s.buckets, d_keys, d_tmp, n, kb, is_float, s.ctrl, err, stream, mark);
-    if (decided && by_buckets) {
+    if (words && by_buckets) {
       for (int p = 3; p <= passes && e == cudaSuccess; ++p) e = m();  // (no LSD launches, no final copy)
       return e;
     }
     // decided here: the LSD passes alone; on the device: behind the bucket
     // sort, where they find `off` set and do nothing if it ran
-    off = decided ? nullptr : &s.buckets.map->on;
+    off = words ? nullptr : &s.buckets.map->on;
     if (e == cudaSuccess) e = launch_clear(s.zero_begin, s.zero_bytes, off, stream);
   } else {
     e = cudaMemsetAsync(s.zero_begin, 0, s.zero_bytes, stream);
     if (e == cudaSuccess) e = m();
   }
   auto lsd_mark = [&]() { return off ? cudaSuccess : m(); };
-  const bool window = s.window.state && decided && kb == 8 && rb == 8;
-  if (decided) *reinterpret_cast<volatile uint32_t*>(decided) = 0;  // (kSortAgain comes after the passes)
+  const bool window = s.window.state && words && kb == 8 && rb == 8;
   // With the tables (and 16-byte aligned keys) the histogram also prepares
   // the first pass's tile offsets.
   const bool prepared = s.tile_prefix && kb == 4 && rb == 8 && !has_vals && n < ((size_t)1 << 30) &&
@@ -1051,7 +1080,7 @@ cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32
   if (e == cudaSuccess) e = launch_final_copy(d_keys, d_tmp, d_vals, d_tvals, n, kb, s.ctrl, stream);
   if (e == cudaSuccess && window) {
     WindowScratch w = s.window;
-    w.fail = decided;
+    w.again = &words->again;
     e = enqueue_window_mend(w, d_keys, d_tmp, d_vals, d_tvals, n, stream);
   }
   if (e == cudaSuccess) e = m();

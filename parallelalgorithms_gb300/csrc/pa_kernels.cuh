@@ -198,6 +198,18 @@ cudaError_t launch_bucket_sort(const uint32_t* src, const ChunkRuns& chunks, con
 cudaError_t launch_final_copy(void* keys_a, const void* keys_b, uint32_t* vals_a, const uint32_t* vals_b,
                               size_t n, int key_bytes, const SortCtrl* ctrl, cudaStream_t stream);
 
+// Page-locked host memory that a caller of enqueue_sort which waits for its
+// stream lends to the sort; nothing else uses it meanwhile.
+struct SortWords {
+  uint32_t decided;  // whether the sort goes by buckets: the plan's answer, polled while the sort is enqueued
+  uint32_t again;    // once the stream is done: not zero if the sort has to be enqueued again (kAgain...)
+};
+// The bucket counts turned the keys away, nothing was moved: without s.buckets.
+constexpr uint32_t kAgainByDigits = 1;
+// A 64-bit sort by its leading digits was left unfinished, equal keys in their
+// order: without s.buckets and s.window.
+constexpr uint32_t kAgainAllDigits = 2;
+
 // ---- keys-only sorts by buckets (pa_buckets.cu) ----------------------------
 // Where a key goes: t = min(max(key - lo, 0) >> s, 2^32 - 1) and bucket =
 // min((t * mult) >> 32, nb - 1), written by the plan kernel.
@@ -235,10 +247,12 @@ size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s);
 // says "skip" for every LSD pass; and the count behind it, which runs while a
 // caller that waits for the decision learns it and enqueues the rest (1M uniform
 // 32-bit keys 75 -> 70 us a call, 600 K 62 -> 56; keys turned away find one more
-// launch that returns).  decided, when set, is page-locked host memory that
-// receives map->on as soon as it is known.
+// launch that returns).  The exact counts have the last word: where too many keys
+// are in buckets beyond the finish kernel, the count clears map->on, so that no key
+// is moved.  words, when set, receives map->on in `decided` as soon as the plan
+// knows it, and kAgainByDigits in `again` if the count says no after all.
 cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, const void* tmp, size_t n, int key_bytes,
-                                bool is_float, SortCtrl* ctrl, uint32_t* decided, cudaStream_t stream);
+                                bool is_float, SortCtrl* ctrl, SortWords* words, cudaStream_t stream);
 // Enqueues the planned sort (tmp: n keys of scratch; the result is in keys);
 // nothing is moved when map->on is 0.  `mark` runs at once (twice: the count has
 // been enqueued, and there is no scan launch), after each of the two partitions and after the
@@ -268,7 +282,7 @@ struct WindowScratch {
   uint32_t slots_log2 = 0;
   uint32_t* set = nullptr;       // long runs, by their first key
   uint32_t* run = nullptr;       // their first and end
-  uint32_t* fail = nullptr;      // page-locked word set to kSortAgain when the passes must all run after all
+  uint32_t* again = nullptr;     // page-locked word set to kAgainAllDigits when the passes must all run after all
 };
 bool window_sort_supported(size_t n, int key_bytes);
 // `skipped`: zeroed words of the lowest two passes, which are left out whenever
@@ -313,19 +327,15 @@ struct SortScratch {
 size_t sort_scratch_bytes(size_t n, int key_bytes, bool has_vals, int radix_bits = 8);
 // Carves the scratch from `base` (nullptr measures); returns its size.
 size_t sort_scratch_layout(char* base, size_t n, int key_bytes, bool has_vals, SortScratch* s, int radix_bits = 8);
-constexpr uint32_t kSortAgain = 2;  // (not a value of the bucket plan)
 // Enqueues the whole sort of device buffers on `stream` (the LSD chain: memset,
 // histogram, scan, passes, final copy; or by buckets, scratch and sizes
-// permitting); `mark`, when set, runs between launches.  decided (optional):
-// one word of page-locked host memory nothing else uses meanwhile; with it the
-// call waits for the bucket plan's decision and enqueues only what it takes,
-// without it (asynchronous callers) everything is enqueued and decides on the
-// device, which only large sorts do.  A 64-bit sort by its leading digits may
-// leave kSortAgain in *decided once the stream is done: the caller then enqueues
-// the sort again with s.buckets and s.window cleared.
+// permitting); `mark`, when set, runs between launches.  With words the call waits
+// for the bucket plan's decision and enqueues only what it takes, and the caller
+// looks at words->again once the stream is done; without (asynchronous callers)
+// everything is enqueued and decides on the device, which only large sorts do.
 cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32_t* d_vals, uint32_t* d_tvals,
                          size_t n, int key_bytes, bool is_float, uint32_t* err, cudaStream_t stream,
-                         const std::function<cudaError_t()>& mark = {}, uint32_t* decided = nullptr);
+                         const std::function<cudaError_t()>& mark = {}, SortWords* words = nullptr);
 
 // ---- sum (pa_sum.cu) -------------------------------------------------------
 // Element kinds of the sums (the values of pa_gpu.h's PA_ELEM_*).

@@ -197,9 +197,9 @@ __global__ void __launch_bounds__(kLongBlock) window_long_kernel(K* keys, K* tke
   const uint32_t shift = s.state->shift;
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
   if (shift == 0 || s.state->fail) {
-    if (shift && blockIdx.x == 0 && tid == 0 && s.fail) {
+    if (shift && blockIdx.x == 0 && tid == 0 && s.again) {
       __threadfence_system();
-      *reinterpret_cast<volatile uint32_t*>(s.fail) = kSortAgain;
+      *reinterpret_cast<volatile uint32_t*>(s.again) = kAgainAllDigits;
     }
     return;
   }
