@@ -1689,7 +1689,7 @@ __global__ void __launch_bounds__(kSegCountBlock, 3) seg_count_kernel(const Plan
 constexpr int kSegScanBlock = 256;
 __global__ void __launch_bounds__(kSegScanBlock) seg_jobs_kernel(const PlanDev P) {
   __shared__ uint32_t s_warp[kSegScanBlock / 32];
-  __shared__ uint32_t s_over, s_first, s_job0, s_tile0;
+  __shared__ uint32_t s_over, s_first, s_chunk, s_job0, s_tile0;
   const uint32_t L = blockIdx.x, tid = threadIdx.x;
   const uint32_t s = P.sb.of_large[L];
   bool off = s == 0xFFFFFFFFu;
@@ -1751,14 +1751,17 @@ __global__ void __launch_bounds__(kSegScanBlock) seg_jobs_kernel(const PlanDev P
     }
   }
   if (off) {
+    const uint32_t chunks = P.large[L].hist_chunks;
     if (tid == 0) {
+      s_chunk = atomicAdd(&P.declined[seg::kDeclinedChunks], chunks);
       P.declined[seg::kDeclinedHead + atomicAdd(&P.declined[seg::kDeclinedSegs], 1u)] = L;
       s_first = atomicAdd(&P.declined[seg::kDeclinedTiles], (P.large[L].len + seg::kPassTile - 1) / seg::kPassTile);
-      P.declined_first[L] = s_first;
     }
     __syncthreads();
     const uint32_t tiles = (P.large[L].len + seg::kPassTile - 1) / seg::kPassTile;
-    for (uint32_t t = tid; t < tiles; t += kSegScanBlock) P.declined_tile[s_first + t] = L;
+    for (uint32_t t = tid; t < tiles; t += kSegScanBlock)
+      P.declined_tile[s_first + t] = {P.large[L].base, P.large[L].len, L, s_first, {}};
+    for (uint32_t c = tid; c < chunks; c += kSegScanBlock) P.declined_chunk[s_chunk + c] = make_uint2(L, c);
   }
 }
 

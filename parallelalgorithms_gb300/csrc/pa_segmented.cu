@@ -237,46 +237,79 @@ __global__ void __launch_bounds__(kBlock, 2) segsort_kernel(const PlanDev P) {
 // HIST and SCAN item, so no item waits.
 using PassGeometry = Geometry<uint32_t, false, kPassBlock, kPassItems>;
 
+__device__ __forceinline__ void seg_pass_tile(const PlanDev& P, uint32_t pass, const DeclinedTile& t, uint32_t tile,
+                                              size_t words, unsigned char* smem, uint64_t* s_bar, uint32_t& parity) {
+  const bool even = (pass & 1u) == 0;
+  TileJob<uint32_t, uint32_t> job;
+  job.in = (even ? P.keys : P.tmp) + t.base;
+  job.out = (even ? P.tmp : P.keys) + t.base;
+  job.vin = nullptr;
+  job.vout = nullptr;
+  job.n = t.len;
+  job.out_n = t.len;
+  job.tile = tile;
+  job.shift = 8u * pass;
+  job.tin = false;
+  job.tout = false;
+  job.bin_start = P.bin_start + (size_t)t.seg * 4 * 256 + pass * 256;
+  job.status = P.pass_status + words * 256;
+  job.err = P.err;
+  job.spin_limit = kSpinLimit;
+  onesweep_tile_multisplit<uint32_t, false, kPassBlock, kPassItems, uint32_t>(job, smem, s_bar, parity);
+}
+
 __global__ void __launch_bounds__(kPassBlock, 3) seg_pass_kernel(const PlanDev P, uint32_t pass) {
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + PassGeometry::kBarOff);
   uint32_t* s_tile = reinterpret_cast<uint32_t*>(smem + PassGeometry::kTileIdOff);
-  // all large segments' tiles, or those of the segments the bucket sort declined
-  const uint32_t tiles = P.by_buckets ? P.declined[kDeclinedTiles] : P.pass_tiles;
+  if (threadIdx.x == 0) {
+    *s_tile = atomicAdd(P.pass_ticket + pass, 1u);
+    mbar_init(s_bar, 1);
+    mbar_fence_init();
+  }
+  __syncthreads();
+  const uint32_t g = *s_tile;
+  if (g >= P.pass_tiles) {  // a ticket counter that was not cleared
+    if (threadIdx.x == 0) raise_error(P.err, DEVERR_BAD_STATE);
+    return;
+  }
+  const uint32_t seg = P.tile_seg[g];
+  const LargeSeg L = P.large[seg];
+  uint32_t parity = 0;
+  seg_pass_tile(P, pass, {L.base, L.len, seg, L.ptile_base, {}}, g - L.ptile_base, L.ptile_base, smem, s_bar, parity);
+}
+
+// The same over the segments the bucket sort declined.  How many tiles they have
+// is known on the device alone, so resident CTAs take tickets until the tiles are
+// used up: a CTA for each tile there might be would cost evenly spread keys, which
+// leave nothing to the passes, 50 us a pass of 33 K tiles.  (The loop costs the
+// tiles 2 to 3 %: 300 segments of 1M keys.)
+__global__ void __launch_bounds__(kPassBlock, 3) declined_pass_kernel(const PlanDev P, uint32_t pass) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ DeclinedTile s_job;
+  uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + PassGeometry::kBarOff);
+  uint32_t* s_tile = reinterpret_cast<uint32_t*>(smem + PassGeometry::kTileIdOff);
+  const uint32_t tiles = P.declined[kDeclinedTiles];
   if (tiles == 0) return;
   if (threadIdx.x == 0) {
     mbar_init(s_bar, 1);
     mbar_fence_init();
   }
   uint32_t parity = 0;
-  for (;;) {  // resident CTAs take tickets until the tiles are used up
-    if (threadIdx.x == 0) *s_tile = atomicAdd(P.pass_ticket + pass, 1u);
+  for (;;) {
+    if (threadIdx.x == 0) {
+      const uint32_t g = atomicAdd(P.pass_ticket + pass, 1u);
+      *s_tile = g;
+      if (g < tiles) s_job = P.declined_tile[g];
+    }
     __syncthreads();
     const uint32_t g = *s_tile;
     if (g >= tiles) {
       if (g >= tiles + gridDim.x && threadIdx.x == 0) raise_error(P.err, DEVERR_BAD_STATE);  // a counter not cleared
       return;
     }
-    const uint32_t seg = P.by_buckets ? P.declined_tile[g] : P.tile_seg[g];
-    const LargeSeg L = P.large[seg];
-    const uint32_t first = P.by_buckets ? P.declined_first[seg] : L.ptile_base;
-    const bool even = (pass & 1u) == 0;
-    TileJob<uint32_t, uint32_t> job;
-    job.in = (even ? P.keys : P.tmp) + L.base;
-    job.out = (even ? P.tmp : P.keys) + L.base;
-    job.vin = nullptr;
-    job.vout = nullptr;
-    job.n = L.len;
-    job.out_n = L.len;
-    job.tile = g - first;
-    job.shift = 8u * pass;
-    job.tin = false;
-    job.tout = false;
-    job.bin_start = P.bin_start + (size_t)seg * 4 * 256 + pass * 256;
-    job.status = P.pass_status + ((size_t)first + (P.by_buckets && P.status_sets > 1 ? (size_t)pass * P.pass_tiles : 0)) * 256;
-    job.err = P.err;
-    job.spin_limit = kSpinLimit;
-    onesweep_tile_multisplit<uint32_t, false, kPassBlock, kPassItems, uint32_t>(job, smem, s_bar, parity);
+    seg_pass_tile(P, pass, s_job, g - s_job.first, (size_t)s_job.first + (P.status_sets > 1 ? (size_t)pass * P.pass_tiles : 0),
+                  smem, s_bar, parity);
     __syncthreads();
     // (a tile that gave up ends its CTA, as in the plain pass)
     if (*reinterpret_cast<uint32_t*>(smem + PassGeometry::kAbortOff)) return;
@@ -284,8 +317,9 @@ __global__ void __launch_bounds__(kPassBlock, 3) seg_pass_kernel(const PlanDev P
 }
 
 // The segments the bucket sort declined: their tiles' look-back words cleared
-// (sets: passes to clear for), their digit counts (each CTA takes every
-// gridDim.x-th chunk of each) and bin starts.
+// (sets: passes to clear for), their digit counts and bin starts.  The chunks to
+// be counted are one list over all of them: 2000 segments of 20 K keys, each
+// walked by every CTA, cost 0.6 ms of waiting for two loads a segment.
 __device__ __forceinline__ void clear_status(const PlanDev& P, uint32_t sets) {
   const size_t words = (size_t)P.declined[kDeclinedTiles] * 64;  // 16-byte words: 256 counters a tile
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -297,16 +331,13 @@ __device__ __forceinline__ void clear_status(const PlanDev& P, uint32_t sets) {
 
 __global__ void __launch_bounds__(kBlock, 2) declined_counts_kernel(const PlanDev P) {
   extern __shared__ __align__(128) unsigned char smem[];
-  const uint32_t num = P.declined[kDeclinedSegs];
+  const uint32_t num = P.declined[kDeclinedChunks];
   if (num == 0) return;
   clear_status(P, P.status_sets);
-  for (uint32_t d = 0; d < num; ++d) {
-    const uint32_t seg = P.declined[kDeclinedHead + d];
-    const uint32_t chunks = P.large[seg].hist_chunks;
-    for (uint32_t c = (blockIdx.x + d * 61u) % gridDim.x; c < chunks; c += gridDim.x) {
-      hist_item<8>(P, Item{ITEM_HIST, 0, seg, c}, smem);
-      __syncthreads();
-    }
+  for (uint32_t d = blockIdx.x; d < num; d += gridDim.x) {
+    const uint2 c = P.declined_chunk[d];
+    hist_item<8>(P, Item{ITEM_HIST, 0, c.x, c.y}, smem);
+    __syncthreads();
   }
 }
 
@@ -501,8 +532,8 @@ int build_host_plan(const uint64_t* off_host, size_t num_segments, const pa_segs
     hp->o_map = take(std::max<size_t>(hp->bsegs.size(), 1) * sizeof(SegMap));
     hp->o_bjob = take((size_t)std::max<uint32_t>(hp->buckets, 1) * sizeof(SegBucketJob));
     hp->o_tjob = take((size_t)std::max<uint32_t>(hp->part_tiles, 1) * sizeof(SegTileJob));
-    hp->o_dtile = take((size_t)std::max<uint32_t>(hp->pass_tiles, 1) * 4);
-    hp->o_dfirst = take(nl * 4);
+    hp->o_dtile = take((size_t)std::max<uint32_t>(hp->pass_tiles, 1) * sizeof(DeclinedTile));
+    hp->o_dchunk = take((size_t)std::max<uint32_t>(hp->hist_items, 1) * sizeof(uint2));
   }
   hp->bytes = o;
   return PA_OK;
@@ -535,8 +566,8 @@ PlanDev device_view(const HostPlan& hp, char* dev, uint32_t* keys, uint32_t* tmp
     d.status_sets = hp.status_sets;
     d.sb.whole = (uint32_t)hp.bjobs.size();
     d.declined = reinterpret_cast<uint32_t*>(dev + hp.o_decl);
-    d.declined_tile = reinterpret_cast<uint32_t*>(dev + hp.o_dtile);
-    d.declined_first = reinterpret_cast<uint32_t*>(dev + hp.o_dfirst);
+    d.declined_tile = reinterpret_cast<DeclinedTile*>(dev + hp.o_dtile);
+    d.declined_chunk = reinterpret_cast<uint2*>(dev + hp.o_dchunk);
     d.sb.rare = reinterpret_cast<uint32_t*>(dev + hp.o_rare);
     d.sb.num = (uint32_t)hp.bsegs.size();
     d.sb.buckets = hp.buckets;
@@ -591,7 +622,8 @@ cudaError_t upload_plan(const HostPlan& hp, char* dev, cudaStream_t s, void* pin
 
 unsigned plan_grid(const HostPlan& hp) {
   if (ensure_dynamic_smem(hp.kc.fn, hp.kc.smem) != cudaSuccess) cudaGetLastError();  // the launch reports it
-  if (hp.split && ensure_dynamic_smem(seg_pass_kernel, PassGeometry::kBytes) != cudaSuccess) cudaGetLastError();
+  if (hp.split && ensure_dynamic_smem(hp.by_buckets ? declined_pass_kernel : seg_pass_kernel, PassGeometry::kBytes) != cudaSuccess)
+    cudaGetLastError();
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hp.kc.fn, kBlock, hp.kc.smem) != cudaSuccess) {
     cudaGetLastError();
@@ -607,7 +639,6 @@ cudaError_t launch_plan(const HostPlan& hp, const PlanDev& pd, char* dev, unsign
   cudaError_t e = cudaMemsetAsync(dev + hp.o_head, 0, hp.o_pticket + 256 - hp.o_head, s);
   if (e != cudaSuccess) return e;
   const unsigned sms = (unsigned)device_info().sm_count;
-  const unsigned pass_grid = std::min<unsigned>(hp.pass_tiles, sms * 3);
   if (hp.by_buckets) {
     e = launch_seg_buckets(pd, hp.off.empty() ? 0 : (size_t)hp.off.back(), s);
     if (e != cudaSuccess || hp.pass_tiles == 0) return e;
@@ -616,12 +647,12 @@ cudaError_t launch_plan(const HostPlan& hp, const PlanDev& pd, char* dev, unsign
     const size_t hist_smem = (size_t)4 * 256 * hist_lanes<8>() * 4;
     declined_counts_kernel<<<sms * 2, kBlock, hist_smem, s>>>(pd);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    declined_scan_kernel<<<std::min<unsigned>(hp.num_large, sms), kBlock, 0, s>>>(pd);
+    declined_scan_kernel<<<std::min<unsigned>(hp.num_large, sms * 4), kBlock, 0, s>>>(pd);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     for (uint32_t p = 0; p < hp.passes && e == cudaSuccess; ++p) {
       if (p > 0 && hp.status_sets == 1) declined_clear_kernel<<<sms * 4, 256, 0, s>>>(pd);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
-      seg_pass_kernel<<<pass_grid, kPassBlock, PassGeometry::kBytes, s>>>(pd, p);
+      declined_pass_kernel<<<std::min<unsigned>(hp.pass_tiles, sms * 3), kPassBlock, PassGeometry::kBytes, s>>>(pd, p);
       e = cudaGetLastError();
     }
     return e;
@@ -634,7 +665,7 @@ cudaError_t launch_plan(const HostPlan& hp, const PlanDev& pd, char* dev, unsign
   for (uint32_t p = 0; p < hp.passes && e == cudaSuccess; ++p) {
     e = cudaMemsetAsync(dev + hp.o_pstatus, 0, (size_t)hp.pass_tiles * 256 * 4, s);
     if (e == cudaSuccess) {
-      seg_pass_kernel<<<pass_grid, kPassBlock, PassGeometry::kBytes, s>>>(pd, p);
+      seg_pass_kernel<<<hp.pass_tiles, kPassBlock, PassGeometry::kBytes, s>>>(pd, p);
       e = cudaGetLastError();
     }
   }

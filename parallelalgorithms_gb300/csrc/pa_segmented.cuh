@@ -82,10 +82,28 @@ struct __align__(16) SegBucketJob {
   uint32_t edge;
   uint32_t cell_shift, pad;
 };
-// Words of PlanDev::declined, zeroed per run: declined segments and their pass
-// tiles; jobs of the others' buckets (behind the whole segments') and tiles; jobs
-// of counted buckets (from the job array's end on); then the declined segments.
-enum : uint32_t { kDeclinedSegs = 0, kDeclinedTiles = 1, kJobBuckets = 2, kJobTiles = 3, kJobCounted = 4, kDeclinedHead = 5 };
+// A pass tile of a declined segment: all a pass needs to know, so that a CTA waits
+// for one load between its ticket and its keys.
+struct __align__(16) DeclinedTile {
+  unsigned long long base;  // first key of its segment
+  uint32_t len;             // keys of its segment
+  uint32_t seg;             // its LargeSeg
+  uint32_t first;           // the segment's first tile among the declined ones'
+  uint32_t pad[3];
+};
+// Words of PlanDev::declined, zeroed per run: declined segments, their pass tiles
+// and their count chunks; jobs of the others' buckets (behind the whole segments')
+// and tiles; jobs of counted buckets (from the job array's end on); then the
+// declined segments.
+enum : uint32_t {
+  kDeclinedSegs = 0,
+  kDeclinedTiles = 1,
+  kJobBuckets = 2,
+  kJobTiles = 3,
+  kJobCounted = 4,
+  kDeclinedChunks = 5,
+  kDeclinedHead = 6
+};
 struct SegBucketsDev {
   uint32_t num;                 // segments of several buckets
   uint32_t whole;               // segments that are one bucket: the first jobs, uploaded with the plan
@@ -137,8 +155,8 @@ struct PlanDev {
   uint32_t num_large;
   uint32_t* declined;              // [kDeclinedHead + large]
   uint32_t status_sets;            // look-back words for that many passes (one: cleared between passes)
-  uint32_t* declined_tile;         // [pass_tiles] segment of each of their tiles
-  uint32_t* declined_first;        // [large] a segment's first tile among them
+  DeclinedTile* declined_tile;     // [pass_tiles]
+  uint2* declined_chunk;           // [count chunks] segment and chunk of each to be counted
   SegBucketsDev sb;
 };
 
@@ -178,7 +196,7 @@ struct HostPlan {
   std::vector<SegBucketJob> bjobs;
   uint32_t hist_items = 0, buckets = 0, part_tiles = 0, status_sets = 1;
   size_t o_bseg = 0, o_of_large = 0, o_bjob = 0, o_map = 0, o_count = 0, o_tjob = 0, o_decl = 0, o_rare = 0, o_dtile = 0,
-         o_dfirst = 0;
+         o_dchunk = 0;
   size_t o_items = 0, o_off = 0, o_large = 0, o_tile_seg = 0, o_bins = 0, o_err = 0, o_head = 0, o_done = 0,
          o_hist = 0, o_status = 0, o_pticket = 0, o_pstatus = 0, bytes = 0;
 };
