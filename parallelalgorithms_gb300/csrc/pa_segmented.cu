@@ -686,7 +686,7 @@ struct pa_segsort_plan {
   unsigned grid = 0;
   char* dev = nullptr;
   PlanDev pd{};
-  uint32_t* err_host = nullptr;
+  uint32_t* err_host = nullptr;  // page-locked, the device's error word: read without a copy when the stream is done
   cudaStream_t cap_stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -780,6 +780,8 @@ int pa_segsort_plan_create(const uint64_t* seg_offsets, size_t num_segments, con
   }
   p->grid = plan_grid(p->hp);
   p->pd = device_view(p->hp, p->dev, nullptr, nullptr);
+  *p->err_host = 0;
+  p->pd.err = p->err_host;
   *out = p;
   return PA_OK;
 }
@@ -828,11 +830,9 @@ int pa_segsort_plan_run(pa_segsort_plan* p, uint32_t* keys, uint32_t* tmp, const
 int pa_segsort_plan_sync(pa_segsort_plan* p, void* stream) {
   if (!p) return record_error(PA_ERR_ARG, "plan is NULL");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  PA_SEG_CUDA(cudaMemcpyAsync(p->err_host, p->pd.err, 4, cudaMemcpyDeviceToHost, s));
   PA_SEG_CUDA(cudaStreamSynchronize(s));
-  if (*p->err_host) {
-    PA_SEG_CUDA(cudaMemsetAsync(p->pd.err, 0, 4, s));
-    PA_SEG_CUDA(cudaStreamSynchronize(s));
+  if (*const_cast<volatile uint32_t*>(p->err_host)) {
+    *const_cast<volatile uint32_t*>(p->err_host) = 0;
     return record_error(PA_ERR_TIMEOUT, "a bounded device-side wait of the batched sort gave up");
   }
   return PA_OK;
