@@ -2051,7 +2051,7 @@ cudaError_t enqueue_bucket_sort(const BucketScratch& s, void* keys, void* tmp, s
 
 namespace seg {
 
-cudaError_t launch_seg_buckets(const PlanDev& pd, size_t total_keys, cudaStream_t s) {
+cudaError_t launch_seg_plan(const PlanDev& pd, cudaStream_t s) {
   const unsigned sms = (unsigned)device_info().sm_count;
   cudaError_t e = cudaSuccess;
   if (pd.sb.num) {
@@ -2062,8 +2062,14 @@ cudaError_t launch_seg_buckets(const PlanDev& pd, size_t total_keys, cudaStream_
   }
   if (pd.num_large) {
     seg_jobs_kernel<<<pd.num_large, kSegScanBlock, 0, s>>>(pd);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = cudaGetLastError();
   }
+  return e;
+}
+
+cudaError_t launch_seg_buckets(const PlanDev& pd, size_t total_keys, cudaStream_t s) {
+  const unsigned sms = (unsigned)device_info().sm_count;
+  cudaError_t e = cudaSuccess;
   if (pd.sb.tiles) {
     if ((e = ensure_dynamic_smem(seg_scatter_kernel, sizeof(SegScatterSmem))) != cudaSuccess) return e;
     seg_scatter_kernel<<<std::min(pd.sb.tiles, sms * kScatterPerSm), kScatterBlock, sizeof(SegScatterSmem), s>>>(pd);

@@ -3,12 +3,12 @@
 //
 // Public plans with 8-bit digits sort by buckets (launch_seg_buckets,
 // pa_buckets.cu); only the segments that declines go through the digit passes
-// here (declined_*_kernel, seg_pass_kernel over a list made on the device).  4096
-// arrays of 1 K to 4 M uniform keys, 2.0 G keys: 15.9 ms against 36.0 with four
-// digit passes; 64 arrays of 1 K to 50 K keys 39 us against 58.  Skewed keys pay
-// for the maps and counts they are declined on (the 2.0 G keys skewed: 37.9 ms
-// against 36.1; 300 arrays of up to 1 M keys 1.01 ms against 0.86; the 64 small
-// arrays 97 us against 58, most of it launches).
+// here (declined_*_kernel, over lists made on the device).  A run that waits, by
+// four digit passes alone -> now (us): 4096 arrays of 1 K to 4 M uniform keys, 2.0 G
+// keys, 36040 -> 15800; 300 of 1 K to 1 M 894 -> 379; 64 of 1 K to 50 K 89 -> 60.
+// Skewed keys pay for the maps and counts they are declined on: 1000 arrays of 1 M
+// 16370 -> 17080, 2000 of 20 K 857 -> 903, 300 of 1 K to 1 M 907 -> 927, 64 of 1 K to
+// 50 K 89 -> 93, 64 of 3000 42 -> 40.
 //
 // 11-bit plans, and the plans other sorts build for their groups, run ONE
 // persistent kernel fed by a device work queue (8-bit ones then a launch per
@@ -282,8 +282,9 @@ __global__ void __launch_bounds__(kPassBlock, 3) seg_pass_kernel(const PlanDev P
 // The same over the segments the bucket sort declined.  How many tiles they have
 // is known on the device alone, so resident CTAs take tickets until the tiles are
 // used up: a CTA for each tile there might be would cost evenly spread keys, which
-// leave nothing to the passes, 50 us a pass of 33 K tiles.  (The loop costs the
-// tiles 2 to 3 %: 300 segments of 1M keys.)
+// leave nothing to the passes, 50 us a pass of 33 K tiles.  (The loop costs tiles
+// of long segments 3 %: 300 of 1M keys 1123 to 1185 us a pass against 1088 to 1148;
+// a tile's code called instead of inlined 1165 to 1240.)
 __global__ void __launch_bounds__(kPassBlock, 3) declined_pass_kernel(const PlanDev P, uint32_t pass) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ DeclinedTile s_job;
@@ -635,26 +636,57 @@ unsigned plan_grid(const HostPlan& hp) {
   return grid;
 }
 
-cudaError_t launch_plan(const HostPlan& hp, const PlanDev& pd, char* dev, unsigned grid, cudaStream_t s) {
+namespace {
+
+// Keys of a batch whose declined segments get a stream of their own: above,
+// launches are long and nothing is gained.
+constexpr size_t kForkMostKeys = (size_t)1 << 27;
+
+// The declined segments' digit passes (launches that return at once when there
+// are none).
+cudaError_t launch_declined(const HostPlan& hp, const PlanDev& pd, cudaStream_t s) {
+  const unsigned sms = (unsigned)device_info().sm_count;
+  const size_t hist_smem = (size_t)4 * 256 * hist_lanes<8>() * 4;
+  declined_counts_kernel<<<sms * 2, kBlock, hist_smem, s>>>(pd);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  declined_scan_kernel<<<std::min<unsigned>(hp.num_large, sms * 4), kBlock, 0, s>>>(pd);
+  e = cudaGetLastError();
+  for (uint32_t p = 0; p < hp.passes && e == cudaSuccess; ++p) {
+    if (p > 0 && hp.status_sets == 1) declined_clear_kernel<<<sms * 4, 256, 0, s>>>(pd);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    declined_pass_kernel<<<std::min<unsigned>(hp.pass_tiles, sms * 3), kPassBlock, PassGeometry::kBytes, s>>>(pd, p);
+    e = cudaGetLastError();
+  }
+  return e;
+}
+
+}  // namespace
+
+cudaError_t launch_plan(const HostPlan& hp, const PlanDev& pd, char* dev, unsigned grid, cudaStream_t s,
+                        const PlanFork* fork) {
   cudaError_t e = cudaMemsetAsync(dev + hp.o_head, 0, hp.o_pticket + 256 - hp.o_head, s);
   if (e != cudaSuccess) return e;
-  const unsigned sms = (unsigned)device_info().sm_count;
   if (hp.by_buckets) {
-    e = launch_seg_buckets(pd, hp.off.empty() ? 0 : (size_t)hp.off.back(), s);
-    if (e != cudaSuccess || hp.pass_tiles == 0) return e;
-    // the declined segments' digit passes (launches that return at once when
-    // there are none)
-    const size_t hist_smem = (size_t)4 * 256 * hist_lanes<8>() * 4;
-    declined_counts_kernel<<<sms * 2, kBlock, hist_smem, s>>>(pd);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    declined_scan_kernel<<<std::min<unsigned>(hp.num_large, sms * 4), kBlock, 0, s>>>(pd);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    for (uint32_t p = 0; p < hp.passes && e == cudaSuccess; ++p) {
-      if (p > 0 && hp.status_sets == 1) declined_clear_kernel<<<sms * 4, 256, 0, s>>>(pd);
-      if ((e = cudaGetLastError()) != cudaSuccess) return e;
-      declined_pass_kernel<<<std::min<unsigned>(hp.pass_tiles, sms * 3), kPassBlock, PassGeometry::kBytes, s>>>(pd, p);
-      e = cudaGetLastError();
+    const size_t total = hp.off.empty() ? 0 : (size_t)hp.off.back();
+    if ((e = launch_seg_plan(pd, s)) != cudaSuccess) return e;
+    if (hp.pass_tiles == 0) return launch_seg_buckets(pd, total, s);
+    if (!fork || total > kForkMostKeys) {
+      e = launch_seg_buckets(pd, total, s);
+      return e != cudaSuccess ? e : launch_declined(hp, pd, s);
     }
+    // From here on the two kinds of segments share neither keys nor tables, and in
+    // small batches each launch is mostly latency: side by side.  (us a run, one
+    // behind the other -> beside: 64 arrays of 1 K to 50 K skewed keys 122 -> 94, 300
+    // of 1 K to 1 M 950 -> 925, uniform 379 -> 379; 1000 of 1 M 17.1 ms both ways.)
+    if ((e = cudaEventRecord(fork->leave, s)) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(fork->side, fork->leave, 0)) != cudaSuccess) return e;
+    e = launch_declined(hp, pd, fork->side);
+    const cudaError_t e2 = launch_seg_buckets(pd, total, s);
+    // (always back, so that nothing outlives the call's place in its stream)
+    const cudaError_t e3 = cudaEventRecord(fork->back, fork->side), e4 = cudaStreamWaitEvent(s, fork->back, 0);
+    for (const cudaError_t x : {e2, e3, e4})
+      if (e == cudaSuccess) e = x;
     return e;
   }
   if (!hp.items.empty()) {
@@ -688,6 +720,7 @@ struct pa_segsort_plan {
   PlanDev pd{};
   uint32_t* err_host = nullptr;  // page-locked, the device's error word: read without a copy when the stream is done
   cudaStream_t cap_stream = nullptr;
+  PlanFork fork;  // (plans by buckets with segments that may be declined)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   uint32_t* g_keys = nullptr;
@@ -729,7 +762,7 @@ void destroy_graph(pa_segsort_plan* p) {
 }
 
 int enqueue(pa_segsort_plan* p, cudaStream_t s) {
-  PA_SEG_CUDA(launch_plan(p->hp, p->pd, p->dev, p->grid, s));
+  PA_SEG_CUDA(launch_plan(p->hp, p->pd, p->dev, p->grid, s, p->fork.back ? &p->fork : nullptr));
   // an odd number of passes (11-bit digits: three) leaves every segment in tmp
   if (p->hp.passes & 1u)
     PA_SEG_CUDA(cudaMemcpyAsync(p->pd.keys, p->pd.tmp, (size_t)p->total_keys * 4, cudaMemcpyDeviceToDevice, s));
@@ -774,6 +807,11 @@ int pa_segsort_plan_create(const uint64_t* seg_offsets, size_t num_segments, con
   if (e == cudaSuccess) e = upload_plan(p->hp, p->dev, (cudaStream_t)0);
   if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)0);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking);
+  if (p->hp.by_buckets && p->hp.pass_tiles) {
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->fork.side, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->fork.leave, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->fork.back, cudaEventDisableTiming);
+  }
   if (e != cudaSuccess) {
     pa_segsort_plan_destroy(p);
     return cfail(e, "plan set-up");
@@ -842,6 +880,9 @@ int pa_segsort_plan_destroy(pa_segsort_plan* p) {
   if (!p) return PA_OK;
   destroy_graph(p);
   if (p->cap_stream) cudaStreamDestroy(p->cap_stream);
+  if (p->fork.side) cudaStreamDestroy(p->fork.side);
+  if (p->fork.leave) cudaEventDestroy(p->fork.leave);
+  if (p->fork.back) cudaEventDestroy(p->fork.back);
   if (p->dev) cudaFree(p->dev);
   if (p->err_host) cudaFreeHost(p->err_host);
   delete p;

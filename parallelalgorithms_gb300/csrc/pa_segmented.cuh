@@ -147,7 +147,7 @@ struct PlanDev {
   // pass launches (8-bit plans)
   const uint32_t* tile_seg;        // [pass_tiles] large segment of each tile
   uint32_t pass_tiles;
-  uint32_t* pass_ticket;           // zeroed before each pass
+  uint32_t* pass_ticket;           // one per pass, zeroed per run
   uint32_t* pass_status;           // [pass_tiles][256], zeroed before each pass
   // Plans that sort by buckets: the digit passes' segments are listed on the
   // device (`by_buckets` not zero).
@@ -210,8 +210,10 @@ struct HostPlan {
 // device memory: 64 bytes a bucket and 32 a tile).
 int build_host_plan(const uint64_t* off_host, size_t num_segments, const pa_segsort_config* cfg, HostPlan* hp,
                     int passes = kPasses, bool by_buckets = false);
-// The bucket part of a run (pa_buckets.cu): maps, counts, partition and the
-// sort of every bucket; segments it declines are listed in pd.declined.
+// The bucket part of a run (pa_buckets.cu): maps and counts, with which every
+// segment is either given buckets or listed in pd.declined; then the partition and
+// the sort of every bucket.
+cudaError_t launch_seg_plan(const PlanDev& pd, cudaStream_t s);
 cudaError_t launch_seg_buckets(const PlanDev& pd, size_t total_keys, cudaStream_t s);
 // Pointers of a device block laid out by `hp` (keys / tmp: the batch's keys).
 PlanDev device_view(const HostPlan& hp, char* dev, uint32_t* keys, uint32_t* tmp);
@@ -228,9 +230,16 @@ cudaError_t upload_plan(const HostPlan& hp, char* dev, cudaStream_t s, void* pin
 size_t plan_image_bytes(const HostPlan& hp);
 // Persistent grid for the plan's kernel on the current device.
 unsigned plan_grid(const HostPlan& hp);
+// A second stream, and events to leave for it and to come back.
+struct PlanFork {
+  cudaStream_t side = nullptr;
+  cudaEvent_t leave = nullptr, back = nullptr;
+};
 // Clears the per-run state and launches the persistent kernel (and, for an
-// 8-bit plan, the pass launches after it).
-cudaError_t launch_plan(const HostPlan& hp, const PlanDev& pd, char* dev, unsigned grid, cudaStream_t s);
+// 8-bit plan, the pass launches after it); or a plan by buckets, with `fork` the
+// segments it declined beside the others.
+cudaError_t launch_plan(const HostPlan& hp, const PlanDev& pd, char* dev, unsigned grid, cudaStream_t s,
+                        const PlanFork* fork = nullptr);
 
 }  // namespace seg
 }  // namespace pa
