@@ -153,7 +153,7 @@ __device__ __forceinline__ size_t sample_place(uint32_t i, int log2, size_t n) {
 // first.
 template <typename K>
 __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
-    bucket_plan_kernel(const K* __restrict__ keys, size_t n, int is_float, BucketArgs a, BucketLimits most) {
+    bucket_plan_kernel(const K* __restrict__ keys, size_t n, BucketArgs a, BucketLimits most) {
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ uint32_t s_hist[kBucketsMax / kPlanCtas];
   __shared__ K s_lo[32], s_hi[32];
@@ -168,7 +168,7 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
 #pragma unroll
   for (int j = 0; j < kPlanPer; ++j) {
     const uint32_t i = ((uint32_t)j * kPlanCtas + rank) * kPlanBlock + tid;
-    k[j] = to_ordered(keys[sample_place(i, kSampleLog2, n)], is_float != 0);
+    k[j] = keys[sample_place(i, kSampleLog2, n)];
     lo = min(lo, k[j]);
     hi = max(hi, k[j]);
   }
@@ -324,7 +324,7 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
 // its tile tables: 0.113 ms).
 constexpr int kCountBlock = 1024;
 
-template <typename K, bool FLT>
+template <typename K>
 __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* __restrict__ keys, size_t n,
                                                                       BucketArgs a, BucketLimits most) {
   extern __shared__ __align__(16) uint32_t s_cnt[];
@@ -344,8 +344,7 @@ __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* _
     constexpr bool PLAIN = decltype(plainc)::value;
     const K lo = (K)m.lo;
     const uint32_t shift = 32u - a.nb_bits;
-    auto bucket = [&](K raw) {
-      const K key = to_ordered(raw, FLT);
+    auto bucket = [&](K key) {
       if constexpr (PLAIN) return top_word(key) >> shift;
       else return map_bucket(map_t<K>(key, lo, m.s), m.mult, last);
     };
@@ -502,7 +501,7 @@ template <typename K>
 constexpr uint32_t kScatterTile = (uint32_t)kScatterBlock * kScatterItems<K>;
 
 // PLAIN: the map is the key's top bits (BucketMap::plain).
-template <typename K, bool GROUPED, bool FLT, bool PLAIN>
+template <typename K, bool GROUPED, bool PLAIN>
 __device__ __forceinline__ void scatter_tiles(const K* in, K* out, uint32_t n, const BucketArgs& a, const BucketMap& m,
                                               K* s_keys, uint32_t* s_cnt, uint32_t* s_start, uint32_t* s_base,
                                               uint32_t* s_warp, uint32_t* s_one, const uint32_t* s_first) {
@@ -573,10 +572,6 @@ __device__ __forceinline__ void scatter_tiles(const K* in, K* out, uint32_t n, c
   for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     if (tid < kGroups) s_cnt[tid] = 0;
     if (tid == 0) *s_one = 0;
-    if constexpr (FLT) {
-#pragma unroll
-      for (int j = 0; j < ITEMS; ++j) k[j] = to_ordered(k[j], true);
-    }
     __syncthreads();
     uint32_t r[(ITEMS + 1) / 2];  // ranks in the tile's bins, two 16-bit halves per word
 #pragma unroll
@@ -671,7 +666,7 @@ __device__ __forceinline__ void scatter_tiles(const K* in, K* out, uint32_t n, c
   }
 }
 
-template <typename K, bool GROUPED, bool FLT>
+template <typename K, bool GROUPED>
 __global__ void __launch_bounds__(kScatterBlock, kScatterPerSm) bucket_scatter_kernel(const K* in, K* out, size_t n, BucketArgs a) {
   __shared__ __align__(16) K s_keys[kScatterTile<K>];
   __shared__ uint32_t s_cnt[kGroups], s_start[kGroups], s_base[kGroups];
@@ -687,9 +682,9 @@ __global__ void __launch_bounds__(kScatterBlock, kScatterPerSm) bucket_scatter_k
     __syncthreads();
   }
   if (m.plain)
-    scatter_tiles<K, GROUPED, FLT, true>(in, out, (uint32_t)n, a, m, s_keys, s_cnt, s_start, s_base, s_warp, &s_one, s_first);
+    scatter_tiles<K, GROUPED, true>(in, out, (uint32_t)n, a, m, s_keys, s_cnt, s_start, s_base, s_warp, &s_one, s_first);
   else
-    scatter_tiles<K, GROUPED, FLT, false>(in, out, (uint32_t)n, a, m, s_keys, s_cnt, s_start, s_base, s_warp, &s_one, s_first);
+    scatter_tiles<K, GROUPED, false>(in, out, (uint32_t)n, a, m, s_keys, s_cnt, s_start, s_base, s_warp, &s_one, s_first);
 }
 
 // ---------------------------------------------------------------------------
@@ -1250,7 +1245,7 @@ __device__ void finish_slow(K* a, K* b, uint32_t m, bool into_a, unsigned char* 
 
 // A bucket of at most CAP keys that span fewer than kBucketBins values from
 // `first` on: counted per value, and placed from each value's end down.
-template <typename K, bool FLT>
+template <typename K>
 __device__ void finish_counted(const K* in, K* out, uint32_t cnt, K first, unsigned char* smem, uint32_t* s_warp) {
   constexpr int B = kRareBlock;
   constexpr int PER = (int)kBucketBins / B;  // values per thread in the scan
@@ -1292,7 +1287,7 @@ __device__ void finish_counted(const K* in, K* out, uint32_t cnt, K first, unsig
     s_keys[(atomicSub(s_bin + bin_at(bin_of(key)), 1u) - 1u) & (kFinishCap - 1)] = key;
   }
   __syncthreads();  // (every key of `in` has been read)
-  for (uint32_t i = tid; i < cnt; i += B) out[i] = from_ordered(s_keys[i], FLT);
+  for (uint32_t i = tid; i < cnt; i += B) out[i] = s_keys[i];
 }
 
 // A bucket of at most CAP keys, crowded (many keys equal or nearly so): stable
@@ -1316,13 +1311,13 @@ __device__ void finish_nibbles(const K* in, K* out, uint32_t cnt, K diff, unsign
 }
 
 // job_of(b): bucket b's job.
-template <typename K, bool FLT, typename JobOf>
+template <typename K, typename JobOf>
 __device__ __forceinline__ void rare_buckets(const uint32_t* rare, JobOf&& job_of) {
   constexpr int W = kRareBlock / 32;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint32_t s_warp[W];
   __shared__ K s_edge[2 * W];
-  const uint32_t num = rare[0], tid = threadIdx.x;
+  const uint32_t num = rare[0];
   for (uint32_t i = blockIdx.x; i < num; i += gridDim.x) {
     FinishJob<K> job{};
     job_of(rare[1 + i], job);
@@ -1330,13 +1325,11 @@ __device__ __forceinline__ void rare_buckets(const uint32_t* rare, JobOf&& job_o
       K lo, hi;
       block_minmax<K, kRareBlock>(job.src, job.cnt, false, s_edge, lo, hi);
       if (hi - lo < (K)kBucketBins)
-        finish_counted<K, FLT>(job.src, job.dst, job.cnt, lo, smem, s_warp);
+        finish_counted<K>(job.src, job.dst, job.cnt, lo, smem, s_warp);
       else
-        finish_nibbles<K, FLT>(job.src, job.dst, job.cnt, lo ^ hi, smem, s_warp);
+        finish_nibbles<K, false>(job.src, job.dst, job.cnt, lo ^ hi, smem, s_warp);
     } else {
       finish_slow<K>(job.src, job.other, job.cnt, job.src == job.dst, smem);
-      if (FLT)
-        for (uint32_t j = tid; j < job.cnt; j += kRareBlock) job.dst[j] = from_ordered(job.dst[j], true);
     }
     __syncthreads();
   }
@@ -1367,7 +1360,7 @@ __device__ __forceinline__ void plain_job(const BucketArgs& a, const BucketMap& 
   job.number = b;
 }
 
-template <typename K, bool FLT>
+template <typename K>
 __global__ void __launch_bounds__(kFinishBlock, kFinishPerSm<K>)
     bucket_finish_kernel(K* in, K* out, K* other, size_t n, BucketArgs a) {
   chain_wait();
@@ -1388,17 +1381,17 @@ __global__ void __launch_bounds__(kFinishBlock, kFinishPerSm<K>)
     }
   };
   if (m.counts)
-    finish_buckets<K, FLT, kFinishBlock, kFinishCap, kCellBits, false, true>(a.nb, a.rare, a.err, next);
+    finish_buckets<K, false, kFinishBlock, kFinishCap, kCellBits, false, true>(a.nb, a.rare, a.err, next);
   else
-    finish_buckets<K, FLT>(a.nb, a.rare, a.err, next);
+    finish_buckets<K, false>(a.nb, a.rare, a.err, next);
 }
 
-template <typename K, bool FLT>
+template <typename K>
 __global__ void __launch_bounds__(kRareBlock) bucket_rare_kernel(K* in, K* out, K* other, size_t n, BucketArgs a) {
   chain_wait();
   const BucketMap m = *a.map;
   if (!m.on) return;
-  rare_buckets<K, FLT>(a.rare, [&](uint32_t b, FinishJob<K>& job) {
+  rare_buckets<K>(a.rare, [&](uint32_t b, FinishJob<K>& job) {
     plain_job<K>(a, m, b, a.start[b], a.start[b + 1], in, out, other, n, job);
   });
 }
@@ -1501,14 +1494,14 @@ BucketLimits make_limits(uint32_t nb, size_t n) {
 }
 
 template <typename K>
-cudaError_t plan_t(const BucketArgs& a, const K* keys, size_t n, bool is_float, cudaStream_t stream) {
-  bucket_plan_kernel<K><<<kPlanCtas, kPlanBlock, 0, stream>>>(keys, n, is_float ? 1 : 0, a, make_limits(a.nb, n));
+cudaError_t plan_t(const BucketArgs& a, const K* keys, size_t n, cudaStream_t stream) {
+  bucket_plan_kernel<K><<<kPlanCtas, kPlanBlock, 0, stream>>>(keys, n, a, make_limits(a.nb, n));
   return cudaGetLastError();
 }
 
-template <typename K, bool FLT>
+template <typename K>
 cudaError_t count_t(const BucketArgs& a, const K* keys, size_t n, cudaStream_t stream) {
-  auto kern = bucket_count_kernel<K, FLT>;
+  auto kern = bucket_count_kernel<K>;
   const size_t smem = (size_t)std::max<uint32_t>(a.nb, 1024) * 4;
   cudaError_t e = ensure_dynamic_smem(kern, (size_t)kBucketsMax * 4);
   if (e != cudaSuccess) return e;
@@ -1517,7 +1510,7 @@ cudaError_t count_t(const BucketArgs& a, const K* keys, size_t n, cudaStream_t s
   return launch_chained(kern, (unsigned)grid, kCountBlock, smem, stream, keys, n, a, make_limits(a.nb, n));
 }
 
-template <typename K, bool FLT>
+template <typename K>
 cudaError_t sort_t(const BucketArgs& a, K* keys, K* tmp, size_t n, cudaStream_t stream,
                    const std::function<cudaError_t()>& mark) {
   const unsigned sms = (unsigned)device_info().sm_count;
@@ -1526,25 +1519,25 @@ cudaError_t sort_t(const BucketArgs& a, K* keys, K* tmp, size_t n, cudaStream_t 
   if ((e = m()) != cudaSuccess) return e;
   if ((e = m()) != cudaSuccess) return e;
   const size_t tiles = ceil_div(n, (size_t)kScatterTile<K>) + 1;
-  e = launch_chained(bucket_scatter_kernel<K, false, FLT>, (unsigned)std::min<size_t>(tiles, sms * kScatterPerSm),
+  e = launch_chained(bucket_scatter_kernel<K, false>, (unsigned)std::min<size_t>(tiles, sms * kScatterPerSm),
                      kScatterBlock, 0, stream, keys, tmp, n, a);
   if (e != cudaSuccess) return e;
   if ((e = m()) != cudaSuccess) return e;
   K* in = tmp;
   if (a.low_bits) {
-    e = launch_chained(bucket_scatter_kernel<K, true, false>,
+    e = launch_chained(bucket_scatter_kernel<K, true>,
                        (unsigned)std::min<size_t>(tiles + kGroups, sms * kScatterPerSm), kScatterBlock, 0, stream, tmp, keys, n,
                        a);
     if (e != cudaSuccess) return e;
     in = keys;
   }
   if ((e = m()) != cudaSuccess) return e;
-  auto kern = bucket_finish_kernel<K, FLT>;
+  auto kern = bucket_finish_kernel<K>;
   if ((e = ensure_dynamic_smem(kern, finish_smem<K>())) != cudaSuccess) return e;
   e = launch_chained(kern, std::min<unsigned>(a.nb, sms * kFinishPerSm<K>), kFinishBlock, finish_smem<K>(), stream, in, keys,
                      a.low_bits ? tmp : keys, n, a);
   if (e != cudaSuccess) return e;
-  auto rare = bucket_rare_kernel<K, FLT>;
+  auto rare = bucket_rare_kernel<K>;
   if ((e = ensure_dynamic_smem(rare, rare_smem<K>())) != cudaSuccess) return e;
   e = launch_chained(rare, std::min<unsigned>(a.nb, sms * 2), kRareBlock, rare_smem<K>(), stream, in, keys,
                      a.low_bits ? tmp : keys, n, a);
@@ -1923,13 +1916,13 @@ __device__ __forceinline__ void seg_job(const PlanDev& P, size_t total, const Se
 
 // Whole segments and buckets at the job array's front, then the counted ones at
 // its end.
-template <bool FLT, typename Make>
+template <typename Make>
 __device__ __forceinline__ void seg_finish(const PlanDev& P, Make&& make) {
   // (thread 0) the next bucket's job, read a bucket ahead
   const uint32_t jobs = P.sb.whole + P.declined[seg::kJobBuckets];
   SegBucketJob nj{};
   if (threadIdx.x == 0 && blockIdx.x < jobs) nj = P.sb.bucket_job[blockIdx.x];
-  finish_buckets<uint32_t, FLT>(jobs, P.sb.rare, P.err, [&](uint32_t b, FinishJob<uint32_t>& job) {
+  finish_buckets<uint32_t, false>(jobs, P.sb.rare, P.err, [&](uint32_t b, FinishJob<uint32_t>& job) {
     make(nj, job);
     job.number = b;
     if (b + gridDim.x < jobs) nj = P.sb.bucket_job[b + gridDim.x];
@@ -1938,7 +1931,7 @@ __device__ __forceinline__ void seg_finish(const PlanDev& P, Make&& make) {
   if (counted == 0) return;
   __syncthreads();
   if (threadIdx.x == 0 && blockIdx.x < counted) nj = P.sb.bucket_job[first + blockIdx.x];
-  finish_buckets<uint32_t, FLT, kFinishBlock, kFinishCap, kCellBits, false, true>(
+  finish_buckets<uint32_t, false, kFinishBlock, kFinishCap, kCellBits, false, true>(
       counted, P.sb.rare, P.err, [&](uint32_t b, FinishJob<uint32_t>& job) {
         make(nj, job);
         job.number = first + b;
@@ -1947,11 +1940,11 @@ __device__ __forceinline__ void seg_finish(const PlanDev& P, Make&& make) {
 }
 
 __global__ void __launch_bounds__(kFinishBlock, kFinishPerSm<uint32_t>) seg_finish_kernel(const PlanDev P, size_t total) {
-  seg_finish<false>(P, [&](const SegBucketJob& j, FinishJob<uint32_t>& job) { seg_job(P, total, j, job); });
+  seg_finish(P, [&](const SegBucketJob& j, FinishJob<uint32_t>& job) { seg_job(P, total, j, job); });
 }
 
 __global__ void __launch_bounds__(kRareBlock) seg_rare_kernel(const PlanDev P, size_t total) {
-  rare_buckets<uint32_t, false>(P.sb.rare, [&](uint32_t b, FinishJob<uint32_t>& job) {
+  rare_buckets<uint32_t>(P.sb.rare, [&](uint32_t b, FinishJob<uint32_t>& job) {
     seg_job(P, total, P.sb.bucket_job[b], job);
   });
 }
@@ -2020,33 +2013,33 @@ size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s) {
   return off;
 }
 
-cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, const void* tmp, size_t n, int key_bytes,
-                                bool is_float, SortCtrl* ctrl, SortWords* words, cudaStream_t stream) {
-  if (key_bytes == 8) {
-    BucketArgs a = make_args(s, static_cast<const unsigned long long*>(tmp), n, ctrl, nullptr);
-    a.words = words;
-    const auto* k = static_cast<const unsigned long long*>(keys);
-    const cudaError_t e = plan_t(a, k, n, false, stream);
-    return e != cudaSuccess ? e : count_t<unsigned long long, false>(a, k, n, stream);
-  }
-  BucketArgs a = make_args(s, static_cast<const uint32_t*>(tmp), n, ctrl, nullptr);
+namespace {
+
+template <typename K>
+cudaError_t plan_and_count(const BucketScratch& s, const void* keys, const void* tmp, size_t n, SortCtrl* ctrl,
+                           SortWords* words, cudaStream_t stream) {
+  BucketArgs a = make_args(s, static_cast<const K*>(tmp), n, ctrl, nullptr);
   a.words = words;
-  const auto* k = static_cast<const uint32_t*>(keys);
-  const cudaError_t e = plan_t(a, k, n, is_float, stream);
-  if (e != cudaSuccess) return e;
-  return is_float ? count_t<uint32_t, true>(a, k, n, stream) : count_t<uint32_t, false>(a, k, n, stream);
+  const cudaError_t e = plan_t(a, static_cast<const K*>(keys), n, stream);
+  return e != cudaSuccess ? e : count_t(a, static_cast<const K*>(keys), n, stream);
 }
 
-cudaError_t enqueue_bucket_sort(const BucketScratch& s, void* keys, void* tmp, size_t n, int key_bytes, bool is_float,
-                                SortCtrl* ctrl, uint32_t* err, cudaStream_t stream,
-                                const std::function<cudaError_t()>& mark) {
+}  // namespace
+
+cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, const void* tmp, size_t n, int key_bytes,
+                                SortCtrl* ctrl, SortWords* words, cudaStream_t stream) {
+  return key_bytes == 8 ? plan_and_count<unsigned long long>(s, keys, tmp, n, ctrl, words, stream)
+                        : plan_and_count<uint32_t>(s, keys, tmp, n, ctrl, words, stream);
+}
+
+cudaError_t enqueue_bucket_sort(const BucketScratch& s, void* keys, void* tmp, size_t n, int key_bytes, SortCtrl* ctrl,
+                                uint32_t* err, cudaStream_t stream, const std::function<cudaError_t()>& mark) {
   if (key_bytes == 8) {
     auto *k = static_cast<unsigned long long*>(keys), *t = static_cast<unsigned long long*>(tmp);
-    return sort_t<unsigned long long, false>(make_args(s, t, n, ctrl, err), k, t, n, stream, mark);
+    return sort_t(make_args(s, t, n, ctrl, err), k, t, n, stream, mark);
   }
   auto *k = static_cast<uint32_t*>(keys), *t = static_cast<uint32_t*>(tmp);
-  const BucketArgs a = make_args(s, t, n, ctrl, err);
-  return is_float ? sort_t<uint32_t, true>(a, k, t, n, stream, mark) : sort_t<uint32_t, false>(a, k, t, n, stream, mark);
+  return sort_t(make_args(s, t, n, ctrl, err), k, t, n, stream, mark);
 }
 
 namespace seg {

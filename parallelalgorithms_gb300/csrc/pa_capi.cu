@@ -1018,11 +1018,11 @@ cudaError_t enqueue_sort(const SortScratch& s, void* d_keys, void* d_tmp, uint32
   if (s.buckets.nb && !has_vals && !is_float && (words || n >= (kb == 4 ? kBucketAsyncMin32 : kBucketAsyncMin64))) {
     e = m();
     if (words) *const_cast<volatile uint32_t*>(&words->decided) = kUndecided;
-    if (e == cudaSuccess) e = enqueue_bucket_plan(s.buckets, d_keys, d_tmp, n, kb, is_float, s.ctrl, words, stream);
+    if (e == cudaSuccess) e = enqueue_bucket_plan(s.buckets, d_keys, d_tmp, n, kb, s.ctrl, words, stream);
     uint32_t by_buckets = 1;
     if (words && e == cudaSuccess) e = wait_decided(&words->decided, stream, &by_buckets);
     if (by_buckets && e == cudaSuccess)
-      e = enqueue_bucket_sort(s.buckets, d_keys, d_tmp, n, kb, is_float, s.ctrl, err, stream, mark);
+      e = enqueue_bucket_sort(s.buckets, d_keys, d_tmp, n, kb, s.ctrl, err, stream, mark);
     if (words && by_buckets) {
       for (int p = 3; p <= passes && e == cudaSuccess; ++p) e = m();  // (no LSD launches, no final copy)
       return e;

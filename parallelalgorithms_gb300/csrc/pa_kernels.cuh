@@ -252,14 +252,13 @@ size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s);
 // is moved.  words, when set, receives map->on in `decided` as soon as the plan
 // knows it, and kAgainByDigits in `again` if the count says no after all.
 cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, const void* tmp, size_t n, int key_bytes,
-                                bool is_float, SortCtrl* ctrl, SortWords* words, cudaStream_t stream);
+                                SortCtrl* ctrl, SortWords* words, cudaStream_t stream);
 // Enqueues the planned sort (tmp: n keys of scratch; the result is in keys);
 // nothing is moved when map->on is 0.  `mark` runs at once (twice: the count has
 // been enqueued, and there is no scan launch), after each of the two partitions and after the
 // sort of the buckets.
-cudaError_t enqueue_bucket_sort(const BucketScratch& s, void* keys, void* tmp, size_t n, int key_bytes, bool is_float,
-                                SortCtrl* ctrl, uint32_t* err, cudaStream_t stream,
-                                const std::function<cudaError_t()>& mark = {});
+cudaError_t enqueue_bucket_sort(const BucketScratch& s, void* keys, void* tmp, size_t n, int key_bytes, SortCtrl* ctrl,
+                                uint32_t* err, cudaStream_t stream, const std::function<cudaError_t()>& mark = {});
 // Whole sort of n <= small_sort_max_keys(key_bytes, false) keys by one CTA, in
 // place (launch_small_sort's result; a bulk-copy wait that gives up raises a bit
 // in *err).
