@@ -8,8 +8,8 @@ partitioned into buckets that are (or, where their keys crowd, by the onesweep
 passes).  A plan is built once per segmentation and replayed through a captured
 CUDA graph.
 
-The autotuner times every candidate configuration (small/large cutoff and
-digit width; the onesweep tile of 11-bit plans) on the caller's own data and
+The autotuner times every candidate configuration (digit width, and the
+onesweep tile of 11-bit plans) on the caller's own data and
 remembers the fastest per (GPU, workload shape) in a JSON file, so later
 plans for the same shape start from the tuned choice without measuring
 again.
@@ -47,11 +47,9 @@ class SegSortChoice:
         return c
 
 
-# the small/large cutoff with 8-bit digits (whose passes use the plain
-# sort's tile), and 11-bit digits (three passes of 2048 bins) at the default
-# cutoff with either tile
-CANDIDATES = ([SegSortChoice(c, 8192) for c in (2048, 4096, 8192)] +
-              [SegSortChoice(4096, t, 11) for t in (4096, 8192)])
+# 8-bit digits (by buckets, which read neither the cutoff nor the tile: one
+# candidate), and 11-bit digits (three passes of 2048 bins) with either tile
+CANDIDATES = [SegSortChoice()] + [SegSortChoice(4096, t, 11) for t in (4096, 8192)]
 
 
 def _ptr(x) -> int:
