@@ -1,9 +1,9 @@
 #!/usr/bin/env python3
 """Benchmark of the GB300 radix hot path.
 
-Headline workload: stable LSD radix sort of 100,000,000 uniform uint32 keys
-((uint32)std::mt19937_64(1234)(), the reference's recipe) on one GPU, 8-bit
-digits (4 passes).  One step = one sort of the whole array with the keys
+Headline workload: radix sort of 100,000,000 uniform uint32 keys
+((uint32)std::mt19937_64(1234)(), the reference's recipe) on one GPU.  One
+step = one sort of the whole array with the keys
 already resident in HBM; the input is restored from a pristine device copy
 before each step, outside the step's CUDA events.  The 400 MB input is
 larger than the 129 MB L2, so no L2 flush is needed between steps.
@@ -309,7 +309,7 @@ def cpu_reference_sort(keys: np.ndarray, steps: int, warmup: int) -> dict:
 
 def workload_config(n: int, world: int) -> dict:
     """The `config` both arms print (same workload, same keys)."""
-    return {"workload": f"LSD radix sort of {n} uniform uint32 keys (mt19937_64 seed 1234), 8-bit digits, 4 passes",
+    return {"workload": f"radix sort of {n} uniform uint32 keys (mt19937_64 seed 1234)",
             "keys_per_gpu": n, "key_type": "uint32", "distribution": "uniform mt19937_64(1234)", "digit_bits": 8,
             "l2": "inputs (400 MB) larger than L2; no flush",
             "parallelism": "replicas" if world > 1 else "single GPU"}
@@ -413,20 +413,25 @@ def gb300_arm(args) -> None:
                      P(phases.ctypes.data), 16, _native.opts(stream.cuda_stream))
         acc += phases
     acc /= reps
-    # keys alone are sorted by buckets: plan + counts, two partitions, the sort
-    # of each bucket; then the LSD launches, which find nothing to do
-    names = ["plan_and_count", "scan", "partition_high", "partition_low", "bucket_sort", "lsd_launches", "final_copy"]
-    phase = {name: float(x) for name, x in zip(names, acc)}
+    # keys alone are sorted by buckets (plan + counts, two partitions, the sort of
+    # each bucket, no further launch), or by digit passes, the last of which is
+    # then not empty
+    by_buckets = acc[5] < 0.01 * acc[:5].sum()
+    if by_buckets:
+        names = {0: "plan_and_count", 2: "partition_high", 3: "partition_low", 4: "bucket_sort"}
+    else:
+        names = dict(enumerate(["histogram", "scan", "pass_0", "pass_1", "pass_2", "pass_3", "final_copy"]))
+    phase = {name: float(acc[i]) for i, name in names.items()}
     peak, peak_kind = measured_peak_gbs()
-    top = max(("partition_high", "partition_low", "bucket_sort"), key=phase.get)
+    top = max((names[i] for i in names if 2 <= i < 6), key=phase.get)
     achieved = 8.0 * n / (phase[top] / 1e3) / 1e9
     roofline = {"bound": "shared memory pipe", "kernel": f"{top} (uint32 keys)", "achieved": achieved,
                 "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": None,
                 "peak_source": f"{peak_kind} hbm_gbs (MEASURED_PEAKS.json)" if peak_kind == "measured"
                 else "fallback 6800 GB/s",
                 "bytes_per_launch": 8 * n, "launch_ms": phase[top]}
-    sort_bytes = 28.0 * n
-    whole = {"bytes_per_key": 28, "achieved_gbs": sort_bytes / (ms / 1e3) / 1e9,
+    sort_bytes = (28.0 if by_buckets else 36.0) * n
+    whole = {"bytes_per_key": sort_bytes / n, "achieved_gbs": sort_bytes / (ms / 1e3) / 1e9,
              "frac": sort_bytes / (ms / 1e3) / 1e9 / peak, "phase_ms": phase}
 
     # end to end through the C ABI with pinned host buffers
@@ -459,7 +464,10 @@ def gb300_arm(args) -> None:
         cb = cpu_reference_sort(keys, args.cpu_steps, 1)
         cpu = {k: cb[k] for k in ("value", "unit", "cores", "kind", "sample")}
 
-    launches_per_step = 1 + 1 + 4 + 1  # histogram, scan, 4 digit passes, final copy
+    # histogram, scan, 4 digit passes, final copy; a large asynchronous call has the
+    # bucket sort's six (plan, count, two partitions, buckets, listed buckets) and a
+    # clearing launch before them
+    launches_per_step = 7 + (7 if (1 << 26) <= n <= 32768 * 3072 else 0)
     if rank == 0:
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -551,8 +559,10 @@ def batched_extra(lib, _native, workloads, stream, peak) -> dict:
     wall_plain = (time.perf_counter() - t0) * 1e3
     _native.call("pa_stream_check", P(stream.cuda_stream))
     plain_ms = s.elapsed_time(e)
-    small = sizes <= choice.small_cutoff
-    model_bytes = float(8 * sizes[small].sum() + 36 * sizes[~small].sum())
+    # long segments: 8-bit plans count (4), partition (8) and sort buckets (8); 11-bit
+    # plans count (4), run three passes (24) and copy back (8)
+    small, long_bytes = (sizes <= 4096, 20) if choice.digit_bits == 8 else (sizes <= choice.small_cutoff, 36)
+    model_bytes = float(8 * sizes[small].sum() + long_bytes * sizes[~small].sum())
     plan.close()
     del src, d, t
     torch.cuda.empty_cache()
@@ -563,7 +573,7 @@ def batched_extra(lib, _native, workloads, stream, peak) -> dict:
             "autotune_ms": tune["ms"], "plan": info, "graph": True,
             "plain_per_array_ms": plain_ms, "plain_per_array_wall_ms": wall_plain,
             "speedup_vs_plain_per_array": plain_ms / ms,
-            "bytes_model": "8 B/key for shared-memory segments, 36 B/key for onesweep segments",
+            "bytes_model": f"8 B/key for shared-memory segments, {long_bytes} B/key for longer ones",
             "achieved_gbs": model_bytes / (ms / 1e3) / 1e9, "frac": model_bytes / (ms / 1e3) / 1e9 / peak}
 
 
@@ -746,7 +756,7 @@ def run_extras(pa, lib, _native, workloads, n, stream, peak) -> dict:
         del src, k, tk, v, tv, vsrc
         torch.cuda.empty_cache()
 
-    sort_case("sort_u32_presorted", workloads.presorted_u32(n))
+    sort_case("sort_u32_presorted", workloads.presorted_u32(n), bytes_per_key=28)
     sort_case("sort_u32_constant42", workloads.constant_u32(n, 42))
     sort_case("sort_kv_u64_uniform_u32payload", workloads.uniform_u64(n), np.arange(n, dtype=np.uint32),
               "pa_sort_kv_u64", 200)

@@ -103,12 +103,12 @@ int pa_sort_two_phase_u32(uint32_t* a, uint32_t* b, size_t n, const pa_opts* opt
  * and phase_ms[i] receives the device time in milliseconds of each kernel,
  * from CUDA events recorded between the launches: [0] the one-read digit
  * histogram, [1] the bin-offset scan, [2 + p] digit pass p (one per
- * digit), [2 + passes] the final copy.  Keys alone of the sizes that are sorted
- * by buckets (csrc/pa_buckets.cu): [0] the plan and the bucket counts, [2] and
- * [3] the two partition passes, [4] the sort of each bucket, [5] every LSD
- * launch behind them (nearly nothing, unless the keys were too unevenly spread
- * for buckets; then [0] to [4] are), [2 + passes] the final copy, the others
- * nothing.  phase_cap bounds the entries written.
+ * digit), [2 + passes] the final copy.  Keys alone that are sorted by buckets
+ * (csrc/pa_buckets.cu): [0] the plan and the bucket counts, [2] and [3] the two
+ * partition passes, [4] the sort of each bucket, the others nothing.  Keys that
+ * the plan turns away have it in [0], before the histogram; where the counts do,
+ * or a 64-bit sort by its leading digits runs all passes after all, the phases are
+ * those of the digit passes that then sort.  phase_cap bounds the entries written.
  * GPU form of the per-phase timers the reference keeps commented out in its
  * sort (RadixSortLsdParallel.h:255-258, 287, 307-308). */
 enum { PA_KEY_U32 = 0, PA_KEY_U64 = 1, PA_KEY_F32 = 2 };

@@ -293,7 +293,7 @@ cudaError_t enqueue_window_test(const WindowScratch& s, const void* keys, void* 
   // A share p of all pairs agreeing in the window and no further makes sample^2
   // p / 2 hits.  The window is used up to p = 1 / (2 n), where places out of order
   // are a fair part of all keys and a run of sqrt(n / 2) keys would explain them
-  // (64 hits at 2^19, 42 at 100M, where evenly spread keys have 2).
+  // (128 hits at 2^19, 64 at 2^20, 42 at 100M, where evenly spread keys have 2).
   uint32_t lg = 12;
   while (lg < kTestMostLog2 && ((size_t)1 << (2 * lg)) < 256 * n) ++lg;
   const size_t sample = (size_t)1 << lg;
