@@ -210,6 +210,19 @@ inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned 
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// The place of sample key i of 1 << log2 in an array of n keys: somewhere in the
+// i-th stride.  At even places keys that repeat a pattern whose period divides the
+// stride (a matrix, records, channels) would be seen in one phase only: 2^24 keys,
+// every second one small, looked evenly spread and 31 ms went into one bucket.
+__device__ __forceinline__ size_t sample_place(uint32_t i, int log2, size_t n) {
+  const size_t lo = (size_t)(((unsigned long long)i * n) >> log2);
+  const size_t hi = (size_t)((((unsigned long long)i + 1) * n) >> log2);
+  uint32_t h = i * 0x9E3779B9u;  // (2^32 / golden ratio; its product folded, twice)
+  h = (h ^ (h >> 15)) * 0x9E3779B9u;
+  h ^= h >> 13;
+  return lo + (size_t)__umul64hi((unsigned long long)h << 32, hi - lo);
+}
+
 // Streaming 16-byte load that does not allocate in L1.
 __device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
   uint4 v;

@@ -6,7 +6,7 @@
 // keys together (MoveOutsideOfKthBinIn, :36-55), recurse into the bin.  The
 // result is the same order statistic; here the input is read once in the
 // usual case and never moved:
-//   sample   a cluster of eight CTAs takes kSample keys at even strides and its
+//   sample   a cluster of eight CTAs takes kSample keys, one of each stride, and its
 //            first CTA finds, by the same MSD digit narrowing in shared memory,
 //            the sample's keys `lo` and `hi` a few standard deviations below and
 //            above rank k (the extreme ranks give the key type's minimum /
@@ -191,7 +191,7 @@ __device__ void pick_bin(SelectState* st, const unsigned long long* h, uint32_t 
   if (t == 0) st->ticket = 0;
 }
 
-// The bracket: kSample keys at even strides, and their order statistics at
+// The bracket: kSample keys, one of each stride, and their order statistics at
 // the ranks kBracketSigmas standard deviations either side of rank k's
 // image, both found at once by MSD digit narrowing over the sample in
 // shared memory.  A cluster gathers the sample (strided loads over the whole
@@ -210,11 +210,11 @@ __global__ void __cluster_dims__(kSampleCtas, 1, 1) __launch_bounds__(kSampleThr
   __shared__ bool s_lo_min, s_hi_max;
   const uint32_t tid = threadIdx.x;
   const uint32_t ns = (uint32_t)(n < (size_t)kSample ? n : (size_t)kSample);
-  // key j of the sample sits at (j n + n / 2) / ns: a shift when ns is the
-  // full sample (a power of two), j itself when the input is smaller
+  // key j of the sample sits somewhere in the j-th of ns strides; j itself when the
+  // input is smaller
   const uint32_t j0 = cluster.block_rank() * kSampleThreads + tid;
   K mine = 0;
-  if (j0 < ns) mine = keys[ns == (uint32_t)kSample ? ((size_t)j0 * n + n / 2) >> kSampleLog2 : (size_t)j0];
+  if (j0 < ns) mine = keys[ns == (uint32_t)kSample ? sample_place(j0, kSampleLog2, n) : (size_t)j0];
   for (uint32_t i = j0; i < (uint32_t)kLinBins; i += kSample) st->lin_bins[i] = 0;
   for (uint32_t i = j0; i < 256u; i += kSample) st->hist[i] = 0;
   cluster.sync();  // (the first CTA runs before its memory is written)

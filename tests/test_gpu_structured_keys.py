@@ -56,3 +56,25 @@ def test_period_of_a_stride(pa, torch_cuda, kind, n, wide):
     flip = torch.iinfo(src.dtype).min
     assert torch.equal(got ^ flip, torch.sort(src ^ flip)[0])
     assert took < 10 * even, f"{took * 1e6:.0f} us against {even * 1e6:.0f}"
+
+
+@pytest.mark.parametrize("kind", ["pairs", "rows"])
+@pytest.mark.parametrize("share", [0.0, 0.2, 0.5, 0.9])
+@pytest.mark.parametrize("n", [1 << 20, 1 << 26])
+def test_select_of_a_pattern(pa, torch_cuda, kind, share, n):
+    """The order statistic of such keys, in at most three times what evenly spread
+    keys take: their sample brackets it as well."""
+    torch = torch_cuda
+    took = {}
+    for k in ("even", kind):
+        src = structured(k, n, torch)
+        rank = int(n * share)
+        want = int((torch.sort(src ^ -(1 << 31))[0][rank] ^ -(1 << 31)).item()) & 0xFFFFFFFF
+        took[k] = 1e9
+        for _ in range(4):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            got = pa.select(src, rank)
+            took[k] = min(took[k], time.perf_counter() - t)
+        assert got == want
+    assert took[kind] < 3 * took["even"], took

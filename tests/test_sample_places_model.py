@@ -1,4 +1,4 @@
-"""CPU model of the bucket plan's sample (sample_place, csrc/pa_buckets.cu): a place
+"""CPU model of the samples of bucket plans and selects (sample_place, csrc/pa_common.cuh): a place
 in every stride, and every phase of a pattern that repeats seen in proportion."""
 import numpy as np
 import pytest
