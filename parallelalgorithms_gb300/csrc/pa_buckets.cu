@@ -10,13 +10,15 @@
 // partition, bucket sort) against 1 + 2 * 4 (1 + 2 * 8 for 64-bit keys).
 //
 //   bucket_plan_kernel     one cluster of 8 CTAs reads 16384 keys, one at a
-//                          random place of each stride, takes the range they span, and lays nb
-//                          equal buckets over it (BucketMap); counts the
-//                          sample per bucket to judge the fit: a sample that
-//                          crowds into few buckets leaves the sort to the LSD
-//                          passes, which do not mind how keys are spread;
-//   bucket_count_kernel    one read: exact keys per bucket; the last CTA turns
-//                          the counts into bucket starts and cursors;
+//                          random place of each stride, takes the range they
+//                          span, and lays nb equal buckets over it (BucketMap);
+//                          counts the sample per bucket to judge the fit: a
+//                          sample that crowds into few buckets leaves the sort
+//                          to the LSD passes, which do not mind how keys are
+//                          spread;
+//   bucket_count_kernel    one read: exact keys per bucket, and the cells of a few
+//                          buckets; the last CTA turns the counts into bucket
+//                          starts and cursors, or the sort away;
 //   bucket_scatter_kernel  one tile at a time: rank, reserve, stage by bin,
 //                          write out in bin-contiguous runs.  First on the
 //                          bucket's high bits (keys -> tmp), then, bucket
@@ -65,6 +67,18 @@ constexpr int kCellBits = 16, kBinBits = 12;
 constexpr uint32_t kCells = 1u << kCellBits;      // cells of the finish kernel's bitmap
 constexpr uint32_t kCountSpan = 1u << (kCellBits - 3);  // values a counted bucket may span
 constexpr uint32_t kBucketBins = 1u << kBinBits;  // values a crowded bucket may span to be counted instead
+constexpr int kFinishBlock = 256;
+constexpr uint32_t kEntryHits = 6;  // keys of one entry of the bitmap that found their cell taken, at most
+// Keys may crowd into few cells of every bucket however evenly these fill (multiples
+// of some number, few prefixes with small numbers behind them, clusters): the finish
+// kernel then leaves nearly all of them to bucket_rare_kernel.  So the count kernel
+// lays out half of the cells of kCrowdBuckets buckets (an entry: 32 cells' bits,
+// and its keys, as the finish kernel has them), and turns the sort away where those
+// with too many keys in taken cells hold more than 3/8 of their keys.
+constexpr int kCrowdLog2 = 3;
+constexpr uint32_t kCrowdBuckets = 1u << kCrowdLog2;
+constexpr uint32_t kCrowdEntries = kCells / 32 / 2;
+constexpr uint32_t kCrowdHits = kFinishBlock / 2;  // keys in taken cells of half of a bucket's, at most
 
 struct BucketArgs {
   BucketMap* map;
@@ -93,6 +107,7 @@ struct BucketLimits {
   uint32_t dense_above;  // sample keys above which a 64th of the buckets looks too full
   uint32_t most_keys;   // keys no bucket may exceed
   uint32_t most_over;   // keys that may lie in buckets beyond the finish kernel
+  uint2* crowd;         // [kCrowdBuckets][kCrowdEntries] in the scratch array, not yet in use (may be null)
 };
 
 // t: the key's distance from the bottom of the map, in 32 bits.
@@ -113,6 +128,22 @@ __device__ __forceinline__ uint32_t map_bucket(uint32_t t, uint32_t mult, uint32
 // The key's top 32 bits: its distance from the bottom of a plain map.
 __device__ __forceinline__ uint32_t top_word(uint32_t key) { return key; }
 __device__ __forceinline__ uint32_t top_word(unsigned long long key) { return (uint32_t)(key >> 32); }
+
+// Adds a key's cell to a bucket's laid out half: one entry in two, by the parity of
+// all bits of its number and the bucket's (`part`), so that multiples of a power of
+// two do not all miss it.
+__device__ __forceinline__ void crowd_add(uint2* crowd, uint32_t cell, uint32_t part) {
+  const uint32_t entry = (cell / 32) & (2 * kCrowdEntries - 1);
+  if ((__popc(entry) ^ part) & 1u) return;
+  atomicOr(&crowd[entry / 2].x, 1u << (cell & 31u));
+  atomicAdd(&crowd[entry / 2].y, 1u);
+}
+// Whether the finish kernel would leave the bucket (its keys: cnt) to the rare launch,
+// as far as its half tells: too many keys in taken cells, an entry with too many of
+// them, or the half's share of the keys missing, which are then crowded elsewhere.
+__device__ __forceinline__ bool crowd_listed(uint32_t cnt, uint32_t hits, uint32_t full, uint32_t seen) {
+  return hits > kCrowdHits || full != 0 || (cnt > 256 && seen < cnt / 4);
+}
 
 // Elements from the 16-byte boundary at or below p to p.
 template <typename K>
@@ -299,6 +330,9 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
   }
   // (last, so that no cluster barrier waits for these stores)
   for (uint32_t i = rank * kPlanBlock + tid; i < a.nb; i += kPlanCtas * kPlanBlock) a.count[i] = 0;
+  if (most.crowd)
+    for (uint32_t i = rank * kPlanBlock + tid; i < kCrowdBuckets * kCrowdEntries; i += kPlanCtas * kPlanBlock)
+      most.crowd[i] = make_uint2(0u, 0u);
 }
 
 // ---------------------------------------------------------------------------
@@ -311,22 +345,29 @@ __global__ void __cluster_dims__(kPlanCtas, 1, 1) __launch_bounds__(kPlanBlock)
 // its tile tables: 0.113 ms).
 constexpr int kCountBlock = 1024;
 
-template <typename K>
+template <typename K, bool CROWD>
 __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* __restrict__ keys, size_t n,
                                                                       BucketArgs a, BucketLimits most) {
   extern __shared__ __align__(16) uint32_t s_cnt[];
   __shared__ uint32_t s_warp[kCountBlock / 32];
   __shared__ uint32_t s_last, s_over;
+  __shared__ uint32_t s_hits[kCrowdBuckets], s_full[kCrowdBuckets], s_seen[kCrowdBuckets];
   constexpr int V = 16 / (int)sizeof(K);
   const uint32_t tid = threadIdx.x;
   for (uint32_t i = tid; i < a.nb; i += kCountBlock) s_cnt[i] = 0;
   if (tid == 0) s_over = 0;
+  if (tid < kCrowdBuckets) s_hits[tid] = s_full[tid] = s_seen[tid] = 0;
   chain_wait();
   chain_next();
   const BucketMap m = *a.map;
   if (!m.on) return;
   __syncthreads();
   const uint32_t last = a.nb - 1;
+  // the buckets whose cells are laid out: one in nb / kCrowdBuckets, none of them at
+  // the map's ends (pick beyond every bucket: none at all)
+  const bool crowd = CROWD && !m.counts;
+  const uint32_t crowd_mask = a.nb / kCrowdBuckets - 1;
+  const uint32_t pick = crowd ? (crowd_mask * 5) >> 3 : 0xFFFFFFFFu;
   auto count = [&](auto plainc) {
     constexpr bool PLAIN = decltype(plainc)::value;
     const K lo = (K)m.lo;
@@ -334,6 +375,19 @@ __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* _
     auto bucket = [&](K key) {
       if constexpr (PLAIN) return top_word(key) >> shift;
       else return map_bucket(map_t<K>(key, lo, m.s), m.mult, last);
+    };
+    auto look = [&](const K* k) {  // a vector's keys (few have one that is looked at)
+      if constexpr (CROWD) {
+        bool any = false;
+#pragma unroll
+        for (int e = 0; e < V; ++e) any = any || (bucket(k[e]) & crowd_mask) == pick;
+        if (!any) return;
+        for (int e = 0; e < V; ++e) {
+          const uint32_t b = bucket(k[e]), j = b >> (a.nb_bits - kCrowdLog2);
+          if ((b & crowd_mask) == pick)
+            crowd_add(most.crowd + j * kCrowdEntries, (uint32_t)((PLAIN ? k[e] : k[e] - lo) >> m.cell_shift), j);
+        }
+      }
     };
     const uintptr_t addr = reinterpret_cast<uintptr_t>(keys);
     size_t head = ((16u - (addr & 15u)) & 15u) / sizeof(K);
@@ -369,11 +423,13 @@ __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* _
           for (int e = 1; e < V; ++e) one = one && bucket(k[e]) == d0;
           if (__all_sync(kFull, one)) {
             if ((tid & 31u) == 0) atomicAdd(s_cnt + d0, 32u * V);
+            if ((d0 & crowd_mask) == pick) look(k);
             continue;
           }
         }
 #pragma unroll
         for (int e = 0; e < V; ++e) atomicAdd(s_cnt + bucket(k[e]), 1u);
+        look(k);
       }
       i = nx;
     }
@@ -383,6 +439,7 @@ __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* _
         const K* k = reinterpret_cast<const K*>(&w);
 #pragma unroll
         for (int e = 0; e < V; ++e) atomicAdd(s_cnt + bucket(k[e]), 1u);
+        look(k);
       }
     }
     if (blockIdx.x == 0) {  // head and tail: fewer than 2 * V keys
@@ -410,6 +467,29 @@ __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* _
   // The last CTA: whether the buckets fit after all, their starts, cursors of both
   // passes, and the second pass's tiles per group (tile_first).
   const uint32_t per = max(1u, a.nb / kCountBlock);  // buckets per thread
+  if (crowd) {  // four warps a laid out bucket: its keys in taken cells, entries with too many of them
+    constexpr uint32_t kWarps = kCountBlock / 32 / kCrowdBuckets;
+    constexpr uint32_t kPer = kCrowdEntries / 2 / kWarps;  // 16-byte words, two entries, per warp
+    const uint32_t j = (tid >> 5) / kWarps;
+    const uint4* e = reinterpret_cast<const uint4*>(most.crowd + j * kCrowdEntries) + ((tid >> 5) % kWarps) * kPer;
+    uint32_t hits = 0, full = 0, seen = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < kPer / 32; ++q) {
+      const uint4 x = __ldcg(e + q * 32 + (tid & 31u));
+      const uint32_t h0 = x.y - __popc(x.x), h1 = x.w - __popc(x.z);
+      hits += h0 + h1;
+      seen += x.y + x.w;
+      full |= max(h0, h1) > kEntryHits ? 1u : 0u;
+    }
+    hits = __reduce_add_sync(kFull, hits);
+    full = __reduce_or_sync(kFull, full);
+    seen = __reduce_add_sync(kFull, seen);
+    if ((tid & 31u) == 0) {
+      atomicAdd(&s_hits[j], hits);
+      atomicOr(&s_full[j], full);
+      atomicAdd(&s_seen[j], seen);
+    }
+  }
   if (a.nb >= (uint32_t)kCountBlock) {
     for (uint32_t j = tid * 4; j < a.nb; j += kCountBlock * 4)
       *reinterpret_cast<uint4*>(s_cnt + j) = __ldcg(reinterpret_cast<const uint4*>(a.count + j));
@@ -427,6 +507,14 @@ __global__ void __launch_bounds__(kCountBlock, 1) bucket_count_kernel(const K* _
       large |= c > most.most_keys;
     }
   if (over) atomicAdd(&s_over, over);
+  if (crowd && tid < 32) {
+    uint32_t c = 0, listed = 0;
+    if (tid < kCrowdBuckets) {
+      c = s_cnt[tid * (crowd_mask + 1) + pick];
+      listed = crowd_listed(c, s_hits[tid], s_full[tid], s_seen[tid]) ? c : 0u;
+    }
+    large |= __reduce_add_sync(kFull, listed) > __reduce_add_sync(kFull, c) / 8 * 3;
+  }
   if (__syncthreads_or(large) || s_over > most.most_over) {
     if (tid == 0) {
       a.map->on = 0;  // (every other CTA is past its look at it; the launches behind find nothing to do)
@@ -696,10 +784,8 @@ __global__ void __launch_bounds__(kScatterBlock, kScatterPerSm) bucket_scatter_k
 // 0.33.  Four CTAs per SM of 64 registers: five (48 registers) spill and lose
 // more than they hide; 512 threads with the keys re-read from shared memory
 // 0.41.  64-bit keys need 88 KB a CTA: two per SM.
-constexpr int kFinishBlock = 256;
 template <typename K>
 constexpr int kFinishPerSm = sizeof(K) == 4 ? 4 : 2;
-constexpr uint32_t kEntryHits = 6;  // keys of one entry that found their cell taken, at most
 
 // The least t with umulhi(t, mult) >= b (b < nb), from the rounded-down
 // reciprocal inv = 2^63 / mult: the estimate is at most two short.
@@ -1313,6 +1399,8 @@ __device__ __forceinline__ void rare_buckets(const uint32_t* rare, JobOf&& job_o
       block_minmax<K, kRareBlock>(job.src, job.cnt, false, s_edge, lo, hi);
       if (hi - lo < (K)kBucketBins)
         finish_counted<K>(job.src, job.dst, job.cnt, lo, smem, s_warp);
+      else if (job.cnt <= kFinishCap / 2)  // (every pass takes the places there are, not the keys)
+        finish_nibbles<K, false, kRareBlock, kFinishCap / 2>(job.src, job.dst, job.cnt, lo ^ hi, smem, s_warp);
       else
         finish_nibbles<K, false>(job.src, job.dst, job.cnt, lo ^ hi, smem, s_warp);
     } else {
@@ -1469,8 +1557,21 @@ BucketArgs make_args(const BucketScratch& s, const K* tmp, size_t n, SortCtrl* c
   return a;
 }
 
-BucketLimits make_limits(uint32_t nb, size_t n) {
+// Least keys from which the buckets' crowding is looked at, at about 1 us a call
+// (below, the launch for listed buckets is as fast as the digit passes).  Keys of
+// which a tenth come 20 times each, by digit passes alone / left to that launch / turned
+// away (us a call): 32-bit 2M 135 / 138 / 122, 4M 181 / 203 / 177; 100M multiples of 64
+// 1803 / 2363 / 1848; 64-bit 1M 195 / 185 / 155, 5M 372 / 502 / 264; 67M of 2^20 prefixes
+// 3010 / 6798 / 2090, of 2^24 values 1564 / 7430 / 1600.
+template <typename K>
+constexpr size_t kCrowdLeast = (size_t)1 << (sizeof(K) == 4 ? 21 : 20);
+
+template <typename K>
+BucketLimits make_limits(uint32_t nb, size_t n, const K* tmp) {
   BucketLimits m{};
+  if (n >= kCrowdLeast<K>)
+    m.crowd = reinterpret_cast<uint2*>((reinterpret_cast<uintptr_t>(tmp) + 15) & ~(uintptr_t)15);
+  static_assert(kCrowdLeast<K> * sizeof(K) >= kCrowdBuckets * kCrowdEntries * sizeof(uint2) + 16, "fits the scratch array");
   m.dense_above = (uint32_t)((double)kFinishCap * (nb / kPlanParts) * (double)kSample / (double)n);
   // One CTA sorts such a bucket, at about 2 ns a key and byte; by then the count
   // has been paid for, a fifteenth of the digit passes: n / 1024 keys, 0.6 ms at
@@ -1481,20 +1582,20 @@ BucketLimits make_limits(uint32_t nb, size_t n) {
 }
 
 template <typename K>
-cudaError_t plan_t(const BucketArgs& a, const K* keys, size_t n, cudaStream_t stream) {
-  bucket_plan_kernel<K><<<kPlanCtas, kPlanBlock, 0, stream>>>(keys, n, a, make_limits(a.nb, n));
+cudaError_t plan_t(const BucketArgs& a, const BucketLimits& most, const K* keys, size_t n, cudaStream_t stream) {
+  bucket_plan_kernel<K><<<kPlanCtas, kPlanBlock, 0, stream>>>(keys, n, a, most);
   return cudaGetLastError();
 }
 
 template <typename K>
-cudaError_t count_t(const BucketArgs& a, const K* keys, size_t n, cudaStream_t stream) {
-  auto kern = bucket_count_kernel<K>;
+cudaError_t count_t(const BucketArgs& a, const BucketLimits& most, const K* keys, size_t n, cudaStream_t stream) {
+  auto kern = most.crowd ? bucket_count_kernel<K, true> : bucket_count_kernel<K, false>;
   const size_t smem = (size_t)std::max<uint32_t>(a.nb, 1024) * 4;
   cudaError_t e = ensure_dynamic_smem(kern, (size_t)kBucketsMax * 4);
   if (e != cudaSuccess) return e;
   const size_t work = ceil_div(n, (size_t)kCountBlock * (16 / sizeof(K)) * 2);
   const size_t grid = std::min<size_t>(std::max<size_t>(work, 1), (size_t)device_info().sm_count);
-  return launch_chained(kern, (unsigned)grid, kCountBlock, smem, stream, keys, n, a, make_limits(a.nb, n));
+  return launch_chained(kern, (unsigned)grid, kCountBlock, smem, stream, keys, n, a, most);
 }
 
 template <typename K>
@@ -1553,11 +1654,31 @@ __device__ __forceinline__ uint32_t seg_bucket(uint32_t key, uint32_t lo, uint32
   return mult == 0 ? key >> (32u - nb_bits) : map_bucket(map_t<uint32_t>(key, lo, 0u), mult, (1u << nb_bits) - 1u);
 }
 
+// Crowding in a segment (as in bucket_count_kernel): where it is long enough to pay
+// for it, half of the cells of one bucket, in the scratch array at the segment's
+// own place; in shorter ones, by the sample's keys that share a cell.  (us a run by
+// digit passes alone / left to the launch for listed buckets / declined, a tenth of a
+// segment's keys 20 times each: 2000 of 20 K keys 854 / 1439 / 885, 300 of 100 K 573 / 1459 /
+// 613, 30 of 1 M 585 / 1071 / 623; evenly spread 300 of 1 K to 1 M 376 -> 383, 1000 of 1 M
+// 7.36 -> 7.40 ms, shorter ones 1 to 2 % more.  A bucket's cells for 100 K keys too: 4 %
+// more for evenly spread ones.)
+constexpr uint32_t kSegCrowdLeast = 1u << 17;
+__device__ __forceinline__ uint2* seg_crowd(const PlanDev& P, const BucketSeg& g) {
+  return reinterpret_cast<uint2*>((reinterpret_cast<uintptr_t>(P.tmp + g.base) + 7) & ~(uintptr_t)7);
+}
+constexpr int kSegCellLog2 = 11;  // slots for the sample's cells
+// Whether its buckets are counted: they span at most ceil(2^32 / mult) values.
+__device__ __forceinline__ bool seg_counted(const SegMap& m) { return ((1ull << 32) + m.mult - 1) / m.mult <= kCountSpan; }
+
 // One CTA per segment of several buckets: the range a sample of 1024 keys spans.
 constexpr int kSegPlanBlock = 256;
-__global__ void __launch_bounds__(kSegPlanBlock) seg_map_kernel(const uint32_t* __restrict__ keys, SegBucketsDev sb) {
+__global__ void __launch_bounds__(kSegPlanBlock) seg_map_kernel(const PlanDev P) {
+  const uint32_t* __restrict__ keys = P.keys;
+  const SegBucketsDev& sb = P.sb;
   __shared__ uint32_t s_lo[kSegPlanBlock / 32], s_hi[kSegPlanBlock / 32];
   __shared__ uint32_t s_cnt[kSegBins];
+  __shared__ __align__(16) uint32_t s_cell[1u << kSegCellLog2];
+  __shared__ uint32_t s_hits, s_most_hits, s_mult, s_shift, s_wide, s_off, s_most;
   const BucketSeg g = sb.seg[blockIdx.x];
   uint32_t lo = 0xFFFFFFFFu, hi = 0;
   uint32_t k[4];
@@ -1569,6 +1690,10 @@ __global__ void __launch_bounds__(kSegPlanBlock) seg_map_kernel(const uint32_t* 
     hi = max(hi, k[j]);
   }
   for (uint32_t i = threadIdx.x; i < (1u << g.nb_bits); i += kSegPlanBlock) s_cnt[i] = 0;
+  if (g.len < kSegCrowdLeast)
+    for (uint32_t i = threadIdx.x; i < (1u << kSegCellLog2) / 4; i += kSegPlanBlock)
+      reinterpret_cast<uint4*>(s_cell)[i] = make_uint4(kFull, kFull, kFull, kFull);
+  if (threadIdx.x == 0) s_hits = 0;
   lo = __reduce_min_sync(kFull, lo);
   hi = __reduce_max_sync(kFull, hi);
   if ((threadIdx.x & 31u) == 0) {
@@ -1589,18 +1714,54 @@ __global__ void __launch_bounds__(kSegPlanBlock) seg_map_kernel(const uint32_t* 
     lo = 0;
     hi = 0xFFFFFFFFu;
   }
-  const unsigned long long range = (unsigned long long)(hi - lo) + 1;
-  const uint32_t mult = (uint32_t)min(0xFFFFFFFFull, ((unsigned long long)1 << (32 + g.nb_bits)) / range);
+  if (threadIdx.x < 32) {  // (the divisions, by one warp)
+    const unsigned long long range = (unsigned long long)(hi - lo) + 1;
+    const uint32_t mult = (uint32_t)min(0xFFFFFFFFull, ((unsigned long long)1 << (32 + g.nb_bits)) / range);
+    const unsigned long long width = ((1ull << 32) + mult - 1) / mult, per = g.len >> g.nb_bits;
+    uint32_t cell_shift = 0;
+    while (((width - 1) >> cell_shift) >= kCells) ++cell_shift;
+    // Keys of the sample in taken cells: what evenly spread ones have, and what they
+    // have where buckets reach the finish kernel's limit.
+    const float nb = (float)(1u << g.nb_bits), pairs = 1024.f * 1024.f / 2.f, len = (float)g.len;
+    const float even = pairs / (nb * (float)(width >> cell_shift)), full = 2.f * kFinishBlock * pairs * nb / (len * len);
+    if (threadIdx.x == 0) {
+      s_mult = mult;
+      s_shift = cell_shift;
+      s_wide = width > kCountSpan ? 1u : 0u;
+      // (few values a bucket, but too many to count: as in bucket_plan_kernel)
+      s_off = width > kCountSpan && per * per > 400 * width ? 1u : 0u;
+      s_most = 12u + (uint32_t)(((unsigned long long)(4 * kFinishCap) << 10) / g.len);
+      s_most_hits = (uint32_t)fmaxf(even + 3.f * sqrtf(even) + 2.f, 0.8f * full);
+    }
+  }
+  __syncthreads();
+  const uint32_t mult = s_mult, cell_shift = s_shift, most = s_most;
+  const bool cells = s_wide && g.len < kSegCrowdLeast;
   // The fullest bucket of the sample: a segment with one far beyond the finish
   // kernel is left to the digit passes before its keys are counted.
-  uint32_t mx = 0;
+  uint32_t mx = 0, hits = 0;
 #pragma unroll
-  for (uint32_t j = 0; j < 4; ++j)
-    mx = max(mx, atomicAdd(s_cnt + map_bucket(map_t<uint32_t>(k[j], lo, 0u), mult, (1u << g.nb_bits) - 1u), 1u) + 1u);
-  const uint32_t most = 12u + (uint32_t)(((unsigned long long)(4 * kFinishCap) << 10) / g.len);
-  const unsigned long long width = ((1ull << 32) + mult - 1) / mult, per = g.len >> g.nb_bits;
-  // (few values a bucket, but too many to count: as in bucket_plan_kernel)
-  const bool off = __syncthreads_or(mx > most || (width > kCountSpan && per * per > 400 * width)) != 0;
+  for (uint32_t j = 0; j < 4; ++j) {
+    const uint32_t t = map_t<uint32_t>(k[j], lo, 0u);
+    const uint32_t c = atomicAdd(s_cnt + map_bucket(t, mult, (1u << g.nb_bits) - 1u), 1u) + 1u;
+    mx = max(mx, c);
+    if (!cells || c > most) continue;
+    // (up to two keys a cell, so that a few frequent values, which crowd one bucket,
+    // weigh little)
+    constexpr uint32_t kOne = 1u << 30, kTwo = 1u << 31;
+    const uint32_t cell = t >> cell_shift;
+    uint32_t* slot = s_cell + ((cell * 0x9E3779B9u) >> (32 - kSegCellLog2));
+    const uint32_t old = atomicCAS(slot, kFull, cell);
+    if (old != kFull && (old & ~(kOne | kTwo)) == cell)
+      hits += !(atomicOr(slot, kOne) & kOne) || !(atomicOr(slot, kTwo) & kTwo) ? 1u : 0u;
+  }
+  if (cells) {
+    hits = __reduce_add_sync(kFull, hits);
+    if (hits && (threadIdx.x & 31u) == 0) atomicAdd(&s_hits, hits);
+  }
+  const bool off = __syncthreads_or(mx > most || s_off) != 0 || s_hits > s_most_hits;
+  if (!off && !cells && s_wide)
+    for (uint32_t i = threadIdx.x; i < kCrowdEntries; i += kSegPlanBlock) seg_crowd(P, g)[i] = make_uint2(0u, 0u);
   if (threadIdx.x != 0) return;
   SegMap m{};
   m.off = off ? 1u : 0u;
@@ -1608,7 +1769,7 @@ __global__ void __launch_bounds__(kSegPlanBlock) seg_map_kernel(const uint32_t* 
   m.mult = mult;
   m.plain = lo == 0 && hi == 0xFFFFFFFFu ? 1u : 0u;
   m.inv = (1ull << 63) / mult;
-  while (((width - 1) >> m.cell_shift) >= kCells) ++m.cell_shift;
+  m.cell_shift = cell_shift;
   sb.map[blockIdx.x] = m;
 }
 
@@ -1632,7 +1793,24 @@ __global__ void __launch_bounds__(kSegCountBlock, 3) seg_count_kernel(const Plan
     const uint32_t head = min(len, (4u - skew_of(src)) & 3u);
     const uint32_t nvec = (len - head) / 4u, tail = head + nvec * 4u;
     const uint4* vec = reinterpret_cast<const uint4*>(src + head);
-    auto add = [&](uint32_t key) { atomicAdd(s_cnt + seg_bucket(key, m.lo, mult, g.nb_bits), 1u); };
+    const uint32_t pick = g.len < kSegCrowdLeast || seg_counted(m) ? 0xFFFFFFFFu : nb / 2;
+    auto bucket = [&](uint32_t key) { return seg_bucket(key, m.lo, mult, g.nb_bits); };
+    auto look = [&](uint32_t key, uint32_t b) {
+      if (b == pick) crowd_add(seg_crowd(P, g), (key - m.lo) >> m.cell_shift, s);
+    };
+    auto add = [&](const uint4& q) {
+      const uint32_t b0 = bucket(q.x), b1 = bucket(q.y), b2 = bucket(q.z), b3 = bucket(q.w);
+      atomicAdd(s_cnt + b0, 1u);
+      atomicAdd(s_cnt + b1, 1u);
+      atomicAdd(s_cnt + b2, 1u);
+      atomicAdd(s_cnt + b3, 1u);
+      if (b0 == pick || b1 == pick || b2 == pick || b3 == pick) {
+        look(q.x, b0);
+        look(q.y, b1);
+        look(q.z, b2);
+        look(q.w, b3);
+      }
+    };
     constexpr uint32_t U = 4;
     uint32_t v = threadIdx.x;
     for (; v + (U - 1) * kSegCountBlock < nvec; v += U * kSegCountBlock) {
@@ -1640,22 +1818,11 @@ __global__ void __launch_bounds__(kSegCountBlock, 3) seg_count_kernel(const Plan
 #pragma unroll
       for (uint32_t u = 0; u < U; ++u) q[u] = ld_stream_v4(vec + v + u * kSegCountBlock);
 #pragma unroll
-      for (uint32_t u = 0; u < U; ++u) {
-        add(q[u].x);
-        add(q[u].y);
-        add(q[u].z);
-        add(q[u].w);
-      }
+      for (uint32_t u = 0; u < U; ++u) add(q[u]);
     }
-    for (; v < nvec; v += kSegCountBlock) {
-      const uint4 q = ld_stream_v4(vec + v);
-      add(q.x);
-      add(q.y);
-      add(q.z);
-      add(q.w);
-    }
-    if (threadIdx.x < head) add(src[threadIdx.x]);
-    if (threadIdx.x < len - tail) add(src[tail + threadIdx.x]);
+    for (; v < nvec; v += kSegCountBlock) add(ld_stream_v4(vec + v));
+    if (threadIdx.x < head) atomicAdd(s_cnt + bucket(src[threadIdx.x]), 1u);
+    if (threadIdx.x < len - tail) atomicAdd(s_cnt + bucket(src[tail + threadIdx.x]), 1u);
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < nb; i += kSegCountBlock)
       if (s_cnt[i]) atomicAdd(P.sb.count + g.first_bucket + i, s_cnt[i]);
@@ -1669,7 +1836,7 @@ __global__ void __launch_bounds__(kSegCountBlock, 3) seg_count_kernel(const Plan
 constexpr int kSegScanBlock = 256;
 __global__ void __launch_bounds__(kSegScanBlock) seg_jobs_kernel(const PlanDev P) {
   __shared__ uint32_t s_warp[kSegScanBlock / 32];
-  __shared__ uint32_t s_over, s_first, s_chunk, s_job0, s_tile0;
+  __shared__ uint32_t s_over, s_hits, s_seen, s_first, s_chunk, s_job0, s_tile0;
   const uint32_t L = blockIdx.x, tid = threadIdx.x;
   const uint32_t s = P.sb.of_large[L];
   bool off = s == 0xFFFFFFFFu;
@@ -1678,7 +1845,7 @@ __global__ void __launch_bounds__(kSegScanBlock) seg_jobs_kernel(const PlanDev P
     const SegMap m = P.sb.map[s];
     const uint32_t nb = 1u << g.nb_bits;
     uint32_t* cnt = P.sb.count + g.first_bucket;
-    if (tid == 0) s_over = 0;
+    if (tid == 0) s_over = s_hits = s_seen = 0;
     __syncthreads();
     uint32_t over = 0;
     for (uint32_t i = tid; i < nb; i += kSegScanBlock) {
@@ -1686,13 +1853,30 @@ __global__ void __launch_bounds__(kSegScanBlock) seg_jobs_kernel(const PlanDev P
       if (c > kFinishCap) over += c > 4 * kFinishCap ? g.len : c;
     }
     if (over) atomicAdd(&s_over, min(over, g.len));
+    const bool counted = seg_counted(m);
+    bool crowded = false;
+    if (!m.off && !counted && g.len >= kSegCrowdLeast) {
+      uint32_t hits = 0, full = 0, seen = 0;
+      for (uint32_t i = tid; i < kCrowdEntries; i += kSegScanBlock) {
+        const uint2 e = seg_crowd(P, g)[i];
+        hits += e.y - __popc(e.x);
+        seen += e.y;
+        full |= e.y - __popc(e.x) > kEntryHits ? 1u : 0u;
+      }
+      hits = __reduce_add_sync(kFull, hits);
+      seen = __reduce_add_sync(kFull, seen);
+      if ((tid & 31u) == 0) {
+        atomicAdd(&s_hits, hits);
+        atomicAdd(&s_seen, seen);
+      }
+      full = __syncthreads_or((int)full) != 0 ? 1u : 0u;
+      crowded = crowd_listed(cnt[nb / 2], s_hits, full, s_seen);
+    }
     __syncthreads();
-    off = m.off || s_over > g.len / 32;
+    off = m.off || crowded || s_over > g.len / 32;
     if (!off) {
       // room for its jobs behind those of the segments before it
       const uint32_t tiles = (g.len + 3u + kSegTile - 1u) / kSegTile;
-      // (a bucket's values, at most: ceil(2^32 / mult))
-      const bool counted = ((1ull << 32) + m.mult - 1) / m.mult <= kCountSpan;
       if (tid == 0) {
         s_job0 = counted ? P.sb.buckets - nb - atomicAdd(&P.declined[seg::kJobCounted], nb)
                          : P.sb.whole + atomicAdd(&P.declined[seg::kJobBuckets], nb);
@@ -2003,17 +2187,18 @@ size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s) {
 namespace {
 
 template <typename K>
-cudaError_t plan_and_count(const BucketScratch& s, const void* keys, const void* tmp, size_t n, SortCtrl* ctrl,
+cudaError_t plan_and_count(const BucketScratch& s, const void* keys, void* tmp, size_t n, SortCtrl* ctrl,
                            SortWords* words, cudaStream_t stream) {
   BucketArgs a = make_args(s, static_cast<const K*>(tmp), n, ctrl, nullptr);
   a.words = words;
-  const cudaError_t e = plan_t(a, static_cast<const K*>(keys), n, stream);
-  return e != cudaSuccess ? e : count_t(a, static_cast<const K*>(keys), n, stream);
+  const BucketLimits most = make_limits(a.nb, n, static_cast<const K*>(tmp));
+  const cudaError_t e = plan_t(a, most, static_cast<const K*>(keys), n, stream);
+  return e != cudaSuccess ? e : count_t(a, most, static_cast<const K*>(keys), n, stream);
 }
 
 }  // namespace
 
-cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, const void* tmp, size_t n, int key_bytes,
+cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, void* tmp, size_t n, int key_bytes,
                                 SortCtrl* ctrl, SortWords* words, cudaStream_t stream) {
   return key_bytes == 8 ? plan_and_count<unsigned long long>(s, keys, tmp, n, ctrl, words, stream)
                         : plan_and_count<uint32_t>(s, keys, tmp, n, ctrl, words, stream);
@@ -2035,7 +2220,7 @@ cudaError_t launch_seg_plan(const PlanDev& pd, cudaStream_t s) {
   const unsigned sms = (unsigned)device_info().sm_count;
   cudaError_t e = cudaSuccess;
   if (pd.sb.num) {
-    seg_map_kernel<<<pd.sb.num, kSegPlanBlock, 0, s>>>(pd.keys, pd.sb);
+    seg_map_kernel<<<pd.sb.num, kSegPlanBlock, 0, s>>>(pd);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     seg_count_kernel<<<std::min(pd.sb.chunks, sms * 3), kSegCountBlock, 0, s>>>(pd);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;

@@ -248,10 +248,10 @@ size_t bucket_scratch_layout(char* base, size_t n, BucketScratch* s);
 // caller that waits for the decision learns it and enqueues the rest (1M uniform
 // 32-bit keys 75 -> 70 us a call, 600 K 62 -> 56; keys turned away find one more
 // launch that returns).  The exact counts have the last word: where too many keys
-// are in buckets beyond the finish kernel, the count clears map->on, so that no key
-// is moved.  words, when set, receives map->on in `decided` as soon as the plan
+// are in buckets beyond the finish kernel, or crowd in theirs, the count clears
+// map->on, so that no key is moved (tmp is written).  words, when set, receives map->on in `decided` as soon as the plan
 // knows it, and kAgainByDigits in `again` if the count says no after all.
-cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, const void* tmp, size_t n, int key_bytes,
+cudaError_t enqueue_bucket_plan(const BucketScratch& s, const void* keys, void* tmp, size_t n, int key_bytes,
                                 SortCtrl* ctrl, SortWords* words, cudaStream_t stream);
 // Enqueues the planned sort (tmp: n keys of scratch; the result is in keys);
 // nothing is moved when map->on is 0.  `mark` runs at once (twice: the count has
