@@ -965,10 +965,8 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
       if constexpr (COUNTS) {
         uint32_t* s_half = reinterpret_cast<uint32_t*>(s_entry);
         constexpr uint32_t kWords = kEntries * 2;
-        if (job.edge) {  // (its range is known only now)
-          const bool wide = first > (K)~(K)0 - (kCountSpan - 1) ? false : edge_hi > first + (kCountSpan - 1);
-          if (wide && tid == 0) atomicMax(&s_over, 1u);  // (not over the 2 of a copy that never came)
-        }
+        // (an end bucket's range is known only now, and to every thread)
+        const bool wide = job.edge && (K)(edge_hi - first) > (K)(kCountSpan - 1);
         K k[ITEMS];
         uint32_t r[ITEMS / 2];
 #pragma unroll
@@ -993,7 +991,7 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
           return;
         }
         go_on();
-        if (s_over == 0) {
+        if (!wide) {
           uint4 q[U];
           uint32_t c2[U];
           auto both = [](uint32_t w) { return (w & 0xFFFFu) + (w >> 16); };
@@ -1209,8 +1207,9 @@ __device__ __forceinline__ void finish_buckets(uint32_t nb, uint32_t* rare, uint
     if (!done) {
       if (tid == 0) rare[1 + atomicAdd(rare, 1u)] = job.number;
       // every thread has read s_nhit and s_over, which say which barriers it
-      // takes part in, before thread 0 clears them (write_out has a barrier too)
-      __syncthreads();
+      // takes part in, before thread 0 clears them (write_out has a barrier too;
+      // counted buckets are listed without a look at either)
+      if constexpr (!COUNTS) __syncthreads();
     }
   }
   if (tid == 0) bulk_store_wait_all();
