@@ -757,7 +757,8 @@ def run_extras(pa, lib, _native, workloads, n, stream, peak) -> dict:
         torch.cuda.empty_cache()
 
     sort_case("sort_u32_presorted", workloads.presorted_u32(n), bytes_per_key=28)
-    sort_case("sort_u32_constant42", workloads.constant_u32(n, 42))
+    # (one read: no pass moves a key)
+    sort_case("sort_u32_constant42", workloads.constant_u32(n, 42), bytes_per_key=4)
     sort_case("sort_kv_u64_uniform_u32payload", workloads.uniform_u64(n), np.arange(n, dtype=np.uint32),
               "pa_sort_kv_u64", 200)
     sort_case("sort_kv_u64_zipf_u32payload", workloads.zipf_u64(n), np.arange(n, dtype=np.uint32),

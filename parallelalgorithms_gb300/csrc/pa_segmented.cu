@@ -5,10 +5,10 @@
 // pa_buckets.cu); only the segments that declines go through the digit passes
 // here (declined_*_kernel, over lists made on the device).  A run that waits, by
 // four digit passes alone -> now (us): 4096 arrays of 1 K to 4 M uniform keys, 2.0 G
-// keys, 36040 -> 15800; 300 of 1 K to 1 M 894 -> 379; 64 of 1 K to 50 K 89 -> 60.
+// keys, 36060 -> 15800; 300 of 1 K to 1 M 898 -> 381; 64 of 1 K to 50 K 90 -> 60.
 // Skewed keys pay for the maps and counts they are declined on: 1000 arrays of 1 M
-// 16370 -> 17080, 2000 of 20 K 857 -> 903, 300 of 1 K to 1 M 907 -> 927, 64 of 1 K to
-// 50 K 89 -> 93, 64 of 3000 42 -> 40.
+// 16430 -> 17100, 2000 of 20 K 863 -> 890, 300 of 1 K to 1 M 906 -> 919; 64 of 1 K to
+// 50 K 84 -> 84, 64 of 3000 42 -> 41.
 //
 // 11-bit plans, and the plans other sorts build for their groups, run ONE
 // persistent kernel fed by a device work queue (8-bit ones then a launch per
@@ -677,8 +677,9 @@ cudaError_t launch_plan(const HostPlan& hp, const PlanDev& pd, char* dev, unsign
     }
     // From here on the two kinds of segments share neither keys nor tables, and in
     // small batches each launch is mostly latency: side by side.  (us a run, one
-    // behind the other -> beside: 64 arrays of 1 K to 50 K skewed keys 122 -> 94, 300
-    // of 1 K to 1 M 950 -> 925, uniform 379 -> 379; 1000 of 1 M 17.1 ms both ways.)
+    // behind the other -> beside, both before crowding was looked at: 64 arrays of 1 K
+    // to 50 K skewed keys 122 -> 94, 300 of 1 K to 1 M 950 -> 925, uniform 379 -> 379;
+    // 1000 of 1 M 17.1 ms both ways.)
     if ((e = cudaEventRecord(fork->leave, s)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(fork->side, fork->leave, 0)) != cudaSuccess) return e;
     e = launch_declined(hp, pd, fork->side);
